@@ -6,8 +6,10 @@
 
 namespace kvq {
 
-constexpr int kMmaThreads = 128;
-constexpr int kMmaWarps = 4;
+// Eight warps per CTA and two CTAs per SM (128 registers a thread): WARPNOTE
+constexpr int kMmaThreads = 256;
+constexpr int kMmaWarps = 8;
+constexpr int kMmaSmemMax = 115712;                                // dynamic shared memory of a CTA with two of them on an SM
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
@@ -142,46 +144,10 @@ template <> struct VFields<1> {
     }
 };
 
-// Key-side extraction from ONE register that already pairs the same 16-bit half-word of two channel rows (as a
-// transposing ldmatrix delivers them): r[i] = fp16x2 of field i of both half-words, i < 16 / BITS, at bit position
-// Fields<BITS>::pos(i).
-template <int BITS> struct KHalf;
-template <> struct KHalf<4> {
-    static constexpr int N = 4;
-    __device__ static __forceinline__ void unpack(uint32_t x, uint32_t (&r)[4]) {
-        const uint32_t xs = x >> 8;
-        r[0] = x & 0x000f000fu; r[1] = x & 0x00f000f0u; r[2] = xs & 0x000f000fu; r[3] = xs & 0x00f000f0u;
-    }
-};
-template <> struct KHalf<2> {
-    static constexpr int N = 8;
-    __device__ static __forceinline__ void unpack(uint32_t x, uint32_t (&r)[8]) {
-        const uint32_t xs = x >> 10;
-#pragma unroll
-        for (int t = 0; t < 5; ++t) r[t] = x & (0x00030003u << (2 * t));
-#pragma unroll
-        for (int t = 5; t < 8; ++t) r[t] = xs & (0x00030003u << (2 * (t - 5)));
-    }
-};
-template <> struct KHalf<1> {
-    static constexpr int N = 16;
-    __device__ static __forceinline__ void unpack(uint32_t x, uint32_t (&r)[16]) {
-        const uint32_t xs = x >> 10;
-#pragma unroll
-        for (int t = 0; t < 10; ++t) r[t] = x & (0x00010001u << t);
-#pragma unroll
-        for (int t = 10; t < 16; ++t) r[t] = xs & (0x00010001u << (t - 10));
-    }
-};
-template <> struct KHalf<3> {                       // 3-bit keys do not use this path (11 fields do not split into half-words)
-    static constexpr int N = 2;
-    __device__ static __forceinline__ void unpack(uint32_t, uint32_t (&)[2]) {}
-};
-
-// Value-side extraction from ONE register that already pairs two 16-bit half-words along the contraction axis (as
-// a transposing ldmatrix delivers them): r[i] = fp16x2 of field i of both half-words, i < 16 / BITS, each left at
+// Extraction from ONE register that already pairs two 16-bit half-words along the contraction axis (as
+// a transposing ldmatrix delivers them: two tokens of values, two channels of keys): r[i] = fp16x2 of field i of both half-words, i < 16 / BITS, each left at
 // bit position pos(i) >= 4 (>= 2 for 4-bit codes) of its half -- the positions VFields uses, for the same reason.
-template <int BITS> struct VHalf;
+template <int BITS> struct VHalf;     // 3-bit words do not split into half-words
 template <> struct VHalf<4> {
     static constexpr int N = 4;
     __device__ static __forceinline__ int pos(int i) { return (i & 1) ? 6 : 2; }
@@ -216,6 +182,9 @@ template <> struct VHalf<1> {
         for (int t = 10; t < 16; ++t) r[t] = xd & (0x00010001u << (t - 6));
     }
 };
+template <> struct VHalf<3> {
+    static constexpr int N = 2;
+};
 
 // ---------------------------------------------------------------------------------------------
 // Key-side geometry per bit width.  A warp tile is 8 lane-octets x TPO tokens; code words reach the
@@ -227,29 +196,27 @@ template <int KB> struct KGeom {
     static constexpr int WPL = (KB == 4) ? 4 : (KB == 2) ? 2 : 1;     // words per octet: 32 tokens (11 for 3-bit)
     static constexpr int TPO = WPL * FPI;                              // tokens per octet chunk
     static constexpr int WT = 8 * TPO;                                 // tokens per warp tile (256 / 88)
-    static constexpr int KSPS = (KB == 4) ? 1 : 2;                     // k-steps (16 channels) per stage
-    static constexpr int NSTAGE = 8 / KSPS;                            // stages per warp tile: 8 / 4
+    static constexpr int KSPS = (KB == 4 || KB == 2) ? 1 : 2;          // k-steps (16 channels) per stage
+    static constexpr int NSTAGE = 8 / KSPS;                            // stages per warp tile of all channels: 8 / 4
     static constexpr int NMMA = (TPO + 1) / 2;                         // MMAs (token pairs) per octet chunk
     static constexpr int RB = 32 * WPL;                                // code bytes per channel row per warp tile
     static constexpr int RS = RB + 16;                                 // padded row stride in the ring
     static constexpr int ROWS = 16 * KSPS;                             // channel rows per stage
-    static constexpr int STAGE_BYTES = ROWS * RS;                      // 2304 / 2560 / 1536
+    static constexpr int CODE_BYTES = ROWS * RS;                       // 2304 / 1280 / 1536 (4 / 2 / 3 and 1 bits)
     static constexpr int GPR = RB / 16;                                // 16-byte granules per row: 8 / 4 / 2
-    static constexpr int GPL = ROWS * GPR / 32;                        // granules per lane per stage: 4 / 4 / 2
+    static constexpr int GPL = ROWS * GPR / 32;                        // granules per lane per stage: 4 / 2 / 2
     static constexpr int RPI = 32 / GPR;                               // rows between a lane's granules
-    static constexpr int NS = 4;                                       // ring slots (NSTAGE % NS == 0: slots are static)
-    static constexpr int P = NS - 1;                                   // stages in flight
-    static constexpr int SZ_BYTES = 2 * kHeadDim * 16;                 // scale + zero tile: 16 B per channel row
-    static constexpr int WARP_BYTES = NS * STAGE_BYTES + SZ_BYTES;
     static constexpr float MID = (float)((1 << KB) - 1) * 0.5f;        // codes are centred on the group midpoint
 };
 
-template <int WPL> struct WordVec;
-template <> struct WordVec<1> { using T = uint32_t; };
-template <> struct WordVec<2> { using T = uint2; };
-template <> struct WordVec<4> { using T = uint4; };
+// The ring of the key codes: NS slots of one stage (codes, then the scale and zero rows of the stage's channels, SZ bytes).
+template <int KB, int SZ, int NSLOTS> struct KRing {
+    static constexpr int NS = NSLOTS, P = NS - 1;
+    static constexpr int STAGE_BYTES = KGeom<KB>::CODE_BYTES + SZ;
+    static constexpr int BYTES = NS * STAGE_BYTES;
+};
 
-template <int VB> struct VGeom {
+template <int VB, int NSLOTS = (VB == 4) ? 4 : (VB == 2) ? 6 : 8> struct VGeom {
     static constexpr int FPI = fields_per_word(VB);
     static constexpr int RBV = kHeadDim / FPI * 4;                     // code bytes per token row: 64 / 32 / 16
     static constexpr int TPS = 32;                                     // tokens per stage (2 k-steps)
@@ -257,16 +224,12 @@ template <int VB> struct VGeom {
     static constexpr int GPL = (TPS * GPT + 31) / 32;                  // code granules per lane per stage: 4 / 2 / 1
     static constexpr int SZ_OFF = TPS * RBV;                           // scale rows, then zero rows (<= 4 groups each)
     static constexpr int STAGE_BYTES = TPS * RBV + 2 * TPS * 4 * 2;
-    static constexpr int NS = (VB == 4) ? 4 : (VB == 2) ? 6 : 8;
+    static constexpr int NS = NSLOTS;
     static constexpr int P = NS - 1;
     static constexpr int PB_OFF = NS * STAGE_BYTES;                    // operand tile p*scale / p*mid: 16 token pairs x 8 cols
     static constexpr int WARP_BYTES = NS * STAGE_BYTES + 16 * 8 * 4;
     static constexpr float MID = (float)((1 << VB) - 1) * 0.5f;
 };
-
-template <int KB, int VB> constexpr int warp_region_bytes() {
-    return KGeom<KB>::WARP_BYTES > VGeom<VB>::WARP_BYTES ? KGeom<KB>::WARP_BYTES : VGeom<VB>::WARP_BYTES;
-}
 
 template <int BYTES>
 __device__ __forceinline__ void cp_async(uint32_t smem_addr, const void *gmem) {
@@ -295,5 +258,42 @@ __device__ __forceinline__ uint32_t pack_h2_sat(float lo, float hi) {
 }
 __device__ __forceinline__ uint32_t as_u32(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
 __device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
+
+// hi / lo part of the exact product q * s for a pair of channels: even columns carry hi = rn(q * s), odd columns
+// lo = q * s - hi (exact in fp16).  neg_mask is 0 in even-column lanes and all ones in odd-column lanes:
+// fma(q, s, +0) = hi, fma(q, s, -hi) = lo.
+__device__ __forceinline__ uint32_t hilo(__half2 q, __half2 s, uint32_t neg_mask) {
+    const uint32_t hi = as_u32(__hmul2(q, s));
+    return as_u32(__hfma2(q, s, as_h2((hi ^ 0x80008000u) & neg_mask)));
+}
+
+// Four neighbouring scores of the softmax: the channel splits' partial sums added, rounded to fp16 where the call asks for it
+// (upstream's GEMV returns fp16 scores), scaled.
+__device__ __forceinline__ float4 score_quad(const kvq_attn_args &a, const float4 *s, int split_stride4, int ks_log2) {
+    float4 v = *s;
+    for (int p = 1; p < (1 << ks_log2); ++p) {
+        const float4 u = s[p * split_stride4];
+        v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    if (a.round_scores) {
+        const float2 r0 = __half22float2(__floats2half2_rn(v.x, v.y)), r1 = __half22float2(__floats2half2_rn(v.z, v.w));
+        v = make_float4(r0.x, r0.y, r1.x, r1.y);
+    }
+    v.x *= a.softmax_scale; v.y *= a.softmax_scale; v.z *= a.softmax_scale; v.w *= a.softmax_scale;
+    return v;
+}
+// weights + mask, clamped at the fp32 floor
+__device__ __forceinline__ void mask_quad(const kvq_attn_args &a, int b, int h, int t, float4 &v) {
+    v.x = fmaxf(v.x + attn_mask_at(a, b, h, min(t, a.T - 1)), kMaskFloor);
+    v.y = fmaxf(v.y + attn_mask_at(a, b, h, min(t + 1, a.T - 1)), kMaskFloor);
+    v.z = fmaxf(v.z + attn_mask_at(a, b, h, min(t + 2, a.T - 1)), kMaskFloor);
+    v.w = fmaxf(v.w + attn_mask_at(a, b, h, min(t + 3, a.T - 1)), kMaskFloor);
+}
+// the last, partial quad: neutral padding behind its `left` valid scores
+__device__ __forceinline__ void pad_quad(float4 &v, int left) {
+    if (left <= 1) v.y = -INFINITY;
+    if (left <= 2) v.z = -INFINITY;
+    if (left <= 3) v.w = -INFINITY;
+}
 
 }  // namespace kvq

@@ -1,7 +1,7 @@
 // Work plan of the tensor-core attention kernels: which tokens of which head a CTA scores.
 //
 // The token axis of every head (a query head, or the group of query heads that share a kv head) is cut into
-// units of `unit` tokens (one key tile per warp: 256, or 352 = 4 x 88 for 3-bit keys); a head has
+// units of `unit` tokens (a warp's key tile: 256, or four of them for 3-bit keys: 352 = 4 x 88); a head has
 // uph = ceil(T / unit) units, the last one possibly short.  One CTA works one segment = a run of units of one head:
 //   * the first n_whole CTAs take one whole head each (only when a head fits the score buffer); n_whole is a multiple
 //     of the resident-CTA slots of the GPU, so these CTAs fill whole waves;
@@ -24,49 +24,68 @@ struct AttnPlan {
     int k;               // segments per cut head (1: a whole head per CTA here too)
     int seg_units;       // units per segment of a cut head
     int n_scores;        // most tokens in a segment, rounded up to 32
+    int ks_log2;         // the channels of a key tile are shared by 1 << ks_log2 warps (partial scores, summed by the softmax)
 };
 
 constexpr int kSmCount = 148;
+constexpr int kPlanSlots = 2 * kSmCount;       // resident CTAs: two of eight warps per SM
+constexpr int kPlanWarps = 8;
+// Whole heads are launched in multiples of whole waves of two, three, ... CTAs per SM
+constexpr int kWholeWave = 6 * kSmCount;
 // One partial result of a cut head: 128 accumulators, the segment's maximum and sum, padded so that rows stay 16-byte
 // aligned (the merge reads them with 128-bit loads).
 constexpr int kPartStride = 128 + 4;
-// What merging one more segment costs the CTA that finishes last, in tokens' worth of time.
-constexpr int kMergeTokensPerSegment = 4;
-// A CTA costs about this many tokens' worth of time besides the tokens it scores (launch, ring fill of two phases,
-// softmax barriers, warps that get one key tile fewer than their neighbours, merge).  Measured on B200 with 2-bit
-// keys and values at 4096 tokens: 256 heads take 54 us whole, 60 .. 66 us cut in 2 .. 4 (more CTAs than resident
-// slots), and cutting the 272 heads beyond four full waves of a 2048-head launch costs 1 .. 9 % -- so heads are cut
-// only where the score buffer forces it or where whole heads would leave most slots empty.
-constexpr int kCtaOverheadTokens = 2048;
 constexpr int kMaxCtaRounds = 8;       // cut heads are never spread over more CTAs than this many waves (bounds the workspace)
 
-// heads: number of heads (or head groups); max_chunk: most tokens a segment may hold (score buffer); slots: resident
-// CTAs on the whole GPU.
-// units_per_pass: units the warps of a CTA work side by side (4 when a unit is one warp's key tile, 1 when a unit is
-// already a tile per warp): a segment takes as long as its units rounded up to that.
-inline AttnPlan make_attn_plan(int T, int unit, int max_chunk, long long heads, int slots, int units_per_pass = 1) {
+inline int plan_round32(int n) { return (n + 31) / 32 * 32; }
+
+// Channel split of a segment's key tiles.  A warp walks a tile's 128 channels in four steps of 32; where a segment has fewer
+// tiles than the CTA has warps, 2 or 4 warps share a tile's channels and each leaves partial scores.  Steps a warp takes
+// (x 2), with about half a step's time of per-tile overhead; `max_scores` bounds the score buffer (tokens x splits).
+inline int plan_key_steps(int n, int tile, int ks_log2) {
+    const int tiles = (n + tile - 1) / tile;
+    const int passes = ((tiles << ks_log2) + kPlanWarps - 1) / kPlanWarps;
+    return passes * ((8 >> ks_log2) + 1);
+}
+inline int plan_key_split(int n, int tile, int max_scores) {
+    int best = 0;
+    for (int l = 1; l <= 2; ++l)
+        if ((plan_round32(n) << l) <= max_scores && plan_key_steps(n, tile, l) < plan_key_steps(n, tile, best)) best = l;
+    return best;
+}
+
+// SM cycles a segment of n tokens takes (one of two CTAs on its SM; measured with clock stamps inside the kernels on
+// B200): 850 per two half-steps of keys, 850 per 32 tokens of values a warp works, the softmax, and PLANFIXED for
+// the launch, the ring fill, the fp16 tails and the final sum.
+inline long long plan_segment_cycles(int n, int tile, int max_scores) {
+    const int key = plan_key_steps(n, tile, plan_key_split(n, tile, max_scores)) * 850;
+    const int val = (n + 32 * kPlanWarps - 1) / (32 * kPlanWarps) * 850;
+    return key + val + 1500 + n / 2 + 5500;
+}
+// What cutting a head adds to its last CTA: publishing the partials and the merge of k of them.
+inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; }
+
+// heads: number of heads (or head groups); tile: tokens of a warp's key tile; max_scores: tokens the score buffer holds.
+inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long long heads) {
     AttnPlan p;
     p.unit = unit;
     p.uph = (T + unit - 1) / unit;
-    const bool whole_ok = T <= max_chunk;
-    p.n_whole = (int)(whole_ok ? (heads / slots) * slots : 0);
+    const int max_units = max_scores / unit;
+    const bool whole_ok = T <= max_units * unit;
+    p.n_whole = (int)(whole_ok ? (heads / kWholeWave) * kWholeWave : 0);
     p.n_cut = (int)(heads - p.n_whole);
     p.k = 1;
     p.seg_units = p.uph;
     if (p.n_cut > 0) {
-        // candidates: segments of su units; estimated finish = rounds of CTAs x (tokens + overhead)
-        const int su_max = whole_ok ? p.uph : max_chunk / unit;
+        // candidates: segments of su units; estimated finish = rounds of CTAs x cycles of one + merge
         long long best = -1;
-        for (int su = su_max; su >= 1; --su) {
+        for (int su = whole_ok ? p.uph : max_units; su >= 1; --su) {
             const int k = (p.uph + su - 1) / su;
-            if (k > 1 && su < 2 && p.uph > 2) break;                           // at least two units per segment
             const long long ctas = (long long)p.n_cut * k;
-            if (ctas > (long long)kMaxCtaRounds * slots && best >= 0) break;
-            const long long rounds = (ctas + slots - 1) / slots;
-            const long long su_eff = (long long)(su + units_per_pass - 1) / units_per_pass * units_per_pass;
-            const long long tokens = k > 1 ? su_eff * unit : ((long long)su * unit < T ? (long long)su * unit : T);
-            const long long cost = rounds * (tokens + kCtaOverheadTokens) +
-                                   (k > 1 ? kCtaOverheadTokens / 4 + (long long)k * kMergeTokensPerSegment : 0);
+            if (ctas > (long long)kMaxCtaRounds * kPlanSlots && best >= 0) break;
+            const long long rounds = (ctas + kPlanSlots - 1) / kPlanSlots;
+            const int n = su * unit < T ? su * unit : T;
+            const long long cost = rounds * plan_segment_cycles(n, tile, max_scores) + plan_merge_cycles(k);
             if (best < 0 || cost < best) {
                 best = cost;
                 p.k = k;
@@ -78,7 +97,8 @@ inline AttnPlan make_attn_plan(int T, int unit, int max_chunk, long long heads, 
     }
     long long ns = (long long)(p.n_whole ? p.uph : p.seg_units) * unit;
     if (ns > T) ns = T;
-    p.n_scores = (int)((ns + 31) / 32 * 32);
+    p.n_scores = plan_round32((int)ns);
+    p.ks_log2 = plan_key_split((int)ns, tile, max_scores);
     return p;
 }
 

@@ -71,18 +71,19 @@ __device__ __forceinline__ void fused_quant_v_group(const kvq_attn_args &a, int 
     static_cast<__half *>(const_cast<void *>(a.vmn))[zo] = __float2half_rn(lo);
 }
 
-// The update work of one segment [t0, t1) of kv head (b, hk), before its attention phases; every thread of the CTA
+// The update work of one segment [t0, t1) of kv head (b, hk), before its attention phases; every thread of the CTA (2 x 128:
+// the first half quantizes keys, the second values)
 // calls it (it ends with a CTA barrier when it wrote packed data the CTA is about to read).
 template <int KB, int VB>
 __device__ __forceinline__ void fused_cache_update(const kvq_attn_args &a, int b, int hk, int t0, int t1, int tid) {
     if (!a.k_new) return;
     bool wrote = false;
     if (a.k_quant > 0 && t0 <= a.Tkq - a.k_quant && a.Tkq - a.k_quant < t1) {
-        fused_quant_k_group<KB>(a, b, hk, tid);
+        if (tid < kHeadDim) fused_quant_k_group<KB>(a, b, hk, tid);
         wrote = true;
     }
     if (a.v_quant > 0 && t0 <= a.Tvq - a.v_quant && a.Tvq - a.v_quant < t1) {
-        if constexpr (VB != 3) fused_quant_v_group<VB>(a, b, hk, tid);
+        if constexpr (VB != 3) if (tid >= kHeadDim) fused_quant_v_group<VB>(a, b, hk, tid - kHeadDim);
         wrote = true;
     }
     if (t1 == a.T && tid < 32) {                               // the rings receive the new token for the following steps
@@ -167,23 +168,69 @@ __device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, kvq_attn_
     }
 }
 
-// Head-sharded exchange: the rows `vals[i]` (this thread's channel `tid` of `n_heads` consecutive query heads starting
-// at local head h0 of sequence b) go to every rank's gather buffer, then every rank's arrival counter is raised by
-// n_heads.  Every thread of the CTA calls it (CTA barrier inside).  Plain peer stores and one system-scope
+// Head-sharded exchange: the rows `vals[i]` (channel `ch` of n_mine consecutive query heads starting at local head h0 of
+// sequence b) go to every rank's gather buffer, then every rank's arrival counter is raised by the CTA's n_heads.
+// Every thread of the CTA calls it (CTA barrier inside).  Plain peer stores and one system-scope
 // fence + atomic per rank: no multicast, nothing waits here.
 template <int N>
-__device__ __forceinline__ void peer_publish(const kvq_attn_args &a, int b, int h0, int n_heads, const __half (&vals)[N], int tid) {
+__device__ __forceinline__ void peer_publish(const kvq_attn_args &a, int b, int h0, int n_mine, const __half (&vals)[N], int ch,
+                                             int tid, int n_heads) {
     if (a.n_peers <= 0) return;
     for (int p = 0; p < a.n_peers; ++p) {
-        __half *dst = static_cast<__half *>(a.peer_out[p]) + (int64_t)b * a.peer_sB + (int64_t)(a.peer_head0 + h0) * a.peer_sH + tid;
+        __half *dst = static_cast<__half *>(a.peer_out[p]) + (int64_t)b * a.peer_sB + (int64_t)(a.peer_head0 + h0) * a.peer_sH + ch;
 #pragma unroll
         for (int i = 0; i < N; ++i)
-            if (i < n_heads) dst[(int64_t)i * a.peer_sH] = vals[i];
+            if (i < n_mine) dst[(int64_t)i * a.peer_sH] = vals[i];
     }
     __syncthreads();                                           // every thread's stores are issued ...
     if (tid < a.n_peers) {
         __threadfence_system();                                // ... and ordered before the arrival count, system-wide
         atomicAdd_system(a.peer_flag[tid], (unsigned)n_heads);
+    }
+}
+
+// The fp16 value tail is read at the very end of a segment: its rows are fetched into L2 while the packed part is worked.
+__device__ __forceinline__ void prefetch_v_tail(const kvq_attn_args &a, const __half *vf, int b, int hk, int v_lo, int t1, int tid, int threads) {
+    for (int i = tid; i < 2 * (t1 - v_lo); i += threads)
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(v_tail_row(a, vf, b, hk, v_lo + (i >> 1)) + 64 * (i & 1)));
+}
+
+// p . V over the fp16 value tail, tokens [v_lo, t1), for H heads whose probabilities lie `p_stride` floats apart: warp w takes
+// tokens v_lo + w, v_lo + w + 8, ..., a lane owns four channels of every head; the sums are added to the warp's partial
+// results red[H][128] (already complete and visible to the warp).
+template <int H>
+__device__ __forceinline__ void pv_tail(const kvq_attn_args &a, const __half *vf, int b, int hk, const float *p, int p_stride, int t0, int v_lo,
+                                        int t1, float *red, int warp, int n_warps, int lane) {
+    float acc[H][4];
+#pragma unroll
+    for (int h = 0; h < H; ++h) acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f;
+    constexpr int U = 8;                                       // rows in flight per warp
+    for (int t = v_lo + warp; t < t1; t += U * n_warps) {
+        uint2 v[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            v[j] = __ldg(reinterpret_cast<const uint2 *>(v_tail_row(a, vf, b, hk, min(t + j * n_warps, t1 - 1))) + lane);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int tj = t + j * n_warps;
+            const float2 v01 = __half22float2(*reinterpret_cast<const __half2 *>(&v[j].x));
+            const float2 v23 = __half22float2(*reinterpret_cast<const __half2 *>(&v[j].y));
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+                const float ph = tj < t1 ? p[h * p_stride + tj - t0] : 0.f;
+                acc[h][0] = fmaf(ph, v01.x, acc[h][0]);
+                acc[h][1] = fmaf(ph, v01.y, acc[h][1]);
+                acc[h][2] = fmaf(ph, v23.x, acc[h][2]);
+                acc[h][3] = fmaf(ph, v23.y, acc[h][3]);
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+        float4 *r = reinterpret_cast<float4 *>(red + h * kHeadDim) + lane;
+        float4 s = *r;
+        s.x += acc[h][0]; s.y += acc[h][1]; s.z += acc[h][2]; s.w += acc[h][3];
+        *r = s;
     }
 }
 

@@ -22,26 +22,27 @@
 namespace kvq {
 
 constexpr int kQH = 4;                  // query-head slots per CTA
-constexpr int kGqaMaxChunk = 2048;      // tokens per segment: 4 x 2048 fp32 scores (3072 fit too but measured 10 % slower)
-constexpr int kGqaTailOff = 2048;       // per-warp region: [value ring | operand tiles (2 KB) | fp16-tail partial (2 KB)]
+constexpr int kGqaMaxScores = 2048, kGqaMaxScores3 = 2112;   // tokens the score buffer holds (x 4 heads): two CTAs per SM
 
 struct GqaSmem {
-    float *scores;          // [kQH][n_scores]
+    float *scores;          // [1 << ks_log2][kQH][n_scores]
     unsigned char *ring;    // this warp's region
     __half *q;              // [kQH][kHeadDim]
     float *misc;            // [64]
-    int n_scores;
+    int n_scores, ks_log2;
 };
 
-// Scale/zero tiles of a key warp tile are double-buffered (the operands are formed k-step by k-step, so a tile's
-// scales stay in use until its last stage).  3-bit keys: 8 groups per tile, a [128][16 B] scale tile followed by the
-// zero tile; other widths (<= 4 groups per tile): one [128][16 B] tile whose rows hold 4 scales then 4 zeros.
-template <int KB> constexpr int gqa_sz_bytes() { return KB == 3 ? 4096 : 2048; }
-template <int KB> constexpr int gqa_zero_off() { return KB == 3 ? 2048 : 8; }
+// A stage carries the scale and zero rows of its channels behind the codes.  3-bit keys: 8 groups per tile, 16-byte scale
+// rows followed by the zero rows; other widths (<= 4 groups per tile): 16-byte rows that hold 4 scales then 4 zeros.
+template <int KB> constexpr int gqa_zero_off() { return KB == 3 ? KGeom<KB>::ROWS * 16 : 8; }
+template <int KB> using GqaKRing = KRing<KB, KGeom<KB>::ROWS * (KB == 3 ? 32 : 16), (KB == 4 || KB == 3) ? 3 : 4>;
+template <int VB> using GqaVGeom = VGeom<VB, VB == 4 ? 3 : VB == 2 ? 5 : 7>;
+// operand tiles of the values: 512 bytes per channel group (4 / 2 / 2 groups at most)
+template <int VB> constexpr int gqa_op_bytes() { return VB == 4 ? 2048 : 1024; }
 
 template <int KB, int VB> constexpr int gqa_region_bytes() {
-    constexpr int k = KGeom<KB>::NS * KGeom<KB>::STAGE_BYTES + 2 * gqa_sz_bytes<KB>();
-    constexpr int v = VGeom<VB>::NS * VGeom<VB>::STAGE_BYTES + kGqaTailOff + kQH * kHeadDim * 4;
+    constexpr int k = GqaKRing<KB>::BYTES;
+    constexpr int v = GqaVGeom<VB>::NS * GqaVGeom<VB>::STAGE_BYTES + gqa_op_bytes<VB>();
     return k > v ? k : v;
 }
 
@@ -49,14 +50,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     uint2 v;
     asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(addr));
     return v;
-}
-
-// hi / lo part of the exact product q * s for a pair of channels: even columns carry hi = rn(q * s), odd columns
-// lo = q * s - hi (exact in fp16).  neg_mask is 0 in even-column lanes and all ones in odd-column lanes:
-// fma(q, s, +0) = hi, fma(q, s, -hi) = lo.
-__device__ __forceinline__ uint32_t hilo(__half2 q, __half2 s, uint32_t neg_mask) {
-    const uint32_t hi = as_u32(__hmul2(q, s));
-    return as_u32(__hfma2(q, s, as_h2((hi ^ 0x80008000u) & neg_mask)));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -86,40 +79,36 @@ __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half
             mma16816(c, ra[S].z, rb[S].z, ra[S].w, rb[S].w, qf[S].z, qf[S].w);
         }
         if (tig < 2) {                                         // columns 2 tig, 2 tig + 1 = heads 2 tig, 2 tig + 1
-            if (a.round_scores) {
-                const float2 r0 = __half22float2(__floats2half2_rn(c[0], c[1])), r1 = __half22float2(__floats2half2_rn(c[2], c[3]));
-                c[0] = r0.x; c[1] = r0.y; c[2] = r1.x; c[3] = r1.y;
+            for (int p = 0; p < (1 << sm.ks_log2); ++p) {      // the whole score in the first partial, zero in the others
+                float *d0 = sm.scores + (p * kQH + 2 * tig) * sm.n_scores - t0, *d1 = d0 + sm.n_scores;
+                if (ta < t1) { d0[ta] = p ? 0.f : c[0]; d1[ta] = p ? 0.f : c[1]; }
+                if (tb < t1) { d0[tb] = p ? 0.f : c[2]; d1[tb] = p ? 0.f : c[3]; }
             }
-            float *d0 = sm.scores + (2 * tig) * sm.n_scores, *d1 = d0 + sm.n_scores;
-            if (ta < t1) { d0[ta - t0] = c[0] * a.softmax_scale; d1[ta - t0] = c[1] * a.softmax_scale; }
-            if (tb < t1) { d0[tb - t0] = c[2] * a.softmax_scale; d1[tb - t0] = c[3] * a.softmax_scale; }
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same ring and stage geometry as the
-// single-head kernel (KGeom); scores[h][t - t0] receive the scaled scores.
+// q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same stage geometry, tile order and channel
+// splits as the single-head kernel; scores[split][h][t - t0] receive the raw scores.
 template <int KB>
 __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const GqaSmem &sm, int t0, int hi, const __half *kf,
                                               int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
+    using R = GqaKRing<KB>;
     using F = Fields<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int Gk = a.k_group;
     const int n_words = a.Tkq / G::FPI;
-    const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;
-    const int my_tiles = (n_tiles - warp + kMmaWarps - 1) / kMmaWarps;
-    if (my_tiles <= 0) {
-        __syncthreads();                                       // q is in shared memory
-        if (tail_lo < t1) gqa_qk_tail(a, kf, b, hk, sm, t0, tail_lo, t1);
-        return;
-    }
+    const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;                         // <= 0: no packed keys in this segment
+    const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = kMmaWarps >> sm.ks_log2;
+    const int my_tiles = (n_tiles - wt + tile_lanes - 1) / tile_lanes;
+    const int ch0 = split * (kHeadDim >> sm.ks_log2), steps = (kHeadDim / 32) >> sm.ks_log2;   // channels of this warp
+    const int tile_stages = G::NSTAGE >> sm.ks_log2;
     const int kc_sD = (int)a.kc_sD, ks_sD = (int)a.ks_sD;
     const uint32_t ring_s = smem_u32(sm.ring);
-    const uint32_t sz_s = ring_s + G::NS * G::STAGE_BYTES;                    // two scale/zero tile buffers
-    constexpr int SZB = gqa_sz_bytes<KB>(), ZOFF = gqa_zero_off<KB>();
+    constexpr int ZOFF = gqa_zero_off<KB>();
     const int gr = lane % G::GPR, row0 = lane / G::GPR;
     const uint32_t cp_dst = ring_s + row0 * G::RS + gr * 16;
     constexpr int FH = (KB == 3) ? 2 : 16 / KB;                                // fields per half-word: 4 / 8 / 16
@@ -128,14 +117,14 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
     constexpr int NACC = (KB == 3) ? 8 : NBK * MPB;                            // accumulators per tile: 8 words / 16 token pairs
     const uint32_t ldk_s = ring_s + ((lane & 7) + 8 * ((lane >> 3) & 1)) * G::RS + (lane >> 4) * 16;
     const uint32_t w3_s = ring_s + (2 * tig) * G::RS;                          // 3-bit: word rows 2 tig, +1, +8, +9
-    const uint32_t szrow_s = sz_s + (2 * tig) * 16;                            // + buffer + 256 ksx [+16 | +128 | +144] [+ZOFF zero]
-    const uint32_t q_s = smem_u32(sm.q) + (g >> 1) * (kHeadDim * 2) + (2 * tig) * 2;   // this column's head; + 32 ksx [+16]
+    const uint32_t szrow_s = ring_s + G::CODE_BYTES + (2 * tig) * 16;         // + slot + 256 k [+16 | +128 | +144] [+ZOFF zero]
+    const uint32_t szm_s = ring_s + G::CODE_BYTES + (KB == 3 ? ZOFF : 0) + (lane & 15) * 16;   // zero tile as an A operand
+    const uint32_t q_s = smem_u32(sm.q) + (g >> 1) * (kHeadDim * 2) + (ch0 + 2 * tig) * 2;     // this column's head; + 32 per k-step [+16]
     const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;
     const int ngw = (G::WT + Gk - 1) / Gk;                                     // groups per warp tile: 8 (3-bit) / 4 / 2
     const bool wide = Gk >= 128;                                               // 128-token groups (else 64)
-    const uint32_t szcp_dst = sz_s + lane * 16;
-    const int tile_words = kMmaWarps * G::WT / G::FPI;
-    const int tile_groups = kMmaWarps * G::WT / Gk;
+    const int tile_words = tile_lanes * G::WT / G::FPI;
+    const int tile_groups = tile_lanes * G::WT / Gk;
     // 3-bit keys: field g of a word sits at bits 3g..3g+2; one byte permute brings the two bytes that hold it (of both
     // channel words) into the 16-bit halves, a mask isolates it in place at bit p0 = 3g mod 8 (<= 7: linear fp16 range).
     // Fields 8..10 (rows g + 8, g < 3) sit in byte 3 at bits 0, 3, 6 (the last one 2 bits wide).
@@ -147,77 +136,76 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
     const int p1 = 3 * (g < 3 ? g : 0);
     const float sc0 = __int_as_float((151 - p0) << 23), sc1 = __int_as_float((151 - p1) << 23);   // 2^(24 - position)
 
-    const int32_t *tb_cur = kc + (int64_t)row0 * kc_sD + (t0 + warp * G::WT) / G::FPI + 4 * gr;
-    const __half *ks_cur = ks + (int64_t)lane * ks_sD + (t0 + warp * G::WT) / Gk;
-    const __half *kz_cur = kz + (int64_t)lane * ks_sD + (t0 + warp * G::WT) / Gk;
-    int wcol_cur = (t0 + warp * G::WT) / G::FPI + 4 * gr;
-    bool ok_cur = wcol_cur < n_words;
+    // the next stage to issue: its addresses, its word column, its position in its tile and the tiles left.  A stage of 16
+    // channels takes one scale / zero copy per lane (zeros: lanes 16-31), one of 32 channels two.
+    const int32_t *iss = kc + (int64_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr;
+    constexpr bool kOneSz = G::ROWS == 16;
+    const int sz_row = kOneSz ? (lane & 15) : lane;
+    const bool sz_zero = kOneSz && lane >= 16;
+    const __half *iss_s = (sz_zero ? kz : ks) + (int64_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk;
+    const ptrdiff_t sz_gap = kOneSz ? 0 : kz - ks;
+    const uint32_t szcp_dst = ring_s + G::CODE_BYTES + sz_row * 16 + (sz_zero ? ZOFF : 0);
+    int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
+    uint32_t iss_slot = 0, slot = 0;
+    bool iss_ok = iss_col < n_words;
 
-    auto issue_stage = [&](const int32_t *tb, bool ok, int sst) {
-        if (ok) {
-            const uint32_t dst = cp_dst + (sst % G::NS) * G::STAGE_BYTES;
+    auto issue_stage = [&]() {
+        if (iss_tiles > 0) {
+            if (iss_ok) {
 #pragma unroll
-            for (int i = 0; i < G::GPL; ++i)
-                cp_async<16>(dst + i * G::RPI * G::RS, tb + (sst * G::ROWS + i * G::RPI) * kc_sD);
+                for (int i = 0; i < G::GPL; ++i)
+                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, iss + i * G::RPI * kc_sD);
+            }
+            const uint32_t d = szcp_dst + iss_slot;
+            if (KB == 3) { cp_async<16>(d, iss_s); cp_async<16>(d + ZOFF, iss_s + sz_gap); }
+            else if (ngw == 4) { cp_async<8>(d, iss_s); if (!kOneSz) cp_async<8>(d + ZOFF, iss_s + sz_gap); }
+            else { cp_async<4>(d, iss_s); if (!kOneSz) cp_async<4>(d + ZOFF, iss_s + sz_gap); }
+        }
+        cp_async_commit();
+        iss_slot = iss_slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : iss_slot + R::STAGE_BYTES;
+        iss += G::ROWS * kc_sD;
+        iss_s += G::ROWS * ks_sD;
+        if (++iss_st == tile_stages) {
+            iss_st = 0;
+            iss += tile_words - tile_stages * (G::ROWS * kc_sD);
+            iss_s += tile_groups - tile_stages * (G::ROWS * ks_sD);
+            iss_col += tile_words;
+            iss_ok = iss_col < n_words;
+            --iss_tiles;
         }
     };
-    auto issue_sz = [&](const __half *ps, const __half *pz, uint32_t buf) {    // channel rows lane, lane + 32, ...
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int off = 32 * i * ks_sD;
-            const uint32_t d = szcp_dst + buf + i * 512;
-            if (KB == 3) { cp_async<16>(d, ps + off); cp_async<16>(d + ZOFF, pz + off); }
-            else if (ngw == 4) { cp_async<8>(d, ps + off); cp_async<8>(d + ZOFF, pz + off); }
-            else { cp_async<4>(d, ps + off); cp_async<4>(d + ZOFF, pz + off); }
-        }
-    };
 
-    issue_sz(ks_cur, kz_cur, 0u);
-    issue_stage(tb_cur, ok_cur, 0);
-    cp_async_commit();
-    issue_stage(tb_cur, ok_cur, 1);
-    cp_async_commit();
-    issue_stage(tb_cur, ok_cur, 2);
-    cp_async_commit();
+#pragma unroll 1
+    for (int q = 0; q < R::P; ++q) issue_stage();
     __syncthreads();                                           // q is in shared memory (stored by the caller without a barrier)
     if (tail_lo < t1) gqa_qk_tail(a, kf, b, hk, sm, t0, tail_lo, t1);
 
     for (int j = 0; j < my_tiles; ++j) {
-        const int tile0 = t0 + (j * kMmaWarps + warp) * G::WT;
-        const bool have_next = j + 1 < my_tiles;
-        const int32_t *tb_nxt = tb_cur + tile_words;
-        const bool ok_nxt = have_next && (wcol_cur + tile_words < n_words);
-
-        const uint32_t szbuf = (j & 1) ? SZB : 0u;
+        const int tile0 = t0 + (j * tile_lanes + wt) * G::WT;
+        uint32_t q_cur = q_s;
         // groups of this tile that hold tokens below hi: operands of the others are never formed (their scale/zero
         // words lie beyond the packed prefix and may hold anything, and 0 * NaN would poison a shared accumulator)
         const int nvg = min(ngw, (hi - tile0 + Gk - 1) / Gk);
-        // the zero-term MMAs (one per k-step) rotate over four accumulators so that consecutive ones do not wait for each other
-        float acc[NACC][4], accz[4][4];
+        float acc[NACC][4], zsum = 0.f;
 #pragma unroll
         for (int m = 0; m < NACC; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) accz[m][0] = accz[m][1] = accz[m][2] = accz[m][3] = 0.f;
 
+        // LOOPNOTE
+#pragma unroll 1
+        for (int it = 0; it < steps; ++it) {
+          float accz[4] = {0.f, 0.f, 0.f, 0.f};               // zero terms of two k-steps
 #pragma unroll
-        for (int st = 0; st < G::NSTAGE; ++st) {
-            if (st + G::P < G::NSTAGE) {
-                issue_stage(tb_cur, ok_cur, st + G::P);
-            } else {
-                issue_stage(tb_nxt, ok_nxt, st + G::P - G::NSTAGE);
-            }
-            // the next tile's scale/zero tile goes to the other buffer (last read one tile ago)
-            if (st == 0 && have_next) issue_sz(ks_cur + tile_groups, kz_cur + tile_groups, szbuf ^ SZB);
-            cp_async_commit();
-            cp_async_wait<G::P>();                             // stage st has landed (this tile's scale/zero tile long before)
+          for (int s2 = 0; s2 < 2 / G::KSPS; ++s2) {
+            issue_stage();
+            cp_async_wait<R::P>();
             __syncwarp();
-            const uint32_t stage_s = (st % G::NS) * G::STAGE_BYTES;
+            const uint32_t stage_s = slot;
 #pragma unroll
             for (int k = 0; k < G::KSPS; ++k) {
-                const int ksx = st * G::KSPS + k;
-                const uint32_t q01u = lds32(q_s + 32 * ksx), q89u = lds32(q_s + 32 * ksx + 16);
+                const uint32_t q01u = lds32(q_cur), q89u = lds32(q_cur + 16);
+                q_cur += 32;
                 const __half2 q01 = as_h2(q01u), q89 = as_h2(q89u);
-                const uint32_t zrow = szrow_s + szbuf + 256 * ksx;   // scale rows 16 ksx + 2 tig (+1, +8, +9); zeros + ZOFF
+                const uint32_t zrow = szrow_s + slot + 256 * k;      // scale rows 16 k + 2 tig (+1, +8, +9); zeros + ZOFF
                 if constexpr (KB == 3) {
                     // every word is its own group: per word j one B operand and one code MMA (rows = its 11 tokens); words
                     // are taken in pairs so that scales arrive as 32-bit loads.  The zero terms sum_d q[d] * zero[d, j] of
@@ -228,8 +216,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                     {
                         uint32_t za0, za2;
                         asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                                     : "=r"(za0), "=r"(za2) : "r"(sz_s + szbuf + ZOFF + (16 * ksx + (lane & 15)) * 16));
-                        mma16816(accz[ksx & 3], za0, 0u, za2, 0u, q01u & ~neg_mask, q89u & ~neg_mask);
+                                     : "=r"(za0), "=r"(za2) : "r"(szm_s + slot + 256 * k));
+                        mma16816(accz, za0, 0u, za2, 0u, q01u & ~neg_mask, q89u & ~neg_mask);
                     }
 #pragma unroll
                     for (int jp = 0; jp < 4; ++jp) {
@@ -258,8 +246,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                     {
                         uint32_t za0, za2;
                         asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                                     : "=r"(za0), "=r"(za2) : "r"(sz_s + szbuf + (16 * ksx + (lane & 15)) * 16));
-                        mma16816(accz[ksx & 3], za0, 0u, za2, 0u, q01u & ~neg_mask, q89u & ~neg_mask);
+                                     : "=r"(za0), "=r"(za2) : "r"(szm_s + slot + 256 * k));
+                        mma16816(accz, za0, 0u, za2, 0u, q01u & ~neg_mask, q89u & ~neg_mask);
                     }
                     // B operands of the tile's groups (<= 4: k_group >= 64)
                     const uint2 sA = lds64(zrow), sB = lds64(zrow + 16), sC = lds64(zrow + 128), sD = lds64(zrow + 144);
@@ -275,7 +263,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                             b[jk][0] = b[jk][1] = 0u;
                         }
                     }
-                    using H = KHalf<KB>;
+                    using H = VHalf<KB>;
                     const uint32_t lsrc = ldk_s + stage_s + (k * 16) * G::RS;
 #pragma unroll
                     for (int pb2 = 0; pb2 < NBK / 2; ++pb2) {
@@ -298,13 +286,16 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                     }
                 }
             }
-            __syncwarp();                                      // slot st % NS may be refilled
+            __syncwarp();                                      // the slot may be refilled
+            slot = slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : slot + R::STAGE_BYTES;
+          }
+          zsum += accz[0] + accz[1];
         }
 
         // ---- epilogue: lane (g, tig) holds, per accumulator, row g / g + 8 of head tig as (hi, lo) ------------
-        // row g = group g of the tile: its zero term for head tig (hi + lo columns, summed over the rotating accumulators)
-        const float zsum = ((accz[0][0] + accz[0][1]) + (accz[1][0] + accz[1][1])) + ((accz[2][0] + accz[2][1]) + (accz[3][0] + accz[3][1]));
-        float *dst_h = sm.scores + tig * sm.n_scores - t0;
+        // row g = group g of the tile: its zero term for head tig (hi + lo columns)
+        
+        float *dst_h = sm.scores + (split * kQH + tig) * sm.n_scores - t0;
         if constexpr (KB == 3) {
 #pragma unroll
             for (int jw = 0; jw < 8; ++jw) {
@@ -312,14 +303,9 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                 const int ta = tile0 + 11 * jw + g, tb = ta + 8;
                 float s0 = fmaf(acc[jw][0] + acc[jw][1], sc0, corr);
                 float s1 = fmaf(acc[jw][2] + acc[jw][3], sc1, corr);
-                if (a.round_scores) {
-                    const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                    s0 = r.x;
-                    s1 = r.y;
-                }
                 if (11 * jw + tile0 < hi) {                    // words are whole or absent (hi is a group multiple)
-                    dst_h[ta] = s0 * a.softmax_scale;
-                    if (g < 3) dst_h[tb] = s1 * a.softmax_scale;
+                    dst_h[ta] = s0;
+                    if (g < 3) dst_h[tb] = s1;
                 }
             }
         } else {
@@ -335,23 +321,13 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 #pragma unroll
                     for (int ip = 0; ip < MPB; ++ip) {
                         const int m = bb * MPB + ip;
-                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - F::pos(2 * ip))), corr);
-                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - F::pos(2 * ip + 1))), corr);
-                        if (a.round_scores) {
-                            const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                            s0 = r.x;
-                            s1 = r.y;
-                        }
-                        *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0 * a.softmax_scale, s1 * a.softmax_scale);
+                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - VHalf<KB>::pos(2 * ip))), corr);
+                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - VHalf<KB>::pos(2 * ip + 1))), corr);
+                        *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0, s1);
                     }
                 }
             }
         }
-        tb_cur = tb_nxt;
-        ok_cur = ok_nxt;
-        wcol_cur += tile_words;
-        ks_cur += tile_groups;
-        kz_cur += tile_groups;
     }
     cp_async_wait<0>();
 }
@@ -362,7 +338,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 template <int VB, int MODE>
 __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int32_t *vc, const __half *vs,
                                               const __half *vz, const GqaSmem &sm, int t0, int hi) {
-    using G = VGeom<VB>;
+    using G = GqaVGeom<VB>;
     using F = VHalf<VB>;
     constexpr int NB = G::GPT;                                // 16-byte blocks per token row: 1 / 2 / 4
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
@@ -424,12 +400,10 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
 #pragma unroll
     for (int m = 0; m < 8; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
     // 1-bit values in groups of 64 channels: a 16-byte block (128 channels) then spans two groups, and the rows of an
-    // MMA (lane octet g = channels 16 g .. 16 g + 15) lie in group g / 4.  Every code tile is multiplied twice, by the
-    // operands of group 0 and of group 1, and a lane keeps the product of its own group.
+    // MMA (lane octet g = channels 16 g .. 16 g + 15) lie in group g / 4.  Every code tile is multiplied twice, the rows of
+    // group 1 cleared by the operands of group 0 and the other way round, into the same accumulators.
     const bool split = VB == 1 && Gv == 64;
-    float acc2[VB == 1 ? 8 : 1][4];
-#pragma unroll
-    for (int m = 0; m < (VB == 1 ? 8 : 1); ++m) acc2[m][0] = acc2[m][1] = acc2[m][2] = acc2[m][3] = 0.f;
+    const uint32_t rows0 = !split || g < 4 ? 0xffffffffu : 0u, rows1 = g >= 4 ? 0xffffffffu : 0u;
     const uint32_t ones = 0x3c003c00u;
     constexpr int kFlush = 16;                                 // short accumulation chains (see the single-head kernel)
     float sum[8][2], sumz[2] = {0.f, 0.f};
@@ -438,15 +412,8 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     auto flush = [&]() {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
-            if constexpr (VB == 1) {
-                const bool second = split && g >= 4;
-                sum[m][0] += second ? acc2[m][0] : acc[m][0];
-                sum[m][1] += second ? acc2[m][2] : acc[m][2];
-                acc2[m][0] = acc2[m][1] = acc2[m][2] = acc2[m][3] = 0.f;
-            } else {
-                sum[m][0] += acc[m][0];
-                sum[m][1] += acc[m][2];
-            }
+            sum[m][0] += acc[m][0];
+            sum[m][1] += acc[m][2];
             acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
         }
         sumz[0] += accz[0][0] + accz[1][0];
@@ -520,8 +487,8 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
 #pragma unroll
             for (int bb = 0; bb < NB; ++bb) {
                 uint32_t rlo[F::N], rhi[F::N];
-                F::unpack(x[bb][0], rlo);
-                F::unpack(x[bb][1], rhi);
+                F::unpack(VB == 1 ? x[bb][0] & rows0 : x[bb][0], rlo);
+                F::unpack(VB == 1 ? x[bb][1] & rows0 : x[bb][1], rhi);
                 // the block's channel group: v_group is 32 (4-bit values only), 64 or 128
                 const int j32 = (bb * CPB) / 32 < 4 ? (bb * CPB) / 32 : 3, j64 = (bb * CPB) / 64;
                 const uint32_t bx = Gv == 32 ? b[j32][0] : Gv == 64 ? b[j64][0] : b[0][0];
@@ -531,9 +498,11 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
                     mma16816(acc[bb * MPB + i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], bx, by);
                 if constexpr (VB == 1) {
                     if (split) {
+                        F::unpack(x[bb][0] & rows1, rlo);
+                        F::unpack(x[bb][1] & rows1, rhi);
 #pragma unroll
                         for (int i = 0; i < F::N; i += 2)
-                            mma16816(acc2[i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b[1][0], b[1][1]);
+                            mma16816(acc[i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b[1][0], b[1][1]);
                     }
                 }
             }
@@ -570,7 +539,7 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of head group s (sequence b, kv head hk, quad of query heads); segment `seg` of `cnt`.
 template <int KB, int VB>
-__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int qhv, int s, int t0, int t1, int seg,
+__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int ks_log2, int qhv, int s, int t0, int t1, int seg,
                                             int cnt, int n_whole, float *__restrict__ parts,
                                             unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -578,12 +547,12 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     constexpr int kRegion = gqa_region_bytes<KB, VB>();
     GqaSmem sm;
     sm.n_scores = n_scores;
+    sm.ks_log2 = ks_log2;
     sm.scores = reinterpret_cast<float *>(smem_raw);
-    unsigned char *after_scores = smem_raw + (size_t)kQH * n_scores * 4;
+    unsigned char *after_scores = smem_raw + ((size_t)kQH * n_scores << ks_log2) * 4;
     sm.ring = after_scores + warp * kRegion;
     sm.q = reinterpret_cast<__half *>(after_scores + kMmaWarps * kRegion);
     sm.misc = reinterpret_cast<float *>(sm.q + kQH * kHeadDim);
-    float *tail_part = reinterpret_cast<float *>(sm.ring + VGeom<VB>::NS * VGeom<VB>::STAGE_BYTES + kGqaTailOff);
 
     const int n_rep = a.nh / a.nh_kv, nq = n_rep / qhv;                // quads per kv head
     const int b = s / (a.nh_kv * nq), hk = (s / nq) % a.nh_kv, h_first = hk * n_rep + (s % nq) * qhv;
@@ -591,76 +560,48 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     // q of the quad (head slots beyond qhv repeat the last head: their columns are computed and dropped)
     {
-        const int hs = min(tid >> 5, qhv - 1);                          // warp w stores head slot w
+        const int slot = tid >> 6, hs = min(slot, qhv - 1);              // two warps store a head slot
         const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + hs) * a.q_sH;
-        *reinterpret_cast<uint2 *>(sm.q + warp * kHeadDim + 4 * lane) = *reinterpret_cast<const uint2 *>(q + 4 * lane);
+        *reinterpret_cast<uint32_t *>(sm.q + slot * kHeadDim + 2 * (tid & 63)) = *reinterpret_cast<const uint32_t *>(q + 2 * (tid & 63));
     }
+    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
+    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
+    prefetch_v_tail(a, vf, b, hk, v_lo, t1, tid, kMmaThreads);
 
     // ---- 1. scores ------------------------------------------------------------------------------
     const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
     {
-        const int hi = min(t1, a.Tkq);
-        if (t0 < hi) {
-            const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
-            const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-            const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-            gqa_qk_packed<KB>(a, kc, ks, kz, sm, t0, hi, kf, max(t0, a.Tkq), t1, b, hk);
-        } else {
-            __syncthreads();
-            if (t0 < t1) gqa_qk_tail(a, kf, b, hk, sm, t0, t0, t1);
-        }
+        const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
+        const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
+        const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
+        gqa_qk_packed<KB>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
-    const int v_hi = min(t1, a.Tvq);
-    if (t0 < v_hi) gqa_pv_packed<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);   // start filling this warp's value ring now
+    gqa_pv_packed<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
-    // ---- 2. softmax numerators: warp w owns head slot w -------------------------------------------
-    // The fp16 value tail of this segment is fetched into registers first (its latency is spent under the softmax).
-    const int n = t1 - t0;
-    const int v_lo = max(t0, a.Tvq);
-    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
-    const int co = tid & 15, tl = tid >> 4;
-    uint4 vt[16];
-    auto load_tail_round = [&](int base) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int t = base + tl + 8 * j;
-            vt[j] = (t < t1) ? __ldg(reinterpret_cast<const uint4 *>(v_tail_row(a, vf, b, hk, t)) + co) : make_uint4(0u, 0u, 0u, 0u);
-        }
-    };
-    if (v_lo < t1) load_tail_round(v_lo);
-
-    const int h_mine = h_first + min(warp, qhv - 1);
+    // ---- 2. softmax numerators: two warps per head slot --------------------------------------------
+    const int n = t1 - t0, n4 = (n + 3) >> 2, hs_mine = warp >> 1;
+    const int h_mine = h_first + min(hs_mine, qhv - 1);
     float m = kMaskFloor;
-    const int n4 = (n + 3) >> 2;
-    float4 *sc4 = reinterpret_cast<float4 *>(sm.scores + warp * n_scores);
-#pragma unroll 4
-    for (int i = lane; i < n4; i += 32) {
-        float4 v = sc4[i];
-        if (a.mask) {
-            const int t = t0 + 4 * i;
-            v.x = fmaxf(v.x + attn_mask_at(a, b, h_mine, min(t, a.T - 1)), kMaskFloor);
-            v.y = fmaxf(v.y + attn_mask_at(a, b, h_mine, min(t + 1, a.T - 1)), kMaskFloor);
-            v.z = fmaxf(v.z + attn_mask_at(a, b, h_mine, min(t + 2, a.T - 1)), kMaskFloor);
-            v.w = fmaxf(v.w + attn_mask_at(a, b, h_mine, min(t + 3, a.T - 1)), kMaskFloor);
-            sc4[i] = v;
-        }
-        if (4 * i + 3 >= n) {
-            if (4 * i + 1 >= n) v.y = -INFINITY;
-            if (4 * i + 2 >= n) v.z = -INFINITY;
-            v.w = -INFINITY;
-            sc4[i] = v;
-        }
+    float4 *sc4 = reinterpret_cast<float4 *>(sm.scores + hs_mine * n_scores);
+#pragma unroll 2
+    for (int i = tid & 63; i < n4; i += 64) {
+        float4 v = score_quad(a, sc4 + i, kQH * (n_scores >> 2), ks_log2);
+        if (a.mask) mask_quad(a, b, h_mine, t0 + 4 * i, v);
+        if (4 * i + 3 >= n) pad_quad(v, n - 4 * i);
+        sc4[i] = v;
         m = fmaxf(fmaxf(m, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
     m = warp_max(m);
-    __syncwarp();
+    if (lane == 0) sm.misc[warp] = m;
+    __syncthreads();
+    m = fmaxf(sm.misc[2 * hs_mine], sm.misc[2 * hs_mine + 1]);
     float l = 0.f;
-#pragma unroll 4
-    for (int i = lane; i < n4; i += 32) {
+#pragma unroll 2
+    for (int i = tid & 63; i < n4; i += 64) {
         float4 v = sc4[i];
         v.x = __expf(v.x - m);
         v.y = __expf(v.y - m);
@@ -670,88 +611,60 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         l += (v.x + v.y) + (v.z + v.w);
     }
     l = warp_sum(l);
-    if (lane == 0) { sm.misc[warp] = m; sm.misc[4 + warp] = l; }
+    if (lane == 0) sm.misc[8 + warp] = l;
     __syncthreads();
 
     // ---- 3. p . V -----------------------------------------------------------------------------------
-    if (v_lo < t1) {
-#pragma unroll 1
-        for (int hs = 0; hs < kQH; ++hs) {
-            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            const float *ph = sm.scores + hs * n_scores - t0;
-            for (int base = v_lo; base < t1; base += 128) {
-                if (base > v_lo || hs > 0) { if (t1 - v_lo > 128) load_tail_round(base); }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int t = base + tl + 8 * j;
-                    const float p = (t < t1) ? ph[t] : 0.f;
-                    const __half2 *h = reinterpret_cast<const __half2 *>(&vt[j]);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float2 f = __half22float2(h[k]);
-                        acc[2 * k] = fmaf(p, f.x, acc[2 * k]);
-                        acc[2 * k + 1] = fmaf(p, f.y, acc[2 * k + 1]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);
-            if (lane < 16) {
-                float4 *dst = reinterpret_cast<float4 *>(tail_part + hs * kHeadDim + 8 * co);
-                dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-            }
-        }
-    } else {
-        for (int i = lane; i < kQH * kHeadDim; i += 32) tail_part[i] = 0.f;
-    }
-    if (t0 < v_hi) gqa_pv_packed<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
-    else for (int i = lane; i < kQH * kHeadDim; i += 32) reinterpret_cast<float *>(sm.ring)[i] = 0.f;
+    gqa_pv_packed<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    __syncwarp();
+    if (v_lo < t1) pv_tail<kQH>(a, vf, b, hk, sm.scores, n_scores, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();
 
-    // ---- 4. finish / merge: thread tid owns channel tid of every head ----------------------------------
+    // ---- 4. finish / merge: a thread owns channel ch of head slots 2 hp, 2 hp + 1 -------------------------
     constexpr int kPart = kPartStride;
-    float o[kQH];
+    const int ch = tid & (kHeadDim - 1), hp = tid >> 7, n_mine = max(0, min(2, qhv - 2 * hp));
+    float o[2];
+    __half res[2] = {};
 #pragma unroll
-    for (int hs = 0; hs < kQH; ++hs) {
+    for (int i = 0; i < 2; ++i) {
         float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < kMmaWarps; ++w) {
-            const unsigned char *reg = after_scores + w * kRegion;
-            v += reinterpret_cast<const float *>(reg)[hs * kHeadDim + tid] +
-                 reinterpret_cast<const float *>(reg + VGeom<VB>::NS * VGeom<VB>::STAGE_BYTES + kGqaTailOff)[hs * kHeadDim + tid];
-        }
-        o[hs] = v;
+        for (int w = 0; w < kMmaWarps; ++w) v += reinterpret_cast<const float *>(after_scores + w * kRegion)[(2 * hp + i) * kHeadDim + ch];
+        o[i] = v;
     }
-    __half res[kQH];
+    __half *out = static_cast<__half *>(a.out) + (int64_t)b * a.o_sB + (int64_t)(h_first + 2 * hp) * a.o_sH + ch;
     if (cnt == 1) {
 #pragma unroll
-        for (int hs = 0; hs < kQH; ++hs) {
-            if (hs < qhv) {
-                __half *out = static_cast<__half *>(a.out) + (int64_t)b * a.o_sB + (int64_t)(h_first + hs) * a.o_sH;
-                res[hs] = __float2half_rn(o[hs] / sm.misc[4 + hs]);
-                out[tid] = res[hs];
+        for (int i = 0; i < 2; ++i) {
+            if (i < n_mine) {
+                const int hs = 2 * hp + i;
+                res[i] = __float2half_rn(o[i] / (sm.misc[8 + 2 * hs] + sm.misc[9 + 2 * hs]));
+                out[(int64_t)i * a.o_sH] = res[i];
             }
         }
-        peer_publish(ac, b, h_first, qhv, res, tid);
+        peer_publish(ac, b, h_first + 2 * hp, n_mine, res, ch, tid, qhv);
         return;
     }
     float *part = parts + ((int64_t)(s - n_whole) * cnt + seg) * qhv * kPart;    // partials of the cut head groups only
 #pragma unroll
-    for (int hs = 0; hs < kQH; ++hs) {
-        if (hs < qhv) {
-            part[hs * kPart + tid] = o[hs];
-            if (tid == 0) { part[hs * kPart + kHeadDim] = sm.misc[hs]; part[hs * kPart + kHeadDim + 1] = sm.misc[4 + hs]; }
+    for (int i = 0; i < 2; ++i) {
+        if (i < n_mine) {
+            const int hs = 2 * hp + i;
+            part[hs * kPart + ch] = o[i];
+            if (ch == 0) {
+                part[hs * kPart + kHeadDim] = fmaxf(sm.misc[2 * hs], sm.misc[2 * hs + 1]);
+                part[hs * kPart + kHeadDim + 1] = sm.misc[8 + 2 * hs] + sm.misc[9 + 2 * hs];
+            }
         }
     }
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        sm.misc[8] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
+        sm.misc[16] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
         __threadfence();
     }
     __syncthreads();
-    if (sm.misc[8] == 0.f) return;
+    if (sm.misc[16] == 0.f) return;
     // The last CTA merges the cnt segments of its head group.  A long context over few heads means a hundred or more
     // segments, and a merge that walks them one dependent round trip at a time becomes the kernel, so many 128-bit loads
     // are kept in flight: warp w merges head slot w, lane l owning channels 4l .. 4l + 3; the maximum over the segments
@@ -783,15 +696,14 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     }
     __syncthreads();
 #pragma unroll
-    for (int hs = 0; hs < kQH; ++hs) {
-        if (hs < qhv) {
-            __half *out = static_cast<__half *>(a.out) + (int64_t)b * a.o_sB + (int64_t)(h_first + hs) * a.o_sH;
-            res[hs] = stage[hs * kHeadDim + tid];
-            out[tid] = res[hs];
+    for (int i = 0; i < 2; ++i) {
+        if (i < n_mine) {
+            res[i] = stage[(2 * hp + i) * kHeadDim + ch];
+            out[(int64_t)i * a.o_sH] = res[i];
         }
     }
     if (tid == 0) counters[s] = 0u;
-    peer_publish(ac, b, h_first, qhv, res, tid);
+    peer_publish(ac, b, h_first + 2 * hp, n_mine, res, ch, tid, qhv);
 }
 
 template <int KB, int VB, bool DEV>
@@ -805,10 +717,10 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_gqa_kernel(const _
         dev_state_step(a, b);
         plan_cta(plan, b.T, blockIdx.x, group, t0, t1, seg, cnt);
         if (cnt > 1) cnt = min(cnt, (b.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < b.T) gqa_segment<KB, VB>(b, a, plan.n_scores, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        if (t0 < b.T) gqa_segment<KB, VB>(b, a, plan.n_scores, plan.ks_log2, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     } else {
         plan_cta(plan, a.T, blockIdx.x, group, t0, t1, seg, cnt);
-        gqa_segment<KB, VB>(a, a, plan.n_scores, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        gqa_segment<KB, VB>(a, a, plan.n_scores, plan.ks_log2, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     }
 }
 
@@ -828,24 +740,23 @@ int gqa_heads_per_cta(const kvq_attn_args &a) {
 }
 
 AttnPlan plan_attn_gqa(int T, int k_bits, long long head_groups) {
-    const int unit = (k_bits == 3) ? 352 : 256;
-    const int max_chunk = (k_bits == 3) ? 2816 : kGqaMaxChunk;     // whole units of 352 / 256 tokens
-    return make_attn_plan(T, unit, max_chunk, head_groups, kSmCount * 2, k_bits == 3 ? 1 : kMmaWarps);
+    return k_bits == 3 ? make_attn_plan(T, 352, KGeom<3>::WT, kGqaMaxScores3, head_groups)
+                       : make_attn_plan(T, 256, KGeom<4>::WT, kGqaMaxScores, head_groups);
 }
 
 template <int KB, int VB>
 static int launch_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, float *parts, unsigned int *counters,
                       cudaStream_t st) {
-    const size_t smem = (size_t)kQH * plan.n_scores * 4 + (size_t)kMmaWarps * gqa_region_bytes<KB, VB>() +
+    const size_t smem = ((size_t)kQH * plan.n_scores << plan.ks_log2) * 4 + (size_t)kMmaWarps * gqa_region_bytes<KB, VB>() +
                         kQH * kHeadDim * 2 + 64 * 4;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+            e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }

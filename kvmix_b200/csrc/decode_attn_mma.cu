@@ -32,17 +32,22 @@
 namespace kvq {
 
 struct MmaSmem {
-    float *scores;          // [n_scores]
+    float *scores;          // [1 << ks_log2][n_scores]
     unsigned char *ring;    // this warp's region
-    float *tailred;         // [kMmaWarps][kHeadDim] partial sums of the fp16 value tail
     __half *q;              // [kHeadDim]
-    float *misc;            // [16]
+    float *misc;            // [32]
+    int n_scores, ks_log2;
 };
+template <int KB> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, 4>;        // scale rows, then zero rows, 16 B each
+template <int KB, int VB> constexpr int warp_region_bytes() {
+    return MmaKRing<KB>::BYTES > VGeom<VB>::WARP_BYTES ? MmaKRing<KB>::BYTES : VGeom<VB>::WARP_BYTES;
+}
 
 // ---------------------------------------------------------------------------------------------
-// q . K^T over packed keys for tokens [t0, hi) (t0 is a multiple of 1024, or 352 for 3-bit keys).
-// Scores (already multiplied by softmax_scale) go to sm.scores[t - t0].  Warps work independently:
-// warp w takes warp tiles w, w+4, ... and streams their code words through its own ring.
+// q . K^T over packed keys for tokens [t0, hi) (t0 is a multiple of 256, or 352 for 3-bit keys).
+// Raw fp32 scores go to sm.scores[split][t - t0].  Warps work independently: with `ns` = 1 << ks_log2 channel splits, warp w
+// takes channels [128 / ns * (w % ns), ..) of the warp tiles w / ns, w / ns + 8 / ns, ... and streams their code words
+// through its own ring.
 __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half *kf, int b, int hk, const MmaSmem &sm,
                                             int t0, int lo, int t1);
 
@@ -53,22 +58,20 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                                               const __half *kz, const MmaSmem &sm, int t0, int hi,
                                               const __half *kf, int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
+    using R = MmaKRing<KB>;
     using F = Fields<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int Gk = a.k_group;
     const int n_words = a.Tkq / G::FPI;                       // valid code words per channel row
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;
-    const int my_tiles = (n_tiles - warp + kMmaWarps - 1) / kMmaWarps;   // tiles warp, warp+4, ...
-    if (my_tiles <= 0) {
-        __syncthreads();                                       // q is in shared memory (see below)
-        if (tail_lo < t1) qk_tail_mma(a, kf, b, hk, sm, t0, tail_lo, t1);
-        return;
-    }
+    const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = kMmaWarps >> sm.ks_log2;
+    const int my_tiles = (n_tiles - wt + tile_lanes - 1) / tile_lanes;   // <= 0: none
+    const int ch0 = split * (kHeadDim >> sm.ks_log2), steps = (kHeadDim / 32) >> sm.ks_log2;   // channels of this warp
+    const int tile_stages = G::NSTAGE >> sm.ks_log2;
 
     const int kc_sD = (int)a.kc_sD, ks_sD = (int)a.ks_sD;
     // ---- per-lane constants --------------------------------------------------------------------
     const uint32_t ring_s = smem_u32(sm.ring);
-    const uint32_t sz_s = ring_s + G::NS * G::STAGE_BYTES;                    // [2][128][8] halfs
     const int gr = lane % G::GPR, row0 = lane / G::GPR;
     const uint32_t cp_dst = ring_s + row0 * G::RS + gr * 16;                   // + slot*STAGE + i*RPI*RS
     // 3-bit: octet g owns the word of group g (11 tokens), fetched with plain 32-bit loads.
@@ -85,129 +88,119 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     constexpr int HW = 2;                                                      // 4-bit: code words per octet per half
     const uint32_t frag_s = ring_s + (2 * tig) * G::RS + ((KB == 4) ? 8 * g : 4 * g);   // 3-bit and 4-bit (plain loads)
     const uint32_t ldk_s = ring_s + ((lane & 7) + 8 * ((lane >> 3) & 1)) * G::RS + (lane >> 4) * 16;   // + k*16*RS + 32*pair
-    // ldmatrix.x4 row addresses: lanes 0-7 scale rows 16ksx+0..7, 8-15 scale rows +8..15, 16-31 the same of the zero tile
-    const uint32_t ldm_s = sz_s + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16 + (lane >> 4) * 2048;
-    const uint32_t q_s = smem_u32(sm.q) + (2 * tig) * 2;                       // + 32 ksx [+16]
+    // ldmatrix.x4 row addresses: lanes 0-7 scale rows 0..7 of a k-step, 8-15 scale rows 8..15, 16-31 the same of the zero rows
+    const uint32_t ldm_s = ring_s + G::CODE_BYTES + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16 + (lane >> 4) * (G::ROWS * 16);
+    const uint32_t q_s = smem_u32(sm.q) + (ch0 + 2 * tig) * 2;                 // + 32 per k-step [+16]
     const int ngw = (G::WT + Gk - 1) / Gk;                                     // groups per warp tile: 8 / 4 / 2
-    const uint32_t szcp_dst = sz_s + lane * 16;                                // + i*512
-    const int tile_words = kMmaWarps * G::WT / G::FPI;                         // word-column distance between my tiles
-    const int tile_groups = kMmaWarps * G::WT / Gk;
+    const uint32_t szcp_dst = ring_s + G::CODE_BYTES + lane * 16;                  // one granule per lane (16 channels a stage) or two
+    const int tile_words = tile_lanes * G::WT / G::FPI;                        // word-column distance between my tiles
+    const int tile_groups = tile_lanes * G::WT / Gk;
 
-    const int32_t *tb_cur = kc + (int64_t)row0 * kc_sD + (t0 + warp * G::WT) / G::FPI + 4 * gr;
-    const __half *ks_cur = ks + (int64_t)lane * ks_sD + (t0 + warp * G::WT) / Gk;
-    const __half *kz_cur = kz + (int64_t)lane * ks_sD + (t0 + warp * G::WT) / Gk;
-    int wcol_cur = (t0 + warp * G::WT) / G::FPI + 4 * gr;                      // this lane's granule word column
-    bool ok_cur = wcol_cur < n_words;
+    // the next stage to issue: its addresses, its word column, its position in its tile and the tiles left.  Stages
+    // carry the scale and zero rows of their own channels, so the operands are formed k-step by k-step and the loop over
+    // a tile's stages stays rolled: LOOPNOTE
+    const int32_t *iss = kc + (int64_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr;
+    constexpr bool kOneSz = 2 * G::ROWS == 32;                                 // 16 channels: lanes 16-31 fetch the zero rows
+    const int sz_row = kOneSz ? (lane & 15) : lane;
+    const int64_t sz0 = (int64_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk;
+    const __half *iss_s = (kOneSz && lane >= 16 ? kz : ks) + sz0;
+    const ptrdiff_t sz_gap = kOneSz ? 0 : kz - ks;                             // zero row behind the scale row
+    int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
+    uint32_t iss_slot = 0, slot = 0;                                            // byte offsets of the slot being filled / read
+    bool iss_ok = iss_col < n_words;
 
-    auto issue_stage = [&](const int32_t *tb, bool ok, int sst) {              // sst: compile-time stage of the tile
-        if (ok) {
-            const uint32_t dst = cp_dst + (sst % G::NS) * G::STAGE_BYTES;
+    auto issue_stage = [&]() {
+        if (iss_tiles > 0) {
+            if (iss_ok) {
 #pragma unroll
-            for (int i = 0; i < G::GPL; ++i)
-                cp_async<16>(dst + i * G::RPI * G::RS, tb + (sst * G::ROWS + i * G::RPI) * kc_sD);
+                for (int i = 0; i < G::GPL; ++i)
+                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, iss + i * G::RPI * kc_sD);
+            }
+            const uint32_t d = szcp_dst + iss_slot;
+            if (ngw == 8) { cp_async<16>(d, iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, iss_s + sz_gap); }
+            else if (ngw == 4) { cp_async<8>(d, iss_s); if (!kOneSz) cp_async<8>(d + G::ROWS * 16, iss_s + sz_gap); }
+            else { cp_async<4>(d, iss_s); if (!kOneSz) cp_async<4>(d + G::ROWS * 16, iss_s + sz_gap); }
+        }
+        cp_async_commit();
+        iss_slot = iss_slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : iss_slot + R::STAGE_BYTES;
+        iss += G::ROWS * kc_sD;
+        iss_s += G::ROWS * ks_sD;
+        if (++iss_st == tile_stages) {
+            iss_st = 0;
+            iss += tile_words - tile_stages * (G::ROWS * kc_sD);
+            iss_s += tile_groups - tile_stages * (G::ROWS * ks_sD);
+            iss_col += tile_words;
+            iss_ok = iss_col < n_words;
+            --iss_tiles;
         }
     };
-    auto issue_sz = [&](const __half *ps, const __half *pz) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int off = 32 * i * ks_sD;
-            if (ngw == 8) { cp_async<16>(szcp_dst + i * 512, ps + off); cp_async<16>(szcp_dst + 2048 + i * 512, pz + off); }
-            else if (ngw == 4) { cp_async<8>(szcp_dst + i * 512, ps + off); cp_async<8>(szcp_dst + 2048 + i * 512, pz + off); }
-            else { cp_async<4>(szcp_dst + i * 512, ps + off); cp_async<4>(szcp_dst + 2048 + i * 512, pz + off); }
-        }
-    };
 
-    issue_sz(ks_cur, kz_cur);
-    issue_stage(tb_cur, ok_cur, 0);
-    cp_async_commit();
-    issue_stage(tb_cur, ok_cur, 1);
-    cp_async_commit();
-    issue_stage(tb_cur, ok_cur, 2);
-    cp_async_commit();
+#pragma unroll 1
+    for (int q = 0; q < R::P; ++q) issue_stage();
     // The caller stored q to shared memory just before this call without a barrier, so that the first code stages
     // are in flight while q arrives; every warp passes exactly one barrier here before anything reads q.
     __syncthreads();
     if (tail_lo < t1) qk_tail_mma(a, kf, b, hk, sm, t0, tail_lo, t1);
 
     for (int j = 0; j < my_tiles; ++j) {
-        const int tile0 = t0 + (j * kMmaWarps + warp) * G::WT;
-        const bool have_next = j + 1 < my_tiles;
-        const int32_t *tb_nxt = tb_cur + tile_words;
-        const bool ok_nxt = have_next && (wcol_cur + tile_words < n_words);
+        const int tile0 = t0 + (j * tile_lanes + wt) * G::WT;
+        uint32_t q_cur = q_s;
 
-        // the scale/zero tile of this warp tile was committed at least 3 groups ago
-        cp_async_wait<2>();
-        __syncwarp();
         // ---- B fragments q*scale and the zero term sum_d q[d]*zero[d,g] ----------------------------------
         // q*scale needs 22 bits; it is carried as an fp16 pair hi + lo (lo = fma(q, s, -hi) is exact), so the key
         // side adds no rounding beyond the fp32 accumulation.
         // 3-bit keys: b0 = hi and b1 = lo of the eight groups of the tile, every code tile is multiplied by both.
         // Other widths: b0 / b1 serve the first / second half of the tile; column n carries group (n / 2) of that
         // half, hi in even and lo in odd columns, so one MMA per code tile yields both parts.
-        uint32_t b0[8][2], b1[8][2];
-        float accz[4] = {0.f, 0.f, 0.f, 0.f}, accy[4] = {0.f, 0.f, 0.f, 0.f};
+        float zsum = 0.f;
         const int gph = ngw > 1 ? ngw / 2 : 1;                 // groups per half tile: 4 / 2 / 1
         const int src0 = 4 * ((g >> 1) % gph) + tig;           // lane holding group (n / 2) of the first half
         const int src1 = src0 + 4 * (ngw / 2);
-        const bool odd = g & 1;
-#pragma unroll
-        for (int ksx = 0; ksx < 8; ++ksx) {
-            const uint32_t q01u = lds32(q_s + 32 * ksx), q89u = lds32(q_s + 32 * ksx + 16);
-            const __half2 q01 = as_h2(q01u), q89 = as_h2(q89u);
-            // the tile rows are 8 groups x fp16 = one 8x8 matrix per 8 channels: a transposing ldmatrix hands
-            // lane (g, tig) exactly {row 2tig, row 2tig+1} x column g, i.e. its B-fragment pairs of group g, in one go
-            // (with fewer than 8 groups per tile the columns past the last group are stale and feed unused columns)
-            uint32_t r0, r1, r2, r3;
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                         : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(ldm_s + ksx * 256));
-            // The zero terms: the same two registers are also the A fragment of the transposed zero tile (row = group g,
-            // k = channels 2tig, 2tig+1 / +8), so ONE MMA with B = q (in every column) leaves sum_d q[d] * zero[d, g] in
-            // row g; fp16 x fp16 products are exact in the tensor core, no hi / lo split is needed.  Two accumulators
-            // alternate to keep the chains short.  A stale group only spoils its own row.
-            if (ksx & 1) mma16816(accy, r2, 0u, r3, 0u, q01u, q89u);
-            else mma16816(accz, r2, 0u, r3, 0u, q01u, q89u);
-            if constexpr (KB == 3) {
-                const __half2 s01 = as_h2(r0), s89 = as_h2(r1);
-                const __half2 p01 = __hmul2(q01, s01), p89 = __hmul2(q89, s89);
-                b0[ksx][0] = as_u32(p01);
-                b0[ksx][1] = as_u32(p89);
-                b1[ksx][0] = as_u32(__hfma2(q01, s01, __hneg2(p01)));
-                b1[ksx][1] = as_u32(__hfma2(q89, s89, __hneg2(p89)));
-            } else {
-                const __half2 sa01 = as_h2(__shfl_sync(0xffffffffu, r0, src0)), sa89 = as_h2(__shfl_sync(0xffffffffu, r1, src0));
-                const __half2 sb01 = as_h2(__shfl_sync(0xffffffffu, r0, src1)), sb89 = as_h2(__shfl_sync(0xffffffffu, r1, src1));
-                const __half2 pa01 = __hmul2(q01, sa01), pa89 = __hmul2(q89, sa89);
-                const __half2 pb01 = __hmul2(q01, sb01), pb89 = __hmul2(q89, sb89);
-                b0[ksx][0] = odd ? as_u32(__hfma2(q01, sa01, __hneg2(pa01))) : as_u32(pa01);
-                b0[ksx][1] = odd ? as_u32(__hfma2(q89, sa89, __hneg2(pa89))) : as_u32(pa89);
-                b1[ksx][0] = odd ? as_u32(__hfma2(q01, sb01, __hneg2(pb01))) : as_u32(pb01);
-                b1[ksx][1] = odd ? as_u32(__hfma2(q89, sb89, __hneg2(pb89))) : as_u32(pb89);
-            }
-        }
-        __syncwarp();                                          // everyone has read the tile: it may be refilled
-#pragma unroll
-        for (int i = 0; i < 4; ++i) accz[i] += accy[i];
+        const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;  // odd columns: the lo part
 
         float acc[G::NMMA][4];
 #pragma unroll
         for (int m = 0; m < G::NMMA; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
 
+#pragma unroll 1
+        for (int it = 0; it < steps; ++it) {
+          float accz[4] = {0.f, 0.f, 0.f, 0.f};               // zero terms of two k-steps
 #pragma unroll
-        for (int st = 0; st < G::NSTAGE; ++st) {
-            // issue stage st+P (of this tile or the next); the next tile's scale/zero tile rides with its first stage
-            if (st + G::P < G::NSTAGE) {
-                issue_stage(tb_cur, ok_cur, st + G::P);
-            } else {
-                issue_stage(tb_nxt, ok_nxt, st + G::P - G::NSTAGE);
-            }
-            if (st == 0 && have_next) issue_sz(ks_cur + tile_groups, kz_cur + tile_groups);
-            cp_async_commit();
-            cp_async_wait<G::P>();
+          for (int s2 = 0; s2 < 2 / G::KSPS; ++s2) {
+            issue_stage();
+            cp_async_wait<R::P>();
             __syncwarp();
-            const uint32_t src = frag_s + (st % G::NS) * G::STAGE_BYTES;
+            const uint32_t src = frag_s + slot;
 #pragma unroll
             for (int k = 0; k < G::KSPS; ++k) {
-                const int ksx = st * G::KSPS + k;
+                const uint32_t q01u = lds32(q_cur), q89u = lds32(q_cur + 16);
+                q_cur += 32;
+                const __half2 q01 = as_h2(q01u), q89 = as_h2(q89u);
+                // the tile rows are 8 groups x fp16 = one 8x8 matrix per 8 channels: a transposing ldmatrix hands
+                // lane (g, tig) exactly {row 2tig, row 2tig+1} x column g, i.e. its B-fragment pairs of group g, in one go
+                // (with fewer than 8 groups per tile the columns past the last group are stale and feed unused columns)
+                uint32_t r0, r1, r2, r3;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                             : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(ldm_s + slot + k * 256));
+                // The zero terms: the same two registers are also the A fragment of the transposed zero tile (row = group g,
+                // k = channels 2tig, 2tig+1 / +8), so ONE MMA with B = q (in every column) leaves sum_d q[d] * zero[d, g] in
+                // row g; fp16 x fp16 products are exact in the tensor core, no hi / lo split is needed.  Chains of
+                // two MMAs (the tensor core truncates as it accumulates).  A stale group only spoils its own row.
+                mma16816(accz, r2, 0u, r3, 0u, q01u, q89u);
+                uint32_t b0[2], b1[2];
+                if constexpr (KB == 3) {
+                    const __half2 s01 = as_h2(r0), s89 = as_h2(r1);
+                    const __half2 p01 = __hmul2(q01, s01), p89 = __hmul2(q89, s89);
+                    b0[0] = as_u32(p01);
+                    b0[1] = as_u32(p89);
+                    b1[0] = as_u32(__hfma2(q01, s01, __hneg2(p01)));
+                    b1[1] = as_u32(__hfma2(q89, s89, __hneg2(p89)));
+                } else {
+                    b0[0] = hilo(q01, as_h2(__shfl_sync(0xffffffffu, r0, src0)), neg_mask);
+                    b0[1] = hilo(q89, as_h2(__shfl_sync(0xffffffffu, r1, src0)), neg_mask);
+                    b1[0] = hilo(q01, as_h2(__shfl_sync(0xffffffffu, r0, src1)), neg_mask);
+                    b1[1] = hilo(q89, as_h2(__shfl_sync(0xffffffffu, r1, src1)), neg_mask);
+                }
                 if constexpr (KB == 3) {
                     uint32_t w[4];
 #pragma unroll
@@ -218,12 +211,12 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 #pragma unroll
                     for (int i = 0; i < F::N; i += 2) {
                         const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
-                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b0[ksx][0], b0[ksx][1]);
+                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b0[0], b0[1]);
                     }
 #pragma unroll
                     for (int i = 0; i < F::N; i += 2) {
                         const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
-                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b1[ksx][0], b1[ksx][1]);
+                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b1[0], b1[1]);
                     }
                 } else if constexpr (KB == 4) {
                     // 4-bit keys: two words (16 tokens) per octet and half, plain 64-bit loads + byte permutes (measured 1.5 %
@@ -245,14 +238,14 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 #pragma unroll
                             for (int i = 0; i < NF; i += 2) {
                                 const int m = h * 8 + (x * NF + i) / 2;
-                                if (h == 0) mma16816(acc[m], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b0[ksx][0], b0[ksx][1]);
-                                else mma16816(acc[m], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b1[ksx][0], b1[ksx][1]);
+                                if (h == 0) mma16816(acc[m], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b0[0], b0[1]);
+                                else mma16816(acc[m], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b1[0], b1[1]);
                             }
                         }
                     }
                 } else {
-                    using H = KHalf<KB>;
-                    const uint32_t lsrc = ldk_s + (st % G::NS) * G::STAGE_BYTES + (k * 16) * G::RS;
+                    using H = VHalf<KB>;
+                    const uint32_t lsrc = ldk_s + slot + (k * 16) * G::RS;
 #pragma unroll
                     for (int pb2 = 0; pb2 < NBK / 2; ++pb2) {              // two blocks per load
                         uint32_t x[2][2];
@@ -264,8 +257,8 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                             uint32_t rlo[H::N], rhi[H::N];
                             H::unpack(x[u][0], rlo);                        // channels 2tig, 2tig+1  -> k cols 2tig, 2tig+1
                             H::unpack(x[u][1], rhi);                        // channels 2tig+8, +9    -> k cols 2tig+8, 2tig+9
-                            const uint32_t bx = (bb >= NBK / 2) ? b1[ksx][0] : b0[ksx][0];
-                            const uint32_t by = (bb >= NBK / 2) ? b1[ksx][1] : b0[ksx][1];
+                            const uint32_t bx = (bb >= NBK / 2) ? b1[0] : b0[0];
+                            const uint32_t by = (bb >= NBK / 2) ? b1[1] : b0[1];
 #pragma unroll
                             for (int i = 0; i < H::N; i += 2)
                                 mma16816(acc[bb * MPB + i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], bx, by);
@@ -273,29 +266,28 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                     }
                 }
             }
-            __syncwarp();                                      // slot st % NS is free for the stage NS ahead
+            __syncwarp();                                      // the slot may be refilled
+            slot = slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : slot + R::STAGE_BYTES;
+          }
+          zsum += accz[0];
         }
 
+        float *dst0 = sm.scores + split * sm.n_scores - t0;
         // ---- epilogue ----------------------------------------------------------------------------------
         if constexpr (KB == 3) {
             // the octet's column is n = g, held by the lane with tig == g/2
             const int tok0 = tile0 + g * G::TPO;               // first token of this octet's chunk
             if (tok0 < hi && tig == (g >> 1)) {                // chunks are whole or absent (hi is a group multiple)
                 const bool sel = g & 1;
-                const float corr = accz[0];                    // row g of the zero-term product = group g = this octet's word
-                float *dst = sm.scores + (tok0 - t0);
+                const float corr = zsum;                    // row g of the zero-term product = group g = this octet's word
+                float *dst = dst0 + tok0;
 #pragma unroll
                 for (int m = 0; m < G::NMMA; ++m) {
                     const int i0 = 2 * m, i1 = 2 * m + 1;
                     float s0 = fmaf(sel ? acc[m][1] : acc[m][0], (float)(1 << (24 - F::pos(i0 % F::N))), corr);
                     float s1 = (i1 < G::TPO) ? fmaf(sel ? acc[m][3] : acc[m][2], (float)(1 << (24 - F::pos(i1 % F::N))), corr) : 0.f;
-                    if (a.round_scores) {
-                        const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                        s0 = r.x;
-                        s1 = r.y;
-                    }
-                    dst[i0] = s0 * a.softmax_scale;
-                    if (i1 < G::TPO) dst[i1] = s1 * a.softmax_scale;
+                    dst[i0] = s0;
+                    if (i1 < G::TPO) dst[i1] = s1;
                 }
             }
         } else if constexpr (KB == 4) {
@@ -306,21 +298,16 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int grp = h * gph + cp;
-                const float corr = __shfl_sync(0xffffffffu, accz[0], 4 * grp);    // row grp of the zero-term product
+                const float corr = __shfl_sync(0xffffffffu, zsum, 4 * grp);    // row grp of the zero-term product
                 const int tok0 = tile0 + 128 * h + 16 * g;
                 if (tok0 < hi && tig == cp) {                  // 16-token chunks are whole or absent (hi is a group multiple)
-                    float *dst = sm.scores + (tok0 - t0);
+                    float *dst = dst0 + tok0;
 #pragma unroll
                     for (int m = 0; m < 8; ++m) {
                         const int i0 = (2 * m) % NF, i1 = (2 * m + 1) % NF;
                         float s0 = fmaf(acc[h * 8 + m][0] + acc[h * 8 + m][1], (float)(1 << (24 - F::pos(i0))), corr);
                         float s1 = fmaf(acc[h * 8 + m][2] + acc[h * 8 + m][3], (float)(1 << (24 - F::pos(i1))), corr);
-                        if (a.round_scores) {
-                            const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                            s0 = r.x;
-                            s1 = r.y;
-                        }
-                        *reinterpret_cast<float2 *>(dst + 2 * m) = make_float2(s0 * a.softmax_scale, s1 * a.softmax_scale);
+                        *reinterpret_cast<float2 *>(dst + 2 * m) = make_float2(s0, s1);
                     }
                 }
             }
@@ -335,30 +322,20 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                 const int h = bb / kHalfBlocks;
                 const int cp = (((bb % kHalfBlocks) * 8 * FH) + g * FH) >> lgk;
                 const int grp = h * gph + cp;
-                const float corr = __shfl_sync(0xffffffffu, accz[0], 4 * grp);    // row grp of the zero-term product
+                const float corr = __shfl_sync(0xffffffffu, zsum, 4 * grp);    // row grp of the zero-term product
                 const int tok0 = tile0 + bb * 8 * FH + g * FH;
                 if (tok0 < hi && tig == cp) {                  // FH-token chunks are whole or absent (hi is a group multiple)
-                    float *dst = sm.scores + (tok0 - t0);
+                    float *dst = dst0 + tok0;
 #pragma unroll
                     for (int ip = 0; ip < MPB; ++ip) {
                         const int m = bb * MPB + ip;
-                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - F::pos(2 * ip))), corr);
-                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - F::pos(2 * ip + 1))), corr);
-                        if (a.round_scores) {
-                            const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                            s0 = r.x;
-                            s1 = r.y;
-                        }
-                        *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0 * a.softmax_scale, s1 * a.softmax_scale);
+                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - VHalf<KB>::pos(2 * ip))), corr);
+                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - VHalf<KB>::pos(2 * ip + 1))), corr);
+                        *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0, s1);
                     }
                 }
             }
         }
-        tb_cur = tb_nxt;
-        ok_cur = ok_nxt;
-        wcol_cur += tile_words;
-        ks_cur += tile_groups;
-        kz_cur += tile_groups;
     }
     cp_async_wait<0>();
 }
@@ -383,7 +360,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int Gv = a.v_group;
     const int ngv = kHeadDim / Gv;                            // channel groups: 4 / 2 / 1
-    const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;
+    const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;      // <= 0: no packed values in this segment
     const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
     float *my_red = reinterpret_cast<float *>(sm.ring);
     if (my_blocks <= 0) {
@@ -590,14 +567,11 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
             mma16816(c, ra[S].z, rb[S].z, ra[S].w, rb[S].w, qf[S].z, qf[S].w);
         }
         if (tig == 0) {
-            float s0 = c[0], s1 = c[2];
-            if (a.round_scores) {
-                const float2 r = __half22float2(__floats2half2_rn(s0, s1));
-                s0 = r.x;
-                s1 = r.y;
+            for (int p = 0; p < (1 << sm.ks_log2); ++p) {      // the whole score in the first partial, zero in the others
+                float *dst = sm.scores + p * sm.n_scores - t0;
+                if (ta < t1) dst[ta] = p ? 0.f : c[0];
+                if (tb < t1) dst[tb] = p ? 0.f : c[2];
             }
-            if (ta < t1) sm.scores[ta - t0] = s0 * a.softmax_scale;
-            if (tb < t1) sm.scores[tb - t0] = s1 * a.softmax_scale;
         }
     }
 }
@@ -605,17 +579,18 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of query head (b, h); segment `seg` of the `cnt` the head is cut into.
 template <int KB, int VB>
-__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int s, int t0, int t1, int seg,
+__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int ks_log2, int s, int t0, int t1, int seg,
                                              int cnt, int n_whole, float *__restrict__ parts,
                                              unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     MmaSmem sm;
+    sm.n_scores = n_scores;
+    sm.ks_log2 = ks_log2;
     sm.scores = reinterpret_cast<float *>(smem_raw);
-    unsigned char *after_scores = smem_raw + (size_t)n_scores * 4;
+    unsigned char *after_scores = smem_raw + ((size_t)n_scores << ks_log2) * 4;
     sm.ring = after_scores + warp * warp_region_bytes<KB, VB>();
-    sm.tailred = reinterpret_cast<float *>(after_scores + kMmaWarps * warp_region_bytes<KB, VB>());
-    sm.q = reinterpret_cast<__half *>(sm.tailred + kMmaWarps * kHeadDim);
+    sm.q = reinterpret_cast<__half *>(after_scores + kMmaWarps * warp_region_bytes<KB, VB>());
     sm.misc = reinterpret_cast<float *>(sm.q + kHeadDim);
     const int b = s / a.nh, h = s % a.nh;
     // grouped queries: each query head is its own segment and reads kv head hk; the heads of one kv head are
@@ -625,76 +600,44 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)h * a.q_sH;
     if (tid < kHeadDim) sm.q[tid] = q[tid];
-    for (int i = tid; i < kMmaWarps * kHeadDim; i += kMmaThreads) sm.tailred[i] = 0.f;
+    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
+    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
+    prefetch_v_tail(a, vf, b, hk, v_lo, t1, tid, kMmaThreads);
 
     // ---- 1. scores ------------------------------------------------------------------------------
     {
-        const int hi = min(t1, a.Tkq);
-        if (t0 < hi) {
-            const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
-            const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-            const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-            const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
-            qk_packed_mma<KB>(a, kc, ks, kz, sm, t0, hi, kf, max(t0, a.Tkq), t1, b, hk);
-        } else {
-            __syncthreads();                                   // q is in shared memory
-            const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
-            if (t0 < t1) qk_tail_mma(a, kf, b, hk, sm, t0, t0, t1);
-        }
+        const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
+        const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
+        const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
+        const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
+        qk_packed_mma<KB>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
-    const int v_hi = min(t1, a.Tvq);
-    if (t0 < v_hi) pv_packed_mma<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);   // start filling this warp's value ring now
+    pv_packed_mma<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
     // ---- 2. softmax numerators ------------------------------------------------------------------
-    // The fp16 value tail of this split (the window: usually <= 128 tokens) is fetched into registers first, so its
-    // global-load latency is spent under the two softmax passes.  Thread (co, tl) owns 8 channels and tokens
-    // v_lo + tl + 8 j; rounds of 128 tokens, the first one preloaded.
-    const int n = t1 - t0;
-    const int v_lo = max(t0, a.Tvq);
-    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
-    const int co = tid & 15, tl = tid >> 4;
-    uint4 vt[16];
-    auto load_tail_round = [&](int base) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int t = base + tl + 8 * j;
-            vt[j] = (t < t1) ? __ldg(reinterpret_cast<const uint4 *>(v_tail_row(a, vf, b, hk, t)) + co) : make_uint4(0u, 0u, 0u, 0u);
-        }
-    };
-    if (v_lo < t1) load_tail_round(v_lo);
-
+    // upstream rounds the raw score to fp16 before scaling it (round_scores)
+    const int n = t1 - t0, n4 = (n + 3) >> 2;
     float m = kMaskFloor;                                      // a fully masked range then weighs uniformly, as upstream's does
-    const int n4 = (n + 3) >> 2;
     float4 *sc4 = reinterpret_cast<float4 *>(sm.scores);
-#pragma unroll 4
+#pragma unroll 2
     for (int i = tid; i < n4; i += kMmaThreads) {
-        float4 v = sc4[i];
-        if (a.mask) {                                          // weights + mask, clamped at the fp32 floor
-            const int t = t0 + 4 * i;
-            v.x = fmaxf(v.x + attn_mask_at(a, b, h, min(t, a.T - 1)), kMaskFloor);
-            v.y = fmaxf(v.y + attn_mask_at(a, b, h, min(t + 1, a.T - 1)), kMaskFloor);
-            v.z = fmaxf(v.z + attn_mask_at(a, b, h, min(t + 2, a.T - 1)), kMaskFloor);
-            v.w = fmaxf(v.w + attn_mask_at(a, b, h, min(t + 3, a.T - 1)), kMaskFloor);
-            sc4[i] = v;
-        }
-        if (4 * i + 3 >= n) {                                  // the last, partial quad: neutral padding
-            if (4 * i + 1 >= n) v.y = -INFINITY;
-            if (4 * i + 2 >= n) v.z = -INFINITY;
-            v.w = -INFINITY;
-            sc4[i] = v;
-        }
+        float4 v = score_quad(a, sc4 + i, n_scores >> 2, ks_log2);
+        if (a.mask) mask_quad(a, b, h, t0 + 4 * i, v);
+        if (4 * i + 3 >= n) pad_quad(v, n - 4 * i);
+        sc4[i] = v;
         m = fmaxf(fmaxf(m, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
     m = warp_max(m);
     if (lane == 0) sm.misc[warp] = m;
     __syncthreads();
-    m = fmaxf(fmaxf(sm.misc[0], sm.misc[1]), fmaxf(sm.misc[2], sm.misc[3]));
+    m = sm.misc[lane & (kMmaWarps - 1)];
+    m = warp_max(m);
     float l = 0.f;
-#pragma unroll 4
+#pragma unroll 2
     for (int i = tid; i < n4; i += kMmaThreads) {
         float4 v = sc4[i];
         v.x = __expf(v.x - m);
@@ -705,87 +648,69 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
         l += (v.x + v.y) + (v.z + v.w);
     }
     l = warp_sum(l);
-    if (lane == 0) sm.misc[4 + warp] = l;
+    if (lane == 0) sm.misc[8 + warp] = l;
     __syncthreads();
-    l = (sm.misc[4] + sm.misc[5]) + (sm.misc[6] + sm.misc[7]);
 
     // ---- 3. p.V -----------------------------------------------------------------------------------
-    if (v_lo < t1) {
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int base = v_lo; base < t1; base += 128) {
-            if (base > v_lo) load_tail_round(base);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int t = base + tl + 8 * j;
-                const float p = (t < t1) ? sm.scores[t - t0] : 0.f;
-                const __half2 *h = reinterpret_cast<const __half2 *>(&vt[j]);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float2 f = __half22float2(h[k]);
-                    acc[2 * k] = fmaf(p, f.x, acc[2 * k]);
-                    acc[2 * k + 1] = fmaf(p, f.y, acc[2 * k + 1]);
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 16);   // the warp's two token lanes
-        if (lane < 16) {
-            float4 *dst = reinterpret_cast<float4 *>(sm.tailred + warp * kHeadDim + 8 * co);
-            dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-        }
-    }
-    if (t0 < v_hi) pv_packed_mma<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    pv_packed_mma<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    __syncwarp();
+    if (v_lo < t1) pv_tail<1>(a, vf, b, hk, sm.scores, 0, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();
 
     // ---- 4. finish / merge --------------------------------------------------------------------------
-    float o = (sm.tailred[tid] + sm.tailred[kHeadDim + tid]) + (sm.tailred[2 * kHeadDim + tid] + sm.tailred[3 * kHeadDim + tid]);
-    if (t0 < min(t1, a.Tvq)) {                               // each warp left its packed-value partial at its region base
+    const bool own = tid < kHeadDim;                           // thread tid owns channel tid
+    float o = 0.f, l_all = 0.f;
+    if (own) {
 #pragma unroll
-        for (int w = 0; w < kMmaWarps; ++w)
-            o += reinterpret_cast<const float *>(after_scores + w * warp_region_bytes<KB, VB>())[tid];
+        for (int w = 0; w < kMmaWarps; ++w) o += reinterpret_cast<const float *>(after_scores + w * warp_region_bytes<KB, VB>())[tid];
     }
+#pragma unroll
+    for (int w = 0; w < kMmaWarps; ++w) l_all += sm.misc[8 + w];
     __half *out = static_cast<__half *>(a.out) + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH;
     if (cnt == 1) {
-        const __half r[1] = {__float2half_rn(o / l)};
-        out[tid] = r[0];
-        peer_publish(ac, b, h, 1, r, tid);
+        const __half r[1] = {__float2half_rn(o / l_all)};
+        if (own) out[tid] = r[0];
+        peer_publish(ac, b, h, own ? 1 : 0, r, tid & (kHeadDim - 1), tid, 1);
         return;
     }
     constexpr int kPart = kPartStride;
     float *part = parts + ((int64_t)(s - n_whole) * cnt + seg) * kPart;          // partials of the cut heads only
-    part[tid] = o;
-    if (tid == 0) { part[kHeadDim] = m; part[kHeadDim + 1] = l; }
+    if (own) part[tid] = o;
+    if (tid == 0) { part[kHeadDim] = m; part[kHeadDim + 1] = l_all; }
     __syncthreads();
     if (tid == 0) {
         // one cumulative device-scope fence after the CTA barrier publishes every thread's partial before the count;
         // the fence after the count orders the merging CTA's reads (ld.cg, from L2) behind the other CTAs' fences
         __threadfence();
-        sm.misc[8] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
+        sm.misc[16] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
         __threadfence();
     }
     __syncthreads();
-    if (sm.misc[8] == 0.f) return;
+    if (sm.misc[16] == 0.f) return;
     const float *base = parts + (int64_t)(s - n_whole) * cnt * kPart;
     float M = kMaskFloor;
-    for (int i = 0; i < cnt; ++i) M = fmaxf(M, __ldcg(base + i * kPart + kHeadDim));
+    for (int i = lane; i < cnt; i += 32) M = fmaxf(M, __ldcg(base + i * kPart + kHeadDim));
+    M = warp_max(M);
     float L = 0.f, acc = 0.f;
+    const int ch = tid & (kHeadDim - 1);
+#pragma unroll 8
     for (int i = 0; i < cnt; ++i) {
-        const float w = __expf(__ldcg(base + i * kPart + kHeadDim) - M);
-        L = fmaf(__ldcg(base + i * kPart + kHeadDim + 1), w, L);
-        acc = fmaf(__ldcg(base + i * kPart + tid), w, acc);
+        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(base + i * kPart + kHeadDim));
+        const float w = __expf(ml.x - M);
+        L = fmaf(ml.y, w, L);
+        acc = fmaf(__ldcg(base + i * kPart + ch), w, acc);
     }
     const __half r[1] = {__float2half_rn(acc / L)};
-    out[tid] = r[0];
+    if (own) out[tid] = r[0];
     if (tid == 0) counters[s] = 0u;                          // the head is done: its counter is ready for the next launch
-    peer_publish(ac, b, h, 1, r, tid);
+    peer_publish(ac, b, h, own ? 1 : 0, r, ch, tid, 1);
 }
 
 // CTA = one segment (see attn_plan.cuh): a whole head, or one of the k pieces of a head that is cut.
 // DEV: lengths and ring starts come from the device-resident state (attn_update.cuh); the plan was laid out for an
 // upper bound of the length, so segments beyond the real length are empty and a head counts fewer of them.
 template <int KB, int VB, bool DEV>
-__global__ void __launch_bounds__(kMmaThreads, 3) decode_attn_mma_kernel(const __grid_constant__ kvq_attn_args a,
+__global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_mma_kernel(const __grid_constant__ kvq_attn_args a,
                                                                      const __grid_constant__ AttnPlan plan,
                                                                      float *__restrict__ parts,
                                                                      unsigned int *__restrict__ counters) {
@@ -795,10 +720,10 @@ __global__ void __launch_bounds__(kMmaThreads, 3) decode_attn_mma_kernel(const _
         dev_state_step(a, b);
         plan_cta(plan, b.T, blockIdx.x, head, t0, t1, seg, cnt);
         if (cnt > 1) cnt = min(cnt, (b.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < b.T) attn_segment<KB, VB>(b, a, plan.n_scores, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        if (t0 < b.T) attn_segment<KB, VB>(b, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     } else {
         plan_cta(plan, a.T, blockIdx.x, head, t0, t1, seg, cnt);
-        attn_segment<KB, VB>(a, a, plan.n_scores, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        attn_segment<KB, VB>(a, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     }
 }
 
@@ -833,16 +758,16 @@ bool mma_path_eligible(const kvq_attn_args &a) {
 template <int KB, int VB>
 static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
                       cudaStream_t st) {
-    const size_t smem = (size_t)plan.n_scores * 4 + (size_t)kMmaWarps * warp_region_bytes<KB, VB>() +
-                        kMmaWarps * kHeadDim * 4 + kHeadDim * 2 + 16 * 4;
+    const size_t smem = ((size_t)plan.n_scores << plan.ks_log2) * 4 + (size_t)kMmaWarps * warp_region_bytes<KB, VB>() +
+                        kHeadDim * 2 + 32 * 4;
     static bool attr_set[64] = {};                           // per device: the opt-in is sticky for the process
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+        e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+            e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
@@ -866,9 +791,8 @@ int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *
 
 // Plan of the tensor-core kernel for B * nh query heads (one head per segment).
 AttnPlan plan_attn_mma(int T, int k_bits, long long heads) {
-    const int unit = (k_bits == 3) ? 352 : 256;              // one key tile per warp
-    const int max_chunk = (k_bits == 3) ? 8096 : 8192;       // scores held in shared memory
-    return make_attn_plan(T, unit, max_chunk, heads, kSmCount * 3, k_bits == 3 ? 1 : kMmaWarps);
+    // score buffers that leave room for two CTAs per SM
+    return k_bits == 3 ? make_attn_plan(T, 352, KGeom<3>::WT, 7040, heads) : make_attn_plan(T, 256, KGeom<4>::WT, 6144, heads);
 }
 
 }  // namespace kvq
