@@ -6,7 +6,10 @@
 
 namespace kvq {
 
-// Eight warps per CTA and two CTAs per SM (128 registers a thread): WARPNOTE
+// Eight warps per CTA and two CTAs per SM (128 registers a thread): with four warps of 168-208
+// registers the SM held 8-12 warps and a warp issued once in 7 cycles, a CTA's time hardly depending on its neighbours; eight
+// warps per CTA make 16 and halve the chain of every CTA (32 heads x 8 sequences at 4096 tokens: 279 -> 247 us a step of five
+// layers; grouped queries at 32k tokens 840 -> 655 us).
 constexpr int kMmaThreads = 256;
 constexpr int kMmaWarps = 8;
 constexpr int kMmaSmemMax = 115712;                                // dynamic shared memory of a CTA with two of them on an SM
@@ -186,6 +189,22 @@ template <> struct VHalf<3> {
     static constexpr int N = 2;
 };
 
+// The same for the keys.  2-bit codes: a byte swap of the halves instead of the two shifts, positions 2 .. 8 -- keys
+// have no probabilities of very different size side by side, and a shift less per eight fields counts.
+template <int BITS> struct KHalf : VHalf<BITS> {};
+template <> struct KHalf<2> {
+    static constexpr int N = 8;
+    __device__ static __forceinline__ int pos(int i) { return i == 0 ? 8 : i < 5 ? 2 * i : 2 * i - 8; }
+    __device__ static __forceinline__ void unpack(uint32_t x, uint32_t (&r)[8]) {
+        const uint32_t y = prmt(x, x, 0x2301);
+        r[0] = y & 0x03000300u;
+#pragma unroll
+        for (int t = 1; t < 5; ++t) r[t] = x & (0x00030003u << (2 * t));
+#pragma unroll
+        for (int t = 5; t < 8; ++t) r[t] = y & (0x00030003u << (2 * t - 8));
+    }
+};
+
 // ---------------------------------------------------------------------------------------------
 // Key-side geometry per bit width.  A warp tile is 8 lane-octets x TPO tokens; code words reach the
 // warp through its own ring of cp.async stages in shared memory (padded rows so the fragment loads
@@ -196,15 +215,15 @@ template <int KB> struct KGeom {
     static constexpr int WPL = (KB == 4) ? 4 : (KB == 2) ? 2 : 1;     // words per octet: 32 tokens (11 for 3-bit)
     static constexpr int TPO = WPL * FPI;                              // tokens per octet chunk
     static constexpr int WT = 8 * TPO;                                 // tokens per warp tile (256 / 88)
-    static constexpr int KSPS = (KB == 4 || KB == 2) ? 1 : 2;          // k-steps (16 channels) per stage
+    static constexpr int KSPS = (KB == 4) ? 1 : 2;          // k-steps (16 channels) per stage
     static constexpr int NSTAGE = 8 / KSPS;                            // stages per warp tile of all channels: 8 / 4
     static constexpr int NMMA = (TPO + 1) / 2;                         // MMAs (token pairs) per octet chunk
     static constexpr int RB = 32 * WPL;                                // code bytes per channel row per warp tile
     static constexpr int RS = RB + 16;                                 // padded row stride in the ring
     static constexpr int ROWS = 16 * KSPS;                             // channel rows per stage
-    static constexpr int CODE_BYTES = ROWS * RS;                       // 2304 / 1280 / 1536 (4 / 2 / 3 and 1 bits)
+    static constexpr int CODE_BYTES = ROWS * RS;                       // 2304 / 2560 / 1536 (4 / 2 / 3 and 1 bits)
     static constexpr int GPR = RB / 16;                                // 16-byte granules per row: 8 / 4 / 2
-    static constexpr int GPL = ROWS * GPR / 32;                        // granules per lane per stage: 4 / 2 / 2
+    static constexpr int GPL = ROWS * GPR / 32;                        // granules per lane per stage: 4 / 4 / 2
     static constexpr int RPI = 32 / GPR;                               // rows between a lane's granules
     static constexpr float MID = (float)((1 << KB) - 1) * 0.5f;        // codes are centred on the group midpoint
 };

@@ -55,7 +55,7 @@ inline int plan_key_split(int n, int tile, int max_scores) {
 }
 
 // SM cycles a segment of n tokens takes (one of two CTAs on its SM; measured with clock stamps inside the kernels on
-// B200): 850 per two half-steps of keys, 850 per 32 tokens of values a warp works, the softmax, and PLANFIXED for
+// B200): 850 per two half-steps of keys, 850 per 32 tokens of values a warp works, the softmax, and 5500 for
 // the launch, the ring fill, the fp16 tails and the final sum.
 inline long long plan_segment_cycles(int n, int tile, int max_scores) {
     const int key = plan_key_steps(n, tile, plan_key_split(n, tile, max_scores)) * 850;

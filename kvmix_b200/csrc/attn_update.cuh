@@ -189,47 +189,65 @@ __device__ __forceinline__ void peer_publish(const kvq_attn_args &a, int b, int 
     }
 }
 
-// The fp16 value tail is read at the very end of a segment: its rows are fetched into L2 while the packed part is worked.
-__device__ __forceinline__ void prefetch_v_tail(const kvq_attn_args &a, const __half *vf, int b, int hk, int v_lo, int t1, int tid, int threads) {
-    for (int i = tid; i < 2 * (t1 - v_lo); i += threads)
+// The fp16 tails are read between the packed phases (keys) and at the very end (values): the CTA asks for their rows before it
+// fills its rings, so that they are in L2 by then.  A launch of 256 CTAs over 4096 tokens spent 12 k of a CTA's 67 k
+// cycles waiting for them before.
+__device__ __forceinline__ void prefetch_tails(const kvq_attn_args &a, const __half *kf, const __half *vf, int b, int hk, int t0, int t1, int tid, int threads) {
+    const int k_lo = max(t0, a.Tkq), nk = 2 * max(0, t1 - k_lo), v_lo = max(t0, a.Tvq), nv = 2 * max(0, t1 - v_lo);
+    for (int i = tid; i < nk; i += threads)
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(k_tail_row(a, kf, b, hk, k_lo + (i >> 1)) + 64 * (i & 1)));
+    for (int i = tid; i < nv; i += threads)
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(v_tail_row(a, vf, b, hk, v_lo + (i >> 1)) + 64 * (i & 1)));
 }
 
-// p . V over the fp16 value tail, tokens [v_lo, t1), for H heads whose probabilities lie `p_stride` floats apart: warp w takes
-// tokens v_lo + w, v_lo + w + 8, ..., a lane owns four channels of every head; the sums are added to the warp's partial
+// p . V over the fp16 value tail, tokens [v_lo, t1), for H heads whose probabilities lie `p_stride` floats apart: the CTA's
+// half-warps take tokens in turn, a lane owns eight channels of every head; the sums are added to the warp's partial
 // results red[H][128] (already complete and visible to the warp).
 template <int H>
 __device__ __forceinline__ void pv_tail(const kvq_attn_args &a, const __half *vf, int b, int hk, const float *p, int p_stride, int t0, int v_lo,
                                         int t1, float *red, int warp, int n_warps, int lane) {
-    float acc[H][4];
+    float acc[H][8];
 #pragma unroll
-    for (int h = 0; h < H; ++h) acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.f;
-    constexpr int U = 8;                                       // rows in flight per warp
-    for (int t = v_lo + warp; t < t1; t += U * n_warps) {
-        uint2 v[U];
+    for (int h = 0; h < H; ++h)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[h][c] = 0.f;
+    constexpr int U = H == 1 ? 10 : 6;                         // rows in flight: a 128-token window with a part of a group in one / two rounds
+    const int l16 = lane & 15, step = 2 * n_warps;
+    for (int t = v_lo + 2 * warp + (lane >> 4); t < t1; t += U * step) {
+        uint4 v[U];
 #pragma unroll
         for (int j = 0; j < U; ++j)
-            v[j] = __ldg(reinterpret_cast<const uint2 *>(v_tail_row(a, vf, b, hk, min(t + j * n_warps, t1 - 1))) + lane);
+            if (t + j * step < t1) v[j] = __ldg(reinterpret_cast<const uint4 *>(v_tail_row(a, vf, b, hk, t + j * step)) + l16);
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-            const int tj = t + j * n_warps;
-            const float2 v01 = __half22float2(*reinterpret_cast<const __half2 *>(&v[j].x));
-            const float2 v23 = __half22float2(*reinterpret_cast<const __half2 *>(&v[j].y));
+            const int tj = t + j * step;
+            if (tj >= t1) break;
+            const __half2 *hv = reinterpret_cast<const __half2 *>(&v[j]);
+            float2 f[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) f[c] = __half22float2(hv[c]);
 #pragma unroll
             for (int h = 0; h < H; ++h) {
-                const float ph = tj < t1 ? p[h * p_stride + tj - t0] : 0.f;
-                acc[h][0] = fmaf(ph, v01.x, acc[h][0]);
-                acc[h][1] = fmaf(ph, v01.y, acc[h][1]);
-                acc[h][2] = fmaf(ph, v23.x, acc[h][2]);
-                acc[h][3] = fmaf(ph, v23.y, acc[h][3]);
+                const float ph = p[h * p_stride + tj - t0];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    acc[h][2 * c] = fmaf(ph, f[c].x, acc[h][2 * c]);
+                    acc[h][2 * c + 1] = fmaf(ph, f[c].y, acc[h][2 * c + 1]);
+                }
             }
         }
     }
+    __syncwarp();
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-        float4 *r = reinterpret_cast<float4 *>(red + h * kHeadDim) + lane;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[h][c] += __shfl_xor_sync(0xffffffffu, acc[h][c], 16);
+        // the lower half-warp adds the first four channels, the upper one the others
+        float4 *r = reinterpret_cast<float4 *>(red + h * kHeadDim) + 2 * l16 + (lane >> 4);
         float4 s = *r;
-        s.x += acc[h][0]; s.y += acc[h][1]; s.z += acc[h][2]; s.w += acc[h][3];
+        const bool up = lane >= 16;
+        s.x += up ? acc[h][4] : acc[h][0]; s.y += up ? acc[h][5] : acc[h][1];
+        s.z += up ? acc[h][6] : acc[h][2]; s.w += up ? acc[h][7] : acc[h][3];
         *r = s;
     }
 }

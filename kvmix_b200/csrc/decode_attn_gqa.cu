@@ -35,7 +35,7 @@ struct GqaSmem {
 // A stage carries the scale and zero rows of its channels behind the codes.  3-bit keys: 8 groups per tile, 16-byte scale
 // rows followed by the zero rows; other widths (<= 4 groups per tile): 16-byte rows that hold 4 scales then 4 zeros.
 template <int KB> constexpr int gqa_zero_off() { return KB == 3 ? KGeom<KB>::ROWS * 16 : 8; }
-template <int KB> using GqaKRing = KRing<KB, KGeom<KB>::ROWS * (KB == 3 ? 32 : 16), (KB == 4 || KB == 3) ? 3 : 4>;
+template <int KB> using GqaKRing = KRing<KB, KGeom<KB>::ROWS * (KB == 3 ? 32 : 16), KB == 1 ? 4 : 3>;
 template <int VB> using GqaVGeom = VGeom<VB, VB == 4 ? 3 : VB == 2 ? 5 : 7>;
 // operand tiles of the values: 512 bytes per channel group (4 / 2 / 2 groups at most)
 template <int VB> constexpr int gqa_op_bytes() { return VB == 4 ? 2048 : 1024; }
@@ -138,37 +138,41 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 
     // the next stage to issue: its addresses, its word column, its position in its tile and the tiles left.  A stage of 16
     // channels takes one scale / zero copy per lane (zeros: lanes 16-31), one of 32 channels two.
-    const int32_t *iss = kc + (int64_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr;
+    uint32_t iss = 4u * ((uint32_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr);   // bytes from the head's first word
     constexpr bool kOneSz = G::ROWS == 16;
     const int sz_row = kOneSz ? (lane & 15) : lane;
     const bool sz_zero = kOneSz && lane >= 16;
-    const __half *iss_s = (sz_zero ? kz : ks) + (int64_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk;
-    const ptrdiff_t sz_gap = kOneSz ? 0 : kz - ks;
+    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk);
+    const char *sz_b = reinterpret_cast<const char *>(sz_zero ? kz : ks);
     const uint32_t szcp_dst = ring_s + G::CODE_BYTES + sz_row * 16 + (sz_zero ? ZOFF : 0);
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
     uint32_t iss_slot = 0, slot = 0;
     bool iss_ok = iss_col < n_words;
+
+    const char *kc_b = reinterpret_cast<const char *>(kc), *kz_b = reinterpret_cast<const char *>(kz);
+    const uint32_t row_step = (uint32_t)(G::RPI * 4) * kc_sD, stage_step = (uint32_t)(G::ROWS * 4) * kc_sD, sz_step = (uint32_t)(G::ROWS * 2) * ks_sD;
+    const uint32_t tile_step = 4 * tile_words - tile_stages * stage_step, tile_sz_step = 2 * tile_groups - tile_stages * sz_step;
 
     auto issue_stage = [&]() {
         if (iss_tiles > 0) {
             if (iss_ok) {
 #pragma unroll
                 for (int i = 0; i < G::GPL; ++i)
-                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, iss + i * G::RPI * kc_sD);
+                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, kc_b + (iss + i * row_step));
             }
             const uint32_t d = szcp_dst + iss_slot;
-            if (KB == 3) { cp_async<16>(d, iss_s); cp_async<16>(d + ZOFF, iss_s + sz_gap); }
-            else if (ngw == 4) { cp_async<8>(d, iss_s); if (!kOneSz) cp_async<8>(d + ZOFF, iss_s + sz_gap); }
-            else { cp_async<4>(d, iss_s); if (!kOneSz) cp_async<4>(d + ZOFF, iss_s + sz_gap); }
+            if (KB == 3) { cp_async<16>(d, sz_b + iss_s); cp_async<16>(d + ZOFF, kz_b + iss_s); }
+            else if (ngw == 4) { cp_async<8>(d, sz_b + iss_s); if (!kOneSz) cp_async<8>(d + ZOFF, kz_b + iss_s); }
+            else { cp_async<4>(d, sz_b + iss_s); if (!kOneSz) cp_async<4>(d + ZOFF, kz_b + iss_s); }
         }
         cp_async_commit();
         iss_slot = iss_slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : iss_slot + R::STAGE_BYTES;
-        iss += G::ROWS * kc_sD;
-        iss_s += G::ROWS * ks_sD;
+        iss += stage_step;
+        iss_s += sz_step;
         if (++iss_st == tile_stages) {
             iss_st = 0;
-            iss += tile_words - tile_stages * (G::ROWS * kc_sD);
-            iss_s += tile_groups - tile_stages * (G::ROWS * ks_sD);
+            iss += tile_step;
+            iss_s += tile_sz_step;
             iss_col += tile_words;
             iss_ok = iss_col < n_words;
             --iss_tiles;
@@ -190,7 +194,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 #pragma unroll
         for (int m = 0; m < NACC; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
 
-        // LOOPNOTE
+        // two k-steps a turn: unrolled over all eight the loop missed the instruction cache (2.7 of 7.3 cycles per issued
+        // instruction at 2 bits were fetch stalls)
 #pragma unroll 1
         for (int it = 0; it < steps; ++it) {
           float accz[4] = {0.f, 0.f, 0.f, 0.f};               // zero terms of two k-steps
@@ -263,7 +268,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                             b[jk][0] = b[jk][1] = 0u;
                         }
                     }
-                    using H = VHalf<KB>;
+                    using H = KHalf<KB>;
                     const uint32_t lsrc = ldk_s + stage_s + (k * 16) * G::RS;
 #pragma unroll
                     for (int pb2 = 0; pb2 < NBK / 2; ++pb2) {
@@ -321,8 +326,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 #pragma unroll
                     for (int ip = 0; ip < MPB; ++ip) {
                         const int m = bb * MPB + ip;
-                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - VHalf<KB>::pos(2 * ip))), corr);
-                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - VHalf<KB>::pos(2 * ip + 1))), corr);
+                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - KHalf<KB>::pos(2 * ip))), corr);
+                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - KHalf<KB>::pos(2 * ip + 1))), corr);
                         *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0, s1);
                     }
                 }
@@ -373,14 +378,16 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     const float *pa = sm.scores + (2 * hh) * sm.n_scores + warp * G::TPS + bt0, *pb = pa + sm.n_scores;
 
     const int block_stride = kMmaWarps * G::TPS;
-    const char *src_codes = reinterpret_cast<const char *>(vc + (int64_t)(t0 + warp * G::TPS) * a.vc_sT) + lane * 16;
+    const char *vc_b = reinterpret_cast<const char *>(vc);                               // 32-bit byte offsets from the head's first row
+    uint32_t src_codes = (uint32_t)(t0 + warp * G::TPS) * G::RBV + lane * 16;
     const int ngran = 4 * ngv;
     const int sz_arr = lane >= ngran ? 1 : 0;
     const int sz_off = (lane - sz_arr * ngran) * 16;
     const bool sz_on = lane < 2 * ngran;
-    const char *src_sz = reinterpret_cast<const char *>((sz_arr ? vz : vs) + (int64_t)(t0 + warp * G::TPS) * a.vs_sT) + sz_off;
+    const char *sz_b = reinterpret_cast<const char *>(sz_arr ? vz : vs);
+    uint32_t src_sz = (uint32_t)(t0 + warp * G::TPS) * (ngv * 2) + sz_off;
     const uint32_t sz_dst = ring_s + G::SZ_OFF + sz_arr * (G::TPS * 4 * 2) + sz_off;
-    const int64_t codes_step = (int64_t)block_stride * G::RBV, sz_step = (int64_t)block_stride * ngv * 2;
+    const uint32_t codes_step = block_stride * G::RBV, sz_step = block_stride * ngv * 2;
 
     int to_issue = my_blocks;
     auto issue_stage = [&](uint32_t slot_off) {
@@ -388,8 +395,8 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
 #pragma unroll
             for (int i = 0; i < G::GPL; ++i)
                 if (G::TPS * G::GPT % 32 == 0 || lane + 32 * i < G::TPS * G::GPT)
-                    cp_async<16>(cp_dst + slot_off + i * (32 / G::GPT) * G::RBV, src_codes + i * 512);
-            if (sz_on) cp_async<16>(sz_dst + slot_off, src_sz);
+                    cp_async<16>(cp_dst + slot_off + i * (32 / G::GPT) * G::RBV, vc_b + (src_codes + i * 512));
+            if (sz_on) cp_async<16>(sz_dst + slot_off, sz_b + src_sz);
         }
         --to_issue;
         src_codes += codes_step;
@@ -557,6 +564,10 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     const int n_rep = a.nh / a.nh_kv, nq = n_rep / qhv;                // quads per kv head
     const int b = s / (a.nh_kv * nq), hk = (s / nq) % a.nh_kv, h_first = hk * n_rep + (s % nq) * qhv;
 
+    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
+    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
+    const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
+    prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, kMmaThreads);
     fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     // q of the quad (head slots beyond qhv repeat the last head: their columns are computed and dropped)
     {
@@ -564,12 +575,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + hs) * a.q_sH;
         *reinterpret_cast<uint32_t *>(sm.q + slot * kHeadDim + 2 * (tid & 63)) = *reinterpret_cast<const uint32_t *>(q + 2 * (tid & 63));
     }
-    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
-    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
-    prefetch_v_tail(a, vf, b, hk, v_lo, t1, tid, kMmaThreads);
 
     // ---- 1. scores ------------------------------------------------------------------------------
-    const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
     {
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;

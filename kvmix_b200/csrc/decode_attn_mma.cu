@@ -38,7 +38,7 @@ struct MmaSmem {
     float *misc;            // [32]
     int n_scores, ks_log2;
 };
-template <int KB> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, 4>;        // scale rows, then zero rows, 16 B each
+template <int KB> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, KB == 2 ? 3 : 4>;        // scale rows, then zero rows, 16 B each
 template <int KB, int VB> constexpr int warp_region_bytes() {
     return MmaKRing<KB>::BYTES > VGeom<VB>::WARP_BYTES ? MmaKRing<KB>::BYTES : VGeom<VB>::WARP_BYTES;
 }
@@ -98,37 +98,41 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 
     // the next stage to issue: its addresses, its word column, its position in its tile and the tiles left.  Stages
     // carry the scale and zero rows of their own channels, so the operands are formed k-step by k-step and the loop over
-    // a tile's stages stays rolled: LOOPNOTE
-    const int32_t *iss = kc + (int64_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr;
+    // a tile's stages stays rolled (two k-steps a turn; unrolled over all
+    // eight it missed the instruction cache: 1.6 of 7.9 cycles per issued instruction were fetch stalls, 0.4 now).
+    uint32_t iss = 4u * ((uint32_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr);   // bytes from the head's first word
     constexpr bool kOneSz = 2 * G::ROWS == 32;                                 // 16 channels: lanes 16-31 fetch the zero rows
     const int sz_row = kOneSz ? (lane & 15) : lane;
-    const int64_t sz0 = (int64_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk;
-    const __half *iss_s = (kOneSz && lane >= 16 ? kz : ks) + sz0;
-    const ptrdiff_t sz_gap = kOneSz ? 0 : kz - ks;                             // zero row behind the scale row
+    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk);
+    const char *sz_b = reinterpret_cast<const char *>(kOneSz && lane >= 16 ? kz : ks);
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
     uint32_t iss_slot = 0, slot = 0;                                            // byte offsets of the slot being filled / read
     bool iss_ok = iss_col < n_words;
+
+    const char *kc_b = reinterpret_cast<const char *>(kc), *kz_b = reinterpret_cast<const char *>(kz);
+    const uint32_t row_step = (uint32_t)(G::RPI * 4) * kc_sD, stage_step = (uint32_t)(G::ROWS * 4) * kc_sD, sz_step = (uint32_t)(G::ROWS * 2) * ks_sD;
+    const uint32_t tile_step = 4 * tile_words - tile_stages * stage_step, tile_sz_step = 2 * tile_groups - tile_stages * sz_step;
 
     auto issue_stage = [&]() {
         if (iss_tiles > 0) {
             if (iss_ok) {
 #pragma unroll
                 for (int i = 0; i < G::GPL; ++i)
-                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, iss + i * G::RPI * kc_sD);
+                    cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, kc_b + (iss + i * row_step));
             }
             const uint32_t d = szcp_dst + iss_slot;
-            if (ngw == 8) { cp_async<16>(d, iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, iss_s + sz_gap); }
-            else if (ngw == 4) { cp_async<8>(d, iss_s); if (!kOneSz) cp_async<8>(d + G::ROWS * 16, iss_s + sz_gap); }
-            else { cp_async<4>(d, iss_s); if (!kOneSz) cp_async<4>(d + G::ROWS * 16, iss_s + sz_gap); }
+            if (ngw == 8) { cp_async<16>(d, sz_b + iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, kz_b + iss_s); }
+            else if (ngw == 4) { cp_async<8>(d, sz_b + iss_s); if (!kOneSz) cp_async<8>(d + G::ROWS * 16, kz_b + iss_s); }
+            else { cp_async<4>(d, sz_b + iss_s); if (!kOneSz) cp_async<4>(d + G::ROWS * 16, kz_b + iss_s); }
         }
         cp_async_commit();
         iss_slot = iss_slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : iss_slot + R::STAGE_BYTES;
-        iss += G::ROWS * kc_sD;
-        iss_s += G::ROWS * ks_sD;
+        iss += stage_step;
+        iss_s += sz_step;
         if (++iss_st == tile_stages) {
             iss_st = 0;
-            iss += tile_words - tile_stages * (G::ROWS * kc_sD);
-            iss_s += tile_groups - tile_stages * (G::ROWS * ks_sD);
+            iss += tile_step;
+            iss_s += tile_sz_step;
             iss_col += tile_words;
             iss_ok = iss_col < n_words;
             --iss_tiles;
@@ -244,7 +248,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                         }
                     }
                 } else {
-                    using H = VHalf<KB>;
+                    using H = KHalf<KB>;
                     const uint32_t lsrc = ldk_s + slot + (k * 16) * G::RS;
 #pragma unroll
                     for (int pb2 = 0; pb2 < NBK / 2; ++pb2) {              // two blocks per load
@@ -329,8 +333,8 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 #pragma unroll
                     for (int ip = 0; ip < MPB; ++ip) {
                         const int m = bb * MPB + ip;
-                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - VHalf<KB>::pos(2 * ip))), corr);
-                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - VHalf<KB>::pos(2 * ip + 1))), corr);
+                        float s0 = fmaf(acc[m][0] + acc[m][1], (float)(1 << (24 - KHalf<KB>::pos(2 * ip))), corr);
+                        float s1 = fmaf(acc[m][2] + acc[m][3], (float)(1 << (24 - KHalf<KB>::pos(2 * ip + 1))), corr);
                         *reinterpret_cast<float2 *>(dst + 2 * ip) = make_float2(s0, s1);
                     }
                 }
@@ -398,14 +402,16 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     const uint32_t pb_wr = pb_s + (pi * 8 + 4 * ch) * 4;
 
     const int block_stride = kMmaWarps * G::TPS;
-    const char *src_codes = reinterpret_cast<const char *>(vc + (int64_t)(t0 + warp * G::TPS) * a.vc_sT) + lane * 16;
+    const char *vc_b = reinterpret_cast<const char *>(vc);                               // 32-bit byte offsets from the head's first row
+    uint32_t src_codes = (uint32_t)(t0 + warp * G::TPS) * G::RBV + lane * 16;
     const int ngran = 4 * ngv;                                                           // 16-byte granules per array per stage
     const int sz_arr = lane >= ngran ? 1 : 0;                                            // 0: scale rows, 1: zero rows
     const int sz_off = (lane - sz_arr * ngran) * 16;
     const bool sz_on = lane < 2 * ngran;
-    const char *src_sz = reinterpret_cast<const char *>((sz_arr ? vz : vs) + (int64_t)(t0 + warp * G::TPS) * a.vs_sT) + sz_off;
+    const char *sz_b = reinterpret_cast<const char *>(sz_arr ? vz : vs);
+    uint32_t src_sz = (uint32_t)(t0 + warp * G::TPS) * (ngv * 2) + sz_off;
     const uint32_t sz_dst = ring_s + G::SZ_OFF + sz_arr * (G::TPS * 4 * 2) + sz_off;
-    const int64_t codes_step = (int64_t)block_stride * G::RBV, sz_step = (int64_t)block_stride * ngv * 2;
+    const uint32_t codes_step = block_stride * G::RBV, sz_step = block_stride * ngv * 2;
 
     int to_issue = my_blocks;                                                            // blocks not yet issued
     auto issue_stage = [&](uint32_t slot_off) {
@@ -413,8 +419,8 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
 #pragma unroll
             for (int i = 0; i < G::GPL; ++i)
                 if (G::TPS * G::GPT % 32 == 0 || lane + 32 * i < G::TPS * G::GPT)
-                    cp_async<16>(cp_dst + slot_off + i * (32 / G::GPT) * G::RBV, src_codes + i * 512);
-            if (sz_on) cp_async<16>(sz_dst + slot_off, src_sz);
+                    cp_async<16>(cp_dst + slot_off + i * (32 / G::GPT) * G::RBV, vc_b + (src_codes + i * 512));
+            if (sz_on) cp_async<16>(sz_dst + slot_off, sz_b + src_sz);
         }
         --to_issue;
         src_codes += codes_step;
@@ -597,19 +603,19 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     // neighbouring units of work, so the cache is fetched from HBM once and re-read from L2
     const int hk = h / (a.nh / a.nh_kv);
 
+    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
+    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
+    const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
+    prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, kMmaThreads);
     fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)h * a.q_sH;
     if (tid < kHeadDim) sm.q[tid] = q[tid];
-    const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
-    const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
-    prefetch_v_tail(a, vf, b, hk, v_lo, t1, tid, kMmaThreads);
 
     // ---- 1. scores ------------------------------------------------------------------------------
     {
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
         qk_packed_mma<KB>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
@@ -746,6 +752,8 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     if (a.Tkq > 0) {
         if (!al16(a.kcode) || a.kc_sB % 4 || a.kc_sH % 4 || a.kc_sD % 4) return false;
         if (!al16(a.kscale) || !al16(a.kmn) || a.ks_sB % 8 || a.ks_sH % 8 || a.ks_sD % 8) return false;
+        // a head's keys are addressed by 32-bit byte offsets (128 rows)
+        if (a.kc_sD < 0 || a.kc_sD >= (1 << 22) || a.ks_sD < 0 || a.ks_sD >= (1 << 23)) return false;
     }
     if (a.Tvq > 0) {
         const int fv = fields_per_word(a.v_bits);
