@@ -2,15 +2,23 @@
 //
 //   out[n] = fp16( sum_k in[k] * (scale[k, n/G] * code[k, n] + zero[k, n/G]) ),  fp32 accumulation
 //
+// Two kernels:
+//   gemv_mma_kernel   1, 2 and 4 bits, groups of 32 / 64 / 128: the codes go to mma.sync as fp16 subnormals, as in the
+//                     attention kernels; rows (k) are the contraction, so q . K^T (K = head_dim rows, thousands of columns)
+//                     and p . V (thousands of rows, 128 columns) are the same loop, split differently over the warps.
+//   gemv_kernel       everything else (3-bit words, other groups): one thread per word column.
+#include <cooperative_groups.h>
+
+#include "attn_mma_common.cuh"
+
+namespace kvq {
+
+// ---------------------------------------------------------------------------------------------
 // The zero term is hoisted: sum_k in[k]*zero[k,g] is accumulated once per packed word instead of
 // once per field, and in[k]*scale[k,g] is formed once per word.  A CTA is WX word columns x KY
 // k-lanes; lanes along the word axis read consecutive words (coalesced) for both uses of the
 // routine: q.K^T (K = head_dim rows, thousands of word columns) and p.V (thousands of rows,
 // head_dim/fpi word columns).
-#include "common.cuh"
-
-namespace kvq {
-
 template <int BITS>
 __global__ void __launch_bounds__(256) gemv_kernel(kvq_gemv_args a, int wx_log2, int nblk) {
     constexpr int FPI = fields_per_word(BITS);
@@ -55,6 +63,304 @@ __global__ void __launch_bounds__(256) gemv_kernel(kvq_gemv_args a, int wx_log2,
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Tensor-core form.  A warp works tiles of 128 columns (16 * BITS bytes of a row) x 32 rows a stage:
+//   A (16x16)  codes, rows = columns n of the result, k = 16 rows of the matrix (transposing ldmatrix, fields left in place);
+//   B (16x8)   column 2j / 2j + 1 = hi / lo of in[k] * scale[k, group j], j < 4 groups: the product of two fp16 numbers needs
+//              22 bits and is carried as an fp16 pair, so what is left is the fp32 accumulation, as before.  `in` is first
+//              divided by a power of two >= its largest magnitude in the chunk, so that no product overflows and the small
+//              probabilities of a long softmax keep their low part (absolute error 2^-25 of the largest).
+//   Every other 16 rows use the complement of the codes with the operand's sign turned, c = MAX - (MAX - c): the tensor core cuts
+//   products off downwards (codes are subnormal: 2^-20 of a product), which over thousands of rows of non-negative
+//   probabilities adds up to 3e-6 of the magnitude summed; with opposite signs the two halves cancel.
+//   zeros      one MMA per 16 rows with the [4 scales | 4 zeros] rows read transposed as A and `in` as B: row 4 + j of the
+//              product is the zero term of group j (and row j the sum of in * scale that the complemented rows need).
+// Bound by the instruction stream (0.6 logic operations a code); 16 sequences x 32 heads x 4096 tokens, q . K^T
+// and p . V together: 105 us at 2 bits and 115 us at 4 bits, 229 and 318 us with one thread per word column.
+template <int BITS> struct GemvGeom {
+    static constexpr int RB = 16 * BITS;                       // code bytes of a tile row
+    static constexpr int RS = BITS == 1 ? RB : RB + 16;        // padded: conflict-free ldmatrix
+    static constexpr int CODE_BYTES = 32 * RS;
+    static constexpr int STAGE_BYTES = CODE_BYTES + 32 * 16;
+    static constexpr int NS = BITS == 4 ? 3 : 4;
+    static constexpr int WARP_BYTES = NS * STAGE_BYTES;
+};
+constexpr int kGemvWarps = 8, kGemvThreads = 32 * kGemvWarps;
+constexpr int kGemvChunk = 2048;                               // rows whose `in` is held (and normalised) at a time
+constexpr int kGemvFlush = 8;                                  // stages between flushes of the MMA accumulators (short chains)
+
+struct GemvPlan {
+    int wk_log2;         // warps that share a column tile (the other factor of 8: column tiles of a CTA)
+    int col_ctas;        // CTAs per head along the columns
+    int kc;              // CTAs of a cluster, each with rows_per_cta rows
+    int rows_per_cta;
+    int code_align;      // 16, 8 or 4: what every row of a tile is aligned to
+    int sz_vec;          // scale / zero rows of a whole tile can be copied as one vector
+};
+
+template <int CG, int BITS>
+__device__ __forceinline__ void gemv_copy_codes(uint32_t dst, const int32_t *src, int64_t q_sK, int rows, int words, int lane) {
+    using G = GemvGeom<BITS>;
+    constexpr int GPR = G::RB / CG;                            // granules per row
+#pragma unroll
+    for (int i = 0; i < GPR; ++i) {
+        const int x = lane + 32 * i, row = x / GPR, col = x % GPR;
+        if (row < rows && col * (CG / 4) < words) cp_async<CG>(dst + row * G::RS + col * CG, src + row * q_sK + col * (CG / 4));
+    }
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_constant__ kvq_gemv_args a,
+                                                                   const __grid_constant__ GemvPlan plan) {
+    using G = GemvGeom<BITS>;
+    using F = VHalf<BITS>;
+    constexpr int FPI = fields_per_word(BITS), FH = 16 / BITS, MPB = FH / 2, NBLK = BITS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float *red = reinterpret_cast<float *>(smem);                               // [kGemvWarps][128] tile sums
+    __half *xs = reinterpret_cast<__half *>(red + kGemvWarps * 128);            // [kGemvChunk] normalised `in`
+    float *misc = reinterpret_cast<float *>(xs + kGemvChunk);                   // [8]
+    unsigned char *ring = reinterpret_cast<unsigned char *>(misc + 8) + 96;     // 128-byte aligned
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
+    const int WK = 1 << plan.wk_log2, wk = warp & (WK - 1), wc = warp >> plan.wk_log2, WC = kGemvWarps >> plan.wk_log2;
+    const int rank = blockIdx.x % plan.kc, job = blockIdx.x / plan.kc;
+    const int64_t s = job / plan.col_ctas;
+    const int b = (int)(s / a.nh), h = (int)(s % a.nh), hk = h / (int)(a.nh / a.nh_kv);
+    const int N = (int)(a.n_groups * a.group), n_pack = N / FPI;
+    const int n0 = ((job % plan.col_ctas) * WC + wc) * 128;                     // this warp's first column
+    const int k_beg = rank * plan.rows_per_cta, k_end = min((int)a.K, k_beg + plan.rows_per_cta);
+    const int grp0 = n0 / a.group, ngw = 128 / a.group;
+    const int words = min(128 / FPI, n_pack - n0 / FPI);                        // <= 0: no such tile
+    const __half *in = static_cast<const __half *>(a.fA) + b * a.a_sB + h * a.a_sH;
+    const int32_t *qb = a.qB + b * a.q_sB + hk * a.q_sH + n0 / FPI;
+    const int64_t zo = b * a.s_sB + hk * a.s_sH + grp0;
+    const __half *sp = static_cast<const __half *>(a.scale) + zo, *zp = static_cast<const __half *>(a.zero) + zo;
+    const int groups = min(ngw, (int)a.n_groups - grp0);
+    const bool vec = plan.sz_vec && groups == ngw;
+
+    const uint32_t ring_s = smem_u32(ring) + warp * G::WARP_BYTES;
+    const uint32_t sz_dst = ring_s + G::CODE_BYTES + lane * 16;
+    const uint32_t szm_s = ring_s + G::CODE_BYTES + (lane & 15) * 16;
+    const uint32_t ldk_s = ring_s + (lane & 15) * G::RS + (BITS == 1 ? 0 : (lane >> 4) * 16);
+    const uint32_t x_s = smem_u32(xs) + (2 * tig) * 2;
+    const int src = 4 * (g >> 1) + tig;                                         // lane holding group (column / 2)
+    const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;
+
+    float acc[8][4], sum[8][2], accz[2][4] = {}, zsum = 0.f;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) { acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f; sum[m][0] = sum[m][1] = 0.f; }
+
+    for (int c0 = k_beg; c0 < k_end; c0 += kGemvChunk) {
+        const int rows = min(kGemvChunk, k_end - c0), n_st = (rows + 31) / 32;
+        // ---- in / 2^e, 2^e >= the largest magnitude of the chunk (an infinity or NaN is left as it is) -----------
+        if (c0 > k_beg) __syncthreads();                                        // the previous chunk has been read
+        float mx = 0.f;
+        for (int i = tid; i < rows; i += kGemvThreads) mx = fmaxf(mx, fabsf(__half2float(__ldg(in + c0 + i))));
+        mx = warp_max(mx);
+        if (lane == 0) misc[warp] = mx;
+        __syncthreads();
+        mx = warp_max(misc[lane & 7]);
+        int e = 0;
+        if (mx > 0.f && mx <= 65504.f) e = (int)((__float_as_uint(mx) >> 23) & 255u) - 126;   // mx < 2^e
+        const float down = __uint_as_float((uint32_t)(127 - e) << 23), up = __uint_as_float((uint32_t)(127 + e) << 23);
+        for (int i = tid; i < n_st * 32; i += kGemvThreads)
+            xs[i] = i < rows ? __float2half_rn(__half2float(__ldg(in + c0 + i)) * down) : __float2half_rn(0.f);
+        __syncthreads();
+        if (words <= 0) continue;
+
+        auto issue = [&](int st, uint32_t slot) {
+            if (st < n_st) {
+                const int left = rows - 32 * st;                                // rows of the stage that exist
+                const int64_t r0 = c0 + 32 * st;
+                const int32_t *p = qb + r0 * a.q_sK;
+                if (plan.code_align == 16) gemv_copy_codes<16, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                else if (plan.code_align == 8) gemv_copy_codes<8, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                else gemv_copy_codes<4, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                const __half *ps = sp + (r0 + lane) * a.s_sK, *pz = zp + (r0 + lane) * a.s_sK;
+                const uint32_t d = sz_dst + slot;
+                if (lane < left && vec && ngw > 1) {
+                    if (ngw == 4) { cp_async<8>(d, ps); cp_async<8>(d + 8, pz); }
+                    else { cp_async<4>(d, ps); cp_async<4>(d + 8, pz); }
+                } else {                                                        // odd group counts, one group a tile, missing rows: zeros
+                    uint32_t v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int jj = j & 1;
+                        const __half *q = j < 2 ? ps : pz;
+                        const bool ok0 = lane < left && 2 * jj < groups, ok1 = lane < left && 2 * jj + 1 < groups;
+                        const uint32_t lo = ok0 ? __half_as_ushort(__ldg(q + 2 * jj)) : 0u, hi = ok1 ? __half_as_ushort(__ldg(q + 2 * jj + 1)) : 0u;
+                        v[j] = lo | (hi << 16);
+                    }
+                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+                }
+            }
+            cp_async_commit();
+        };
+        auto flush = [&]() {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                sum[m][0] = fmaf(acc[m][0] + acc[m][1], up, sum[m][0]);
+                sum[m][1] = fmaf(acc[m][2] + acc[m][3], up, sum[m][1]);
+                acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+            }
+            // lanes of rows 4 .. 7: zero terms of all rows; of rows 0 .. 3: sums of in * scale of the complemented rows
+            zsum = fmaf(g < 4 ? accz[1][0] : accz[0][0] + accz[1][0], up, zsum);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) accz[0][i] = accz[1][i] = 0.f;
+        };
+
+        uint32_t iss_slot = 0, slot = 0;
+        int iss_st = wk;
+#pragma unroll 1
+        for (int q = 0; q < G::NS - 1; ++q) { issue(iss_st, iss_slot); iss_st += WK; iss_slot += G::STAGE_BYTES; }
+        int since = 0;
+#pragma unroll 1
+        for (int st = wk; st < n_st; st += WK) {
+            issue(iss_st, iss_slot);
+            iss_st += WK;
+            iss_slot = iss_slot == (G::NS - 1) * G::STAGE_BYTES ? 0u : iss_slot + G::STAGE_BYTES;
+            cp_async_wait<G::NS - 1>();
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t xa = x_s + (32 * st + 16 * k) * 2;
+                const uint32_t x01u = lds32(xa), x89u = lds32(xa + 16);
+                uint32_t r0, r1;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                             : "=r"(r0), "=r"(r1) : "r"(szm_s + slot + k * 256));
+                mma16816(accz[k], r0, 0u, r1, 0u, x01u, x89u);
+                const uint32_t flip = k ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
+                // an infinite product gives hi = inf and lo = NaN: the minimum keeps a number there, and the sum infinite
+                const __half2 big = __floats2half2_rn(65504.f, 65504.f);
+                const uint32_t h0 = hilo(as_h2(x01u ^ sign), as_h2(__shfl_sync(0xffffffffu, r0, src)), neg_mask);
+                const uint32_t h1 = hilo(as_h2(x89u ^ sign), as_h2(__shfl_sync(0xffffffffu, r1, src)), neg_mask);
+                const uint32_t b0 = (as_u32(__hmin2(as_h2(h0), big)) & neg_mask) | (h0 & ~neg_mask);
+                const uint32_t b1 = (as_u32(__hmin2(as_h2(h1), big)) & neg_mask) | (h1 & ~neg_mask);
+                uint32_t x[NBLK][2];
+                const uint32_t ad = ldk_s + slot + (16 * k) * G::RS;
+                if constexpr (BITS == 1) {
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(x[0][0]), "=r"(x[0][1]) : "r"(ad));
+                } else {
+#pragma unroll
+                    for (int p = 0; p < NBLK / 2; ++p)
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                                     : "=r"(x[2 * p][0]), "=r"(x[2 * p][1]), "=r"(x[2 * p + 1][0]), "=r"(x[2 * p + 1][1]) : "r"(ad + 32 * p));
+                }
+#pragma unroll
+                for (int bb = 0; bb < NBLK; ++bb) {
+                    uint32_t rlo[F::N], rhi[F::N];
+                    F::unpack(x[bb][0] ^ flip, rlo);
+                    F::unpack(x[bb][1] ^ flip, rhi);
+#pragma unroll
+                    for (int i = 0; i < F::N; i += 2)
+                        mma16816(acc[bb * MPB + i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b0, b1);
+                }
+            }
+            __syncwarp();
+            slot = slot == (G::NS - 1) * G::STAGE_BYTES ? 0u : slot + G::STAGE_BYTES;
+            if (++since == kGemvFlush) { flush(); since = 0; }
+        }
+        flush();
+        cp_async_wait<0>();
+        __syncwarp();
+    }
+
+    // ---- tile sums: octet g of block bb owns columns bb * 8 FH + g * FH .. + FH - 1, their group's pair of B columns is held by
+    // the lane with tig == group, its zero term by row 4 + group
+    if (words > 0) {
+#pragma unroll
+        for (int bb = 0; bb < NBLK; ++bb) {
+            const int c = bb * 8 * FH + g * FH, cp = c / a.group;
+            constexpr float kMax = (float)((1 << BITS) - 1);
+            const float corr = fmaf(kMax, __shfl_sync(0xffffffffu, zsum, 4 * cp), __shfl_sync(0xffffffffu, zsum, 4 * (4 + cp)));
+            if (tig == cp) {
+#pragma unroll
+                for (int ip = 0; ip < MPB; ++ip) {
+                    red[warp * 128 + c + 2 * ip] = fmaf(sum[bb * MPB + ip][0], (float)(1 << (24 - F::pos(2 * ip))), corr);
+                    red[warp * 128 + c + 2 * ip + 1] = fmaf(sum[bb * MPB + ip][1], (float)(1 << (24 - F::pos(2 * ip + 1))), corr);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    __half *out = static_cast<__half *>(a.out) + b * a.o_sB + h * a.o_sH;
+    const int col0 = (job % plan.col_ctas) * WC * 128;
+    namespace cg = cooperative_groups;
+    if (plan.kc > 1) {                                                          // every rank: the sums over its warps; rank 0 adds the ranks
+        for (int i = tid; i < WC * 128; i += kGemvThreads) {
+            float v = 0.f;
+            for (int j = 0; j < WK; ++j) v += red[((i >> 7) * WK + j) * 128 + (i & 127)];
+            red[((i >> 7) * WK) * 128 + (i & 127)] = v;                         // only this thread reads or writes these entries
+        }
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        if (rank == 0) {
+            for (int i = tid; i < WC * 128; i += kGemvThreads) {
+                float v = 0.f;
+                for (int r = 0; r < plan.kc; ++r) v += cluster.map_shared_rank(red, r)[((i >> 7) * WK) * 128 + (i & 127)];
+                if (col0 + i < N) out[col0 + i] = __float2half_rn(v);
+            }
+        }
+        cluster.sync();                                                         // nobody leaves while its sums are read
+    } else {
+        for (int i = tid; i < WC * 128; i += kGemvThreads) {
+            float v = 0.f;
+            for (int j = 0; j < WK; ++j) v += red[((i >> 7) * WK + j) * 128 + (i & 127)];
+            if (col0 + i < N) out[col0 + i] = __float2half_rn(v);
+        }
+    }
+}
+
+template <int BITS>
+static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned grid, cudaStream_t st) {
+    const size_t smem = kGemvWarps * 128 * 4 + kGemvChunk * 2 + 8 * 4 + 96 + (size_t)kGemvWarps * GemvGeom<BITS>::WARP_BYTES;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return record_cuda_error(e);
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        e = cudaFuncSetAttribute(gemv_mma_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return record_cuda_error(e);
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kGemvThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)p.kc;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = p.kc > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<BITS>, a, p);
+    if (e != cudaSuccess) return record_cuda_error(e);
+    return check_launch();
+}
+
+// The split of the work: a CTA's eight warps take as many column tiles as there are (p . V has one) and share each tile's rows
+// with the rest; where heads x column CTAs leave half of the resident CTAs (296) idle, clusters of up to eight CTAs cut
+// the rows further, at least 512 a CTA.
+static bool gemv_mma_plan(const kvq_gemv_args &a, int64_t n_pack, GemvPlan &p, int64_t &grid) {
+    if (a.bits == 3 || (a.group != 32 && a.group != 64 && a.group != 128)) return false;
+    if (a.K <= 0 || a.K > (1 << 30) || a.n_groups * a.group > (1 << 30)) return false;
+    const int64_t tiles = (a.n_groups * a.group + 127) / 128;
+    p.wk_log2 = tiles > 4 ? 0 : tiles > 2 ? 1 : tiles > 1 ? 2 : 3;
+    const int wc = kGemvWarps >> p.wk_log2;
+    p.col_ctas = (int)((tiles + wc - 1) / wc);
+    const int64_t jobs = a.B * a.nh * p.col_ctas;
+    p.kc = 1;
+    while (p.kc < 8 && jobs * p.kc * 2 <= 2 * 148 && a.K >= 512LL * p.kc * 2) p.kc *= 2;
+    p.rows_per_cta = (int)((a.K + 32LL * p.kc - 1) / (32LL * p.kc) * 32);
+    const uint64_t bits = reinterpret_cast<uintptr_t>(a.qB) | (uint64_t)(4 * (a.q_sB | a.q_sH | a.q_sK | n_pack));
+    p.code_align = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 4;
+    const int ngw = 128 / a.group;
+    p.sz_vec = (reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.zero)) % (2 * ngw) == 0 &&
+               a.s_sB % ngw == 0 && a.s_sH % ngw == 0 && a.s_sK % ngw == 0;
+    grid = jobs * p.kc;
+    return grid <= 2147483647LL;
+}
+
 }  // namespace kvq
 
 extern "C" int kvq_gemv(const kvq_gemv_args *a, kvq_stream_t stream) {
@@ -71,13 +377,22 @@ extern "C" int kvq_gemv(const kvq_gemv_args *a, kvq_stream_t stream) {
     if (a->B * a->nh == 0 || n_pack == 0) return KVQ_OK;
     if (!a->fA || !a->out) return KVQ_ERR_NULL;
     if (a->K > 0 && (!a->qB || !a->scale || !a->zero)) return KVQ_ERR_NULL;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    GemvPlan p;
+    int64_t mma_grid = 0;
+    if (gemv_mma_plan(*a, n_pack, p, mma_grid)) {
+        switch (a->bits) {
+            case 1: return launch_gemv_mma<1>(*a, p, (unsigned)mma_grid, st);
+            case 2: return launch_gemv_mma<2>(*a, p, (unsigned)mma_grid, st);
+            default: return launch_gemv_mma<4>(*a, p, (unsigned)mma_grid, st);
+        }
+    }
     int wx_log2 = 5;
     while (wx_log2 > 2 && (1 << (wx_log2 - 1)) >= n_pack) --wx_log2;
     const int WX = 1 << wx_log2;
     const int64_t nblk = (n_pack + WX - 1) / WX;
     if (nblk * a->B * a->nh > 2147483647LL) return KVQ_ERR_UNSUPPORTED;
     dim3 grid((unsigned)(nblk * a->B * a->nh));
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     switch (a->bits) {
         case 1: gemv_kernel<1><<<grid, 256, 0, st>>>(*a, wx_log2, (int)nblk); break;
         case 2: gemv_kernel<2><<<grid, 256, 0, st>>>(*a, wx_log2, (int)nblk); break;
