@@ -88,6 +88,7 @@ class KVmixLayerCache:
                              vc.data_ptr(), vc.stride(0), vc.stride(1), vc.stride(2),
                              vs.data_ptr(), self.vmn.data_ptr(), vs.stride(0), vs.stride(1), vs.stride(2),
                              vf.data_ptr(), vf.stride(0), vf.stride(1), vf.stride(2), self.v_cap, 0, 0, 0)
+        self._att_ref = C.byref(self._att)
         self._ws = {}
         self._fused = None               # None: not tried yet; False: the library does not fuse this geometry
         # device_state=True: lengths and ring starts also live in device memory ({T, Tkq, Tvq, k_start, v_start}, then the
@@ -216,7 +217,7 @@ class KVmixLayerCache:
         a.vscale, a.vmn, a.vs_sB, a.vs_sH, a.vs_sT = vs.data_ptr(), self.vmn.data_ptr(), vs.stride(0), vs.stride(1), vs.stride(2)
         a.kfull, a.kf_sB, a.kf_sH, a.kf_sT = kf.data_ptr(), kf.stride(0), kf.stride(1), kf.stride(2)
         a.vfull, a.vf_sB, a.vf_sH, a.vf_sT = vf.data_ptr(), vf.stride(0), vf.stride(1), vf.stride(2)
-        _lib.check(self._lib.kvq_prefill(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        _lib.check(self._lib.kvq_prefill(C.byref(a), ops.raw_stream()))
         ops.LAUNCHES[0] += (nk > 0) + (nv > 0) + (nk < L or nv < L)
         self.tkq, self.tvq = nk, nv
         self.k_start = self.v_start = 0
@@ -237,7 +238,7 @@ class KVmixLayerCache:
         a.v_new, a.vn_sB, a.vn_sH = v_new.data_ptr(), v_new.stride(0), v_new.stride(1)
         a.k_slot = (self.k_start + self.k_len) % self.k_cap
         a.v_slot = (self.v_start + self.v_len) % self.v_cap
-        _lib.check(self._lib.kvq_append_kv(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        _lib.check(self._lib.kvq_append_kv(C.byref(a), ops.raw_stream()))
         ops.LAUNCHES[0] += 1
         self.k_len += 1
         self.v_len += 1
@@ -267,8 +268,8 @@ class KVmixLayerCache:
         if q.stride(3) != 1 or q.dtype != torch.float16:
             q = q.to(torch.float16).contiguous()
         if out is None:
-            out = torch.empty((B, nh, 1, D), dtype=torch.float16, device=q.device)
-        stream = torch.cuda.current_stream().cuda_stream
+            out = q.new_empty((B, nh, 1, D))
+        stream = ops.raw_stream()
         ws = self._workspace(nh, stream, q.device)
         a = self._att
         a.nh, a.T, a.Tkq, a.Tvq = nh, self.tkq + self.k_len, self.tkq, self.tvq
@@ -280,7 +281,7 @@ class KVmixLayerCache:
         a.mask, a.mask_sB, a.mask_sH, a.mask_is_f32 = ops.mask_fields(attention_mask, B, nh, a.T)
         if peers is not None:
             peers.fill(a)
-        rc = self._lib.kvq_decode_attn(C.byref(a), C.c_void_p(stream))
+        rc = self._lib.kvq_decode_attn(self._att_ref, stream)
         a.n_peers = 0
         _lib.check(rc)
         ops.LAUNCHES[0] += 1
@@ -315,11 +316,19 @@ class KVmixLayerCache:
         nv = split_point(self.v_len + 1, self.v_group, self.rv, self.window)
         if nk not in (0, self.k_group) or nv not in (0, self.v_group) or nk > self.k_len or nv > self.v_len:
             return None                                         # more than one group due (a freshly adopted cache): unfused
-        fix = lambda t: t if (t.stride(3) == 1 and t.dtype == torch.float16) else t.to(torch.float16).contiguous()
-        q, k_new, v_new = fix(q), fix(k_new), fix(v_new)
+        qs, ks, vs = q.stride(), k_new.stride(), v_new.stride()
+        if qs[3] != 1 or q.dtype != torch.float16:
+            q = q.to(torch.float16).contiguous()
+            qs = q.stride()
+        if ks[3] != 1 or k_new.dtype != torch.float16:
+            k_new = k_new.to(torch.float16).contiguous()
+            ks = k_new.stride()
+        if vs[3] != 1 or v_new.dtype != torch.float16:
+            v_new = v_new.to(torch.float16).contiguous()
+            vs = v_new.stride()
         if out is None:
-            out = torch.empty((B, nh, 1, D), dtype=torch.float16, device=q.device)
-        stream = torch.cuda.current_stream().cuda_stream
+            out = q.new_empty((B, nh, 1, D))
+        stream = ops.raw_stream()
         ws = self._workspace(nh, stream, q.device)
         a = self._att
         a.nh, a.T, a.Tkq, a.Tvq = nh, self.kv_seq_len + 1, self.tkq + nk, self.tvq + nv
@@ -336,17 +345,21 @@ class KVmixLayerCache:
             a.window = -1 if self.window is None else int(self.window)
             a.k_ratio, a.v_ratio = float(self.rk or 0.0), float(self.rv or 0.0)
         a.round_scores = int(bool(round_scores))
-        a.q, a.q_sB, a.q_sH = q.data_ptr(), q.stride(0), q.stride(1)
-        a.out, a.o_sB, a.o_sH = out.data_ptr(), out.stride(0), out.stride(1)
+        os = out.stride()
+        a.q, a.q_sB, a.q_sH = q.data_ptr(), qs[0], qs[1]
+        a.out, a.o_sB, a.o_sH = out.data_ptr(), os[0], os[1]
         a.kf_start, a.vf_start = (self.k_start + nk) % self.k_cap, (self.v_start + nv) % self.v_cap
         a.workspace, a.workspace_bytes, a.flags = ws.data_ptr(), ws.numel(), _lib.ATTN_WORKSPACE_READY
-        a.mask, a.mask_sB, a.mask_sH, a.mask_is_f32 = ops.mask_fields(attention_mask, B, nh, self.kv_seq_len + 1)
-        a.k_new, a.kn_sB, a.kn_sH = k_new.data_ptr(), k_new.stride(0), k_new.stride(1)
-        a.v_new, a.vn_sB, a.vn_sH = v_new.data_ptr(), v_new.stride(0), v_new.stride(1)
+        if attention_mask is None:
+            a.mask = None
+        else:
+            a.mask, a.mask_sB, a.mask_sH, a.mask_is_f32 = ops.mask_fields(attention_mask, B, nh, self.kv_seq_len + 1)
+        a.k_new, a.kn_sB, a.kn_sH = k_new.data_ptr(), ks[0], ks[1]
+        a.v_new, a.vn_sB, a.vn_sH = v_new.data_ptr(), vs[0], vs[1]
         a.k_quant, a.v_quant, a.k_quant_slot, a.v_quant_slot = nk, nv, self.k_start, self.v_start
         if peers is not None:
             peers.fill(a)
-        rc = self._lib.kvq_decode_attn(C.byref(a), C.c_void_p(stream))
+        rc = self._lib.kvq_decode_attn(self._att_ref, stream)
         a.k_new = a.v_new = a.state = None
         a.k_quant = a.v_quant = a.n_peers = 0
         if rc == -11:                                           # this geometry is not served fused: remember and fall back
