@@ -448,14 +448,15 @@ extern "C" int kvq_decode_attn(const kvq_attn_args *a, kvq_stream_t stream) {
     if (L.ctas > 2147483647LL) return KVQ_ERR_UNSUPPORTED;
     if (a->n_peers != 0) {                                     // head-sharded exchange (see the header)
         if (a->n_peers < 0 || a->n_peers > KVQ_MAX_PEERS || a->peer_head0 < 0) return KVQ_ERR_SHAPE;
-        if (!L.use_mma) return KVQ_ERR_UNSUPPORTED;
+        if (!L.use_mma || a->v_bits == 3) return KVQ_ERR_UNSUPPORTED;
         for (int p = 0; p < a->n_peers; ++p)
             if (!a->peer_out[p] || !a->peer_flag[p]) return KVQ_ERR_NULL;
     }
     if (a->k_new || a->v_new) {                                // fused decode step (see the header)
         if (!a->k_new || !a->v_new) return KVQ_ERR_NULL;
         const int n_rep = a->nh / a->nh_kv;
-        if (!L.use_mma || (L.qhv ? n_rep != L.qhv : n_rep != 1)) return KVQ_ERR_UNSUPPORTED;   // one CTA per kv head and segment
+        // one CTA per kv head and segment; the update of 3-bit values is not fused
+        if (!L.use_mma || a->v_bits == 3 || (L.qhv ? n_rep != L.qhv : n_rep != 1)) return KVQ_ERR_UNSUPPORTED;
         if (!dev_state) {
             if (Rk < 1 || Rv < 1) return KVQ_ERR_TOKENS;       // the new token stays in the fp16 tails
             if ((a->k_quant != 0 && a->k_quant != a->k_group) || (a->v_quant != 0 && a->v_quant != a->v_group)) return KVQ_ERR_TOKENS;

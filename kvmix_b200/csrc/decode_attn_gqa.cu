@@ -40,10 +40,15 @@ template <int VB> using GqaVGeom = VGeom<VB, VB == 4 ? 3 : VB == 2 ? 5 : 7>;
 // operand tiles of the values: 512 bytes per channel group (4 / 2 / 2 groups at most)
 template <int VB> constexpr int gqa_op_bytes() { return VB == 4 ? 2048 : 1024; }
 
+// 3-bit values (the short-last-group extension: 12 words and 12 groups a token): 48 + 2 x 24 bytes a token, two slots, operand
+// tiles of four groups and the tile of the probabilities
+constexpr int kV3Words = (kHeadDim + 10) / 11;
+constexpr int kV3Stage = 32 * (kV3Words * 4 + 2 * kV3Words * 2), kV3Slots = 2, kV3SzOff = 32 * kV3Words * 4;
+constexpr int kV3Region = kV3Slots * kV3Stage + 4 * 512 + 512;
+template <int VB> constexpr int gqa_v_region() { return GqaVGeom<VB>::NS * GqaVGeom<VB>::STAGE_BYTES + gqa_op_bytes<VB>(); }
+template <> constexpr int gqa_v_region<3>() { return kV3Region; }
 template <int KB, int VB> constexpr int gqa_region_bytes() {
-    constexpr int k = GqaKRing<KB>::BYTES;
-    constexpr int v = GqaVGeom<VB>::NS * GqaVGeom<VB>::STAGE_BYTES + gqa_op_bytes<VB>();
-    return k > v ? k : v;
+    return GqaKRing<KB>::BYTES > gqa_v_region<VB>() ? GqaKRing<KB>::BYTES : gqa_v_region<VB>();
 }
 
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
@@ -412,23 +417,7 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     const bool split = VB == 1 && Gv == 64;
     const uint32_t rows0 = !split || g < 4 ? 0xffffffffu : 0u, rows1 = g >= 4 ? 0xffffffffu : 0u;
     const uint32_t ones = 0x3c003c00u;
-    constexpr int kFlush = 16;                                 // short accumulation chains (see the single-head kernel)
-    float sum[8][2], sumz[2] = {0.f, 0.f};
-#pragma unroll
-    for (int m = 0; m < 8; ++m) sum[m][0] = sum[m][1] = 0.f;
-    auto flush = [&]() {
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            sum[m][0] += acc[m][0];
-            sum[m][1] += acc[m][2];
-            acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
-        }
-        sumz[0] += accz[0][0] + accz[1][0];
-        sumz[1] += accz[0][1] + accz[1][1];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) accz[u][0] = accz[u][1] = accz[u][2] = accz[u][3] = 0.f;
-    };
-
+    // accumulation chains stay short by themselves (see the single-head kernel): 2112 tokens are at most nine blocks a warp
     if (MODE != 2) {
 #pragma unroll
         for (int q = 0; q < G::P; ++q) { issue_stage(q * G::STAGE_BYTES); cp_async_commit(); }
@@ -519,14 +508,12 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
         issue_st = (issue_st + G::STAGE_BYTES == G::NS * G::STAGE_BYTES) ? 0u : issue_st + G::STAGE_BYTES;
         pa += block_stride;
         pb += block_stride;
-        if ((q % kFlush) == kFlush - 1) flush();
     }
-    flush();
     cp_async_wait<0>();
     __syncwarp();
     // epilogue: lane (g, tig) holds channels of rows g / g + 8 for head tig (column 2 tig); row jv of the ones-MMAs holds
     // (sum p*scale, sum p*mid) of channel group jv for head tig
-    const float corr_mine = (sumz[1] - G::MID * sumz[0]) * (1.f / 256.f);
+    const float corr_mine = ((accz[0][1] + accz[1][1]) - G::MID * (accz[0][0] + accz[1][0])) * (1.f / 256.f);
     float cj[4];
 #pragma unroll
     for (int jv = 0; jv < 4; ++jv) cj[jv] = __shfl_sync(0xffffffffu, corr_mine, 4 * jv + tig);
@@ -537,9 +524,161 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
                          : Gv == 64 ? (VB == 1 ? (g >= 4 ? cj[1] : cj[0]) : cj[(bb * CPB) / 64]) : cj[0];
 #pragma unroll
         for (int ip = 0; ip < MPB; ++ip) {
-            my_red[tig * kHeadDim + c0 + 2 * ip] = fmaf(sum[bb * MPB + ip][0], (float)(1 << (16 - F::pos(2 * ip))), corr);
-            my_red[tig * kHeadDim + c0 + 2 * ip + 1] = fmaf(sum[bb * MPB + ip][1], (float)(1 << (16 - F::pos(2 * ip + 1))), corr);
+            my_red[tig * kHeadDim + c0 + 2 * ip] = fmaf(acc[bb * MPB + ip][0], (float)(1 << (16 - F::pos(2 * ip))), corr);
+            my_red[tig * kHeadDim + c0 + 2 * ip + 1] = fmaf(acc[bb * MPB + ip][2], (float)(1 << (16 - F::pos(2 * ip + 1))), corr);
         }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// p . V over 3-bit values: twelve words a token, each its own group of 11 channels (the last of 7).  As for 3-bit keys the
+// channels of a word are the rows of an MMA (11 of 16 used); p * scale is carried as an fp16 pair hi + lo of the fp32
+// product, columns 2h / 2h + 1 of head h (4 p, saturating only together: 65504 + 65504 is above 4 * 18715, the largest
+// scale a group of fp16 numbers can have), the zero terms come from one MMA per 16 tokens (rows = groups, B = p hi / lo).
+// Every other 16 tokens use the complemented codes and the operands' sign turned, so that what the tensor core cuts off
+// the products (codes are subnormal) cancels instead of adding up; the sums of p * scale this needs are one more such MMA.
+// Bound by the operand tiles (12 groups x 4 heads of p * scale for 352 bytes of a token pair).  8 x 8 kv heads, 32768
+// tokens, 3-bit keys and values: 210 us a layer, 735 us with the CUDA-core kernel.
+template <int MODE>
+__device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int32_t *vc, const __half *vs, const __half *vz,
+                                               const GqaSmem &sm, int t0, int hi) {
+    constexpr int W = kV3Words;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int n_blocks = (hi - t0 + 31) / 32;
+    const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
+    float *my_red = reinterpret_cast<float *>(sm.ring);
+    if (my_blocks <= 0) {
+        if (MODE != 1)
+            for (int i = lane; i < kQH * kHeadDim; i += 32) my_red[i] = 0.f;
+        return;
+    }
+    const uint32_t ring_s = smem_u32(sm.ring);
+    const uint32_t op_s = ring_s + kV3Slots * kV3Stage, pp_s = op_s + 4 * 512;
+    const char *vc_b = reinterpret_cast<const char *>(vc);
+    uint32_t src_codes = (uint32_t)(t0 + warp * 32) * (W * 4) + lane * 16;
+    // granules lane, lane + 32, lane + 64 of the 48 + 48 of a stage's scale and zero rows
+    uint32_t src_sz = (uint32_t)(t0 + warp * 32) * (W * 2);
+    constexpr uint32_t codes_step = kMmaWarps * 32 * W * 4, sz_step = kMmaWarps * 32 * W * 2;
+    int to_issue = my_blocks;
+    auto issue_stage = [&](uint32_t slot) {
+        if (to_issue > 0) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                cp_async<16>(ring_s + slot + lane * 16 + i * 512, vc_b + (src_codes + i * 512));
+                const int x = lane + 32 * i, z = x >= 48;
+                cp_async<16>(ring_s + slot + kV3SzOff + x * 16, reinterpret_cast<const char *>(z ? vz : vs) + (src_sz + (x - 48 * z) * 16));
+            }
+        }
+        cp_async_commit();
+        --to_issue;
+        src_codes += codes_step;
+        src_sz += sz_step;
+    };
+    if (MODE == 1) {
+        issue_stage(0);
+        return;
+    }
+    --to_issue;
+    src_codes += codes_step;
+    src_sz += sz_step;
+
+    // field g / g + 8 of a word (see gqa_qk_packed)
+    const int byte0 = (3 * g) >> 3, p0 = 3 * g - 8 * byte0;
+    const uint32_t sel0 = (uint32_t)(byte0 | ((byte0 + 1) << 4) | ((4 + byte0) << 8) | ((5 + byte0) << 12));
+    const uint32_t msk0 = 0x00070007u << p0, sel1 = 0x7733u;
+    const uint32_t msk1 = g == 0 ? 0x00070007u : g == 1 ? 0x00380038u : g == 2 ? 0x00c000c0u : 0u;
+    const int p1 = 3 * (g < 3 ? g : 0);
+    // operand build: lane -> token pair pi = lane & 15, head pair hh = lane >> 4
+    const int pi = lane & 15, hh = lane >> 4;
+    const int bt0 = 16 * (pi >> 3) + 8 * ((pi >> 2) & 1) + 2 * (pi & 3);
+    const uint32_t sz_rd = ring_s + kV3SzOff + bt0 * (W * 2);
+    const uint32_t op_wr = op_s + (pi * 8 + 4 * hh) * 4, op_rd = op_s + (tig * 8 + g) * 4;
+    const float *pa = sm.scores + (2 * hh) * sm.n_scores + warp * 32 + bt0, *pb = pa + sm.n_scores;
+    const uint32_t w_rd = ring_s + (2 * tig) * (W * 4);
+    const uint32_t g_rd = ring_s + kV3SzOff + (2 * tig) * (W * 2) + 2 * g;            // scale of (token 2 tig, group g); zeros + 768
+
+    float acc[W][4], accz[4] = {0.f, 0.f, 0.f, 0.f}, accs[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < W; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    auto put = [&](uint32_t addr, float x0, float x1, float y0, float y1) {           // hi, lo of (x0, x1), then of (y0, y1)
+        const uint32_t hx = pack_h2_sat(x0, x1), hy = pack_h2_sat(y0, y1);
+        const float2 fx = __half22float2(as_h2(hx)), fy = __half22float2(as_h2(hy));
+        const uint32_t lx = pack_h2_sat(x0 - fx.x, x1 - fx.y), ly = pack_h2_sat(y0 - fy.x, y1 - fy.y);
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(hx), "r"(lx), "r"(hy), "r"(ly));
+    };
+    // A fragment of a [token][group] tile read transposed: rows g, g + 8 = groups (12 of 16), k = 16 tokens
+    auto group_rows = [&](uint32_t addr, uint32_t (&r)[4]) {
+        const uint32_t n = W * 2;
+        r[0] = lds16(addr) | (lds16(addr + n) << 16);
+        r[2] = lds16(addr + 8 * n) | (lds16(addr + 9 * n) << 16);
+        r[1] = r[3] = 0u;
+        if (g < W - 8) {
+            r[1] = lds16(addr + 16) | (lds16(addr + n + 16) << 16);
+            r[3] = lds16(addr + 8 * n + 16) | (lds16(addr + 9 * n + 16) << 16);
+        }
+    };
+
+    uint32_t st = 0;
+#pragma unroll 1
+    for (int q = 0; q < my_blocks; ++q) {
+        issue_stage(kV3Stage - st);
+        cp_async_wait<1>();
+        __syncwarp();
+        const float2 fa = *reinterpret_cast<const float2 *>(pa), fb = *reinterpret_cast<const float2 *>(pb);
+        const float a0 = 4.f * fa.x, a1 = 4.f * fa.y, b0 = 4.f * fb.x, b1 = 4.f * fb.y;
+        put(pp_s + (pi * 8 + 4 * hh) * 4, a0, a1, b0, b1);
+#pragma unroll
+        for (int r = 0; r < W / 4; ++r) {
+#pragma unroll
+            for (int jv = 0; jv < 4; ++jv) {
+                const float s0 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * (4 * r + jv))));
+                const float s1 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * (4 * r + jv) + W * 2)));
+                put(op_wr + jv * 512, a0 * s0, a1 * s1, b0 * s0, b1 * s1);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {
+                const uint32_t flip = h2 ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
+                if (r == 0) {
+                    const uint32_t pp_rd = pp_s + (tig * 8 + g + 64 * h2) * 4, x0 = lds32(pp_rd), x1 = lds32(pp_rd + 128);
+                    uint32_t z[4];
+                    group_rows(g_rd + st + h2 * 16 * (W * 2) + 32 * (W * 2), z);
+                    mma16816(accz, z[0], z[1], z[2], z[3], x0, x1);
+                    if (h2) {
+                        group_rows(g_rd + st + h2 * 16 * (W * 2), z);
+                        mma16816(accs, z[0], z[1], z[2], z[3], x0, x1);
+                    }
+                }
+                uint32_t w[4][4];                              // tokens 2 tig, 2 tig + 1, + 8, + 9 of the k-step, words 4 r ..
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(w[i][0]), "=r"(w[i][1]), "=r"(w[i][2]), "=r"(w[i][3])
+                                 : "r"(w_rd + st + (16 * h2 + (i & 1) + 8 * (i >> 1)) * (W * 4) + 16 * r));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t b_lo = lds32(op_rd + u * 512 + 256 * h2) ^ sign, b_hi = lds32(op_rd + u * 512 + 256 * h2 + 128) ^ sign;
+                    mma16816(acc[4 * r + u], (prmt(w[0][u], w[1][u], sel0) ^ flip) & msk0, (prmt(w[0][u], w[1][u], sel1) ^ flip) & msk1,
+                             (prmt(w[2][u], w[3][u], sel0) ^ flip) & msk0, (prmt(w[2][u], w[3][u], sel1) ^ flip) & msk1, b_lo, b_hi);
+                }
+            }
+            __syncwarp();                                      // the operand tiles (and at the end the slot) may be overwritten
+        }
+        st = kV3Stage - st;
+        pa += kMmaWarps * 32;
+        pb += kMmaWarps * 32;
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    // lane (g, tig): channels of rows g, g + 8 for head tig; the group's zero term and complement sum sit in the lanes of row j
+    const float sc0 = __int_as_float((151 - 2 - p0) << 23), sc1 = __int_as_float((151 - 2 - p1) << 23);   // 2^(24 - position) / 4
+    const float z0 = accz[0] + accz[1], z1 = accz[2] + accz[3], s0 = accs[0] + accs[1], s1 = accs[2] + accs[3];
+    const float max1 = g == 2 ? 3.f : 7.f;                     // the 11th field has two bits
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        const int from = 4 * (j & 7) + tig;
+        const float z = 0.25f * __shfl_sync(0xffffffffu, j < 8 ? z0 : z1, from), sv = 0.25f * __shfl_sync(0xffffffffu, j < 8 ? s0 : s1, from);
+        if (11 * j + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + g] = fmaf(acc[j][0] + acc[j][1], sc0, fmaf(7.f, sv, z));
+        if (g < 3 && 11 * j + 8 + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + 8 + g] = fmaf(acc[j][2] + acc[j][3], sc1, fmaf(max1, sv, z));
     }
 }
 
@@ -586,7 +725,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
-    gqa_pv_packed<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
+    if constexpr (VB == 3) gqa_pv_packed3<1>(a, vc, vs, vz, sm, t0, v_hi);
+    else gqa_pv_packed<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
     // ---- 2. softmax numerators: two warps per head slot --------------------------------------------
@@ -622,7 +762,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     __syncthreads();
 
     // ---- 3. p . V -----------------------------------------------------------------------------------
-    gqa_pv_packed<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    if constexpr (VB == 3) gqa_pv_packed3<2>(a, vc, vs, vz, sm, t0, v_hi);
+    else gqa_pv_packed<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
     __syncwarp();
     if (v_lo < t1) pv_tail<kQH>(a, vf, b, hk, sm.scores, n_scores, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();
@@ -686,15 +827,24 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         M = warp_max(M);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         float L = 0.f;
-#pragma unroll 16
-        for (int i = 0; i < cnt; ++i) {
-            const float *pi = bh + (int64_t)i * stride;
-            const float2 ml = __ldcg(reinterpret_cast<const float2 *>(pi + kHeadDim));
-            const float4 p = __ldcg(reinterpret_cast<const float4 *>(pi) + lane);
-            const float w = __expf(ml.x - M);
-            L = fmaf(ml.y, w, L);
-            acc.x = fmaf(p.x, w, acc.x); acc.y = fmaf(p.y, w, acc.y);
-            acc.z = fmaf(p.z, w, acc.z); acc.w = fmaf(p.w, w, acc.w);
+        constexpr int U = 16;                                  // loads in flight; behind the last segment it is read again, as zeros
+        for (int i0 = 0; i0 < cnt; i0 += U) {
+            float2 ml[U];
+            float4 p[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float *pi = bh + (int64_t)min(i0 + u, cnt - 1) * stride;
+                ml[u] = __ldcg(reinterpret_cast<const float2 *>(pi + kHeadDim));
+                p[u] = __ldcg(reinterpret_cast<const float4 *>(pi) + lane);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = i0 + u < cnt;
+                const float w = __expf(ml[u].x - M);
+                L = fmaf(in ? ml[u].y : 0.f, w, L);
+                acc.x = fmaf(in ? p[u].x : 0.f, w, acc.x); acc.y = fmaf(in ? p[u].y : 0.f, w, acc.y);
+                acc.z = fmaf(in ? p[u].z : 0.f, w, acc.z); acc.w = fmaf(in ? p[u].w : 0.f, w, acc.w);
+            }
         }
         const float inv = 1.f / L;
         __half2 *dst = reinterpret_cast<__half2 *>(stage + warp * kHeadDim + 4 * lane);
@@ -740,7 +890,7 @@ int gqa_heads_per_cta(const kvq_attn_args &a) {
     const int n_rep = a.nh / a.nh_kv;
     if (n_rep != 2 && n_rep % 4 != 0) return 0;
     const int kmin = a.k_bits == 1 ? 128 : a.k_bits == 2 ? 64 : a.k_bits == 4 ? 64 : 11;
-    const int vmin = a.v_bits == 1 ? 64 : a.v_bits == 2 ? 64 : 32;     // 1-bit values at group 64: two MMAs per code tile
+    const int vmin = a.v_bits == 1 ? 64 : a.v_bits == 2 ? 64 : a.v_bits == 3 ? 11 : 32;     // 1-bit values at group 64: two MMAs per code tile
     if (a.k_bits != 3 && a.k_group < kmin) return 0;
     if (a.v_group < vmin) return 0;
     return n_rep == 2 ? 2 : 4;
@@ -762,13 +912,13 @@ static int launch_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, flo
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
         e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
+        if (VB != 3 && e == cudaSuccess)
+            e = cudaFuncSetAttribute(decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const unsigned grid = (unsigned)(plan.n_whole + plan.n_cut * plan.k);
-    if (a.state) decode_attn_gqa_kernel<KB, VB, true><<<grid, kMmaThreads, smem, st>>>(a, plan, qhv, parts, counters);
+    if (VB != 3 && a.state) decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true><<<grid, kMmaThreads, smem, st>>>(a, plan, qhv, parts, counters);
     else decode_attn_gqa_kernel<KB, VB, false><<<grid, kMmaThreads, smem, st>>>(a, plan, qhv, parts, counters);
     return check_launch();
 }
@@ -781,6 +931,7 @@ int launch_decode_attn_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv
     KVQ_GQA_CASE(3, 4) KVQ_GQA_CASE(3, 2) KVQ_GQA_CASE(3, 1)
     KVQ_GQA_CASE(2, 4) KVQ_GQA_CASE(2, 2) KVQ_GQA_CASE(2, 1)
     KVQ_GQA_CASE(1, 4) KVQ_GQA_CASE(1, 2) KVQ_GQA_CASE(1, 1)
+    KVQ_GQA_CASE(4, 3) KVQ_GQA_CASE(3, 3) KVQ_GQA_CASE(2, 3) KVQ_GQA_CASE(1, 3)
 #undef KVQ_GQA_CASE
     return KVQ_ERR_UNSUPPORTED;
 }

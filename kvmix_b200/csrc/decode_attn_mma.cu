@@ -699,12 +699,23 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     M = warp_max(M);
     float L = 0.f, acc = 0.f;
     const int ch = tid & (kHeadDim - 1);
-#pragma unroll 8
-    for (int i = 0; i < cnt; ++i) {
-        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(base + i * kPart + kHeadDim));
-        const float w = __expf(ml.x - M);
-        L = fmaf(ml.y, w, L);
-        acc = fmaf(__ldcg(base + i * kPart + ch), w, acc);
+    constexpr int U = 8;                                     // loads in flight; behind the last segment it is read again, as zeros
+    for (int i0 = 0; i0 < cnt; i0 += U) {
+        float2 ml[U];
+        float p[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float *pi = base + min(i0 + u, cnt - 1) * kPart;
+            ml[u] = __ldcg(reinterpret_cast<const float2 *>(pi + kHeadDim));
+            p[u] = __ldcg(pi + ch);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = i0 + u < cnt;
+            const float w = __expf(ml[u].x - M);
+            L = fmaf(in ? ml[u].y : 0.f, w, L);
+            acc = fmaf(in ? p[u] : 0.f, w, acc);
+        }
     }
     const __half r[1] = {__float2half_rn(acc / L)};
     if (own) out[tid] = r[0];
@@ -736,6 +747,8 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_mma_kernel(const _
 // ---------------------------------------------------------------------------------------------
 // The tensor-core path needs a whole number of query heads per kv head, supported group sizes, 16-byte aligned
 // and row-contiguous packed tensors (cp.async granules), and a packed-value length that is a multiple of 32.
+int gqa_heads_per_cta(const kvq_attn_args &a);               // decode_attn_gqa.cu
+
 bool mma_path_eligible(const kvq_attn_args &a) {
     if (a.nh_kv <= 0 || a.nh % a.nh_kv != 0 || a.D != kHeadDim) return false;
     if (a.k_bits == 3) {
@@ -743,8 +756,11 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     } else if (a.k_group != 32 && a.k_group != 64 && a.k_group != 128) {
         return false;
     }
-    if (a.v_bits == 3) return false;
-    if (a.v_group != 32 && a.v_group != 64 && a.v_group != 128) return false;
+    if (a.v_bits == 3) {                                       // only the grouped kernel has 3-bit values
+        if (a.v_group != 11 || gqa_heads_per_cta(a) == 0) return false;
+    } else if (a.v_group != 32 && a.v_group != 64 && a.v_group != 128) {
+        return false;
+    }
     if (a.Tvq % 32 != 0) return false;
     auto al16 = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     if (a.T > a.Tkq && (!al16(a.kfull) || a.kf_sB % 8 || a.kf_sH % 8 || a.kf_sT % 8)) return false;
@@ -756,9 +772,9 @@ bool mma_path_eligible(const kvq_attn_args &a) {
         if (a.kc_sD < 0 || a.kc_sD >= (1 << 22) || a.ks_sD < 0 || a.ks_sD >= (1 << 23)) return false;
     }
     if (a.Tvq > 0) {
-        const int fv = fields_per_word(a.v_bits);
-        if (!al16(a.vcode) || a.vc_sB % 4 || a.vc_sH % 4 || a.vc_sT != kHeadDim / fv) return false;
-        if (!al16(a.vscale) || !al16(a.vmn) || a.vs_sB % 8 || a.vs_sH % 8 || a.vs_sT != kHeadDim / a.v_group) return false;
+        const int fv = fields_per_word(a.v_bits);              // rows back to back (3 bits: 12 words and groups a token)
+        if (!al16(a.vcode) || a.vc_sB % 4 || a.vc_sH % 4 || a.vc_sT != (kHeadDim + fv - 1) / fv) return false;
+        if (!al16(a.vscale) || !al16(a.vmn) || a.vs_sB % 8 || a.vs_sH % 8 || a.vs_sT != (kHeadDim + a.v_group - 1) / a.v_group) return false;
     }
     return true;
 }

@@ -14,7 +14,7 @@ TOKENS = (257, 385, 600, 861, 1023, 2100)
 
 
 @pytest.mark.parametrize("kb,vb,G,nh,hkv", [(4, 2, 32, 2, 2), (2, 4, 64, 2, 2), (3, 1, 32, 2, 2), (1, 2, 128, 2, 2),
-                                            (4, 4, 64, 8, 2), (3, 2, 64, 8, 2), (2, 1, 64, 4, 2), (1, 1, 128, 4, 1)])
+                                            (4, 4, 64, 8, 2), (3, 2, 64, 8, 2), (2, 1, 64, 4, 2), (1, 1, 128, 4, 1), (3, 3, 64, 8, 2), (4, 3, 32, 4, 2), (1, 3, 128, 4, 1)])
 def test_short_and_ragged_contexts(cuda, kb, vb, G, nh, hkv):
     import kvmix_b200 as kv
     for T in TOKENS:
