@@ -8,7 +8,7 @@
 //            3-bit: the 11th element of each group clamps to 3; 0/0 (constant group) -> 0
 //   stored scale = scale32 narrowed to the input dtype, stored mn = mn
 //
-// Three kernels, one result:
+// Four kernels, one result:
 //   quant_contig_kernel   groups run along the contiguous axis (values: [.., T, D], groups over D;
 //                         or keys already transposed to [.., D, T]).  A thread owns one or two output
 //                         words; the threads of a group combine min/max with shuffles.
@@ -17,6 +17,7 @@
 //                         channels, keeps a whole group in registers (all loads in flight at
 //                         once), and the CTA transposes words through shared memory so global
 //                         writes are contiguous runs per channel.
+//   quant_rope_kernel     the same for keys that still have to be rotated (prefill).
 //   quant_generic_kernel  any strides / any group-to-word relation; one thread per word.
 #include "quant_core.cuh"
 
@@ -132,19 +133,10 @@ struct StridedCfg {
     static constexpr int WPAD = WPC + 1;
 };
 
-// Rotary embedding applied while loading (prefill of keys straight from the k_proj output): element (b, s, c) of the
-// cos / sin tables at b * r_sB + s * r_sS + c, fp16.  HF's rotate_half form (the one upstream's model files import):
-// out[c] = k[c] * cos[c] + rot[c] * sin[c] with rot = (-k[c + 64], k[c - 64]) for c < 64 / c >= 64, every product and
-// the sum rounded to fp16 as the framework's fp16 tensor arithmetic rounds them.
-struct RopeTables {
-    const __half *cos, *sin;
-    int64_t r_sB, r_sS;
-};
-
-template <int BITS, int G, bool ROPE>
+template <int BITS, int G>
 __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__restrict__ x, int32_t *__restrict__ code,
                                                             __half *__restrict__ scale, __half *__restrict__ mn,
-                                                            QuantDims d, RopeTables rope) {
+                                                            QuantDims d) {
     using C = StridedCfg<BITS, G>;
     __shared__ int32_t s_code[128 * C::WPAD];
     __shared__ __half s_scale[128 * (C::GPC + 2)];
@@ -158,22 +150,8 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
     const int groups_here = (int)min((int64_t)C::GPC, n_groups - g0);
     const __half *px = x + b * d.x_sB + h * d.x_sH + (a0 + 2 * pair);
     constexpr int QMAX = (1 << BITS) - 1;
-    // element pair (2 pair, 2 pair + 1) of token s of this (b, h) slab, rotated on the way in when ROPE
-    const int partner = (2 * pair < 64) ? 64 : -64;
-    const __half *pcos = ROPE ? rope.cos + b * rope.r_sB + 2 * pair : nullptr;
-    const __half *psin = ROPE ? rope.sin + b * rope.r_sB + 2 * pair : nullptr;
-    auto load = [&](int64_t s) -> __half2 {
-        const __half2 k = __ldg(reinterpret_cast<const __half2 *>(px + s * d.x_sS));
-        if constexpr (ROPE) {
-            __half2 r = __ldg(reinterpret_cast<const __half2 *>(px + s * d.x_sS + partner));
-            if (partner > 0) r = __hneg2(r);
-            const __half2 cs = __ldg(reinterpret_cast<const __half2 *>(pcos + s * rope.r_sS));
-            const __half2 sn = __ldg(reinterpret_cast<const __half2 *>(psin + s * rope.r_sS));
-            return __hadd2_rn(__hmul2_rn(k, cs), __hmul2_rn(r, sn));
-        } else {
-            return k;
-        }
-    };
+    // element pair (2 pair, 2 pair + 1) of token s of this (b, h) slab
+    auto load = [&](int64_t s) -> __half2 { return __ldg(reinterpret_cast<const __half2 *>(px + s * d.x_sS)); };
 
     // tokens held in registers at a time: a whole group up to 32 tokens; longer groups are walked twice anyway (min/max,
     // then codes from L1/L2), and for them 16 at a time measured 5-10 % faster for 2- and 4-bit codes (fewer live
@@ -238,6 +216,147 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
         }
         for (int i = threadIdx.x; i < 128 * groups_here; i += 256) {
             const int ch = i / groups_here, g = i % groups_here;
+            scale[zo + ch * d.z_sA + g] = s_scale[ch * (C::GPC + 2) + g];
+            mn[zo + ch * d.z_sA + g] = s_mn[ch * (C::GPC + 2) + g];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Rotary embedding applied while loading (prefill of keys straight from the k_proj output): element (b, s, c) of the
+// cos / sin tables at b * r_sB + s * r_sS + c, fp16.  HF's rotate_half form (the one upstream's model files import):
+// out[c] = k[c] * cos[c] + rot[c] * sin[c] with rot = (-k[c + 64], k[c - 64]) for c < 64 / c >= 64, every product and
+// the sum rounded to fp16 as the framework's fp16 tensor arithmetic rounds them.
+struct RopeTables {
+    const __half *cos, *sin;
+    int64_t r_sB, r_sS;
+};
+
+
+// Keys straight from the projection.  A CTA rotates 128 tokens (132 for groups of 11) x 128 channels into shared memory -- a
+// lane takes four channels of a row, the rotation partner (64 channels away) is a shuffle, so rows and table rows are
+// read once -- and then works parts of 32 (11) tokens of a channel pair from there; groups of 64 and 128 tokens meet over
+// shared memory.  Loops stay rolled: with a warp's 32 tokens in registers and every word unrolled, tie path included, the same
+// work took 46 .. 71 us, waiting for instructions; read from global memory twice and rotated twice (a thread per
+// pair and group, four loads an element pair) 38 us.  2 x 8 kv heads x 8191 tokens, group 64, 4 bits: 22 us.
+template <int BITS, int G>
+struct RopeCfg {
+    static constexpr int FPI = fields_per_word(BITS);
+    static constexpr int PT = G == 11 ? 11 : 32;              // tokens of a part
+    static constexpr int NP = G == 11 ? 12 : 4;               // parts of a tile
+    static constexpr int TOK = NP * PT;                       // tokens of a tile: 132 / 128
+    static constexpr int PPG = G > 32 ? G / 32 : 1;           // parts of a group
+    static constexpr int GPC = NP / PPG;                      // groups of a tile
+    static constexpr int WPP = PT / FPI;                      // words of a part: 4 / 2 / 1 / 1
+    static constexpr int WPC = NP * WPP, WPAD = WPC + 1;
+};
+
+template <int BITS, int G>
+__global__ void __launch_bounds__(256, 4) quant_rope_kernel(const __half *__restrict__ x, int32_t *__restrict__ code,
+                                                         __half *__restrict__ scale, __half *__restrict__ mn, QuantDims d, RopeTables rope) {
+    using C = RopeCfg<BITS, G>;
+    constexpr int QMAX = (1 << BITS) - 1;
+    __shared__ __align__(16) __half2 s_tile[C::TOK * 64];
+    __shared__ int32_t s_code[128 * C::WPAD];
+    __shared__ __half s_scale[128 * (C::GPC + 2)], s_mn[128 * (C::GPC + 2)];
+    __shared__ __half2 s_lo[C::PPG > 1 ? C::NP * 64 : 1], s_hi[C::PPG > 1 ? C::NP * 64 : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t bh = blockIdx.z, b = bh / d.H, h = bh % d.H;
+    const int64_t g0 = (int64_t)blockIdx.x * C::GPC, n_groups = d.S / G;
+    const int groups_here = (int)min((int64_t)C::GPC, n_groups - g0), tokens = groups_here * G;
+    {
+        const __half *px = x + b * d.x_sB + h * d.x_sH + g0 * G * d.x_sS + 4 * lane;
+        const __half *pc = rope.cos + b * rope.r_sB + g0 * G * rope.r_sS + 4 * lane;
+        const __half *ps = rope.sin + b * rope.r_sB + g0 * G * rope.r_sS + 4 * lane;
+        const uint32_t turn = lane < 16 ? 0x80008000u : 0u;   // rot = (-k[c + 64], k[c - 64])
+        auto h2 = [](const uint32_t &u) { return *reinterpret_cast<const __half2 *>(&u); };
+        constexpr int NB = 4;                                 // rows in flight per warp (x 3 loads)
+#pragma unroll 1
+        for (int t0 = warp; t0 < tokens; t0 += 8 * NB) {
+            uint2 k[NB], cs[NB], sn[NB];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const int64_t t = min(t0 + 8 * i, tokens - 1);
+                k[i] = __ldg(reinterpret_cast<const uint2 *>(px + t * d.x_sS));
+                cs[i] = __ldg(reinterpret_cast<const uint2 *>(pc + t * rope.r_sS));
+                sn[i] = __ldg(reinterpret_cast<const uint2 *>(ps + t * rope.r_sS));
+            }
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                const uint32_t r0 = __shfl_xor_sync(0xffffffffu, k[i].x, 16) ^ turn, r1 = __shfl_xor_sync(0xffffffffu, k[i].y, 16) ^ turn;
+                const __half2 o0 = __hadd2_rn(__hmul2_rn(h2(k[i].x), h2(cs[i].x)), __hmul2_rn(h2(r0), h2(sn[i].x)));
+                const __half2 o1 = __hadd2_rn(__hmul2_rn(h2(k[i].y), h2(cs[i].y)), __hmul2_rn(h2(r1), h2(sn[i].y)));
+                if (t0 + 8 * i < tokens) {
+                    uint2 o;
+                    o.x = *reinterpret_cast<const uint32_t *>(&o0);
+                    o.y = *reinterpret_cast<const uint32_t *>(&o1);
+                    *reinterpret_cast<uint2 *>(&s_tile[(t0 + 8 * i) * 64 + 2 * lane]) = o;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const int pair = threadIdx.x & 63, parts = groups_here * C::PPG;
+    // min / max of a part in fp16x2 (exact: the data are fp16; NaN operands are skipped as by fminf)
+    auto range = [&](int part, __half2 &lo2, __half2 &hi2) {
+        const __half2 *t = s_tile + part * C::PT * 64 + pair;
+        lo2 = hi2 = t[0];
+#pragma unroll
+        for (int i = 1; i < C::PT; ++i) { const __half2 v = t[i * 64]; lo2 = __hmin2(lo2, v); hi2 = __hmax2(hi2, v); }
+    };
+    if constexpr (C::PPG > 1) {                               // four parts: one per thread
+        const int part = threadIdx.x >> 6;
+        if (part < parts) {
+            __half2 lo2, hi2;
+            range(part, lo2, hi2);
+            s_lo[part * 64 + pair] = lo2;
+            s_hi[part * 64 + pair] = hi2;
+        }
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int part = threadIdx.x >> 6; part < parts; part += 4) {
+        __half2 lo2, hi2;
+        if constexpr (C::PPG > 1) {
+            const int p0 = part / C::PPG * C::PPG;
+            lo2 = s_lo[p0 * 64 + pair];
+            hi2 = s_hi[p0 * 64 + pair];
+#pragma unroll
+            for (int p = 1; p < C::PPG; ++p) { lo2 = __hmin2(lo2, s_lo[(p0 + p) * 64 + pair]); hi2 = __hmax2(hi2, s_hi[(p0 + p) * 64 + pair]); }
+        } else {
+            range(part, lo2, hi2);
+        }
+        const float lo0 = __low2float(lo2), lo1 = __high2float(lo2), hi0 = __low2float(hi2), hi1 = __high2float(hi2);
+        const float sc0 = (hi0 - lo0) / (float)QMAX, sc1 = (hi1 - lo1) / (float)QMAX;
+        const float ri0 = __frcp_rn(sc0), ri1 = __frcp_rn(sc1);     // correctly rounded reciprocals
+#pragma unroll 1
+        for (int w = 0; w < C::WPP; ++w) {
+            const __half2 *t = s_tile + (part * C::PT + w * C::FPI) * 64 + pair;
+            __half2 raw[C::FPI];
+#pragma unroll
+            for (int i = 0; i < C::FPI; ++i) raw[i] = t[i * 64];
+            s_code[(2 * pair) * C::WPAD + part * C::WPP + w] = (int32_t)quant_word<BITS>([&](int i) { return __low2float(raw[i]); }, lo0, sc0, ri0);
+            s_code[(2 * pair + 1) * C::WPAD + part * C::WPP + w] = (int32_t)quant_word<BITS>([&](int i) { return __high2float(raw[i]); }, lo1, sc1, ri1);
+        }
+        if (part % C::PPG == 0) {
+            const int g = part / C::PPG, o = (2 * pair) * (C::GPC + 2) + g;
+            s_scale[o] = __float2half_rn(stored_scale<QMAX>(hi0 - lo0, sc0, d.by_div));
+            s_scale[o + C::GPC + 2] = __float2half_rn(stored_scale<QMAX>(hi1 - lo1, sc1, d.by_div));
+            s_mn[o] = __float2half_rn(lo0);
+            s_mn[o + C::GPC + 2] = __float2half_rn(lo1);
+        }
+    }
+    __syncthreads();
+    const int words_here = groups_here * (G / C::FPI);
+    int32_t *dc = code + b * d.c_sB + h * d.c_sH + g0 * (G / C::FPI);
+    const int64_t zo = b * d.z_sB + h * d.z_sH + g0;
+    for (int i = threadIdx.x; i < 128 * C::WPC; i += 256) {
+        const int ch = i / C::WPC, w = i % C::WPC;
+        if (w < words_here) dc[ch * d.c_sA + w] = s_code[ch * C::WPAD + w];
+    }
+    for (int i = threadIdx.x; i < 128 * C::GPC; i += 256) {
+        const int ch = i / C::GPC, g = i % C::GPC;
+        if (g < groups_here) {
             scale[zo + ch * d.z_sA + g] = s_scale[ch * (C::GPC + 2) + g];
             mn[zo + ch * d.z_sA + g] = s_mn[ch * (C::GPC + 2) + g];
         }
@@ -373,8 +492,12 @@ static int launch_bits(const kvq_quant_args *a, const QuantDims &d, cudaStream_t
     {                                                                                              \
         using C = StridedCfg<BITS, GG>;                                                            \
         dim3 grid((unsigned)((ng + C::GPC - 1) / C::GPC), (unsigned)(d.A / 128), (unsigned)(d.B * d.H)); \
-        if (rope) quant_strided_kernel<BITS, GG, true><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d, *rope);      \
-        else quant_strided_kernel<BITS, GG, false><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d, RopeTables{});   \
+        if (rope) {                                                                                \
+            grid.x = (unsigned)((ng + RopeCfg<BITS, GG>::GPC - 1) / RopeCfg<BITS, GG>::GPC);       \
+            quant_rope_kernel<BITS, GG><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d, *rope);      \
+        } else {                                                                                   \
+            quant_strided_kernel<BITS, GG><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d);          \
+        }                                                                                          \
         return check_launch();                                                                     \
     }
             if constexpr (BITS == 3) {
