@@ -71,10 +71,10 @@ __device__ __forceinline__ void fused_quant_v_group(const kvq_attn_args &a, int 
     static_cast<__half *>(const_cast<void *>(a.vmn))[zo] = __float2half_rn(lo);
 }
 
-// The update work of one segment [t0, t1) of kv head (b, hk), before its attention phases; every thread of the CTA (2 x 128:
-// the first half quantizes keys, the second values)
+// The update work of one segment [t0, t1) of kv head (b, hk), before its attention phases; every thread of the CTA (NT: 256,
+// the first half quantizes keys and the second values; or 128, one after the other)
 // calls it (it ends with a CTA barrier when it wrote packed data the CTA is about to read).
-template <int KB, int VB>
+template <int KB, int VB, int NT>
 __device__ __forceinline__ void fused_cache_update(const kvq_attn_args &a, int b, int hk, int t0, int t1, int tid) {
     if (!a.k_new) return;
     bool wrote = false;
@@ -83,7 +83,7 @@ __device__ __forceinline__ void fused_cache_update(const kvq_attn_args &a, int b
         wrote = true;
     }
     if (a.v_quant > 0 && t0 <= a.Tvq - a.v_quant && a.Tvq - a.v_quant < t1) {
-        if constexpr (VB != 3) if (tid >= kHeadDim) fused_quant_v_group<VB>(a, b, hk, tid - kHeadDim);
+        if constexpr (VB != 3) if (tid >= NT - kHeadDim) fused_quant_v_group<VB>(a, b, hk, tid - (NT - kHeadDim));
         wrote = true;
     }
     if (t1 == a.T && tid < 32) {                               // the rings receive the new token for the following steps

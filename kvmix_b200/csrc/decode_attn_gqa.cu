@@ -707,7 +707,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
     const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
     prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, kMmaThreads);
-    fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
+    fused_cache_update<KB, VB, kMmaThreads>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     // q of the quad (head slots beyond qhv repeat the last head: their columns are computed and dropped)
     {
         const int slot = tid >> 6, hs = min(slot, qhv - 1);              // two warps store a head slot

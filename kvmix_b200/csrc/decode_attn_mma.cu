@@ -38,9 +38,12 @@ struct MmaSmem {
     float *misc;            // [32]
     int n_scores, ks_log2;
 };
-template <int KB> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, KB == 2 ? 3 : 4>;        // scale rows, then zero rows, 16 B each
-template <int KB, int VB> constexpr int warp_region_bytes() {
-    return MmaKRing<KB>::BYTES > VGeom<VB>::WARP_BYTES ? MmaKRing<KB>::BYTES : VGeom<VB>::WARP_BYTES;
+// Rings of a CTA of NW warps: the scale rows, then the zero rows of a stage, 16 B each, follow its codes.  Four warps: sized so
+// that four CTAs fit an SM next to 5000 scores each.
+template <int KB, int NW> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, (KB == 2 ? 3 : 4) - (NW == 4)>;
+template <int VB, int NW> using MmaVGeom = VGeom<VB, (VB == 4 ? 4 : VB == 2 ? 6 : 8) - (NW == 4 && VB != 1)>;
+template <int KB, int VB, int NW> constexpr int warp_region_bytes() {
+    return MmaKRing<KB, NW>::BYTES > MmaVGeom<VB, NW>::WARP_BYTES ? MmaKRing<KB, NW>::BYTES : MmaVGeom<VB, NW>::WARP_BYTES;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -48,23 +51,24 @@ template <int KB, int VB> constexpr int warp_region_bytes() {
 // Raw fp32 scores go to sm.scores[split][t - t0].  Warps work independently: with `ns` = 1 << ks_log2 channel splits, warp w
 // takes channels [128 / ns * (w % ns), ..) of the warp tiles w / ns, w / ns + 8 / ns, ... and streams their code words
 // through its own ring.
+template <int NW>
 __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half *kf, int b, int hk, const MmaSmem &sm,
                                             int t0, int lo, int t1);
 
 // If the split also holds fp16 tail keys (tail_lo < t1) they are scored right after the first code stages
 // have been issued, so the tail's global-load latency overlaps the ring fill.
-template <int KB>
+template <int KB, int NW>
 __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const MmaSmem &sm, int t0, int hi,
                                               const __half *kf, int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
-    using R = MmaKRing<KB>;
+    using R = MmaKRing<KB, NW>;
     using F = Fields<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int Gk = a.k_group;
     const int n_words = a.Tkq / G::FPI;                       // valid code words per channel row
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;
-    const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = kMmaWarps >> sm.ks_log2;
+    const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = NW >> sm.ks_log2;
     const int my_tiles = (n_tiles - wt + tile_lanes - 1) / tile_lanes;   // <= 0: none
     const int ch0 = split * (kHeadDim >> sm.ks_log2), steps = (kHeadDim / 32) >> sm.ks_log2;   // channels of this warp
     const int tile_stages = G::NSTAGE >> sm.ks_log2;
@@ -144,7 +148,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     // The caller stored q to shared memory just before this call without a barrier, so that the first code stages
     // are in flight while q arrives; every warp passes exactly one barrier here before anything reads q.
     __syncthreads();
-    if (tail_lo < t1) qk_tail_mma(a, kf, b, hk, sm, t0, tail_lo, t1);
+    if (tail_lo < t1) qk_tail_mma<NW>(a, kf, b, hk, sm, t0, tail_lo, t1);
 
     for (int j = 0; j < my_tiles; ++j) {
         const int tile0 = t0 + (j * tile_lanes + wt) * G::WT;
@@ -353,10 +357,10 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 // ring region (float [128] at the region base).
 // MODE 1 only issues the first stages (called before the softmax, whose latency then hides the ring fill);
 // MODE 2 continues after such a call; MODE 0 does both.
-template <int VB, int MODE>
+template <int VB, int MODE, int NW>
 __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int32_t *vc, const __half *vs,
                                               const __half *vz, const MmaSmem &sm, int t0, int hi) {
-    using G = VGeom<VB>;
+    using G = MmaVGeom<VB, NW>;
     using F = VHalf<VB>;
     constexpr int NB = G::GPT;                                // 16-byte blocks per token row: 1 / 2 / 4
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
@@ -365,7 +369,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     const int Gv = a.v_group;
     const int ngv = kHeadDim / Gv;                            // channel groups: 4 / 2 / 1
     const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;      // <= 0: no packed values in this segment
-    const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
+    const int my_blocks = (n_blocks - warp + NW - 1) / NW;
     float *my_red = reinterpret_cast<float *>(sm.ring);
     if (my_blocks <= 0) {
         if (MODE != 1)
@@ -401,7 +405,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     const uint32_t o10 = ring_s + G::SZ_OFF + (bt1 * ngv + g0) * 2, o11 = ring_s + G::SZ_OFF + (bt1 * ngv + g1) * 2;
     const uint32_t pb_wr = pb_s + (pi * 8 + 4 * ch) * 4;
 
-    const int block_stride = kMmaWarps * G::TPS;
+    const int block_stride = NW * G::TPS;
     const char *vc_b = reinterpret_cast<const char *>(vc);                               // 32-bit byte offsets from the head's first row
     uint32_t src_codes = (uint32_t)(t0 + warp * G::TPS) * G::RBV + lane * 16;
     const int ngran = 4 * ngv;                                                           // 16-byte granules per array per stage
@@ -549,6 +553,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
 // q . K^T over the fp16 tail for tokens [lo, t1): 16-token tiles on the tensor core, straight from
 // global memory (row g and g+8 of a tile per lane-octet, 16-byte loads of 8 channels; the k axis is
 // permuted identically in the q fragments).  Every B column carries q, so each lane sees its rows' sums.
+template <int NW>
 __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half *kf, int b, int hk, const MmaSmem &sm,
                                             int t0, int lo, int t1) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
@@ -556,7 +561,7 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 #pragma unroll
     for (int S = 0; S < 4; ++S) qf[S] = *reinterpret_cast<const uint4 *>(sm.q + 32 * S + 8 * tig);
     const int n_tiles = (t1 - lo + 15) / 16;
-    for (int tile = warp; tile < n_tiles; tile += kMmaWarps) {
+    for (int tile = warp; tile < n_tiles; tile += NW) {
         const int ta = lo + 16 * tile + g, tb = ta + 8;
         const __half *pa = k_tail_row(a, kf, b, hk, min(ta, t1 - 1)) + 8 * tig;
         const __half *pb = k_tail_row(a, kf, b, hk, min(tb, t1 - 1)) + 8 * tig;
@@ -584,7 +589,7 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of query head (b, h); segment `seg` of the `cnt` the head is cut into.
-template <int KB, int VB>
+template <int KB, int VB, int NW>
 __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int ks_log2, int s, int t0, int t1, int seg,
                                              int cnt, int n_whole, float *__restrict__ parts,
                                              unsigned int *__restrict__ counters) {
@@ -595,8 +600,8 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     sm.ks_log2 = ks_log2;
     sm.scores = reinterpret_cast<float *>(smem_raw);
     unsigned char *after_scores = smem_raw + ((size_t)n_scores << ks_log2) * 4;
-    sm.ring = after_scores + warp * warp_region_bytes<KB, VB>();
-    sm.q = reinterpret_cast<__half *>(after_scores + kMmaWarps * warp_region_bytes<KB, VB>());
+    sm.ring = after_scores + warp * warp_region_bytes<KB, VB, NW>();
+    sm.q = reinterpret_cast<__half *>(after_scores + NW * warp_region_bytes<KB, VB, NW>());
     sm.misc = reinterpret_cast<float *>(sm.q + kHeadDim);
     const int b = s / a.nh, h = s % a.nh;
     // grouped queries: each query head is its own segment and reads kv head hk; the heads of one kv head are
@@ -606,8 +611,8 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
     const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
     const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
-    prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, kMmaThreads);
-    fused_cache_update<KB, VB>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
+    prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, (32 * NW));
+    fused_cache_update<KB, VB, 32 * NW>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)h * a.q_sH;
     if (tid < kHeadDim) sm.q[tid] = q[tid];
 
@@ -616,12 +621,12 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        qk_packed_mma<KB>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        qk_packed_mma<KB, NW>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
-    pv_packed_mma<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
+    pv_packed_mma<VB, 1, NW>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
     // ---- 2. softmax numerators ------------------------------------------------------------------
@@ -630,7 +635,7 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     float m = kMaskFloor;                                      // a fully masked range then weighs uniformly, as upstream's does
     float4 *sc4 = reinterpret_cast<float4 *>(sm.scores);
 #pragma unroll 2
-    for (int i = tid; i < n4; i += kMmaThreads) {
+    for (int i = tid; i < n4; i += (32 * NW)) {
         float4 v = score_quad(a, sc4 + i, n_scores >> 2, ks_log2);
         if (a.mask) mask_quad(a, b, h, t0 + 4 * i, v);
         if (4 * i + 3 >= n) pad_quad(v, n - 4 * i);
@@ -640,11 +645,11 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     m = warp_max(m);
     if (lane == 0) sm.misc[warp] = m;
     __syncthreads();
-    m = sm.misc[lane & (kMmaWarps - 1)];
+    m = sm.misc[lane & (NW - 1)];
     m = warp_max(m);
     float l = 0.f;
 #pragma unroll 2
-    for (int i = tid; i < n4; i += kMmaThreads) {
+    for (int i = tid; i < n4; i += (32 * NW)) {
         float4 v = sc4[i];
         v.x = __expf(v.x - m);
         v.y = __expf(v.y - m);
@@ -658,20 +663,20 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     __syncthreads();
 
     // ---- 3. p.V -----------------------------------------------------------------------------------
-    pv_packed_mma<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    pv_packed_mma<VB, 2, NW>(a, vc, vs, vz, sm, t0, v_hi);
     __syncwarp();
-    if (v_lo < t1) pv_tail<1>(a, vf, b, hk, sm.scores, 0, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
+    if (v_lo < t1) pv_tail<1>(a, vf, b, hk, sm.scores, 0, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, NW, lane);
     __syncthreads();
 
     // ---- 4. finish / merge --------------------------------------------------------------------------
-    const bool own = tid < kHeadDim;                           // thread tid owns channel tid
+    const bool own = NW == 4 || tid < kHeadDim;                         // thread tid owns channel tid
     float o = 0.f, l_all = 0.f;
     if (own) {
 #pragma unroll
-        for (int w = 0; w < kMmaWarps; ++w) o += reinterpret_cast<const float *>(after_scores + w * warp_region_bytes<KB, VB>())[tid];
+        for (int w = 0; w < NW; ++w) o += reinterpret_cast<const float *>(after_scores + w * warp_region_bytes<KB, VB, NW>())[tid];
     }
 #pragma unroll
-    for (int w = 0; w < kMmaWarps; ++w) l_all += sm.misc[8 + w];
+    for (int w = 0; w < NW; ++w) l_all += sm.misc[8 + w];
     __half *out = static_cast<__half *>(a.out) + (int64_t)b * a.o_sB + (int64_t)h * a.o_sH;
     if (cnt == 1) {
         const __half r[1] = {__float2half_rn(o / l_all)};
@@ -726,8 +731,8 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
 // CTA = one segment (see attn_plan.cuh): a whole head, or one of the k pieces of a head that is cut.
 // DEV: lengths and ring starts come from the device-resident state (attn_update.cuh); the plan was laid out for an
 // upper bound of the length, so segments beyond the real length are empty and a head counts fewer of them.
-template <int KB, int VB, bool DEV>
-__global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_mma_kernel(const __grid_constant__ kvq_attn_args a,
+template <int KB, int VB, bool DEV, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW) decode_attn_mma_kernel(const __grid_constant__ kvq_attn_args a,
                                                                      const __grid_constant__ AttnPlan plan,
                                                                      float *__restrict__ parts,
                                                                      unsigned int *__restrict__ counters) {
@@ -737,10 +742,10 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_mma_kernel(const _
         dev_state_step(a, b);
         plan_cta(plan, b.T, blockIdx.x, head, t0, t1, seg, cnt);
         if (cnt > 1) cnt = min(cnt, (b.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < b.T) attn_segment<KB, VB>(b, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        if (t0 < b.T) attn_segment<KB, VB, NW>(b, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     } else {
         plan_cta(plan, a.T, blockIdx.x, head, t0, t1, seg, cnt);
-        attn_segment<KB, VB>(a, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        attn_segment<KB, VB, NW>(a, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
     }
 }
 
@@ -779,32 +784,38 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     return true;
 }
 
-template <int KB, int VB>
+template <int KB, int VB, int NW>
 static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
                       cudaStream_t st) {
-    const size_t smem = ((size_t)plan.n_scores << plan.ks_log2) * 4 + (size_t)kMmaWarps * warp_region_bytes<KB, VB>() +
+    const size_t smem = ((size_t)plan.n_scores << plan.ks_log2) * 4 + (size_t)NW * warp_region_bytes<KB, VB, NW>() +
                         kHeadDim * 2 + 32 * 4;
     static bool attr_set[64] = {};                           // per device: the opt-in is sticky for the process
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
+        e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, false, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
+            e = cudaFuncSetAttribute(decode_attn_mma_kernel<KB, VB, true, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmaSmemMax);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const unsigned grid = (unsigned)(plan.n_whole + plan.n_cut * plan.k);
-    if (a.state) decode_attn_mma_kernel<KB, VB, true><<<grid, kMmaThreads, smem, st>>>(a, plan, parts, counters);
-    else decode_attn_mma_kernel<KB, VB, false><<<grid, kMmaThreads, smem, st>>>(a, plan, parts, counters);
+    if (a.state) decode_attn_mma_kernel<KB, VB, true, NW><<<grid, 32 * NW, smem, st>>>(a, plan, parts, counters);
+    else decode_attn_mma_kernel<KB, VB, false, NW><<<grid, 32 * NW, smem, st>>>(a, plan, parts, counters);
     return check_launch();
 }
 
+constexpr int kNarrowScores = 5216;                          // scores of a four-warp CTA with four of them on an SM
+
 int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
                            cudaStream_t st) {
+    // Whole heads in several waves: four warps per CTA and four CTAs per SM.  The same 16 warps per SM, but what a CTA does
+    // once (addresses, ring fill, tails, sums) is done by half as many warps: NARROWNOTE
+    const bool narrow = plan.k == 1 && (int64_t)plan.n_whole + plan.n_cut >= 2 * 4 * kSmCount && plan.n_scores <= kNarrowScores;
 #define KVQ_MMA_CASE(KB, VB) \
-    if (a.k_bits == KB && a.v_bits == VB) return launch_mma<KB, VB>(a, plan, parts, counters, st);
+    if (a.k_bits == KB && a.v_bits == VB)                                                            \
+        return narrow ? launch_mma<KB, VB, 4>(a, plan, parts, counters, st) : launch_mma<KB, VB, 8>(a, plan, parts, counters, st);
     KVQ_MMA_CASE(4, 4) KVQ_MMA_CASE(4, 2) KVQ_MMA_CASE(4, 1)
     KVQ_MMA_CASE(3, 4) KVQ_MMA_CASE(3, 2) KVQ_MMA_CASE(3, 1)
     KVQ_MMA_CASE(2, 4) KVQ_MMA_CASE(2, 2) KVQ_MMA_CASE(2, 1)
