@@ -4,7 +4,7 @@
 // units of `unit` tokens (a warp's key tile: 256, or four of them for 3-bit keys: 352 = 4 x 88); a head has
 // uph = ceil(T / unit) units, the last one possibly short.  One CTA works one segment = a run of units of one head:
 //   * the first n_whole CTAs take one whole head each (only when a head fits the score buffer); n_whole is a multiple
-//     of the resident-CTA slots of the GPU, so these CTAs fill whole waves;
+//     of kWholeWave, so these CTAs fill whole waves;
 //   * every remaining head (n_cut of them) is cut into k segments of seg_units units (the last one shorter), launched
 //     after the whole heads, first segments of all heads first.  k is chosen so that these smaller CTAs, which the
 //     hardware hands to whichever slot frees up, finish as early as possible: the last wave of a grid is then made of
@@ -30,7 +30,7 @@ struct AttnPlan {
 constexpr int kSmCount = 148;
 constexpr int kPlanSlots = 2 * kSmCount;       // resident CTAs: two of eight warps per SM
 constexpr int kPlanWarps = 8;
-// Whole heads are launched in multiples of whole waves of two, three, ... CTAs per SM
+// Whole heads: multiples of two and of three CTAs per SM
 constexpr int kWholeWave = 6 * kSmCount;
 // One partial result of a cut head: 128 accumulators, the segment's maximum and sum, padded so that rows stay 16-byte
 // aligned (the merge reads them with 128-bit loads).
@@ -66,7 +66,10 @@ inline long long plan_segment_cycles(int n, int tile, int max_scores) {
 inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; }
 
 // heads: number of heads (or head groups); tile: tokens of a warp's key tile; max_scores: tokens the score buffer holds.
-inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long long heads) {
+// narrow_scores: tokens up to which a kernel also has four-warp CTAs, four to an SM (0: it has none).  Heads that fill the eight-warp
+// slots more than once and the four-warp ones at most once are then left whole: 320 heads of 4096 tokens at 2 bits
+// take 57 us that way, 68 us cut for the eight-warp CTAs.
+inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long long heads, int narrow_scores = 0) {
     AttnPlan p;
     p.unit = unit;
     p.uph = (T + unit - 1) / unit;
@@ -79,6 +82,7 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
     if (p.n_cut > 0) {
         // candidates: segments of su units; estimated finish = rounds of CTAs x cycles of one + merge
         long long best = -1;
+        const bool one_wave = T <= narrow_scores && heads > kPlanSlots && heads <= 2 * kPlanSlots;
         for (int su = whole_ok ? p.uph : max_units; su >= 1; --su) {
             const int k = (p.uph + su - 1) / su;
             const long long ctas = (long long)p.n_cut * k;
@@ -92,6 +96,7 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
                 p.seg_units = su;
             }
         }
+        if (one_wave) p.k = 1;
         p.seg_units = (p.uph + p.k - 1) / p.k;                                   // even the segments out
         p.k = (p.uph + p.seg_units - 1) / p.seg_units;
     }

@@ -1,4 +1,4 @@
-// Fused decode attention for grouped-query models, tensor-core path: one CTA (4 warps) serves up to FOUR query heads
+// Fused decode attention for grouped-query models, tensor-core path: one CTA (8 warps) serves up to FOUR query heads
 // that share a kv head, so every packed code is fetched, unpacked and fed to the tensor core once for all of them.
 //
 // Same formulation as decode_attn_mma.cu (codes reach mma.sync as fp16 subnormals, q*scale carried as an exact
@@ -14,7 +14,7 @@
 //           in one channel group (a 16-byte block of a token row = 128 / 64 / 32 channels; needs v_group >= that --
 //           except 1-bit values at group 64, where a block spans two groups and every code tile is multiplied by both
 //           groups' operands, each lane keeping the product of the group its rows belong to).
-// Scores of the four heads sit side by side in shared memory ([4][n]); warp w runs the softmax of head w.
+// Scores of the four heads sit side by side in shared memory ([4][n]); two warps run the softmax of a head.
 #include "attn_mma_common.cuh"
 #include "attn_plan.cuh"
 #include "attn_update.cuh"

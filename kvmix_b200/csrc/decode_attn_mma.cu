@@ -1,4 +1,4 @@
-// Fused decode attention, tensor-core path: one CTA (4 warps) per query head and token split; the query heads of a
+// Fused decode attention, tensor-core path: one CTA (8 warps, or 4) per query head and token split; the query heads of a
 // kv head are neighbouring CTAs and share its cache through L2.
 //
 // Why tensor cores for a mat-vec: at the HBM rate a B200 has only ~1-3 issue slots per packed code (2.8 per 2-bit
@@ -808,11 +808,16 @@ static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts
 
 constexpr int kNarrowScores = 5216;                          // scores of a four-warp CTA with four of them on an SM
 
-int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
+int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &given, float *parts, unsigned int *counters,
                            cudaStream_t st) {
-    // Whole heads in several waves: four warps per CTA and four CTAs per SM.  The same 16 warps per SM, but what a CTA does
-    // once (addresses, ring fill, tails, sums) is done by half as many warps: NARROWNOTE
-    const bool narrow = plan.k == 1 && (int64_t)plan.n_whole + plan.n_cut >= 2 * 4 * kSmCount && plan.n_scores <= kNarrowScores;
+    AttnPlan plan = given;
+    // More whole heads than eight-warp CTAs fit the GPU: four warps per CTA and four CTAs per SM.  The same 16 warps per SM, but
+    // what a CTA does once (addresses, ring fill, tails, sums: 20k of the 72k warp instructions of a head of 4096 tokens)
+    // is done by half as many warps.  us a layer of 4096 tokens, 2 bits, eight warps -> four: 2048 heads 275 -> 255 (held by the
+    // power cap), 832 heads 110 -> 105, 576 heads 77.6 -> 73.5; 256 heads want the eight warps.
+    const bool narrow = plan.k == 1 && (int64_t)plan.n_whole + plan.n_cut > kPlanSlots && plan.n_scores <= kNarrowScores;
+    if (narrow) plan.ks_log2 = plan.n_scores > 2 * KGeom<4>::WT ? 0 : plan.ks_log2;      // tiles for four warps without a split
+    if (narrow && (plan.n_scores << plan.ks_log2) > kNarrowScores) plan.ks_log2 = 0;
 #define KVQ_MMA_CASE(KB, VB) \
     if (a.k_bits == KB && a.v_bits == VB)                                                            \
         return narrow ? launch_mma<KB, VB, 4>(a, plan, parts, counters, st) : launch_mma<KB, VB, 8>(a, plan, parts, counters, st);
@@ -827,7 +832,8 @@ int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *
 // Plan of the tensor-core kernel for B * nh query heads (one head per segment).
 AttnPlan plan_attn_mma(int T, int k_bits, long long heads) {
     // score buffers that leave room for two CTAs per SM
-    return k_bits == 3 ? make_attn_plan(T, 352, KGeom<3>::WT, 7040, heads) : make_attn_plan(T, 256, KGeom<4>::WT, 6144, heads);
+    return k_bits == 3 ? make_attn_plan(T, 352, KGeom<3>::WT, 7040, heads, kNarrowScores)
+                       : make_attn_plan(T, 256, KGeom<4>::WT, 6144, heads, kNarrowScores);
 }
 
 }  // namespace kvq

@@ -30,7 +30,7 @@ def features_per_int(bits):
 
 # The current stream of the current device as an integer.  torch.cuda.current_stream() builds a Stream object for it:
 # 3.3 us a call, a sixth of the host time of a one-layer decode step; this is 0.15 us.
-_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 
 
 def raw_stream():
