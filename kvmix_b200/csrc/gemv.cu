@@ -67,16 +67,23 @@ __global__ void __launch_bounds__(256) gemv_kernel(kvq_gemv_args a, int wx_log2,
 // Tensor-core form.  A warp works tiles of 128 columns (16 * BITS bytes of a row) x 32 rows a stage:
 //   A (16x16)  codes, rows = columns n of the result, k = 16 rows of the matrix (transposing ldmatrix, fields left in place);
 //   B (16x8)   column 2j / 2j + 1 = hi / lo of in[k] * scale[k, group j], j < 4 groups: the product of two fp16 numbers needs
-//              22 bits and is carried as an fp16 pair, so what is left is the fp32 accumulation, as before.  `in` is first
-//              divided by a power of two >= its largest magnitude in the chunk, so that no product overflows and the small
-//              probabilities of a long softmax keep their low part (absolute error 2^-25 of the largest).
+//              22 bits and is carried as an fp16 pair.  lo ends at 2^-24 whatever the product, so both factors are first
+//              brought to the upper half of the fp16 range by powers of two: `in` by one per chunk of rows (only upwards, hence
+//              exactly: its largest magnitude to 2^7 .. 2^8), the scales of a group by one per window of stages (the largest
+//              of the first stage to 2^4 .. 2^5, the others below 2^8).  What the pair loses is then at most 2^-36 of the largest
+//              input times the largest scale, 2^-24 of a product 2^12 times smaller; what is left is the fp32 accumulation.
+//              Softmax weights of 0.9 on one row of next to nothing and 0.1 on 2047 others with scales of 0.03: 2e-4 from 64
+//              bits (the fp16 result), 6e-4 (2 bits) and 4e-3 (4 bits) with `in` brought below 1 and the scales as they are.
 //   Every other 16 rows use the complement of the codes with the operand's sign turned, c = MAX - (MAX - c): the tensor core cuts
 //   products off downwards (codes are subnormal: 2^-20 of a product), which over thousands of rows of non-negative
 //   probabilities adds up to 3e-6 of the magnitude summed; with opposite signs the two halves cancel.
 //   zeros      one MMA per 16 rows with the [4 scales | 4 zeros] rows read transposed as A and `in` as B: row 4 + j of the
 //              product is the zero term of group j (and row j the sum of in * scale that the complemented rows need).
-// Bound by the instruction stream (0.6 logic operations a code); 16 sequences x 32 heads x 4096 tokens, q . K^T
-// and p . V together: 105 us at 2 bits and 115 us at 4 bits, 229 and 318 us with one thread per word column.
+//   Infinities and NaN come out as fp32 products and sums give them: a window that holds an infinity works without the complement,
+//              whose two halves would meet as inf - inf.
+// Bound by the instruction stream (0.6 logic operations a code); 16 sequences x 32 heads x 4096 tokens, q . K^T and p . V together
+// at 2 bits: 113 us (105 us without the powers of two), 229 us with one thread per word column; from a flushed L2 123 us at 2
+// bits (115 without) and 135 us at 4 bits (130 without).
 template <int BITS> struct GemvGeom {
     static constexpr int RB = 16 * BITS;                       // code bytes of a tile row
     static constexpr int RS = BITS == 1 ? RB : RB + 16;        // padded: conflict-free ldmatrix
@@ -87,7 +94,9 @@ template <int BITS> struct GemvGeom {
 };
 constexpr int kGemvWarps = 8, kGemvThreads = 32 * kGemvWarps;
 constexpr int kGemvChunk = 2048;                               // rows whose `in` is held (and normalised) at a time
-constexpr int kGemvFlush = 8;                                  // stages between flushes of the MMA accumulators (short chains)
+constexpr int kGemvFlush = 8;                                  // stages between flushes of the MMA accumulators (short chains): a window
+
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 
 struct GemvPlan {
     int wk_log2;         // warps that share a column tile (the other factor of 8: column tiles of a CTA)
@@ -151,7 +160,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
 
     for (int c0 = k_beg; c0 < k_end; c0 += kGemvChunk) {
         const int rows = min(kGemvChunk, k_end - c0), n_st = (rows + 31) / 32;
-        // ---- in / 2^e, 2^e >= the largest magnitude of the chunk (an infinity or NaN is left as it is) -----------
+        // ---- in * 2^up_e: the largest magnitude to 2^7 .. 2^8, larger ones (and a chunk with an infinity) as they are ----
         if (c0 > k_beg) __syncthreads();                                        // the previous chunk has been read
         float mx = 0.f;
         for (int i = tid; i < rows; i += kGemvThreads) mx = fmaxf(mx, fabsf(__half2float(__ldg(in + c0 + i))));
@@ -159,11 +168,13 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
         if (lane == 0) misc[warp] = mx;
         __syncthreads();
         mx = warp_max(misc[lane & 7]);
-        int e = 0;
-        if (mx > 0.f && mx <= 65504.f) e = (int)((__float_as_uint(mx) >> 23) & 255u) - 126;   // mx < 2^e
-        const float down = __uint_as_float((uint32_t)(127 - e) << 23), up = __uint_as_float((uint32_t)(127 + e) << 23);
+        const bool in_finite = mx <= 65504.f;
+        const int in_e = in_finite ? max((int)((__float_as_uint(mx) >> 23) & 255u) - 126, -24) : 16;   // mx < 2^in_e
+        const int up_e = max(8 - in_e, 0);
+        const float up = pow2f(up_e), down = pow2f(-up_e);
+        const int room = 16 - max(in_e, 8);                                     // scales below 2^room: products below 2^16
         for (int i = tid; i < n_st * 32; i += kGemvThreads)
-            xs[i] = i < rows ? __float2half_rn(__half2float(__ldg(in + c0 + i)) * down) : __float2half_rn(0.f);
+            xs[i] = i < rows ? __float2half_rn(__half2float(__ldg(in + c0 + i)) * up) : __float2half_rn(0.f);
         __syncthreads();
         if (words <= 0) continue;
 
@@ -195,24 +206,48 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
             }
             cp_async_commit();
         };
+        // the window's powers of two: of the group of this lane's B column, undone for the group of its C columns; lanes g < 4 watch
+        // that the scales of group g stay below `lim`
+        __half2 s_up = __floats2half2_rn(1.f, 1.f), lim = s_up;
+        float undo = 1.f;
+        uint32_t top = 0u;                                                      // exponent bits of the window's largest scale of the group
+        bool turn = false;                                                      // every other 16 rows complemented
+        int since = 0;
         auto flush = [&]() {
 #pragma unroll
             for (int m = 0; m < 8; ++m) {
-                sum[m][0] = fmaf(acc[m][0] + acc[m][1], up, sum[m][0]);
-                sum[m][1] = fmaf(acc[m][2] + acc[m][3], up, sum[m][1]);
+                sum[m][0] = fmaf(acc[m][0] + acc[m][1], undo, sum[m][0]);
+                sum[m][1] = fmaf(acc[m][2] + acc[m][3], undo, sum[m][1]);
                 acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
             }
             // lanes of rows 4 .. 7: zero terms of all rows; of rows 0 .. 3: sums of in * scale of the complemented rows
-            zsum = fmaf(g < 4 ? accz[1][0] : accz[0][0] + accz[1][0], up, zsum);
+            const float z = g < 4 ? (turn ? accz[1][0] : 0.f) : accz[0][0] + accz[1][0];
+            zsum = fmaf(z, down, zsum);
 #pragma unroll
             for (int i = 0; i < 4; ++i) accz[0][i] = accz[1][i] = 0.f;
+            since = 0;
+        };
+        // A window opens with the largest scales of its first stage (`m`: a lane's largest, four lanes hold a group); a stage with a
+        // scale of more than eight times that closes it early.
+        auto open_window = [&](__half2 m) {
+            if (since) flush();
+            else top = 0u;
+            m = __hmax2(m, as_h2(__shfl_xor_sync(0xffffffffu, as_u32(m), 1)));
+            m = __hmax2(m, as_h2(__shfl_xor_sync(0xffffffffu, as_u32(m), 2)));
+            top = max(top, (uint32_t)__half_as_ushort(__hmax(__low2half(m), __high2half(m))) & 0x7c00u);
+            const uint32_t l = g < ngw && top < 0x7c00u ? min(top + 0x0fffu, 0x7bffu) : 0x7c00u;      // scales up to here are below 2^(exponent - 11)
+            lim = as_h2(l | (l << 16));
+            const float f = pow2f(min(room - ((int)(top >> 10) - 11), 15));
+            const float fb = __shfl_sync(0xffffffffu, f, 4 * (g >> 1)), fc = __shfl_sync(0xffffffffu, f, 4 * tig);
+            s_up = __floats2half2_rn(fb, fb);
+            undo = down * __uint_as_float((254u << 23) - __float_as_uint(fc));
+            turn = in_finite && !__any_sync(0xffffffffu, g < ngw && top == 0x7c00u);
         };
 
         uint32_t iss_slot = 0, slot = 0;
         int iss_st = wk;
 #pragma unroll 1
         for (int q = 0; q < G::NS - 1; ++q) { issue(iss_st, iss_slot); iss_st += WK; iss_slot += G::STAGE_BYTES; }
-        int since = 0;
 #pragma unroll 1
         for (int st = wk; st < n_st; st += WK) {
             issue(iss_st, iss_slot);
@@ -220,21 +255,27 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
             iss_slot = iss_slot == (G::NS - 1) * G::STAGE_BYTES ? 0u : iss_slot + G::STAGE_BYTES;
             cp_async_wait<G::NS - 1>();
             __syncwarp();
+            uint32_t r[2][2];                                                   // scales (lanes g < 4) and zeros of 16 rows, transposed
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                             : "=r"(r[k][0]), "=r"(r[k][1]) : "r"(szm_s + slot + k * 256));
+            const __half2 m = __hmax2(__hmax2(__habs2(as_h2(r[0][0])), __habs2(as_h2(r[0][1]))), __hmax2(__habs2(as_h2(r[1][0])), __habs2(as_h2(r[1][1]))));
+            if (__any_sync(0xffffffffu, since == 0 || __hgt2_mask(m, lim) != 0u)) open_window(m);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const uint32_t xa = x_s + (32 * st + 16 * k) * 2;
                 const uint32_t x01u = lds32(xa), x89u = lds32(xa + 16);
-                uint32_t r0, r1;
-                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                             : "=r"(r0), "=r"(r1) : "r"(szm_s + slot + k * 256));
+                const uint32_t r0 = r[k][0], r1 = r[k][1];
                 mma16816(accz[k], r0, 0u, r1, 0u, x01u, x89u);
-                const uint32_t flip = k ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
-                // an infinite product gives hi = inf and lo = NaN: the minimum keeps a number there, and the sum infinite
-                const __half2 big = __floats2half2_rn(65504.f, 65504.f);
-                const uint32_t h0 = hilo(as_h2(x01u ^ sign), as_h2(__shfl_sync(0xffffffffu, r0, src)), neg_mask);
-                const uint32_t h1 = hilo(as_h2(x89u ^ sign), as_h2(__shfl_sync(0xffffffffu, r1, src)), neg_mask);
-                const uint32_t b0 = (as_u32(__hmin2(as_h2(h0), big)) & neg_mask) | (h0 & ~neg_mask);
-                const uint32_t b1 = (as_u32(__hmin2(as_h2(h1), big)) & neg_mask) | (h1 & ~neg_mask);
+                const uint32_t flip = k && turn ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
+                uint32_t b0 = hilo(as_h2(x01u ^ sign), __hmul2(as_h2(__shfl_sync(0xffffffffu, r0, src)), s_up), neg_mask);
+                uint32_t b1 = hilo(as_h2(x89u ^ sign), __hmul2(as_h2(__shfl_sync(0xffffffffu, r1, src)), s_up), neg_mask);
+                if (!turn) {                                                    // behind an infinite hi the minimum keeps a number, and the sum infinite
+                    const __half2 big = __floats2half2_rn(65504.f, 65504.f);
+                    b0 = (as_u32(__hmin2(as_h2(b0), big)) & neg_mask) | (b0 & ~neg_mask);
+                    b1 = (as_u32(__hmin2(as_h2(b1), big)) & neg_mask) | (b1 & ~neg_mask);
+                }
                 uint32_t x[NBLK][2];
                 const uint32_t ad = ldk_s + slot + (16 * k) * G::RS;
                 if constexpr (BITS == 1) {
@@ -257,9 +298,9 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
             }
             __syncwarp();
             slot = slot == (G::NS - 1) * G::STAGE_BYTES ? 0u : slot + G::STAGE_BYTES;
-            if (++since == kGemvFlush) { flush(); since = 0; }
+            if (++since == kGemvFlush) flush();
         }
-        flush();
+        if (since) flush();
         cp_async_wait<0>();
         __syncwarp();
     }
