@@ -41,10 +41,10 @@ template <int VB> using GqaVGeom = VGeom<VB, VB == 4 ? 3 : VB == 2 ? 5 : 7>;
 template <int VB> constexpr int gqa_op_bytes() { return VB == 4 ? 2048 : 1024; }
 
 // 3-bit values (the short-last-group extension: 12 words and 12 groups a token): 48 + 2 x 24 bytes a token, two slots, operand
-// tiles of four groups and the tile of the probabilities
+// tiles of four groups, the tile of the probabilities and the groups' powers of two
 constexpr int kV3Words = (kHeadDim + 10) / 11;
 constexpr int kV3Stage = 32 * (kV3Words * 4 + 2 * kV3Words * 2), kV3Slots = 2, kV3SzOff = 32 * kV3Words * 4;
-constexpr int kV3Region = kV3Slots * kV3Stage + 4 * 512 + 512;
+constexpr int kV3Region = kV3Slots * kV3Stage + 4 * 512 + 512 + 32;
 template <int VB> constexpr int gqa_v_region() { return GqaVGeom<VB>::NS * GqaVGeom<VB>::STAGE_BYTES + gqa_op_bytes<VB>(); }
 template <> constexpr int gqa_v_region<3>() { return kV3Region; }
 template <int KB, int VB> constexpr int gqa_region_bytes() {
@@ -533,12 +533,17 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
 // ---------------------------------------------------------------------------------------------
 // p . V over 3-bit values: twelve words a token, each its own group of 11 channels (the last of 7).  As for 3-bit keys the
 // channels of a word are the rows of an MMA (11 of 16 used); p * scale is carried as an fp16 pair hi + lo of the fp32
-// product, columns 2h / 2h + 1 of head h (4 p, saturating only together: 65504 + 65504 is above 4 * 18715, the largest
-// scale a group of fp16 numbers can have), the zero terms come from one MMA per 16 tokens (rows = groups, B = p hi / lo).
+// product, columns 2h / 2h + 1 of head h, the zero terms come from one MMA per 16 tokens (rows = groups, B = p hi / lo).
+// lo ends at 2^-24 whatever the product, so p (<= 1) is carried as 2^13 p and the scales of a group times a power of two that
+// brings the largest of this warp's tokens to 2 .. 4 (exactly, but for those 2^-15 of it): what a pair loses is 2^-38 of the
+// largest p and scale.  The largest scales are found by reading the warp's scale rows once ahead (a quarter of a token's bytes,
+// asked for before the softmax and in L2 by then).  Infinite and NaN scales come out as fp32 products give them: a warp whose
+// tokens hold one works without the complement below, whose halves would meet as inf - inf.
 // Every other 16 tokens use the complemented codes and the operands' sign turned, so that what the tensor core cuts off
 // the products (codes are subnormal) cancels instead of adding up; the sums of p * scale this needs are one more such MMA.
 // Bound by the operand tiles (12 groups x 4 heads of p * scale for 352 bytes of a token pair).  8 x 8 kv heads, 32768
-// tokens, 3-bit keys and values: 210 us a layer, 735 us with the CUDA-core kernel.
+// tokens, 3-bit keys and values: 219 us a layer (215 with 4 p and the scales as they are), 735 us with the CUDA-core kernel.
+// 0.99 of the weight on one token of next to nothing, values of sigma 0.03: 2.3e-4 from 64 bits (fp32 products 2.3e-4; 9e-4 so).
 template <int MODE>
 __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int32_t *vc, const __half *vs, const __half *vz,
                                                const GqaSmem &sm, int t0, int hi) {
@@ -574,13 +579,57 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
         src_codes += codes_step;
         src_sz += sz_step;
     };
+    const char *sz_row = reinterpret_cast<const char *>(vs) + src_sz;                 // scale rows of the warp's first block
     if (MODE == 1) {
         issue_stage(0);
+        // the scale rows of the blocks to come, 768 bytes (seven lines at most) each
+        for (int x = lane; x < 7 * my_blocks; x += 32)
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(sz_row + (x / 7) * sz_step + min(128 * (x % 7), 764)));
         return;
     }
     --to_issue;
     src_codes += codes_step;
     src_sz += sz_step;
+
+    const uint32_t up_s = ring_s + kV3Slots * kV3Stage + 4 * 512 + 512;               // [12] fp16 powers of two
+    bool finite;
+    {
+        // granule x of a block's 48 holds halves 8 x .. 8 x + 7, groups 8 (x mod 3) + i (mod 12): lanes 0 .. 23 take granules
+        // lane and lane + 24; magnitudes as integers, 2^-14 at least
+        uint32_t mx[4] = {0x04000400u, 0x04000400u, 0x04000400u, 0x04000400u};
+        if (lane < 24) {
+#pragma unroll 3
+            for (int q = 0; q < my_blocks; ++q) {
+                const uint4 u = __ldg(reinterpret_cast<const uint4 *>(sz_row + q * sz_step) + lane);
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(sz_row + q * sz_step) + lane + 24);
+                mx[0] = __vmaxu2(mx[0], __vmaxu2(u.x & 0x7fff7fffu, v.x & 0x7fff7fffu));
+                mx[1] = __vmaxu2(mx[1], __vmaxu2(u.y & 0x7fff7fffu, v.y & 0x7fff7fffu));
+                mx[2] = __vmaxu2(mx[2], __vmaxu2(u.z & 0x7fff7fffu, v.z & 0x7fff7fffu));
+                mx[3] = __vmaxu2(mx[3], __vmaxu2(u.w & 0x7fff7fffu, v.w & 0x7fff7fffu));
+            }
+        }
+#pragma unroll
+        for (int o = 12; o >= 3; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx[i] = __vmaxu2(mx[i], __shfl_down_sync(0xffffffffu, mx[i], o));
+        // lane 0 holds groups 0 .. 7, lane 1 groups 8 .. 11, 0 .. 3, lane 2 groups 4 .. 11
+        uint32_t up[6];
+        finite = true;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            const uint32_t x = i < 2 ? __vmaxu2(__shfl_sync(0xffffffffu, mx[i], 0), __shfl_sync(0xffffffffu, mx[i + 2], 1))
+                             : i < 4 ? __vmaxu2(__shfl_sync(0xffffffffu, mx[i], 0), __shfl_sync(0xffffffffu, mx[i - 2], 2))
+                                     : __vmaxu2(__shfl_sync(0xffffffffu, mx[i - 4], 1), __shfl_sync(0xffffffffu, mx[i - 2], 2));
+            up[i] = 0x7c007c00u - (x & 0x7c007c00u);           // exponent e of the largest: 2^(16 - e); 0 for infinity and NaN
+            if (!(up[i] & 0xffffu)) { up[i] |= 0x0400u; finite = false; }      // 2^-14: the group's finite scales stay so
+            if (!(up[i] >> 16)) { up[i] |= 0x04000000u; finite = false; }
+        }
+        if (lane == 0) {
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(up_s), "r"(up[0]), "r"(up[1]), "r"(up[2]), "r"(up[3]));
+            asm volatile("st.shared.v2.b32 [%0], {%1,%2};\n" ::"r"(up_s + 16), "r"(up[4]), "r"(up[5]));
+        }
+        __syncwarp();
+    }
 
     // field g / g + 8 of a word (see gqa_qk_packed)
     const int byte0 = (3 * g) >> 3, p0 = 3 * g - 8 * byte0;
@@ -601,10 +650,15 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
 #pragma unroll
     for (int j = 0; j < W; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     auto put = [&](uint32_t addr, float x0, float x1, float y0, float y1) {           // hi, lo of (x0, x1), then of (y0, y1)
-        const uint32_t hx = pack_h2_sat(x0, x1), hy = pack_h2_sat(y0, y1);
+        const uint32_t hx = as_u32(__floats2half2_rn(x0, x1)), hy = as_u32(__floats2half2_rn(y0, y1));
         const float2 fx = __half22float2(as_h2(hx)), fy = __half22float2(as_h2(hy));
-        const uint32_t lx = pack_h2_sat(x0 - fx.x, x1 - fx.y), ly = pack_h2_sat(y0 - fy.x, y1 - fy.y);
-        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(hx), "r"(lx), "r"(hy), "r"(ly));
+        __half2 lx = __floats2half2_rn(x0 - fx.x, x1 - fx.y), ly = __floats2half2_rn(y0 - fy.x, y1 - fy.y);
+        if (!finite) {                                         // behind an infinite hi the minimum keeps a number, and the sum infinite
+            const __half2 big = __floats2half2_rn(65504.f, 65504.f);
+            lx = __hmin2(lx, big);
+            ly = __hmin2(ly, big);
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(hx), "r"(as_u32(lx)), "r"(hy), "r"(as_u32(ly)));
     };
     // A fragment of a [token][group] tile read transposed: rows g, g + 8 = groups (12 of 16), k = 16 tokens
     auto group_rows = [&](uint32_t addr, uint32_t (&r)[4]) {
@@ -625,20 +679,22 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
         cp_async_wait<1>();
         __syncwarp();
         const float2 fa = *reinterpret_cast<const float2 *>(pa), fb = *reinterpret_cast<const float2 *>(pb);
-        const float a0 = 4.f * fa.x, a1 = 4.f * fa.y, b0 = 4.f * fb.x, b1 = 4.f * fb.y;
+        const float a0 = 8192.f * fa.x, a1 = 8192.f * fa.y, b0 = 8192.f * fb.x, b1 = 8192.f * fb.y;
         put(pp_s + (pi * 8 + 4 * hh) * 4, a0, a1, b0, b1);
 #pragma unroll
         for (int r = 0; r < W / 4; ++r) {
+            const uint2 c = lds64(up_s + 8 * r), e0 = lds64(sz_rd + st + 8 * r), e1 = lds64(sz_rd + st + 8 * r + W * 2);
 #pragma unroll
-            for (int jv = 0; jv < 4; ++jv) {
-                const float s0 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * (4 * r + jv))));
-                const float s1 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * (4 * r + jv) + W * 2)));
-                put(op_wr + jv * 512, a0 * s0, a1 * s1, b0 * s0, b1 * s1);
+            for (int half = 0; half < 2; ++half) {             // groups 4 r, 4 r + 1, then 4 r + 2, 4 r + 3
+                const __half2 f = as_h2(half ? c.y : c.x);
+                const float2 s0 = __half22float2(__hmul2(as_h2(half ? e0.y : e0.x), f)), s1 = __half22float2(__hmul2(as_h2(half ? e1.y : e1.x), f));
+                put(op_wr + (2 * half) * 512, a0 * s0.x, a1 * s1.x, b0 * s0.x, b1 * s1.x);
+                put(op_wr + (2 * half + 1) * 512, a0 * s0.y, a1 * s1.y, b0 * s0.y, b1 * s1.y);
             }
             __syncwarp();
 #pragma unroll
             for (int h2 = 0; h2 < 2; ++h2) {
-                const uint32_t flip = h2 ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
+                const uint32_t flip = h2 && finite ? 0xffffffffu : 0u, sign = flip & 0x80008000u;
                 if (r == 0) {
                     const uint32_t pp_rd = pp_s + (tig * 8 + g + 64 * h2) * 4, x0 = lds32(pp_rd), x1 = lds32(pp_rd + 128);
                     uint32_t z[4];
@@ -670,15 +726,17 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
     cp_async_wait<0>();
     __syncwarp();
     // lane (g, tig): channels of rows g, g + 8 for head tig; the group's zero term and complement sum sit in the lanes of row j
-    const float sc0 = __int_as_float((151 - 2 - p0) << 23), sc1 = __int_as_float((151 - 2 - p1) << 23);   // 2^(24 - position) / 4
-    const float z0 = accz[0] + accz[1], z1 = accz[2] + accz[3], s0 = accs[0] + accs[1], s1 = accs[2] + accs[3];
+    const float sc0 = __int_as_float((151 - 13 - p0) << 23), sc1 = __int_as_float((151 - 13 - p1) << 23);   // 2^(24 - position - 13)
+    const float z0 = accz[0] + accz[1], z1 = accz[2] + accz[3], s0 = finite ? accs[0] + accs[1] : 0.f, s1 = finite ? accs[2] + accs[3] : 0.f;
     const float max1 = g == 2 ? 3.f : 7.f;                     // the 11th field has two bits
 #pragma unroll
     for (int j = 0; j < W; ++j) {
         const int from = 4 * (j & 7) + tig;
-        const float z = 0.25f * __shfl_sync(0xffffffffu, j < 8 ? z0 : z1, from), sv = 0.25f * __shfl_sync(0xffffffffu, j < 8 ? s0 : s1, from);
-        if (11 * j + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + g] = fmaf(acc[j][0] + acc[j][1], sc0, fmaf(7.f, sv, z));
-        if (g < 3 && 11 * j + 8 + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + 8 + g] = fmaf(acc[j][2] + acc[j][3], sc1, fmaf(max1, sv, z));
+        constexpr float k = 1.f / 8192.f;
+        const float z = k * __shfl_sync(0xffffffffu, j < 8 ? z0 : z1, from), sv = k * __shfl_sync(0xffffffffu, j < 8 ? s0 : s1, from);
+        const float undo = __int_as_float((127 + 15 - (int)(lds16(up_s + 2 * j) >> 10)) << 23);             // 1 / the group's power of two
+        if (11 * j + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + g] = fmaf(acc[j][0] + acc[j][1], sc0 * undo, fmaf(7.f, sv, z));
+        if (g < 3 && 11 * j + 8 + g < kHeadDim) my_red[tig * kHeadDim + 11 * j + 8 + g] = fmaf(acc[j][2] + acc[j][3], sc1 * undo, fmaf(max1, sv, z));
     }
 }
 
