@@ -4,7 +4,7 @@
 // units of `unit` tokens (a warp's key tile: 256, or four of them for 3-bit keys: 352 = 4 x 88); a head has
 // uph = ceil(T / unit) units, the last one possibly short.  One CTA works one segment = a run of units of one head:
 //   * the first n_whole CTAs take one whole head each (only when a head fits the score buffer); n_whole is a multiple
-//     of kWholeWave, so these CTAs fill whole waves;
+//     of the number of SMs, so these CTAs load all SMs alike;
 //   * every remaining head (n_cut of them) is cut into k segments of seg_units units (the last one shorter), launched
 //     after the whole heads, first segments of all heads first.  k is chosen so that these smaller CTAs, which the
 //     hardware hands to whichever slot frees up, finish as early as possible: the last wave of a grid is then made of
@@ -24,14 +24,14 @@ struct AttnPlan {
     int k;               // segments per cut head (1: a whole head per CTA here too)
     int seg_units;       // units per segment of a cut head
     int n_scores;        // most tokens in a segment, rounded up to 32
+    int warps;           // warps of a CTA: 8 (two CTAs to an SM) or 4 (three or four)
     int ks_log2;         // the channels of a key tile are shared by 1 << ks_log2 warps (partial scores, summed by the softmax)
 };
 
 constexpr int kSmCount = 148;
 constexpr int kPlanSlots = 2 * kSmCount;       // resident CTAs: two of eight warps per SM
 constexpr int kPlanWarps = 8;
-// Whole heads: multiples of two and of three CTAs per SM
-constexpr int kWholeWave = 6 * kSmCount;
+constexpr int kWholeWave = 6 * kSmCount;       // grouped kernel: whole head groups in multiples of three waves
 // One partial result of a cut head: 128 accumulators, the segment's maximum and sum, padded so that rows stay 16-byte
 // aligned (the merge reads them with 128-bit loads).
 constexpr int kPartStride = 128 + 4;
@@ -42,15 +42,15 @@ inline int plan_round32(int n) { return (n + 31) / 32 * 32; }
 // Channel split of a segment's key tiles.  A warp walks a tile's 128 channels in four steps of 32; where a segment has fewer
 // tiles than the CTA has warps, 2 or 4 warps share a tile's channels and each leaves partial scores.  Steps a warp takes
 // (x 2), with about half a step's time of per-tile overhead; `max_scores` bounds the score buffer (tokens x splits).
-inline int plan_key_steps(int n, int tile, int ks_log2) {
+inline int plan_key_steps(int n, int tile, int ks_log2, int warps = kPlanWarps) {
     const int tiles = (n + tile - 1) / tile;
-    const int passes = ((tiles << ks_log2) + kPlanWarps - 1) / kPlanWarps;
+    const int passes = ((tiles << ks_log2) + warps - 1) / warps;
     return passes * ((8 >> ks_log2) + 1);
 }
-inline int plan_key_split(int n, int tile, int max_scores) {
+inline int plan_key_split(int n, int tile, int max_scores, int warps = kPlanWarps) {
     int best = 0;
     for (int l = 1; l <= 2; ++l)
-        if ((plan_round32(n) << l) <= max_scores && plan_key_steps(n, tile, l) < plan_key_steps(n, tile, best)) best = l;
+        if ((plan_round32(n) << l) <= max_scores && plan_key_steps(n, tile, l, warps) < plan_key_steps(n, tile, best, warps)) best = l;
     return best;
 }
 
@@ -65,13 +65,32 @@ inline long long plan_segment_cycles(int n, int tile, int max_scores) {
 // What cutting a head adds to its last CTA: publishing the partials and the merge of k of them.
 inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; }
 
+// Pieces a head is cut into where `heads` of them (fewer than SMs) are left behind whole ones: the SM that gets most of the pieces
+// finishes last; a piece costs its tokens and some 600 more, one whole head by itself on its SM `lone` percent of that.
+inline int plan_left_pieces(int T, int unit, int heads, int lone) {
+    const int uph = (T + unit - 1) / unit;
+    int best_k = 1;
+    long long best = (T + 600) * (long long)lone / 100;
+    for (int k = 2; k <= 8 && k <= uph; ++k) {
+        const int su = (uph + k - 1) / k;
+        const long long cost = (long long)((heads * k + kSmCount - 1) / kSmCount) * (su * unit + 600) + 200;
+        if ((uph + su - 1) / su == k && cost < best) { best = cost; best_k = k; }
+    }
+    return best_k;
+}
+
+inline void plan_finish(AttnPlan &p, int T, int tile, int max_scores) {
+    long long ns = (long long)(p.n_whole ? p.uph : p.seg_units) * p.unit;
+    if (ns > T) ns = T;
+    p.n_scores = plan_round32((int)ns);
+    p.ks_log2 = plan_key_split((int)ns, tile, max_scores, p.warps);
+}
+
 // heads: number of heads (or head groups); tile: tokens of a warp's key tile; max_scores: tokens the score buffer holds.
-// narrow_scores: tokens up to which a kernel also has four-warp CTAs, four to an SM (0: it has none).  Heads that fill the eight-warp
-// slots more than once and the four-warp ones at most once are then left whole: 320 heads of 4096 tokens at 2 bits
-// take 57 us that way, 68 us cut for the eight-warp CTAs.
-inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long long heads, int narrow_scores = 0) {
+inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long long heads) {
     AttnPlan p;
     p.unit = unit;
+    p.warps = kPlanWarps;
     p.uph = (T + unit - 1) / unit;
     const int max_units = max_scores / unit;
     const bool whole_ok = T <= max_units * unit;
@@ -82,7 +101,6 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
     if (p.n_cut > 0) {
         // candidates: segments of su units; estimated finish = rounds of CTAs x cycles of one + merge
         long long best = -1;
-        const bool one_wave = T <= narrow_scores && heads > kPlanSlots && heads <= 2 * kPlanSlots;
         for (int su = whole_ok ? p.uph : max_units; su >= 1; --su) {
             const int k = (p.uph + su - 1) / su;
             const long long ctas = (long long)p.n_cut * k;
@@ -96,14 +114,47 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
                 p.seg_units = su;
             }
         }
-        if (one_wave) p.k = 1;
         p.seg_units = (p.uph + p.k - 1) / p.k;                                   // even the segments out
         p.k = (p.uph + p.seg_units - 1) / p.seg_units;
     }
-    long long ns = (long long)(p.n_whole ? p.uph : p.seg_units) * unit;
-    if (ns > T) ns = T;
-    p.n_scores = plan_round32((int)ns);
-    p.ks_log2 = plan_key_split((int)ns, tile, max_scores);
+    plan_finish(p, T, tile, max_scores);
+    return p;
+}
+
+// The kernel with one query head per CTA, which also comes with four warps per CTA.  narrow_max: most tokens of a segment of those (a
+// multiple of the unit); narrow_split: scores that leave room for four of them on an SM; wide_from: tokens from which eight warps
+// a CTA pay up to seven heads an SM.
+//
+// More heads than eight-warp slots: the multiple of the SM count whole, the others cut (us on B200, whole heads in multiples of 888
+// and eight warps for all that is cut -> this; 4096 tokens: 448 heads 2 bits 78 -> 70, 640 heads 99 -> 91, 1280 heads 173 ->
+// 150, 3-bit keys 1536 heads 260 -> 233; 7000 tokens, 4 bits: 896 heads 235 -> 208, 2048 heads 488 -> 444).  What a CTA does once
+// (addresses, ring fill, tails, sums: 20k of the 72k warp instructions of a head of 4096 tokens) is done by half as many warps
+// in the four-warp form, so it is the better one where there are many CTAs or short ones: 300 tokens 0.76 .. 0.9 of the eight-warp
+// form's time, 2000 tokens 0.9 .. 1.0; at 4096 tokens 320 and 448 heads take 1.10 .. 1.16 of it, 1280 heads 0.92.
+inline AttnPlan make_attn_plan_mma(int T, int unit, int tile, int max_scores, long long heads, int narrow_max, int narrow_split, int wide_from) {
+    const int wide_max = max_scores / unit * unit;
+    const bool many = heads > kPlanSlots;
+    // between one and two heads an SM, too long for the eight-warp form whole: four-warp quarters (256 heads of 8000 tokens, 3-bit keys:
+    // 106 -> 96 us against two eight-warp halves)
+    const bool quarters = !many && heads > kSmCount && T > wide_max;
+    if (T > narrow_max || !(many || quarters)) return make_attn_plan(T, unit, tile, max_scores, heads);
+    AttnPlan p;
+    p.unit = unit;
+    p.uph = (T + unit - 1) / unit;
+    p.warps = many && T >= wide_from && T <= wide_max && heads < 7 * kSmCount ? 8 : 4;
+    // long heads are three to an SM: two or four an SM whole would leave it with one or two for most of the time (592 heads of 8000
+    // tokens, 2 bits: 166 us whole, 143 us as 444 and 148 cut; 320 heads 107 and 86 us all cut in five)
+    const bool three = T > wide_max;
+    int per_sm = quarters ? 0 : (int)(heads / kSmCount);
+    if (three && per_sm == 4) per_sm = 3;
+    if (three && per_sm == 2) per_sm = 0;
+    p.n_whole = per_sm * kSmCount;
+    p.k = quarters ? 4 : per_sm == 0 ? 5 : per_sm == 3 && heads >= 4 * kSmCount ? 3 : plan_left_pieces(T, unit, (int)(heads % kSmCount), three ? 125 : 100);
+    if (p.k == 1) p.n_whole = (int)(heads / kWholeWave * kWholeWave);             // all whole: the same launch wherever the line is drawn
+    p.n_cut = (int)(heads - p.n_whole);
+    p.seg_units = (p.uph + p.k - 1) / p.k;
+    p.k = (p.uph + p.seg_units - 1) / p.seg_units;
+    plan_finish(p, T, tile, p.warps == 4 ? narrow_split : max_scores);
     return p;
 }
 

@@ -312,7 +312,7 @@ int launch_decode_attn_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv
 
 // Upper bound, over every shorter context and every kernel, of the partial results (one per query head and segment)
 // a call may hold: the generic kernel's heads x splits; for the tensor-core kernels either what the score buffers
-// force (a segment holds at most 6144 / 7040 tokens, 2048 / 2112 when four query heads share it) or the planner's own cap of
+// force (segments hold up to 6144 / 7040 tokens where many are needed, 2048 / 2112 when four query heads share it) or the planner's own cap of
 // kMaxCtaRounds waves of CTAs over the cut heads (attn_plan.cuh), whichever is larger.
 static int64_t max_partials_bound(int T, int64_t heads) {
     int64_t n = heads;

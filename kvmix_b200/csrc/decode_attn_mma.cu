@@ -784,11 +784,21 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     return true;
 }
 
+// Score buffers: of an eight-warp CTA, two to an SM; of a four-warp CTA, three to an SM, and four to an SM.
+constexpr int kWideScores = 6144, kWideScores3 = 7040, kNarrowMax = 8192, kNarrowMax3 = 8096, kNarrowScores = 5216;
+
+template <int KB, int VB, int NW> constexpr int mma_smem_bytes(int scores) {
+    return scores * 4 + NW * warp_region_bytes<KB, VB, NW>() + kHeadDim * 2 + 32 * 4;
+}
+
 template <int KB, int VB, int NW>
 static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
                       cudaStream_t st) {
-    const size_t smem = ((size_t)plan.n_scores << plan.ks_log2) * 4 + (size_t)NW * warp_region_bytes<KB, VB, NW>() +
-                        kHeadDim * 2 + 32 * 4;
+    constexpr int kSmSmem = 227 * 1024;                      // of an SM, 1 KB of it taken by every CTA
+    static_assert(NW == 4 || mma_smem_bytes<KB, VB, 8>(KB == 3 ? kWideScores3 : kWideScores) <= kMmaSmemMax, "two eight-warp CTAs");
+    static_assert(NW == 8 || 3 * (mma_smem_bytes<KB, VB, 4>(KB == 3 ? kNarrowMax3 : kNarrowMax) + 1024) <= kSmSmem, "three four-warp CTAs");
+    static_assert(NW == 8 || 4 * (mma_smem_bytes<KB, VB, 4>(kNarrowScores) + 1024) <= kSmSmem, "four four-warp CTAs");
+    const size_t smem = mma_smem_bytes<KB, VB, NW>(plan.n_scores << plan.ks_log2);
     static bool attr_set[64] = {};                           // per device: the opt-in is sticky for the process
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -806,21 +816,11 @@ static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts
     return check_launch();
 }
 
-constexpr int kNarrowScores = 5216;                          // scores of a four-warp CTA with four of them on an SM
-
-int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &given, float *parts, unsigned int *counters,
+int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
                            cudaStream_t st) {
-    AttnPlan plan = given;
-    // More whole heads than eight-warp CTAs fit the GPU: four warps per CTA and four CTAs per SM.  The same 16 warps per SM, but
-    // what a CTA does once (addresses, ring fill, tails, sums: 20k of the 72k warp instructions of a head of 4096 tokens)
-    // is done by half as many warps.  us a layer of 4096 tokens, 2 bits, eight warps -> four: 2048 heads 275 -> 255 (held by the
-    // power cap), 832 heads 110 -> 105, 576 heads 77.6 -> 73.5; 256 heads want the eight warps.
-    const bool narrow = plan.k == 1 && (int64_t)plan.n_whole + plan.n_cut > kPlanSlots && plan.n_scores <= kNarrowScores;
-    if (narrow) plan.ks_log2 = plan.n_scores > 2 * KGeom<4>::WT ? 0 : plan.ks_log2;      // tiles for four warps without a split
-    if (narrow && (plan.n_scores << plan.ks_log2) > kNarrowScores) plan.ks_log2 = 0;
 #define KVQ_MMA_CASE(KB, VB) \
     if (a.k_bits == KB && a.v_bits == VB)                                                            \
-        return narrow ? launch_mma<KB, VB, 4>(a, plan, parts, counters, st) : launch_mma<KB, VB, 8>(a, plan, parts, counters, st);
+        return plan.warps == 4 ? launch_mma<KB, VB, 4>(a, plan, parts, counters, st) : launch_mma<KB, VB, 8>(a, plan, parts, counters, st);
     KVQ_MMA_CASE(4, 4) KVQ_MMA_CASE(4, 2) KVQ_MMA_CASE(4, 1)
     KVQ_MMA_CASE(3, 4) KVQ_MMA_CASE(3, 2) KVQ_MMA_CASE(3, 1)
     KVQ_MMA_CASE(2, 4) KVQ_MMA_CASE(2, 2) KVQ_MMA_CASE(2, 1)
@@ -831,9 +831,8 @@ int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &given, float 
 
 // Plan of the tensor-core kernel for B * nh query heads (one head per segment).
 AttnPlan plan_attn_mma(int T, int k_bits, long long heads) {
-    // score buffers that leave room for two CTAs per SM
-    return k_bits == 3 ? make_attn_plan(T, 352, KGeom<3>::WT, 7040, heads, kNarrowScores)
-                       : make_attn_plan(T, 256, KGeom<4>::WT, 6144, heads, kNarrowScores);
+    return k_bits == 3 ? make_attn_plan_mma(T, 352, KGeom<3>::WT, kWideScores3, heads, kNarrowMax3, kNarrowScores, 1760)
+                       : make_attn_plan_mma(T, 256, KGeom<4>::WT, kWideScores, heads, kNarrowMax, kNarrowScores, 3072);
 }
 
 }  // namespace kvq

@@ -130,7 +130,12 @@ def test_split_plan_invariants_and_workspace_bound():
                     groups = heads // p.heads_per_cta
                     assert p.unit == (352 if kb == 3 else 256) and p.units_per_head == -(-T // p.unit)
                     assert p.n_whole + p.n_cut == groups and p.n_ctas == p.n_whole + p.n_cut * p.segments
-                    slots, cap = (148 * 2, 2816 if kb == 3 else 2048) if grouped else (148 * 3, 8096 if kb == 3 else 8192)
+                    # grouped: two CTAs to an SM, 2048 / 2112 tokens of four heads; per head: 6144 / 7040 tokens in an eight-warp
+                    # CTA (all there is up to 148 heads), 8192 / 8096 in a four-warp one
+                    if grouped:
+                        slots, cap = 148 * 2, 2112 if kb == 3 else 2048
+                    else:
+                        slots, cap = 148, (7040 if kb == 3 else 6144) if groups <= 148 else (8096 if kb == 3 else 8192)
                     assert p.n_whole % slots == 0 and p.max_segment_tokens <= cap
                     assert (p.segments - 1) * p.segment_units < p.units_per_head <= p.segments * p.segment_units
                     if p.n_ctas <= 40000:                                    # walk the small and medium plans fully
@@ -163,3 +168,15 @@ def test_split_plan_prefers_one_split_for_full_grids():
     assert _plan(8, 32, 32768, 4, 1, nh_kv=8, G=32, vb=2).kernel == 1     # 2-bit values at group 32: one head per CTA
     with pytest.raises(Exception):
         _lib.check(_lib.lib().kvq_decode_attn_plan(None, 1, None))
+
+
+def test_split_plan_many_heads():
+    """More heads than eight-warp slots: whole ones in multiples of the SM count, the rest cut, also where a head only fits a
+    four-warp CTA's score buffer."""
+    for B, nh, T, kb, want in [(20, 32, 4096, 2, (592, 48)), (40, 32, 4096, 3, (1184, 96)), (14, 32, 4096, 4, (444, 4)),
+                               (28, 32, 7000, 2, (888, 8)), (48, 32, 8000, 4, (1480, 56)), (20, 32, 7000, 4, (444, 196))]:
+        p = _plan(B, nh, T, kb, 1)
+        assert (p.n_whole, p.n_cut) == want and p.segments > 1 and p.max_segment_tokens >= T
+    assert _plan(64, 32, 600, 2, 1).segments == 1             # 2048 short heads: one CTA each
+    assert _plan(10, 32, 8000, 2, 1).segments == 5            # between two and three an SM, three to an SM at a time: all cut
+    assert _plan(8, 32, 8000, 2, 1).segments == 4 and _plan(64, 32, 9000, 2, 1).max_segment_tokens <= 6144
