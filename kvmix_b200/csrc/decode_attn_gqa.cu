@@ -304,7 +304,6 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 
         // ---- epilogue: lane (g, tig) holds, per accumulator, row g / g + 8 of head tig as (hi, lo) ------------
         // row g = group g of the tile: its zero term for head tig (hi + lo columns)
-        
         float *dst_h = sm.scores + (split * kQH + tig) * sm.n_scores - t0;
         if constexpr (KB == 3) {
 #pragma unroll
@@ -769,8 +768,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     // q of the quad (head slots beyond qhv repeat the last head: their columns are computed and dropped)
     {
         const int slot = tid >> 6, hs = min(slot, qhv - 1);              // two warps store a head slot
-        const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + hs) * a.q_sH;
-        *reinterpret_cast<uint32_t *>(sm.q + slot * kHeadDim + 2 * (tid & 63)) = *reinterpret_cast<const uint32_t *>(q + 2 * (tid & 63));
+        const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + hs) * a.q_sH + 2 * (tid & 63);
+        *reinterpret_cast<__half2 *>(sm.q + slot * kHeadDim + 2 * (tid & 63)) = __halves2half2(q[0], q[1]);   // q rows start at any fp16
     }
 
     // ---- 1. scores ------------------------------------------------------------------------------
