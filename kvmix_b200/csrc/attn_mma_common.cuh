@@ -32,7 +32,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // ---------------------------------------------------------------------------------------------
-// Field extraction.  unpack(wa, wb, r): r[i] = fp16x2 { field i of wa (low), field i of wb (high) }
+// Field extraction from words (3- and 4-bit keys).  unpack(wa, wb, r): r[i] = fp16x2 { field i of wa (low), field i of wb (high) }
 // left at bit position pos(i) inside each 16-bit half, i.e. the subnormal pair
 // { f_a * 2^(pos-24), f_b * 2^(pos-24) }.  inv_scale(i) = 2^(24-pos(i)).
 template <int BITS> struct Fields;
@@ -45,35 +45,6 @@ template <> struct Fields<4> {
         const uint32_t los = lo >> 8, his = hi >> 8;
         r[0] = lo & 0x000f000fu; r[1] = lo & 0x00f000f0u; r[2] = los & 0x000f000fu; r[3] = los & 0x00f000f0u;
         r[4] = hi & 0x000f000fu; r[5] = hi & 0x00f000f0u; r[6] = his & 0x000f000fu; r[7] = his & 0x00f000f0u;
-    }
-};
-
-template <> struct Fields<2> {
-    static constexpr int N = 16;
-    __device__ static __forceinline__ int pos(int i) { const int t = i & 7; return t < 5 ? 2 * t : 2 * (t - 5); }
-    __device__ static __forceinline__ void unpack(uint32_t wa, uint32_t wb, uint32_t (&r)[16]) {
-        const uint32_t lo = prmt(wa, wb, 0x5410), hi = prmt(wa, wb, 0x7632);
-        const uint32_t los = lo >> 10, his = hi >> 10;
-#pragma unroll
-        for (int t = 0; t < 5; ++t) { r[t] = lo & (0x00030003u << (2 * t)); r[8 + t] = hi & (0x00030003u << (2 * t)); }
-#pragma unroll
-        for (int t = 5; t < 8; ++t) {
-            r[t] = los & (0x00030003u << (2 * (t - 5)));
-            r[8 + t] = his & (0x00030003u << (2 * (t - 5)));
-        }
-    }
-};
-
-template <> struct Fields<1> {
-    static constexpr int N = 32;
-    __device__ static __forceinline__ int pos(int i) { const int t = i & 15; return t < 10 ? t : t - 10; }
-    __device__ static __forceinline__ void unpack(uint32_t wa, uint32_t wb, uint32_t (&r)[32]) {
-        const uint32_t lo = prmt(wa, wb, 0x5410), hi = prmt(wa, wb, 0x7632);
-        const uint32_t los = lo >> 10, his = hi >> 10;
-#pragma unroll
-        for (int t = 0; t < 10; ++t) { r[t] = lo & (0x00010001u << t); r[16 + t] = hi & (0x00010001u << t); }
-#pragma unroll
-        for (int t = 10; t < 16; ++t) { r[t] = los & (0x00010001u << (t - 10)); r[16 + t] = his & (0x00010001u << (t - 10)); }
     }
 };
 
@@ -96,60 +67,15 @@ template <> struct Fields<3> {
     }
 };
 
-// Value-side field extraction: same contract as Fields, but every field is moved to bit position >= 4 (>= 2
-// for 4-bit codes) of its 16-bit half.  The tensor core aligns the 16 products of an MMA (and the accumulator) to
-// the largest operand EXPONENT and truncates what falls about 26 bits below it; a subnormal's exponent is fixed at
-// -14 however small its value, so a code parked in the lowest mantissa bits loses low product bits whenever a
-// neighbouring token's probability is larger.  The loss is always downwards, so over a long, diffuse softmax it
-// adds up to a bias (2e-5 of the non-negative code sum for 2-bit codes at position 0, a quarter of that per two
-// positions higher) which the centring of the codes amplifies.  Two more shifts per word pair keep it below the
-// fp32 accumulation error.
-template <int BITS> struct VFields;
-
-template <> struct VFields<4> {
-    static constexpr int N = 8;
-    __device__ static __forceinline__ int pos(int i) { return (i & 1) ? 6 : 2; }
-    __device__ static __forceinline__ void unpack(uint32_t wa, uint32_t wb, uint32_t (&r)[8]) {
-        const uint32_t lo = prmt(wa, wb, 0x5410), hi = prmt(wa, wb, 0x7632);
-        const uint32_t lou = lo << 2, lod = lo >> 6, hiu = hi << 2, hid = hi >> 6;
-        r[0] = lou & 0x003c003cu; r[1] = lou & 0x03c003c0u; r[2] = lod & 0x003c003cu; r[3] = lod & 0x03c003c0u;
-        r[4] = hiu & 0x003c003cu; r[5] = hiu & 0x03c003c0u; r[6] = hid & 0x003c003cu; r[7] = hid & 0x03c003c0u;
-    }
-};
-
-template <> struct VFields<2> {
-    static constexpr int N = 16;
-    __device__ static __forceinline__ int pos(int i) { const int t = i & 7; return t < 2 ? 6 + 2 * t : t < 5 ? 2 * t : 2 * t - 6; }
-    __device__ static __forceinline__ void unpack(uint32_t wa, uint32_t wb, uint32_t (&r)[16]) {
-        const uint32_t lo = prmt(wa, wb, 0x5410), hi = prmt(wa, wb, 0x7632);
-        const uint32_t lou = lo << 6, lod = lo >> 6, hiu = hi << 6, hid = hi >> 6;
-#pragma unroll
-        for (int t = 0; t < 2; ++t) { r[t] = lou & (0x00030003u << (6 + 2 * t)); r[8 + t] = hiu & (0x00030003u << (6 + 2 * t)); }
-#pragma unroll
-        for (int t = 2; t < 5; ++t) { r[t] = lo & (0x00030003u << (2 * t)); r[8 + t] = hi & (0x00030003u << (2 * t)); }
-#pragma unroll
-        for (int t = 5; t < 8; ++t) { r[t] = lod & (0x00030003u << (2 * t - 6)); r[8 + t] = hid & (0x00030003u << (2 * t - 6)); }
-    }
-};
-
-template <> struct VFields<1> {
-    static constexpr int N = 32;
-    __device__ static __forceinline__ int pos(int i) { const int t = i & 15; return t < 4 ? t + 6 : t < 10 ? t : t - 6; }
-    __device__ static __forceinline__ void unpack(uint32_t wa, uint32_t wb, uint32_t (&r)[32]) {
-        const uint32_t lo = prmt(wa, wb, 0x5410), hi = prmt(wa, wb, 0x7632);
-        const uint32_t lou = lo << 6, lod = lo >> 6, hiu = hi << 6, hid = hi >> 6;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) { r[t] = lou & (0x00010001u << (t + 6)); r[16 + t] = hiu & (0x00010001u << (t + 6)); }
-#pragma unroll
-        for (int t = 4; t < 10; ++t) { r[t] = lo & (0x00010001u << t); r[16 + t] = hi & (0x00010001u << t); }
-#pragma unroll
-        for (int t = 10; t < 16; ++t) { r[t] = lod & (0x00010001u << (t - 6)); r[16 + t] = hid & (0x00010001u << (t - 6)); }
-    }
-};
-
 // Extraction from ONE register that already pairs two 16-bit half-words along the contraction axis (as
-// a transposing ldmatrix delivers them: two tokens of values, two channels of keys): r[i] = fp16x2 of field i of both half-words, i < 16 / BITS, each left at
-// bit position pos(i) >= 4 (>= 2 for 4-bit codes) of its half -- the positions VFields uses, for the same reason.
+// a transposing ldmatrix delivers them: two tokens of values, two channels of keys): r[i] = fp16x2 of field i of both
+// half-words, i < 16 / BITS, each moved to bit position pos(i) >= 4 (>= 2 for 4-bit codes) of its half.  The tensor core aligns
+// the 16 products of an MMA (and the accumulator) to the largest operand EXPONENT and truncates what falls about 26 bits below
+// it; a subnormal's exponent is fixed at -14 however small its value, so a code parked in the lowest mantissa bits loses
+// low product bits whenever a neighbouring token's probability is larger.  The loss is always downwards, so over a long,
+// diffuse softmax it adds up to a bias (2e-5 of the non-negative code sum for 2-bit codes at position 0, a quarter of that
+// per two positions higher) which the centring of the codes amplifies.  Two more shifts per register keep it below the
+// fp32 accumulation error.
 template <int BITS> struct VHalf;     // 3-bit words do not split into half-words
 template <> struct VHalf<4> {
     static constexpr int N = 4;

@@ -102,7 +102,6 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                                               int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
     using R = GqaKRing<KB>;
-    using F = Fields<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int Gk = a.k_group;
     const int n_words = a.Tkq / G::FPI;
