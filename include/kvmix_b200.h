@@ -209,7 +209,8 @@ int kvq_prefill(const kvq_prefill_args *a, kvq_stream_t stream);
  * :7-124), reading the caller's layout directly (upstream first transposes codes, scales and
  * zeros on every call, :151-171):
  *   out[b,h,n] = fp16( sum_k fA[b,h,k] * (scale[b,hk,k,n/group] * code[b,hk,k,n] + zero[b,hk,k,n/group]) )
- *   hk = h / (nh / nh_kv), fp32 accumulation.
+ *   hk = h / (nh / nh_kv), fp32 accumulation.  1, 2 and 4 bits at groups of 32, 64 and 128 run on the tensor cores, fA * scale
+ *   carried as an fp16 pair scaled so that it holds the fp32 product; infinities and NaN propagate as in fp32.
  *   fA    [B, nh, K] fp16                 strides a_sB, a_sH, K contiguous
  *   qB    [B, nh_kv, K, n_words] int32    strides q_sB, q_sH, q_sK (words)
  *   scale [B, nh_kv, K, n_groups] fp16    strides s_sB, s_sH, s_sK; zeros alike
@@ -251,16 +252,20 @@ int kvq_gemv(const kvq_gemv_args *a, kvq_stream_t stream);
  *   vcode  [B, nh_kv, Tvq, D/fpi_v]     strides vc_sB, vc_sH, vc_sT (words)
  *   vscale, vmn [B, nh_kv, Tvq, D/v_group] fp16, strides vs_sB, vs_sH, vs_sT
  *   vfull  [B, nh_kv, vf_cap, D] fp16   strides vf_sB, vf_sH, vf_sT, ring like kfull
- * Two kernels serve the call.  The tensor-core kernel takes D = 128, k_group in {32, 64, 128} (11 for 3-bit keys),
- * v_group in {32, 64, 128}, Tvq a multiple of 32, nh a multiple of nh_kv, every packed tensor and fp16 tail 16-byte
- * aligned with row strides that keep rows 16-byte aligned (kc_sD % 4, ks_sD % 8, kf_sT % 8, vf_sT % 8 == 0; value
- * rows contiguous: vc_sT == D/fpi_v, vs_sT == D/v_group) -- what a preallocated cache provides.  Anything else runs
- * on a slower CUDA-core kernel with the same results.
+ * Three kernels serve the call (kvq_decode_attn_plan says which).  The two tensor-core kernels take D = 128, k_group in
+ * {32, 64, 128} (11 for 3-bit keys), v_group in {32, 64, 128}, Tvq a multiple of 32, nh a multiple of nh_kv, every packed
+ * tensor and fp16 tail 16-byte aligned with row strides that keep rows 16-byte aligned (kc_sD % 4, ks_sD % 8, kf_sT % 8,
+ * vf_sT % 8 == 0; value rows contiguous: vc_sT == D/fpi_v, vs_sT == D/v_group) and key rows less than 2^22 words (2^23
+ * groups) apart -- what a preallocated cache provides.  One of them serves the query heads of a kv head together: nh/nh_kv
+ * 2 or a multiple of 4, k_group 128 at 1 bit, >= 64 at 2 and 4 bits, any for 3-bit keys, v_group >= 64 at 1 and 2 bits.
+ * Anything else runs on a slower CUDA-core kernel with the same results.  q and out may start at any fp16.
  * D must be 128.  k_group and v_group must be multiples of the fields per word (k_group == 11 for
  * 3-bit keys).  3-bit values (v_bits == 3, v_group == 11) are an extension without an upstream counterpart --
  * upstream needs D % 11 == 0 for them (quant_cuda/csrc/quantization_cuda.cu:433-434) -- in the layout
  * kvq_quant_lastdim writes with ragged_tail: vcode [B, nh_kv, Tvq, 12], vscale / vmn [B, nh_kv, Tvq, 12], word j
- * holding channels 11j .. min(11j + 10, 127) as its own group; they run on the CUDA-core kernel.
+ * holding channels 11j .. min(11j + 10, 127) as its own group.  They run on the tensor cores where the query heads of a kv
+ * head are served together (value rows of 12 words and 12 groups, the other conditions as above), else on the CUDA-core
+ * kernel; the fused decode step, device-resident state and the exchange do not take them.
  * round_scores != 0 narrows each raw score to fp16 before scaling, as upstream's GEMV and fp16
  * matmul do; everything else accumulates in fp32.
  *
