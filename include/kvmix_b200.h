@@ -255,7 +255,7 @@ int kvq_gemv(const kvq_gemv_args *a, kvq_stream_t stream);
  * Three kernels serve the call (kvq_decode_attn_plan says which).  The two tensor-core kernels take D = 128, k_group in
  * {32, 64, 128} (11 for 3-bit keys), v_group in {32, 64, 128}, Tvq a multiple of 32, nh a multiple of nh_kv, every packed
  * tensor and fp16 tail 16-byte aligned with row strides that keep rows 16-byte aligned (kc_sD % 4, ks_sD % 8, kf_sT % 8,
- * vf_sT % 8 == 0; value rows contiguous: vc_sT == D/fpi_v, vs_sT == D/v_group) and key rows less than 2^22 words (2^23
+ * vf_sT % 8 == 0; value rows contiguous: vc_sT == D/fpi_v, vs_sT == D/v_group) and key rows less than 2^23 words (2^24
  * groups) apart -- what a preallocated cache provides.  One of them serves the query heads of a kv head together: nh/nh_kv
  * 2 or a multiple of 4, k_group 128 at 1 bit, >= 64 at 2 and 4 bits, any for 3-bit keys, v_group >= 64 at 1 and 2 bits.
  * Anything else runs on a slower CUDA-core kernel with the same results.  q and out may start at any fp16.

@@ -957,11 +957,15 @@ AttnPlan plan_attn_gqa(int T, int k_bits, long long head_groups) {
                        : make_attn_plan(T, 256, KGeom<4>::WT, kGqaMaxScores, head_groups);
 }
 
+template <int KB, int VB> constexpr int gqa_smem_bytes(int scores) {
+    return kQH * scores * 4 + kMmaWarps * gqa_region_bytes<KB, VB>() + kQH * kHeadDim * 2 + 64 * 4;
+}
+
 template <int KB, int VB>
 static int launch_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, float *parts, unsigned int *counters,
                       cudaStream_t st) {
-    const size_t smem = ((size_t)kQH * plan.n_scores << plan.ks_log2) * 4 + (size_t)kMmaWarps * gqa_region_bytes<KB, VB>() +
-                        kQH * kHeadDim * 2 + 64 * 4;
+    static_assert(gqa_smem_bytes<KB, VB>(KB == 3 ? kGqaMaxScores3 : kGqaMaxScores) <= kMmaSmemMax, "two CTAs to an SM");
+    const size_t smem = gqa_smem_bytes<KB, VB>(plan.n_scores << plan.ks_log2);
     static bool attr_set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);

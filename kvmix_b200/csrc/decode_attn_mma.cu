@@ -773,8 +773,8 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     if (a.Tkq > 0) {
         if (!al16(a.kcode) || a.kc_sB % 4 || a.kc_sH % 4 || a.kc_sD % 4) return false;
         if (!al16(a.kscale) || !al16(a.kmn) || a.ks_sB % 8 || a.ks_sH % 8 || a.ks_sD % 8) return false;
-        // a head's keys are addressed by 32-bit byte offsets (128 rows)
-        if (a.kc_sD < 0 || a.kc_sD >= (1 << 22) || a.ks_sD < 0 || a.ks_sD >= (1 << 23)) return false;
+        // a head's keys are addressed by 32-bit byte offsets, unsigned (128 rows of 4-byte words, of 2-byte scales)
+        if (a.kc_sD < 0 || a.kc_sD >= (1 << 23) || a.ks_sD < 0 || a.ks_sD >= (1 << 24)) return false;
     }
     if (a.Tvq > 0) {
         const int fv = fields_per_word(a.v_bits);              // rows back to back (3 bits: 12 words and groups a token)

@@ -180,3 +180,16 @@ def test_split_plan_many_heads():
     assert _plan(64, 32, 600, 2, 1).segments == 1             # 2048 short heads: one CTA each
     assert _plan(10, 32, 8000, 2, 1).segments == 5            # between two and three an SM, three to an SM at a time: all cut
     assert _plan(8, 32, 8000, 2, 1).segments == 4 and _plan(64, 32, 9000, 2, 1).max_segment_tokens <= 6144
+
+
+def test_wide_key_rows_keep_their_kernel():
+    """Keys are addressed by unsigned 32-bit byte offsets within a head: 128 rows of up to 2^23 words reach just below 2^32."""
+    for words, groups, kernel in [(1 << 20, 1 << 20, 1), ((1 << 23) - 4, 1 << 20, 1), (1 << 23, 1 << 20, 0), (1 << 20, (1 << 24) - 8, 1), (1 << 20, 1 << 24, 0)]:
+        a = _lib.AttnArgs()
+        a.B, a.nh, a.nh_kv, a.D, a.T, a.Tkq, a.Tvq = 1, 1, 1, 128, 4096, 4096, 4096
+        a.k_bits, a.k_group, a.v_bits, a.v_group = 2, 32, 2, 32
+        a.kcode = a.kscale = a.kmn = a.vcode = a.vscale = a.vmn = 1 << 20
+        a.kc_sD, a.ks_sD, a.vc_sT, a.vs_sT = words, groups, 8, 4
+        p = _lib.AttnPlan()
+        assert _lib.lib().kvq_decode_attn_plan(ctypes.byref(a), -1, ctypes.byref(p)) == 0
+        assert p.kernel == kernel, (words, groups)
