@@ -54,59 +54,62 @@ __device__ __forceinline__ float max_abs(float t, float x, float y) {
 // range.  The word is summed in two fp32 chunks of <= 17 bits (exact) and converted once.  If any element is near
 // a tie or not finite (constant group: 0 * inf), the word is put together element by element and only the elements in
 // question are divided: fp16 data tie often enough that some lane of every eighth warp gets here, and dividing for all
-// elements of the word was a fifth of the quantizers' instructions.
+// elements of the word was a fifth of the quantizers' instructions (1, 2 and 4 bits).
 // Elements go in pairs (f32x2), the tie test is one three-input maximum a pair.  16 x 32 x 8192 x 128 fp16:
-// keys (2 bits, groups of 32 tokens) 353 -> 314 us, values (4 bits, groups of 32) 314 -> 298 us.
+// keys (2 bits, groups of 32 tokens) 348 -> 310 us, values (4 bits, groups of 32) 309 -> 296 us.
+// 3-bit words are worked one element at a time and divided whole: eleven fields in two chunks split badly into pairs, and
+// their lone word a group leaves too little between two tie tests (keys 457 us in pairs with single divisions, 426 us so;
+// contiguous groups 464 and 436 us).
 template <int BITS, typename Get>
 __device__ __forceinline__ uint32_t quant_word(Get get, float lo, float sc, float rinv) {
     constexpr int E = fields_per_word(BITS);
     constexpr int QMAX = (1 << BITS) - 1;
-    constexpr int NLO = (BITS == 3) ? 5 : E / 2;               // fields in the low chunk
-    constexpr int HI_SHIFT = (BITS == 3) ? 15 : BITS * NLO;
     constexpr float kMagic = 12582912.0f;
-    const unsigned long long nlo2 = f32x2(-lo, -lo), rinv2 = f32x2(rinv, rinv), magic2 = f32x2(kMagic, kMagic), minus2 = f32x2(-1.f, -1.f);
-    unsigned long long wl2 = 0ull, wh2 = 0ull;                 // { 0.f, 0.f }
-    float worst = 0.f;
-    // weight of field i in its chunk; pairs (i, i + 1) lie in one chunk but for the 3-bit word's odd low one
-    auto weight = [](int i) -> float {
-        if (BITS == 3) return i < 5 ? (float)(1 << (3 * i)) : i < 10 ? (float)(1 << (3 * (i - 5))) : 32768.f;
-        return (float)(1 << (BITS * (i < NLO ? i : i - NLO)));
-    };
+    if constexpr (BITS == 3) {
+        float wl = 0.f, wh = 0.f, worst = 0.f;
 #pragma unroll
-    for (int i = 0; i + 1 < E; i += 2) {
-        const unsigned long long a = add_f32x2(f32x2(get(i), get(i + 1)), nlo2);
-        const unsigned long long m = fma_f32x2(a, rinv2, magic2);
-        unsigned long long ny = fma_f32x2(m, minus2, magic2);
-        const float2 e = f32x2_split(fma_f32x2(a, rinv2, ny));
-        worst = max_abs(worst, e.x, e.y);
-        if (BITS == 3 && i == 4) {                             // field 4 in the low chunk, 5 in the high one
-            wl2 = fma_f32x2(ny, f32x2(-weight(4), 0.f), wl2);
-            wh2 = fma_f32x2(ny, f32x2(0.f, -weight(5)), wh2);
-        } else if (i < NLO) {
-            wl2 = fma_f32x2(ny, f32x2(-weight(i), -weight(i + 1)), wl2);
-        } else {
-            wh2 = fma_f32x2(ny, f32x2(-weight(i), -weight(i + 1)), wh2);
+        for (int i = 0; i < E; ++i) {
+            const float a = get(i) - lo, m = fmaf(a, rinv, kMagic);
+            float yr = m - kMagic;
+            const float e = fmaf(a, rinv, -yr);
+            worst = max_abs(worst, e, e);
+            if (i == 10) yr = fminf(yr, 3.f);                  // the 11th code of a 3-bit group has two bits
+            if (i < 5) wl = fmaf(yr, (float)(1 << (3 * i)), wl);
+            else wh = fmaf(yr, (float)(1 << (i < 10 ? 3 * (i - 5) : 15)), wh);
         }
-    }
-    const float2 l2 = f32x2_split(wl2), h2 = f32x2_split(wh2);
-    const float wl = l2.x + l2.y;
-    float wh = h2.x + h2.y;
-    if constexpr (BITS == 3) {                                 // the 11th code of a 3-bit group has two bits
-        const float a = get(10) - lo, m = fmaf(a, rinv, kMagic), yr = m - kMagic, e = fmaf(a, rinv, -yr);
-        worst = max_abs(worst, e, e);
-        wh = fmaf(fminf(yr, 3.f), 32768.f, wh);
-    }
-    if (worst <= 0.49999f) return __float2uint_rz(wl) | (__float2uint_rz(wh) << HI_SHIFT);
-    uint32_t word = 0;
+        if (worst <= 0.49999f) return __float2uint_rz(wl) | (__float2uint_rz(wh) << 15);
+        uint32_t word = 0;
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-        const float a = get(i) - lo, m = fmaf(a, rinv, kMagic), e = fmaf(a, rinv, kMagic - m);
-        const int emax = (BITS == 3 && i == 10) ? 3 : QMAX;
-        int q = min((int)(__float_as_uint(m) & 31u), emax);    // the integer sits in the low mantissa bits
-        if (!(fabsf(e) <= 0.49999f)) q = round_code(a / sc, emax);
-        word |= (uint32_t)q << (BITS == 3 ? (i < 10 ? 3 * i : 30) : BITS * i);
+        for (int i = 0; i < E; ++i) word |= (uint32_t)round_code((get(i) - lo) / sc, i < 10 ? 7 : 3) << (i < 10 ? 3 * i : 30);
+        return word;
+    } else {
+        constexpr int NLO = E / 2;                             // fields in the low chunk
+        const unsigned long long nlo2 = f32x2(-lo, -lo), rinv2 = f32x2(rinv, rinv), magic2 = f32x2(kMagic, kMagic), minus2 = f32x2(-1.f, -1.f);
+        unsigned long long wl2 = 0ull, wh2 = 0ull;             // { 0.f, 0.f }
+        float worst = 0.f;
+        auto weight = [](int i) -> float { return (float)(1 << (BITS * (i < NLO ? i : i - NLO))); };   // of field i in its chunk
+#pragma unroll
+        for (int i = 0; i < E; i += 2) {
+            const unsigned long long a = add_f32x2(f32x2(get(i), get(i + 1)), nlo2);
+            const unsigned long long m = fma_f32x2(a, rinv2, magic2);
+            const unsigned long long ny = fma_f32x2(m, minus2, magic2);
+            const float2 e = f32x2_split(fma_f32x2(a, rinv2, ny));
+            worst = max_abs(worst, e.x, e.y);
+            if (i < NLO) wl2 = fma_f32x2(ny, f32x2(-weight(i), -weight(i + 1)), wl2);
+            else wh2 = fma_f32x2(ny, f32x2(-weight(i), -weight(i + 1)), wh2);
+        }
+        const float2 l2 = f32x2_split(wl2), h2 = f32x2_split(wh2);
+        if (worst <= 0.49999f) return __float2uint_rz(l2.x + l2.y) | (__float2uint_rz(h2.x + h2.y) << (BITS * NLO));
+        uint32_t word = 0;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const float a = get(i) - lo, m = fmaf(a, rinv, kMagic), e = fmaf(a, rinv, kMagic - m);
+            int q = min((int)(__float_as_uint(m) & 31u), QMAX);    // the integer sits in the low mantissa bits
+            if (!(fabsf(e) <= 0.49999f)) q = round_code(a / sc, QMAX);
+            word |= (uint32_t)q << (BITS * i);
+        }
+        return word;
     }
-    return word;
 }
 
 template <int QMAX>
