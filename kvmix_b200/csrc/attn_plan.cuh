@@ -68,6 +68,7 @@ inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; 
 // Pieces a head is cut into where `heads` of them (fewer than SMs) are left behind whole ones: the SM that gets most of the pieces
 // finishes last; a piece costs its tokens and some 600 more, one whole head by itself on its SM `lone` percent of that.
 inline int plan_left_pieces(int T, int unit, int heads, int lone) {
+    if (heads == 0) return 1;
     const int uph = (T + unit - 1) / unit;
     int best_k = 1;
     long long best = (T + 600) * (long long)lone / 100;
@@ -123,14 +124,14 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
 
 // The kernel with one query head per CTA, which also comes with four warps per CTA.  narrow_max: most tokens of a segment of those (a
 // multiple of the unit); narrow_split: scores that leave room for four of them on an SM; wide_from: tokens from which eight warps
-// a CTA pay up to seven heads an SM.
+// a CTA pay up to six and a half heads an SM.
 //
 // More heads than eight-warp slots: the multiple of the SM count whole, the others cut (us on B200, whole heads in multiples of 888
 // and eight warps for all that is cut -> this; 4096 tokens: 448 heads 2 bits 78 -> 70, 640 heads 99 -> 91, 1280 heads 173 ->
 // 150, 3-bit keys 1536 heads 260 -> 233; 7000 tokens, 4 bits: 896 heads 235 -> 208, 2048 heads 488 -> 444).  What a CTA does once
 // (addresses, ring fill, tails, sums: 20k of the 72k warp instructions of a head of 4096 tokens) is done by half as many warps
 // in the four-warp form, so it is the better one where there are many CTAs or short ones: 300 tokens 0.76 .. 0.9 of the eight-warp
-// form's time, 2000 tokens 0.9 .. 1.0; at 4096 tokens 320 and 448 heads take 1.10 .. 1.16 of it, 1280 heads 0.92.
+// form's time, 2000 tokens 0.9 .. 1.0; at 4096 tokens 320 and 448 heads take 1.10 .. 1.16 of it, 1024 heads 0.95 .. 0.98, 1280 heads 0.92.
 inline AttnPlan make_attn_plan_mma(int T, int unit, int tile, int max_scores, long long heads, int narrow_max, int narrow_split, int wide_from) {
     const int wide_max = max_scores / unit * unit;
     const bool many = heads > kPlanSlots;
@@ -141,7 +142,7 @@ inline AttnPlan make_attn_plan_mma(int T, int unit, int tile, int max_scores, lo
     AttnPlan p;
     p.unit = unit;
     p.uph = (T + unit - 1) / unit;
-    p.warps = many && T >= wide_from && T <= wide_max && heads < 7 * kSmCount ? 8 : 4;
+    p.warps = many && T >= wide_from && T <= wide_max && 2 * heads <= 13 * kSmCount ? 8 : 4;
     // long heads are three to an SM: two or four an SM whole would leave it with one or two for most of the time (592 heads of 8000
     // tokens, 2 bits: 166 us whole, 143 us as 444 and 148 cut; 320 heads 107 and 86 us all cut in five)
     const bool three = T > wide_max;

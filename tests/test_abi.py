@@ -178,6 +178,7 @@ def test_split_plan_many_heads():
         p = _plan(B, nh, T, kb, 1)
         assert (p.n_whole, p.n_cut) == want and p.segments > 1 and p.max_segment_tokens >= T
     assert _plan(64, 32, 600, 2, 1).segments == 1             # 2048 short heads: one CTA each
+    assert _plan(37, 32, 4096, 2, 1).segments == 1            # 1184 = 8 x 148: nothing is left to cut
     assert _plan(10, 32, 8000, 2, 1).segments == 5            # between two and three an SM, three to an SM at a time: all cut
     assert _plan(8, 32, 8000, 2, 1).segments == 4 and _plan(64, 32, 9000, 2, 1).max_segment_tokens <= 6144
 
