@@ -28,17 +28,18 @@ def features_per_int(bits):
     return 11 if bits == 3 else 32 // bits
 
 
-# torch.cuda.current_stream() builds a Stream object: 3.3 us a call, a sixth of the host time of a one-layer decode step.  Torch's own
-# raw handle takes 0.15 us; these two functions are not part of its documented interface, so a torch without them takes the
-# documented way.
-_raw_stream, _device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+def _stream_getter(c):
+    """A function that returns the current stream of the current device as an integer.  torch.cuda.current_stream() builds
+    a Stream object: 3.3 us a call, a sixth of the host time of a one-layer decode step.  Torch's own raw handle takes
+    0.15 us; its two functions (in `c`) are not part of the documented interface, so a torch without them is asked the
+    documented way."""
+    stream, device = getattr(c, "_cuda_getCurrentRawStream", None), getattr(c, "_cuda_getDevice", None)
+    if stream is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: stream(device())
 
 
-def raw_stream():
-    """The current stream of the current device as an integer."""
-    if _raw_stream is None or _device is None:
-        return torch.cuda.current_stream().cuda_stream
-    return _raw_stream(_device())
+raw_stream = _stream_getter(torch._C)
 
 
 def _need_cuda(*ts):
