@@ -15,6 +15,11 @@
 //           except 1-bit values at group 64, where a block spans two groups and every code tile is multiplied by both
 //           groups' operands, each lane keeping the product of the group its rows belong to).
 // Scores of the four heads sit side by side in shared memory ([4][n]); two warps run the softmax of a head.
+//
+// Bound by the instruction stream around the codes (issue about half busy, the half-rate logic pipe as much), so the loops know their
+// group sizes: conditions on them cost a compare, a branch or a select per group and k-step.  Warp instructions per 32 codes, 2-bit
+// keys and values, group 64: 2.98 with the group sizes looked up, 2.34 so (0.63 of it the isolation of the fields, 0.14 MMAs);
+// 8 x 8 kv heads of 32768 tokens, group 64: 88.7 -> 78.2 us, 4-bit 101.5 -> 87.8, 3-bit keys with 4-bit values 156.3 -> 129.7.
 #include "attn_mma_common.cuh"
 #include "attn_plan.cuh"
 #include "attn_update.cuh"
@@ -96,14 +101,14 @@ __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same stage geometry, tile order and channel
 // splits as the single-head kernel; scores[split][h][t - t0] receive the raw scores.
-template <int KB>
+template <int KB, bool WIDE>
 __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const GqaSmem &sm, int t0, int hi, const __half *kf,
                                               int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
     using R = GqaKRing<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int Gk = a.k_group;
+    constexpr int LGK = WIDE ? 7 : 6, NGW = KB == 3 ? 8 : G::WT >> LGK;         // groups of a tile: 8 (3 bits) / 2 / 4
     const int n_words = a.Tkq / G::FPI;
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;                         // <= 0: no packed keys in this segment
     const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = kMmaWarps >> sm.ks_log2;
@@ -125,10 +130,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
     const uint32_t szm_s = ring_s + G::CODE_BYTES + (KB == 3 ? ZOFF : 0) + (lane & 15) * 16;   // zero tile as an A operand
     const uint32_t q_s = smem_u32(sm.q) + (g >> 1) * (kHeadDim * 2) + (ch0 + 2 * tig) * 2;     // this column's head; + 32 per k-step [+16]
     const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;
-    const int ngw = (G::WT + Gk - 1) / Gk;                                     // groups per warp tile: 8 (3-bit) / 4 / 2
-    const bool wide = Gk >= 128;                                               // 128-token groups (else 64)
     const int tile_words = tile_lanes * G::WT / G::FPI;
-    const int tile_groups = tile_lanes * G::WT / Gk;
+    const int tile_groups = tile_lanes * NGW;
     // 3-bit keys: field g of a word sits at bits 3g..3g+2; one byte permute brings the two bytes that hold it (of both
     // channel words) into the 16-bit halves, a mask isolates it in place at bit p0 = 3g mod 8 (<= 7: linear fp16 range).
     // Fields 8..10 (rows g + 8, g < 3) sit in byte 3 at bits 0, 3, 6 (the last one 2 bits wide).
@@ -146,7 +149,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
     constexpr bool kOneSz = G::ROWS == 16;
     const int sz_row = kOneSz ? (lane & 15) : lane;
     const bool sz_zero = kOneSz && lane >= 16;
-    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk);
+    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (KB == 3 ? (t0 + wt * G::WT) / 11 : (t0 + wt * G::WT) >> LGK));
     const char *sz_b = reinterpret_cast<const char *>(sz_zero ? kz : ks);
     const uint32_t szcp_dst = ring_s + G::CODE_BYTES + sz_row * 16 + (sz_zero ? ZOFF : 0);
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
@@ -166,7 +169,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
             }
             const uint32_t d = szcp_dst + iss_slot;
             if (KB == 3) { cp_async<16>(d, sz_b + iss_s); cp_async<16>(d + ZOFF, kz_b + iss_s); }
-            else if (ngw == 4) { cp_async<8>(d, sz_b + iss_s); if (!kOneSz) cp_async<8>(d + ZOFF, kz_b + iss_s); }
+            else if (NGW == 4) { cp_async<8>(d, sz_b + iss_s); if (!kOneSz) cp_async<8>(d + ZOFF, kz_b + iss_s); }
             else { cp_async<4>(d, sz_b + iss_s); if (!kOneSz) cp_async<4>(d + ZOFF, kz_b + iss_s); }
         }
         cp_async_commit();
@@ -191,9 +194,8 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
     for (int j = 0; j < my_tiles; ++j) {
         const int tile0 = t0 + (j * tile_lanes + wt) * G::WT;
         uint32_t q_cur = q_s;
-        // groups of this tile that hold tokens below hi: operands of the others are never formed (their scale/zero
-        // words lie beyond the packed prefix and may hold anything, and 0 * NaN would poison a shared accumulator)
-        const int nvg = min(ngw, (hi - tile0 + Gk - 1) / Gk);
+        // A group behind the packed prefix (its scale and zero words may hold anything) spoils the accumulators of its own
+        // tokens and its own row of the zero terms, which nothing reads: all groups are formed, without a condition.
         float acc[NACC][4], zsum = 0.f;
 #pragma unroll
         for (int m = 0; m < NACC; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
@@ -237,7 +239,6 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int jw = 2 * jp + u;
-                            if (jw >= nvg) continue;
                             const uint32_t psel = u ? 0x7632u : 0x5410u;
                             const __half2 s01 = as_h2(prmt(sA, sB, psel)), s89 = as_h2(prmt(sC, sD, psel));
                             const uint32_t a_lo = u ? wA.y : wA.x, b_lo = u ? wB.y : wB.x, a_hi = u ? wC.y : wC.x, b_hi = u ? wD.y : wD.x;
@@ -258,19 +259,22 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                                      : "=r"(za0), "=r"(za2) : "r"(szm_s + slot + 256 * k));
                         mma16816(accz, za0, 0u, za2, 0u, q01u & ~neg_mask, q89u & ~neg_mask);
                     }
-                    // B operands of the tile's groups (<= 4: k_group >= 64)
-                    const uint2 sA = lds64(zrow), sB = lds64(zrow + 16), sC = lds64(zrow + 128), sD = lds64(zrow + 144);
-                    uint32_t b[4][2];
+                    // B operands of the tile's groups: two of 128 tokens or four of 64
+                    constexpr int NB = KB == 3 ? 1 : NGW;
+                    uint2 sA, sB, sC, sD;
+                    if constexpr (WIDE) {
+                        sA.x = lds32(zrow); sB.x = lds32(zrow + 16); sC.x = lds32(zrow + 128); sD.x = lds32(zrow + 144);
+                        sA.y = sB.y = sC.y = sD.y = 0u;
+                    } else {
+                        sA = lds64(zrow); sB = lds64(zrow + 16); sC = lds64(zrow + 128); sD = lds64(zrow + 144);
+                    }
+                    uint32_t b[NB][2];
 #pragma unroll
-                    for (int jk = 0; jk < 4; ++jk) {
-                        if (jk < nvg) {
-                            const uint32_t psel = (jk & 1) ? 0x7632u : 0x5410u;
-                            const uint32_t a0 = (jk & 2) ? sA.y : sA.x, a1 = (jk & 2) ? sB.y : sB.x, a2 = (jk & 2) ? sC.y : sC.x, a3 = (jk & 2) ? sD.y : sD.x;
-                            b[jk][0] = hilo(q01, as_h2(prmt(a0, a1, psel)), neg_mask);
-                            b[jk][1] = hilo(q89, as_h2(prmt(a2, a3, psel)), neg_mask);
-                        } else {
-                            b[jk][0] = b[jk][1] = 0u;
-                        }
+                    for (int jk = 0; jk < NB; ++jk) {
+                        const uint32_t psel = (jk & 1) ? 0x7632u : 0x5410u;
+                        const uint32_t a0 = (jk & 2) ? sA.y : sA.x, a1 = (jk & 2) ? sB.y : sB.x, a2 = (jk & 2) ? sC.y : sC.x, a3 = (jk & 2) ? sD.y : sD.x;
+                        b[jk][0] = hilo(q01, as_h2(prmt(a0, a1, psel)), neg_mask);
+                        b[jk][1] = hilo(q89, as_h2(prmt(a2, a3, psel)), neg_mask);
                     }
                     using H = KHalf<KB>;
                     const uint32_t lsrc = ldk_s + stage_s + (k * 16) * G::RS;
@@ -285,9 +289,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                             uint32_t rlo[H::N], rhi[H::N];
                             H::unpack(x[u][0], rlo);
                             H::unpack(x[u][1], rhi);
-                            // the block's group inside the tile: k_group is 64 or 128 here
-                            const int j64 = (bb * 8 * FH) / 64, j128 = (bb * 8 * FH) / 128;
-                            const uint32_t bx = wide ? b[j128][0] : b[j64][0], by = wide ? b[j128][1] : b[j64][1];
+                            const uint32_t bx = b[(bb * 8 * FH) >> LGK][0], by = b[(bb * 8 * FH) >> LGK][1];   // the block's group in the tile
 #pragma unroll
                             for (int i = 0; i < H::N; i += 2)
                                 mma16816(acc[bb * MPB + i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], bx, by);
@@ -317,12 +319,12 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                 }
             }
         } else {
-            float zj[4];
+            float zj[NGW];
 #pragma unroll
-            for (int jk = 0; jk < 4; ++jk) zj[jk] = __shfl_sync(0xffffffffu, zsum, 4 * (4 + jk) + tig);   // rows 4..7
+            for (int jk = 0; jk < NGW; ++jk) zj[jk] = __shfl_sync(0xffffffffu, zsum, 4 * (4 + jk) + tig);   // rows 4..7
 #pragma unroll
             for (int bb = 0; bb < NBK; ++bb) {
-                const float corr = wide ? zj[(bb * 8 * FH) / 128] : zj[(bb * 8 * FH) / 64];
+                const float corr = zj[(bb * 8 * FH) >> LGK];
                 const int tok0 = tile0 + bb * 8 * FH + g * FH;
                 if (tok0 < hi) {                               // FH-token chunks are whole or absent (hi is a group multiple)
                     float *dst = dst_h + tok0;
@@ -343,7 +345,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 // ---------------------------------------------------------------------------------------------
 // p . V over packed values for tokens [t0, hi), (hi - t0) % 32 == 0, for the four heads.  scores[h] hold p_h.  Leaves
 // this warp's partial sums float[kQH][128] at the base of its region.  MODE as in the single-head kernel.
-template <int VB, int MODE>
+template <int VB, int MODE, int NGV>
 __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int32_t *vc, const __half *vs,
                                               const __half *vz, const GqaSmem &sm, int t0, int hi) {
     using G = GqaVGeom<VB>;
@@ -352,8 +354,7 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
     constexpr int MPB = F::N / 2;                             // MMAs per block: 8 / 4 / 2
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int Gv = a.v_group;
-    const int ngv = kHeadDim / Gv;                            // channel groups: 4 / 2 / 1
+    constexpr int ngv = NGV, Gv = kHeadDim / NGV;             // channel groups: 4 / 2 / 1
     const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;
     const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
     float *my_red = reinterpret_cast<float *>(sm.ring);
@@ -412,7 +413,7 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     // 1-bit values in groups of 64 channels: a 16-byte block (128 channels) then spans two groups, and the rows of an
     // MMA (lane octet g = channels 16 g .. 16 g + 15) lie in group g / 4.  Every code tile is multiplied twice, the rows of
     // group 1 cleared by the operands of group 0 and the other way round, into the same accumulators.
-    const bool split = VB == 1 && Gv == 64;
+    constexpr bool split = VB == 1 && Gv == 64;
     const uint32_t rows0 = !split || g < 4 ? 0xffffffffu : 0u, rows1 = g >= 4 ? 0xffffffffu : 0u;
     const uint32_t ones = 0x3c003c00u;
     // accumulation chains stay short by themselves (see the single-head kernel): 2112 tokens are at most nine blocks a warp
@@ -434,35 +435,43 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
         __syncwarp();
         // ---- B operands for the stage: per channel group 16 token pairs x 8 columns (head x {p*scale, p*midpoint}) ----
         {
-            const float2 fa = *reinterpret_cast<const float2 *>(pa), fb = *reinterpret_cast<const float2 *>(pb);
-            const float a0 = fa.x * 256.f, a1 = fa.y * 256.f, b0 = fb.x * 256.f, b1 = fb.y * 256.f;   // p carries 2^8
+            // a lane's two tokens (rows back to back) in pairs: {scale, scale} and {zero, zero} of a group
+            const unsigned long long k256 = f32x2(256.f, 256.f), mid = f32x2(G::MID, G::MID);                    // p carries 2^8
+            const unsigned long long pa2 = mul_f32x2(*reinterpret_cast<const unsigned long long *>(pa), k256);
+            const unsigned long long pb2 = mul_f32x2(*reinterpret_cast<const unsigned long long *>(pb), k256);
+            uint32_t sw[2][2], zw[2][2];                       // [token][pair of groups]
+            if constexpr (NGV == 4) {
+                const uint2 x = lds64(sz_rd + st), y = lds64(sz_rd + st + 8), z = lds64(sz_rd + st + 256), w = lds64(sz_rd + st + 264);
+                sw[0][0] = x.x; sw[0][1] = x.y; sw[1][0] = y.x; sw[1][1] = y.y;
+                zw[0][0] = z.x; zw[0][1] = z.y; zw[1][0] = w.x; zw[1][1] = w.y;
+            } else if constexpr (NGV == 2) {
+                const uint2 x = lds64(sz_rd + st), z = lds64(sz_rd + st + 256);
+                sw[0][0] = x.x; sw[1][0] = x.y; zw[0][0] = z.x; zw[1][0] = z.y;
+            } else {                                           // one group: the two tokens share a word
+                const uint32_t x = lds32(sz_rd + st), z = lds32(sz_rd + st + 256);
+                sw[0][0] = x; sw[1][0] = x >> 16; zw[0][0] = z; zw[1][0] = z >> 16;
+            }
 #pragma unroll
-            for (int jv = 0; jv < 4; ++jv) {
-                if (jv < ngv) {
-                    const float s0 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * jv)));
-                    const float s1 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 2 * (ngv + jv))));
-                    const float z0 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 256 + 2 * jv)));
-                    const float z1 = __half2float(__ushort_as_half((unsigned short)lds16(sz_rd + st + 256 + 2 * (ngv + jv))));
-                    const float m0 = fmaf(G::MID, s0, z0), m1 = fmaf(G::MID, s1, z1);
-                    const uint32_t c0 = pack_h2_sat(a0 * s0, a1 * s1), c1 = pack_h2_sat(a0 * m0, a1 * m1);
-                    const uint32_t c2 = pack_h2_sat(b0 * s0, b1 * s1), c3 = pack_h2_sat(b0 * m0, b1 * m1);
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(pb_wr + jv * 512), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
-                }
+            for (int jv = 0; jv < NGV; ++jv) {
+                auto half_of = [&](uint32_t w) { return (jv & 1) ? __high2float(as_h2(w)) : __low2float(as_h2(w)); };
+                const unsigned long long s2 = f32x2(half_of(sw[0][jv >> 1]), half_of(sw[1][jv >> 1]));
+                const unsigned long long m2 = fma_f32x2(mid, s2, f32x2(half_of(zw[0][jv >> 1]), half_of(zw[1][jv >> 1])));
+                auto pack = [](unsigned long long v) { const float2 f = f32x2_split(v); return pack_h2_sat(f.x, f.y); };
+                const uint32_t c0 = pack(mul_f32x2(pa2, s2)), c1 = pack(mul_f32x2(pa2, m2)), c2 = pack(mul_f32x2(pb2, s2)), c3 = pack(mul_f32x2(pb2, m2));
+                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(pb_wr + jv * 512), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
             }
         }
         __syncwarp();
 #pragma unroll
         for (int h2 = 0; h2 < 2; ++h2) {
-            uint32_t b[4][2];
+            uint32_t b[NGV][2];
 #pragma unroll
-            for (int jv = 0; jv < 4; ++jv) {
-                if (jv < ngv) {
+            for (int jv = 0; jv < NGV; ++jv) {
+                {
                     b[jv][0] = lds32(pb_rd + jv * 512 + (8 * h2) * 32);
                     b[jv][1] = lds32(pb_rd + jv * 512 + (8 * h2 + 4) * 32);
                     const uint32_t row1 = (g == jv) ? ones : 0u;    // sums of group jv land in row jv
                     mma16816(accz[jv & 1], row1, 0u, row1, 0u, b[jv][0], b[jv][1]);
-                } else {
-                    b[jv][0] = b[jv][1] = 0u;
                 }
             }
             uint32_t x[NB][2];
@@ -483,20 +492,17 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
                 uint32_t rlo[F::N], rhi[F::N];
                 F::unpack(VB == 1 ? x[bb][0] & rows0 : x[bb][0], rlo);
                 F::unpack(VB == 1 ? x[bb][1] & rows0 : x[bb][1], rhi);
-                // the block's channel group: v_group is 32 (4-bit values only), 64 or 128
-                const int j32 = (bb * CPB) / 32 < 4 ? (bb * CPB) / 32 : 3, j64 = (bb * CPB) / 64;
-                const uint32_t bx = Gv == 32 ? b[j32][0] : Gv == 64 ? b[j64][0] : b[0][0];
-                const uint32_t by = Gv == 32 ? b[j32][1] : Gv == 64 ? b[j64][1] : b[0][1];
+                const uint32_t bx = b[split ? 0 : bb * CPB / Gv][0], by = b[split ? 0 : bb * CPB / Gv][1];        // the block's channel group
 #pragma unroll
                 for (int i = 0; i < F::N; i += 2)
                     mma16816(acc[bb * MPB + i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], bx, by);
                 if constexpr (VB == 1) {
-                    if (split) {
+                    if constexpr (split) {
                         F::unpack(x[bb][0] & rows1, rlo);
                         F::unpack(x[bb][1] & rows1, rhi);
 #pragma unroll
                         for (int i = 0; i < F::N; i += 2)
-                            mma16816(acc[i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b[1][0], b[1][1]);
+                            mma16816(acc[i / 2], rlo[i], rlo[i + 1], rhi[i], rhi[i + 1], b[NGV - 1][0], b[NGV - 1][1]);
                     }
                 }
             }
@@ -512,20 +518,27 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     // epilogue: lane (g, tig) holds channels of rows g / g + 8 for head tig (column 2 tig); row jv of the ones-MMAs holds
     // (sum p*scale, sum p*mid) of channel group jv for head tig
     const float corr_mine = ((accz[0][1] + accz[1][1]) - G::MID * (accz[0][0] + accz[1][0])) * (1.f / 256.f);
-    float cj[4];
+    float cj[NGV];
 #pragma unroll
-    for (int jv = 0; jv < 4; ++jv) cj[jv] = __shfl_sync(0xffffffffu, corr_mine, 4 * jv + tig);
+    for (int jv = 0; jv < NGV; ++jv) cj[jv] = __shfl_sync(0xffffffffu, corr_mine, 4 * jv + tig);
 #pragma unroll
     for (int bb = 0; bb < NB; ++bb) {
         const int c0 = bb * CPB + g * F::N;
-        const float corr = Gv == 32 ? cj[(bb * CPB) / 32 < 4 ? (bb * CPB) / 32 : 3]
-                         : Gv == 64 ? (VB == 1 ? (g >= 4 ? cj[1] : cj[0]) : cj[(bb * CPB) / 64]) : cj[0];
+        const float corr = split ? (g >= 4 ? cj[NGV - 1] : cj[0]) : cj[bb * CPB / Gv];
 #pragma unroll
         for (int ip = 0; ip < MPB; ++ip) {
             my_red[tig * kHeadDim + c0 + 2 * ip] = fmaf(acc[bb * MPB + ip][0], (float)(1 << (16 - F::pos(2 * ip))), corr);
             my_red[tig * kHeadDim + c0 + 2 * ip + 1] = fmaf(acc[bb * MPB + ip][2], (float)(1 << (16 - F::pos(2 * ip + 1))), corr);
         }
     }
+}
+
+// The loops for the call's number of channel groups: 4 (4-bit values only, gqa_heads_per_cta), 2 or 1.
+template <int VB, int MODE>
+__device__ __forceinline__ void gqa_pv(const kvq_attn_args &a, const int32_t *vc, const __half *vs, const __half *vz, const GqaSmem &sm, int t0, int hi) {
+    if (VB == 4 && a.v_group == 32) gqa_pv_packed<VB, MODE, VB == 4 ? 4 : 2>(a, vc, vs, vz, sm, t0, hi);
+    else if (a.v_group == 64) gqa_pv_packed<VB, MODE, 2>(a, vc, vs, vz, sm, t0, hi);
+    else gqa_pv_packed<VB, MODE, 1>(a, vc, vs, vz, sm, t0, hi);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -776,13 +789,14 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        gqa_qk_packed<KB>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        if (KB != 1 && (KB == 3 || a.k_group == 64)) gqa_qk_packed<KB, false>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        else gqa_qk_packed<KB, KB != 3>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     if constexpr (VB == 3) gqa_pv_packed3<1>(a, vc, vs, vz, sm, t0, v_hi);
-    else gqa_pv_packed<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
+    else gqa_pv<VB, 1>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
     // ---- 2. softmax numerators: two warps per head slot --------------------------------------------
@@ -819,7 +833,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
 
     // ---- 3. p . V -----------------------------------------------------------------------------------
     if constexpr (VB == 3) gqa_pv_packed3<2>(a, vc, vs, vz, sm, t0, v_hi);
-    else gqa_pv_packed<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
+    else gqa_pv<VB, 2>(a, vc, vs, vz, sm, t0, v_hi);
     __syncwarp();
     if (v_lo < t1) pv_tail<kQH>(a, vf, b, hk, sm.scores, n_scores, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();

@@ -57,7 +57,7 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 
 // If the split also holds fp16 tail keys (tail_lo < t1) they are scored right after the first code stages
 // have been issued, so the tail's global-load latency overlaps the ring fill.
-template <int KB, int NW>
+template <int KB, int NW, int LGK>
 __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const MmaSmem &sm, int t0, int hi,
                                               const __half *kf, int tail_lo, int t1, int b, int hk) {
@@ -65,7 +65,6 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     using R = MmaKRing<KB, NW>;
     using F = Fields<KB>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int Gk = a.k_group;
     const int n_words = a.Tkq / G::FPI;                       // valid code words per channel row
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;
     const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = NW >> sm.ks_log2;
@@ -95,10 +94,10 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     // ldmatrix.x4 row addresses: lanes 0-7 scale rows 0..7 of a k-step, 8-15 scale rows 8..15, 16-31 the same of the zero rows
     const uint32_t ldm_s = ring_s + G::CODE_BYTES + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16 + (lane >> 4) * (G::ROWS * 16);
     const uint32_t q_s = smem_u32(sm.q) + (ch0 + 2 * tig) * 2;                 // + 32 per k-step [+16]
-    const int ngw = (G::WT + Gk - 1) / Gk;                                     // groups per warp tile: 8 / 4 / 2
+    constexpr int ngw = KB == 3 ? 8 : G::WT >> LGK;                            // groups per warp tile: 8 / 4 / 2
     const uint32_t szcp_dst = ring_s + G::CODE_BYTES + lane * 16;                  // one granule per lane (16 channels a stage) or two
     const int tile_words = tile_lanes * G::WT / G::FPI;                        // word-column distance between my tiles
-    const int tile_groups = tile_lanes * G::WT / Gk;
+    const int tile_groups = tile_lanes * ngw;
 
     // the next stage to issue: its addresses, its word column, its position in its tile and the tiles left.  Stages
     // carry the scale and zero rows of their own channels, so the operands are formed k-step by k-step and the loop over
@@ -107,7 +106,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     uint32_t iss = 4u * ((uint32_t)(ch0 + row0) * kc_sD + (t0 + wt * G::WT) / G::FPI + 4 * gr);   // bytes from the head's first word
     constexpr bool kOneSz = 2 * G::ROWS == 32;                                 // 16 channels: lanes 16-31 fetch the zero rows
     const int sz_row = kOneSz ? (lane & 15) : lane;
-    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (t0 + wt * G::WT) / Gk);
+    uint32_t iss_s = 2u * ((uint32_t)(ch0 + sz_row) * ks_sD + (KB == 3 ? (t0 + wt * G::WT) / 11 : (t0 + wt * G::WT) >> LGK));
     const char *sz_b = reinterpret_cast<const char *>(kOneSz && lane >= 16 ? kz : ks);
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
     uint32_t iss_slot = 0, slot = 0;                                            // byte offsets of the slot being filled / read
@@ -161,7 +160,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
         // Other widths: b0 / b1 serve the first / second half of the tile; column n carries group (n / 2) of that
         // half, hi in even and lo in odd columns, so one MMA per code tile yields both parts.
         float zsum = 0.f;
-        const int gph = ngw > 1 ? ngw / 2 : 1;                 // groups per half tile: 4 / 2 / 1
+        constexpr int gph = ngw / 2;                           // groups per half tile: 4 / 2 / 1
         const int src0 = 4 * ((g >> 1) % gph) + tig;           // lane holding group (n / 2) of the first half
         const int src1 = src0 + 4 * (ngw / 2);
         const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;  // odd columns: the lo part
@@ -302,7 +301,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
             // octet g of half h is in group h*gph + cp of the tile, cp = 16 g / Gk; its hi and lo sums are the column
             // pair cp, held by the lane with tig == cp; the group's zero term sits in the lanes of octet grp
             constexpr int NF = F::N;
-            const int cp = (16 * g) / Gk;
+            const int cp = (16 * g) >> LGK;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int grp = h * gph + cp;
@@ -323,12 +322,11 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
             // octet g of block bb owns tokens bb*8FH + g*FH ..; in its half of the tile they are in group cp, whose hi and
             // lo sums are the column pair cp, held by the lane with tig == cp; the group's zero term sits in the lanes
             // of octet grp
-            const int lgk = 31 - __clz(Gk);                    // group sizes are powers of two here
 #pragma unroll
             for (int bb = 0; bb < NBK; ++bb) {
                 constexpr int kHalfBlocks = NBK / 2;
                 const int h = bb / kHalfBlocks;
-                const int cp = (((bb % kHalfBlocks) * 8 * FH) + g * FH) >> lgk;
+                const int cp = (((bb % kHalfBlocks) * 8 * FH) + g * FH) >> LGK;
                 const int grp = h * gph + cp;
                 const float corr = __shfl_sync(0xffffffffu, zsum, 4 * grp);    // row grp of the zero-term product
                 const int tok0 = tile0 + bb * 8 * FH + g * FH;
@@ -357,7 +355,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 // ring region (float [128] at the region base).
 // MODE 1 only issues the first stages (called before the softmax, whose latency then hides the ring fill);
 // MODE 2 continues after such a call; MODE 0 does both.
-template <int VB, int MODE, int NW>
+template <int VB, int MODE, int NW, int NGV>
 __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int32_t *vc, const __half *vs,
                                               const __half *vz, const MmaSmem &sm, int t0, int hi) {
     using G = MmaVGeom<VB, NW>;
@@ -366,8 +364,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
     constexpr int MPB = F::N / 2;                             // MMAs (channel pairs per octet) per block: 8 / 4 / 2
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
-    const int Gv = a.v_group;
-    const int ngv = kHeadDim / Gv;                            // channel groups: 4 / 2 / 1
+    constexpr int ngv = NGV, Gv = kHeadDim / NGV;             // channel groups: 4 / 2 / 1
     const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;      // <= 0: no packed values in this segment
     const int my_blocks = (n_blocks - warp + NW - 1) / NW;
     float *my_red = reinterpret_cast<float *>(sm.ring);
@@ -398,11 +395,9 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     const uint32_t pb_rd = pb_s + (tig * 8 + g) * 4;                                     // + (8 h2 + 4 b) * 32
     // operand build: lane -> pair pi = lane & 15, column half ch = lane >> 4 (groups 2ch, 2ch+1)
     const int pi = lane & 15, ch = lane >> 4;
-    const int bt0 = 16 * (pi >> 3) + 8 * ((pi >> 2) & 1) + 2 * (pi & 3), bt1 = bt0 + 1;  // the pair's tokens in the stage
-    // columns beyond the last channel group repeat that group: finite values in C columns nobody reads
-    const int g0 = min(2 * ch, ngv - 1), g1 = min(2 * ch + 1, ngv - 1);
-    const uint32_t o00 = ring_s + G::SZ_OFF + (bt0 * ngv + g0) * 2, o01 = ring_s + G::SZ_OFF + (bt0 * ngv + g1) * 2;
-    const uint32_t o10 = ring_s + G::SZ_OFF + (bt1 * ngv + g0) * 2, o11 = ring_s + G::SZ_OFF + (bt1 * ngv + g1) * 2;
+    const int bt0 = 16 * (pi >> 3) + 8 * ((pi >> 2) & 1) + 2 * (pi & 3);                 // the pair's first token in the stage
+    // (columns beyond the last channel group repeat others: C columns nobody reads)
+    const uint32_t sz_rd = ring_s + G::SZ_OFF + bt0 * (ngv * 2) + (ngv == 4 ? 4 * ch : 0);         // this half's groups of token bt0; zeros + 256
     const uint32_t pb_wr = pb_s + (pi * 8 + 4 * ch) * 4;
 
     const int block_stride = NW * G::TPS;
@@ -477,21 +472,24 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
         {
             // p is scaled by 2^8 before the fp16 rounding so that the many small probabilities of a long, diffuse
             // context stay in the normal fp16 range (p <= 1, so this saturates only if a scale exceeds 255)
-            const float p0 = pp[bt0] * 256.f, p1 = pp[bt1] * 256.f;
-            const float s00 = __half2float(__ushort_as_half((unsigned short)lds16(o00 + st)));
-            const float s01 = __half2float(__ushort_as_half((unsigned short)lds16(o01 + st)));
-            const float s10 = __half2float(__ushort_as_half((unsigned short)lds16(o10 + st)));
-            const float s11 = __half2float(__ushort_as_half((unsigned short)lds16(o11 + st)));
-            const float z00 = __half2float(__ushort_as_half((unsigned short)lds16(o00 + st + 256)));
-            const float z01 = __half2float(__ushort_as_half((unsigned short)lds16(o01 + st + 256)));
-            const float z10 = __half2float(__ushort_as_half((unsigned short)lds16(o10 + st + 256)));
-            const float z11 = __half2float(__ushort_as_half((unsigned short)lds16(o11 + st + 256)));
+            const unsigned long long p01 = mul_f32x2(*reinterpret_cast<const unsigned long long *>(pp + bt0), f32x2(256.f, 256.f)), mid = f32x2(G::MID, G::MID);
+            uint32_t sx, sy, zx, zy;                           // the two groups of tokens bt0 and bt0 + 1
+            if constexpr (NGV == 4) {
+                sx = lds32(sz_rd + st); sy = lds32(sz_rd + st + 8); zx = lds32(sz_rd + st + 256); zy = lds32(sz_rd + st + 264);
+            } else if constexpr (NGV == 2) {
+                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];\n" : "=r"(sx), "=r"(sy) : "r"(sz_rd + st));
+                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];\n" : "=r"(zx), "=r"(zy) : "r"(sz_rd + st + 256));
+            } else {                                           // one group, the two tokens in a word
+                const uint32_t x = lds32(sz_rd + st), z = lds32(sz_rd + st + 256);
+                sx = prmt(x, x, 0x1010); sy = prmt(x, x, 0x3232); zx = prmt(z, z, 0x1010); zy = prmt(z, z, 0x3232);
+            }
             // columns 4ch .. 4ch+3 = (p*scale_g0, p*mid_g0, p*scale_g1, p*mid_g1), each a half2 over the token pair;
             // mid = zero + MID*scale is the midpoint of the group: codes are used as (code - MID)
-            const uint32_t c0 = pack_h2_sat(p0 * s00, p1 * s10);
-            const uint32_t c1 = pack_h2_sat(p0 * fmaf(G::MID, s00, z00), p1 * fmaf(G::MID, s10, z10));
-            const uint32_t c2 = pack_h2_sat(p0 * s01, p1 * s11);
-            const uint32_t c3 = pack_h2_sat(p0 * fmaf(G::MID, s01, z01), p1 * fmaf(G::MID, s11, z11));
+            const unsigned long long s0 = f32x2(__low2float(as_h2(sx)), __low2float(as_h2(sy))), s1 = f32x2(__high2float(as_h2(sx)), __high2float(as_h2(sy)));
+            const unsigned long long m0 = fma_f32x2(mid, s0, f32x2(__low2float(as_h2(zx)), __low2float(as_h2(zy))));
+            const unsigned long long m1 = fma_f32x2(mid, s1, f32x2(__high2float(as_h2(zx)), __high2float(as_h2(zy))));
+            auto pack = [](unsigned long long v) { const float2 f = f32x2_split(v); return pack_h2_sat(f.x, f.y); };
+            const uint32_t c0 = pack(mul_f32x2(p01, s0)), c1 = pack(mul_f32x2(p01, m0)), c2 = pack(mul_f32x2(p01, s1)), c3 = pack(mul_f32x2(p01, m1));
             asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(pb_wr), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
         }
         __syncwarp();
@@ -547,6 +545,15 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
             }
         }
     }
+}
+
+// The loops for the call's number of channel groups (see the keys: 4096 tokens, 64 x 32 heads, 4 bits 257.8 -> 250.4 us, 2 bits
+// 213.3 -> 208.5 with both group sizes known).
+template <int VB, int MODE, int NW>
+__device__ __forceinline__ void pv_mma(const kvq_attn_args &a, const int32_t *vc, const __half *vs, const __half *vz, const MmaSmem &sm, int t0, int hi) {
+    if (a.v_group == 32) pv_packed_mma<VB, MODE, NW, 4>(a, vc, vs, vz, sm, t0, hi);
+    else if (a.v_group == 64) pv_packed_mma<VB, MODE, NW, 2>(a, vc, vs, vz, sm, t0, hi);
+    else pv_packed_mma<VB, MODE, NW, 1>(a, vc, vs, vz, sm, t0, hi);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -621,12 +628,15 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        qk_packed_mma<KB, NW>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        // the loops for the call's group size: looked up, it cost a compare, a branch or a select per group and k-step
+        if (KB == 3 || a.k_group == 32) qk_packed_mma<KB, NW, 5>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        else if (a.k_group == 64) qk_packed_mma<KB, NW, KB == 3 ? 5 : 6>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        else qk_packed_mma<KB, NW, KB == 3 ? 5 : 7>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
     const __half *vz = static_cast<const __half *>(a.vmn) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
-    pv_packed_mma<VB, 1, NW>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
+    pv_mma<VB, 1, NW>(a, vc, vs, vz, sm, t0, v_hi);         // start filling this warp's value ring now
     __syncthreads();
 
     // ---- 2. softmax numerators ------------------------------------------------------------------
@@ -663,7 +673,7 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     __syncthreads();
 
     // ---- 3. p.V -----------------------------------------------------------------------------------
-    pv_packed_mma<VB, 2, NW>(a, vc, vs, vz, sm, t0, v_hi);
+    pv_mma<VB, 2, NW>(a, vc, vs, vz, sm, t0, v_hi);
     __syncwarp();
     if (v_lo < t1) pv_tail<1>(a, vf, b, hk, sm.scores, 0, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, NW, lane);
     __syncthreads();
