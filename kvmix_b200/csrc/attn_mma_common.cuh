@@ -14,6 +14,9 @@ constexpr int kMmaThreads = 256;
 constexpr int kMmaWarps = 8;
 constexpr int kMmaSmemMax = 115712;                                // dynamic shared memory of a CTA with two of them on an SM
 
+// The warp's number, as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"

@@ -81,9 +81,12 @@ __global__ void __launch_bounds__(256) gemv_kernel(kvq_gemv_args a, int wx_log2,
 //              product is the zero term of group j (and row j the sum of in * scale that the complemented rows need).
 //   Infinities and NaN come out as fp32 products and sums give them: a window that holds an infinity works without the complement,
 //              whose two halves would meet as inf - inf.
-// Bound by the instruction stream (0.6 logic operations a code); 16 sequences x 32 heads x 4096 tokens, q . K^T and p . V together
-// at 2 bits: 113 us (105 us without the powers of two), 229 us with one thread per word column; from a flushed L2 123 us at 2
-// bits (115 without) and 135 us at 4 bits (130 without).
+// Bound by the instruction stream: 0.6 logic operations a code, and whatever surrounds them.  A stage of whole rows is copied by
+// 32-bit offsets from the head's first word (64-bit row arithmetic per granule was a quarter of all instructions), the group size is
+// known to the loops, heads and columns are numbered in 32 bits, and where the rows are few (q . K^T) a warp takes up to four
+// column tiles one after the other, the copies running on from tile to tile.  16 sequences x 32 heads x 4096 tokens, group 32, us:
+// q . K^T 2 bits 64 -> 50, 4 bits 68 -> 54, 1 bit (group 128) 60 -> 44; p . V 50 -> 46, 54 -> 52, 48 -> 43 (229 for the 2-bit
+// pair with one thread per word column); warp instructions per 32 codes of q . K^T 4.1 -> 3.6, of p . V 2.8.
 template <int BITS> struct GemvGeom {
     static constexpr int RB = 16 * BITS;                       // code bytes of a tile row
     static constexpr int RS = BITS == 1 ? RB : RB + 16;        // padded: conflict-free ldmatrix
@@ -94,6 +97,9 @@ template <int BITS> struct GemvGeom {
 };
 constexpr int kGemvWarps = 8, kGemvThreads = 32 * kGemvWarps;
 constexpr int kGemvChunk = 2048;                               // rows whose `in` is held (and normalised) at a time
+// A warp takes several column tiles where a tile is short (rows) and the CTAs still fill the GPU: with 128 rows a tile is four stages, and a
+// warp that works only one spends as long on its first copies.
+constexpr int kGemvTileRows = 512, kGemvTiles = 4, kGemvMinCtas = 2 * 296;
 constexpr int kGemvFlush = 8;                                  // stages between flushes of the MMA accumulators (short chains): a window
 
 __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
@@ -101,10 +107,14 @@ __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t
 struct GemvPlan {
     int wk_log2;         // warps that share a column tile (the other factor of 8: column tiles of a CTA)
     int col_ctas;        // CTAs per head along the columns
+    int tpw;             // column tiles a warp takes one after the other
     int kc;              // CTAs of a cluster, each with rows_per_cta rows
     int rows_per_cta;
     int code_align;      // 16, 8 or 4: what every row of a tile is aligned to
     int sz_vec;          // scale / zero rows of a whole tile can be copied as one vector
+    int fast;            // 16-byte granules and vectors, all rows of a head within 32-bit byte offsets
+    int rep;             // query heads per kv head
+    int out_vec;         // output rows are 8-byte aligned
 };
 
 template <int CG, int BITS>
@@ -118,33 +128,32 @@ __device__ __forceinline__ void gemv_copy_codes(uint32_t dst, const int32_t *src
     }
 }
 
-template <int BITS>
+// GS_LOG2: log2 of the group size
+template <int BITS, int GS_LOG2>
 __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_constant__ kvq_gemv_args a,
                                                                    const __grid_constant__ GemvPlan plan) {
     using G = GemvGeom<BITS>;
     using F = VHalf<BITS>;
-    constexpr int FPI = fields_per_word(BITS), FH = 16 / BITS, MPB = FH / 2, NBLK = BITS;
+    constexpr int FPI = fields_per_word(BITS), FH = 16 / BITS, MPB = FH / 2, NBLK = BITS, ngw = 128 >> GS_LOG2, kSzBytes = ngw == 4 ? 8 : 4;
     extern __shared__ __align__(128) unsigned char smem[];
     float *red = reinterpret_cast<float *>(smem);                               // [kGemvWarps][128] tile sums
     __half *xs = reinterpret_cast<__half *>(red + kGemvWarps * 128);            // [kGemvChunk] normalised `in`
     float *misc = reinterpret_cast<float *>(xs + kGemvChunk);                   // [8]
     unsigned char *ring = reinterpret_cast<unsigned char *>(misc + 8) + 96;     // 128-byte aligned
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tig = lane & 3;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31, g = lane >> 2, tig = lane & 3;
     const int WK = 1 << plan.wk_log2, wk = warp & (WK - 1), wc = warp >> plan.wk_log2, WC = kGemvWarps >> plan.wk_log2;
-    const int rank = blockIdx.x % plan.kc, job = blockIdx.x / plan.kc;
-    const int64_t s = job / plan.col_ctas;
-    const int b = (int)(s / a.nh), h = (int)(s % a.nh), hk = h / (int)(a.nh / a.nh_kv);
-    const int N = (int)(a.n_groups * a.group), n_pack = N / FPI;
-    const int n0 = ((job % plan.col_ctas) * WC + wc) * 128;                     // this warp's first column
-    const int k_beg = rank * plan.rows_per_cta, k_end = min((int)a.K, k_beg + plan.rows_per_cta);
-    const int grp0 = n0 / a.group, ngw = 128 / a.group;
-    const int words = min(128 / FPI, n_pack - n0 / FPI);                        // <= 0: no such tile
+    // everything that numbers CTAs, heads and columns fits 32 bits (gemv_mma_plan); 64-bit divisions cost 100 instructions each
+    const uint32_t rank = blockIdx.x % (uint32_t)plan.kc, job = blockIdx.x / (uint32_t)plan.kc;
+    const uint32_t s = job / (uint32_t)plan.col_ctas, col_cta = job - s * (uint32_t)plan.col_ctas;
+    const uint32_t b = s / (uint32_t)a.nh, h = s - b * (uint32_t)a.nh, hk = h / (uint32_t)plan.rep;
+    const int N = (int)(a.n_groups << GS_LOG2), n_pack = N / FPI;
+    const int col0 = (int)col_cta * plan.tpw * WC * 128;                        // the CTA's first column
+    const int k_beg = (int)rank * plan.rows_per_cta, k_end = min((int)a.K, k_beg + plan.rows_per_cta);
     const __half *in = static_cast<const __half *>(a.fA) + b * a.a_sB + h * a.a_sH;
-    const int32_t *qb = a.qB + b * a.q_sB + hk * a.q_sH + n0 / FPI;
-    const int64_t zo = b * a.s_sB + hk * a.s_sH + grp0;
-    const __half *sp = static_cast<const __half *>(a.scale) + zo, *zp = static_cast<const __half *>(a.zero) + zo;
-    const int groups = min(ngw, (int)a.n_groups - grp0);
-    const bool vec = plan.sz_vec && groups == ngw;
+    const int32_t *qh = a.qB + b * a.q_sB + hk * a.q_sH;
+    const __half *sh = static_cast<const __half *>(a.scale) + b * a.s_sB + hk * a.s_sH;
+    const __half *zh = static_cast<const __half *>(a.zero) + b * a.s_sB + hk * a.s_sH;
+    __half *out = static_cast<__half *>(a.out) + b * a.o_sB + h * a.o_sH;
 
     const uint32_t ring_s = smem_u32(ring) + warp * G::WARP_BYTES;
     const uint32_t sz_dst = ring_s + G::CODE_BYTES + lane * 16;
@@ -154,12 +163,113 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
     const int src = 4 * (g >> 1) + tig;                                         // lane holding group (column / 2)
     const uint32_t neg_mask = (g & 1) ? 0xffffffffu : 0u;
 
+    // a stage of the fast path: granule x = lane + 32 i -> row x / GPR, granule x % GPR; bytes from the head's first word / scale
+    constexpr int GPR = G::RB / 16;
+    const uint32_t q_row = (uint32_t)a.q_sK * 4u, s_row = (uint32_t)a.s_sK * 2u;
+    const uint32_t lane_q = (uint32_t)(lane / GPR) * q_row + (lane % GPR) * 16u, lane_s = (uint32_t)lane * s_row;
+    const uint32_t lane_dst = ring_s + (lane / GPR) * G::RS + (lane % GPR) * 16;
+    const char *qh_b = reinterpret_cast<const char *>(qh), *sh_b = reinterpret_cast<const char *>(sh), *zh_b = reinterpret_cast<const char *>(zh);
+
     float acc[8][4], sum[8][2], accz[2][4] = {}, zsum = 0.f;
+    auto clear = [&]() {
 #pragma unroll
-    for (int m = 0; m < 8; ++m) { acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f; sum[m][0] = sum[m][1] = 0.f; }
+        for (int m = 0; m < 8; ++m) sum[m][0] = sum[m][1] = 0.f;
+        zsum = 0.f;
+    };
+    clear();
+#pragma unroll
+    for (int m = 0; m < 8; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
+
+    // tile sums: octet g of block bb owns columns bb * 8 FH + g * FH .. + FH - 1, their group's pair of B columns is held by
+    // the lane with tig == group, its zero term by row 4 + group
+    auto tile_sums = [&]() {
+#pragma unroll
+        for (int bb = 0; bb < NBLK; ++bb) {
+            const int c = bb * 8 * FH + g * FH, cp = c >> GS_LOG2;
+            constexpr float kMax = (float)((1 << BITS) - 1);
+            const float corr = fmaf(kMax, __shfl_sync(0xffffffffu, zsum, 4 * cp), __shfl_sync(0xffffffffu, zsum, 4 * (4 + cp)));
+            if (tig == cp) {
+#pragma unroll
+                for (int ip = 0; ip < MPB; ++ip) {
+                    red[warp * 128 + c + 2 * ip] = fmaf(sum[bb * MPB + ip][0], (float)(1 << (24 - F::pos(2 * ip))), corr);
+                    red[warp * 128 + c + 2 * ip + 1] = fmaf(sum[bb * MPB + ip][1], (float)(1 << (24 - F::pos(2 * ip + 1))), corr);
+                }
+            }
+        }
+    };
 
     for (int c0 = k_beg; c0 < k_end; c0 += kGemvChunk) {
-        const int rows = min(kGemvChunk, k_end - c0), n_st = (rows + 31) / 32;
+        const int rows = min(kGemvChunk, k_end - c0), n_st = (rows + 31) / 32, my_st = (n_st - wk + WK - 1) / WK;
+        // Stages of this warp's tiles in one sequence: the ring runs on from one tile to the next.  (More than one tile only where
+        // all rows are one chunk.)
+        const int n0_first = col0 + wc * 128;
+        int iss_n0 = n0_first, iss_st = wk, iss_left = my_st * plan.tpw;
+        uint32_t iss_q = (uint32_t)(c0 + 32 * wk) * q_row + (uint32_t)(n0_first / FPI) * 4u, iss_s = (uint32_t)(c0 + 32 * wk) * s_row + (uint32_t)(n0_first >> GS_LOG2) * 2u;
+        bool iss_whole = plan.fast && n0_first + 128 <= N;                      // a whole tile, and aligned
+        auto issue_any = [&](uint32_t slot) {                                   // ragged, unaligned or far apart
+            const int words = min(128 / FPI, n_pack - iss_n0 / FPI);            // <= 0: no such tile
+            if (words > 0) {
+                const int left = rows - 32 * iss_st;                            // rows of the stage that exist
+                const int grp0 = iss_n0 >> GS_LOG2, groups = min(ngw, (int)a.n_groups - grp0);
+                const int64_t r0 = c0 + 32 * iss_st;
+                const int32_t *p = qh + iss_n0 / FPI + r0 * a.q_sK;
+                if (plan.code_align == 16) gemv_copy_codes<16, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                else if (plan.code_align == 8) gemv_copy_codes<8, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                else gemv_copy_codes<4, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
+                const __half *ps = sh + grp0 + (r0 + lane) * a.s_sK, *pz = zh + grp0 + (r0 + lane) * a.s_sK;
+                const uint32_t d = sz_dst + slot;
+                if (ngw > 1 && lane < left && plan.sz_vec && groups == ngw) {
+                    cp_async<kSzBytes>(d, ps);
+                    cp_async<kSzBytes>(d + 8, pz);
+                } else {                                                        // odd group counts, one group a tile, missing rows: zeros
+                    uint32_t v[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int jj = j & 1;
+                        const __half *q = j < 2 ? ps : pz;
+                        const bool ok0 = lane < left && 2 * jj < groups, ok1 = lane < left && 2 * jj + 1 < groups;
+                        const uint32_t lo = ok0 ? __half_as_ushort(__ldg(q + 2 * jj)) : 0u, hi = ok1 ? __half_as_ushort(__ldg(q + 2 * jj + 1)) : 0u;
+                        v[j] = lo | (hi << 16);
+                    }
+                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+                }
+            }
+        };
+        auto issue = [&](uint32_t slot) {
+            if (iss_left > 0) {
+                if (iss_whole && 32 * iss_st + 32 <= rows) {
+#pragma unroll
+                    for (int i = 0; i < GPR; ++i)
+                        cp_async<16>(lane_dst + slot + i * (32 / GPR) * G::RS, qh_b + (iss_q + lane_q + i * (32 / GPR) * q_row));
+                    const uint32_t d = sz_dst + slot, o = iss_s + lane_s;
+                    if constexpr (ngw > 1) {
+                        cp_async<kSzBytes>(d, sh_b + o);
+                        cp_async<kSzBytes>(d + 8, zh_b + o);
+                    } else {
+                        const uint32_t v = __half_as_ushort(__ldg(reinterpret_cast<const __half *>(sh_b + o))), z = __half_as_ushort(__ldg(reinterpret_cast<const __half *>(zh_b + o)));
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%2};\n" ::"r"(d), "r"(v), "r"(0u), "r"(z));
+                    }
+                } else {
+                    issue_any(slot);
+                }
+            }
+            cp_async_commit();
+            --iss_left;
+            iss_st += WK;
+            iss_q += 32u * q_row << plan.wk_log2;
+            iss_s += 32u * s_row << plan.wk_log2;
+            if (iss_st >= n_st) {                                               // the next tile
+                iss_n0 += WC * 128;
+                iss_st = wk;
+                iss_q = (uint32_t)(c0 + 32 * wk) * q_row + (uint32_t)(iss_n0 / FPI) * 4u;
+                iss_s = (uint32_t)(c0 + 32 * wk) * s_row + (uint32_t)(iss_n0 >> GS_LOG2) * 2u;
+                iss_whole = plan.fast && iss_n0 + 128 <= N;
+            }
+        };
+        uint32_t iss_slot = 0, slot = 0;
+#pragma unroll 1
+        for (int q = 0; q < G::NS - 1; ++q) { issue(iss_slot); iss_slot += G::STAGE_BYTES; }
+
         // ---- in * 2^up_e: the largest magnitude to 2^7 .. 2^8, larger ones (and a chunk with an infinity) as they are ----
         if (c0 > k_beg) __syncthreads();                                        // the previous chunk has been read
         float mx = 0.f;
@@ -176,36 +286,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
         for (int i = tid; i < n_st * 32; i += kGemvThreads)
             xs[i] = i < rows ? __float2half_rn(__half2float(__ldg(in + c0 + i)) * up) : __float2half_rn(0.f);
         __syncthreads();
-        if (words <= 0) continue;
 
-        auto issue = [&](int st, uint32_t slot) {
-            if (st < n_st) {
-                const int left = rows - 32 * st;                                // rows of the stage that exist
-                const int64_t r0 = c0 + 32 * st;
-                const int32_t *p = qb + r0 * a.q_sK;
-                if (plan.code_align == 16) gemv_copy_codes<16, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
-                else if (plan.code_align == 8) gemv_copy_codes<8, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
-                else gemv_copy_codes<4, BITS>(ring_s + slot, p, a.q_sK, left, words, lane);
-                const __half *ps = sp + (r0 + lane) * a.s_sK, *pz = zp + (r0 + lane) * a.s_sK;
-                const uint32_t d = sz_dst + slot;
-                if (lane < left && vec && ngw > 1) {
-                    if (ngw == 4) { cp_async<8>(d, ps); cp_async<8>(d + 8, pz); }
-                    else { cp_async<4>(d, ps); cp_async<4>(d + 8, pz); }
-                } else {                                                        // odd group counts, one group a tile, missing rows: zeros
-                    uint32_t v[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int jj = j & 1;
-                        const __half *q = j < 2 ? ps : pz;
-                        const bool ok0 = lane < left && 2 * jj < groups, ok1 = lane < left && 2 * jj + 1 < groups;
-                        const uint32_t lo = ok0 ? __half_as_ushort(__ldg(q + 2 * jj)) : 0u, hi = ok1 ? __half_as_ushort(__ldg(q + 2 * jj + 1)) : 0u;
-                        v[j] = lo | (hi << 16);
-                    }
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
-                }
-            }
-            cp_async_commit();
-        };
         // the window's powers of two: of the group of this lane's B column, undone for the group of its C columns; lanes g < 4 watch
         // that the scales of group g stay below `lim`
         __half2 s_up = __floats2half2_rn(1.f, 1.f), lim = s_up;
@@ -244,14 +325,12 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
             turn = in_finite && !__any_sync(0xffffffffu, g < ngw && top == 0x7c00u);
         };
 
-        uint32_t iss_slot = 0, slot = 0;
-        int iss_st = wk;
-#pragma unroll 1
-        for (int q = 0; q < G::NS - 1; ++q) { issue(iss_st, iss_slot); iss_st += WK; iss_slot += G::STAGE_BYTES; }
+        for (int t = 0; t < plan.tpw; ++t) {
+        const int n0 = n0_first + t * WC * 128;
+        if (n0 >= N) break;
 #pragma unroll 1
         for (int st = wk; st < n_st; st += WK) {
-            issue(iss_st, iss_slot);
-            iss_st += WK;
+            issue(iss_slot);
             iss_slot = iss_slot == (G::NS - 1) * G::STAGE_BYTES ? 0u : iss_slot + G::STAGE_BYTES;
             cp_async_wait<G::NS - 1>();
             __syncwarp();
@@ -301,30 +380,30 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
             if (++since == kGemvFlush) flush();
         }
         if (since) flush();
+        if (WK > 1 || plan.kc > 1 || k_end - k_beg > kGemvChunk) continue;
+        // ---- a tile of one warp: its sums are the result
+        tile_sums();
+        __syncwarp();
+        const float4 v = *reinterpret_cast<const float4 *>(red + warp * 128 + 4 * lane);
+        __syncwarp();
+        if (n0 + 128 <= N && plan.out_vec) {
+            const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+            *reinterpret_cast<uint2 *>(out + n0 + 4 * lane) = make_uint2(as_u32(lo), as_u32(hi));
+        } else {
+            const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (n0 + 4 * lane + i < N) out[n0 + 4 * lane + i] = __float2half_rn(e[i]);
+        }
+        clear();
+        }
         cp_async_wait<0>();
         __syncwarp();
     }
+    if (WK == 1 && plan.kc == 1 && k_end - k_beg <= kGemvChunk) return;
 
-    // ---- tile sums: octet g of block bb owns columns bb * 8 FH + g * FH .. + FH - 1, their group's pair of B columns is held by
-    // the lane with tig == group, its zero term by row 4 + group
-    if (words > 0) {
-#pragma unroll
-        for (int bb = 0; bb < NBLK; ++bb) {
-            const int c = bb * 8 * FH + g * FH, cp = c / a.group;
-            constexpr float kMax = (float)((1 << BITS) - 1);
-            const float corr = fmaf(kMax, __shfl_sync(0xffffffffu, zsum, 4 * cp), __shfl_sync(0xffffffffu, zsum, 4 * (4 + cp)));
-            if (tig == cp) {
-#pragma unroll
-                for (int ip = 0; ip < MPB; ++ip) {
-                    red[warp * 128 + c + 2 * ip] = fmaf(sum[bb * MPB + ip][0], (float)(1 << (24 - F::pos(2 * ip))), corr);
-                    red[warp * 128 + c + 2 * ip + 1] = fmaf(sum[bb * MPB + ip][1], (float)(1 << (24 - F::pos(2 * ip + 1))), corr);
-                }
-            }
-        }
-    }
+    if (col0 + wc * 128 < N) tile_sums();
     __syncthreads();
-    __half *out = static_cast<__half *>(a.out) + b * a.o_sB + h * a.o_sH;
-    const int col0 = (job % plan.col_ctas) * WC * 128;
     namespace cg = cooperative_groups;
     if (plan.kc > 1) {                                                          // every rank: the sums over its warps; rank 0 adds the ranks
         for (int i = tid; i < WC * 128; i += kGemvThreads) {
@@ -351,7 +430,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
     }
 }
 
-template <int BITS>
+template <int BITS, int GS_LOG2>
 static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned grid, cudaStream_t st) {
     const size_t smem = kGemvWarps * 128 * 4 + kGemvChunk * 2 + 8 * 4 + 96 + (size_t)kGemvWarps * GemvGeom<BITS>::WARP_BYTES;
     static bool attr_set[64] = {};
@@ -359,7 +438,7 @@ static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned g
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return record_cuda_error(e);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        e = cudaFuncSetAttribute(gemv_mma_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(gemv_mma_kernel<BITS, GS_LOG2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return record_cuda_error(e);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
@@ -374,7 +453,7 @@ static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned g
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = p.kc > 1 ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<BITS>, a, p);
+    e = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<BITS, GS_LOG2>, a, p);
     if (e != cudaSuccess) return record_cuda_error(e);
     return check_launch();
 }
@@ -388,7 +467,10 @@ static bool gemv_mma_plan(const kvq_gemv_args &a, int64_t n_pack, GemvPlan &p, i
     const int64_t tiles = (a.n_groups * a.group + 127) / 128;
     p.wk_log2 = tiles > 4 ? 0 : tiles > 2 ? 1 : tiles > 1 ? 2 : 3;
     const int wc = kGemvWarps >> p.wk_log2;
-    p.col_ctas = (int)((tiles + wc - 1) / wc);
+    // a warp's tiles one after the other where they are short (all rows in one chunk) and there are CTAs enough
+    p.tpw = 1;
+    while (p.wk_log2 == 0 && a.K <= kGemvTileRows && p.tpw < kGemvTiles && a.B * a.nh * ((tiles + 2 * wc * p.tpw - 1) / (2 * wc * p.tpw)) >= kGemvMinCtas) p.tpw *= 2;
+    p.col_ctas = (int)((tiles + (int64_t)wc * p.tpw - 1) / ((int64_t)wc * p.tpw));
     const int64_t jobs = a.B * a.nh * p.col_ctas;
     p.kc = 1;
     while (p.kc < 8 && jobs * p.kc * 2 <= 2 * 148 && a.K >= 512LL * p.kc * 2) p.kc *= 2;
@@ -398,8 +480,12 @@ static bool gemv_mma_plan(const kvq_gemv_args &a, int64_t n_pack, GemvPlan &p, i
     const int ngw = 128 / a.group;
     p.sz_vec = (reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.zero)) % (2 * ngw) == 0 &&
                a.s_sB % ngw == 0 && a.s_sH % ngw == 0 && a.s_sK % ngw == 0;
+    p.fast = p.code_align == 16 && p.sz_vec && a.q_sK >= 0 && a.s_sK >= 0 && a.K * a.q_sK < (1LL << 30) && a.K * a.s_sK < (1LL << 31) &&
+             a.q_sK < (1 << 24) && a.s_sK < (1 << 25);
+    p.rep = (int)(a.nh / a.nh_kv);
+    p.out_vec = (reinterpret_cast<uintptr_t>(a.out) | (uint64_t)(2 * (a.o_sB | a.o_sH))) % 8 == 0;
     grid = jobs * p.kc;
-    return grid <= 2147483647LL;
+    return grid <= 2147483647LL && a.B * a.nh <= 2147483647LL;
 }
 
 }  // namespace kvq
@@ -422,11 +508,12 @@ extern "C" int kvq_gemv(const kvq_gemv_args *a, kvq_stream_t stream) {
     GemvPlan p;
     int64_t mma_grid = 0;
     if (gemv_mma_plan(*a, n_pack, p, mma_grid)) {
-        switch (a->bits) {
-            case 1: return launch_gemv_mma<1>(*a, p, (unsigned)mma_grid, st);
-            case 2: return launch_gemv_mma<2>(*a, p, (unsigned)mma_grid, st);
-            default: return launch_gemv_mma<4>(*a, p, (unsigned)mma_grid, st);
-        }
+#define KVQ_GEMV_CASE(BITS, GS_LOG2) \
+        if (a->bits == BITS && a->group == 1 << GS_LOG2) return launch_gemv_mma<BITS, GS_LOG2>(*a, p, (unsigned)mma_grid, st);
+        KVQ_GEMV_CASE(1, 5) KVQ_GEMV_CASE(1, 6) KVQ_GEMV_CASE(1, 7)
+        KVQ_GEMV_CASE(2, 5) KVQ_GEMV_CASE(2, 6) KVQ_GEMV_CASE(2, 7)
+        KVQ_GEMV_CASE(4, 5) KVQ_GEMV_CASE(4, 6) KVQ_GEMV_CASE(4, 7)
+#undef KVQ_GEMV_CASE
     }
     int wx_log2 = 5;
     while (wx_log2 > 2 && (1 << (wx_log2 - 1)) >= n_pack) --wx_log2;
