@@ -150,7 +150,9 @@ __device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, kvq_attn_
         if ((v0 | v1 | v2 | v3 | v4) >= 0) publish = atomicAdd(reinterpret_cast<unsigned int *>(st + 5), 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    const int T0 = s_state[0], Tkq0 = s_state[1], Tvq0 = s_state[2], ks0 = s_state[3], vs0 = s_state[4];
+    // (as values the compiler knows to be the same in all lanes: loops over tokens then count in uniform registers)
+    auto same = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    const int T0 = same(s_state[0]), Tkq0 = same(s_state[1]), Tvq0 = same(s_state[2]), ks0 = same(s_state[3]), vs0 = same(s_state[4]);
     const int nk = tokens_due(a, T0 - Tkq0 + 1, a.k_group, a.k_ratio);
     const int nv = tokens_due(a, T0 - Tvq0 + 1, a.v_group, a.v_ratio);
     b.T = T0 + 1;

@@ -66,7 +66,7 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
 // fp16 key tail for tokens [lo, t1): 16-token tiles straight from global memory; B column n = query head n.
 __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half *kf, int b, int hk, const GqaSmem &sm,
                                             int t0, int lo, int t1) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     uint4 qf[4];
 #pragma unroll
     for (int S = 0; S < 4; ++S)
@@ -107,7 +107,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
                                               int tail_lo, int t1, int b, int hk) {
     using G = KGeom<KB>;
     using R = GqaKRing<KB>;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     constexpr int LGK = WIDE ? 7 : 6, NGW = KB == 3 ? 8 : G::WT >> LGK;         // groups of a tile: 8 (3 bits) / 2 / 4
     const int n_words = a.Tkq / G::FPI;
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;                         // <= 0: no packed keys in this segment
@@ -353,7 +353,7 @@ __device__ __forceinline__ void gqa_pv_packed(const kvq_attn_args &a, const int3
     constexpr int NB = G::GPT;                                // 16-byte blocks per token row: 1 / 2 / 4
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
     constexpr int MPB = F::N / 2;                             // MMAs per block: 8 / 4 / 2
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     constexpr int ngv = NGV, Gv = kHeadDim / NGV;             // channel groups: 4 / 2 / 1
     const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;
     const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
@@ -559,7 +559,7 @@ template <int MODE>
 __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int32_t *vc, const __half *vs, const __half *vz,
                                                const GqaSmem &sm, int t0, int hi) {
     constexpr int W = kV3Words;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int n_blocks = (hi - t0 + 31) / 32;
     const int my_blocks = (n_blocks - warp + kMmaWarps - 1) / kMmaWarps;
     float *my_red = reinterpret_cast<float *>(sm.ring);
@@ -758,7 +758,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
                                             int cnt, int n_whole, float *__restrict__ parts,
                                             unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     constexpr int kRegion = gqa_region_bytes<KB, VB>();
     GqaSmem sm;
     sm.n_scores = n_scores;

@@ -64,7 +64,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     using G = KGeom<KB>;
     using R = MmaKRing<KB, NW>;
     using F = Fields<KB>;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int n_words = a.Tkq / G::FPI;                       // valid code words per channel row
     const int n_tiles = (hi - t0 + G::WT - 1) / G::WT;
     const int split = warp & ((1 << sm.ks_log2) - 1), wt = warp >> sm.ks_log2, tile_lanes = NW >> sm.ks_log2;
@@ -363,7 +363,7 @@ __device__ __forceinline__ void pv_packed_mma(const kvq_attn_args &a, const int3
     constexpr int NB = G::GPT;                                // 16-byte blocks per token row: 1 / 2 / 4
     constexpr int CPB = kHeadDim / NB;                        // channels per block: 128 / 64 / 32
     constexpr int MPB = F::N / 2;                             // MMAs (channel pairs per octet) per block: 8 / 4 / 2
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     constexpr int ngv = NGV, Gv = kHeadDim / NGV;             // channel groups: 4 / 2 / 1
     const int n_blocks = (hi - t0 + G::TPS - 1) / G::TPS;      // <= 0: no packed values in this segment
     const int my_blocks = (n_blocks - warp + NW - 1) / NW;
@@ -563,7 +563,7 @@ __device__ __forceinline__ void pv_mma(const kvq_attn_args &a, const int32_t *vc
 template <int NW>
 __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half *kf, int b, int hk, const MmaSmem &sm,
                                             int t0, int lo, int t1) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     uint4 qf[4];
 #pragma unroll
     for (int S = 0; S < 4; ++S) qf[S] = *reinterpret_cast<const uint4 *>(sm.q + 32 * S + 8 * tig);
@@ -601,7 +601,7 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
                                              int cnt, int n_whole, float *__restrict__ parts,
                                              unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     MmaSmem sm;
     sm.n_scores = n_scores;
     sm.ks_log2 = ks_log2;
