@@ -47,7 +47,29 @@ __device__ __forceinline__ float attn_mask_at(const kvq_attn_args &a, int b, int
 // upstream clamps masked weights from below at torch.finfo(float32).min (models/modeling_llama_KVmix.py:192)
 constexpr float kMaskFloor = -3.4028234663852886e38f;
 
+// Programmatic launches: a kernel launched by launch_early() may be put on the GPU while the kernel before it in the stream is still
+// running its last CTAs, as soon as each of those has called launch_next(); grid_wait() then holds it until that kernel
+// is complete and its writes are visible.  Nothing before grid_wait() touches global memory.  Behind a kernel that does not call
+// launch_next() it is an ordinary launch.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 int record_cuda_error(cudaError_t e);
 inline int check_launch() { return record_cuda_error(cudaGetLastError()); }
+template <typename... P, typename... A>
+inline int launch_early(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    return e == cudaSuccess ? check_launch() : record_cuda_error(e);
+}
 
 }  // namespace kvq

@@ -838,6 +838,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     if (v_lo < t1) pv_tail<kQH>(a, vf, b, hk, sm.scores, n_scores, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();
 
+    launch_next();                                             // what is left is short: the next launch may come
+
     // ---- 4. finish / merge: a thread owns channel ch of head slots 2 hp, 2 hp + 1 -------------------------
     constexpr int kPart = kPartStride;
     const int ch = tid & (kHeadDim - 1), hp = tid >> 7, n_mine = max(0, min(2, qhv - 2 * hp));
@@ -939,6 +941,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_gqa_kernel(const _
                                                                      float *__restrict__ parts,
                                                                      unsigned int *__restrict__ counters) {
     int group, t0, t1, seg, cnt;
+    grid_wait();
     if constexpr (DEV) {                                       // device-resident cache state: see decode_attn_mma_kernel
         kvq_attn_args b = a;
         dev_state_step(a, b);
@@ -992,9 +995,10 @@ static int launch_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, flo
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     const unsigned grid = (unsigned)(plan.n_whole + plan.n_cut * plan.k);
-    if (VB != 3 && a.state) decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true><<<grid, kMmaThreads, smem, st>>>(a, plan, qhv, parts, counters);
-    else decode_attn_gqa_kernel<KB, VB, false><<<grid, kMmaThreads, smem, st>>>(a, plan, qhv, parts, counters);
-    return check_launch();
+    // launched early (grid_wait): four small layers of 4 x 8 kv heads x 1537 tokens from a host loop 69.5 -> 60.2 us, 131k tokens from a graph
+    // 407 -> 403; let in at the start of the kernel instead of behind p . V the next launch's CTAs cost more than they gain (66.7)
+    if (VB != 3 && a.state) return launch_early(decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
+    return launch_early(decode_attn_gqa_kernel<KB, VB, false>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
 }
 
 int launch_decode_attn_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, float *parts, unsigned int *counters,

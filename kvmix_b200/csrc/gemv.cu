@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
     const uint32_t lane_dst = ring_s + (lane / GPR) * G::RS + (lane % GPR) * 16;
     const char *qh_b = reinterpret_cast<const char *>(qh), *sh_b = reinterpret_cast<const char *>(sh), *zh_b = reinterpret_cast<const char *>(zh);
 
+    grid_wait();
+    launch_next();
     float acc[8][4], sum[8][2], accz[2][4] = {}, zsum = 0.f;
     auto clear = [&]() {
 #pragma unroll
@@ -447,12 +449,14 @@ static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned g
     cfg.blockDim = dim3(kGemvThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)p.kc;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = p.kc > 1 ? 1 : 0;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;            // see grid_wait()
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.kc;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.kc > 1 ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, gemv_mma_kernel<BITS, GS_LOG2>, a, p);
     if (e != cudaSuccess) return record_cuda_error(e);
     return check_launch();

@@ -19,6 +19,8 @@ __global__ void __launch_bounds__(256, 4) prefill_kernel(const __grid_constant__
                                                          const __grid_constant__ QuantDims vd, const __grid_constant__ RopeTables rope,
                                                          const __grid_constant__ PrefillGrid p) {
     int c = blockIdx.x;
+    grid_wait();
+    launch_next();
     if (c < p.k_ctas) {
         const int bh = c / p.k_tiles;
         quant_rope_tile<KB, KG>(static_cast<const __half *>(a.k), a.kcode, static_cast<__half *>(a.kscale), static_cast<__half *>(a.kmn), kd, rope, c - bh * p.k_tiles, bh);
@@ -50,8 +52,7 @@ static int launch_prefill(const kvq_prefill_args &a, const QuantDims &kd, const 
     if (k_ctas + v_ctas + t_ctas > 2147483647LL) return KVQ_ERR_UNSUPPORTED;
     p.k_ctas = (int)k_ctas;
     p.v_ctas = (int)v_ctas;
-    prefill_kernel<KB, KG, VB><<<(unsigned)(k_ctas + v_ctas + t_ctas), 256, 0, st>>>(a, kd, vd, rope, p);
-    return check_launch();
+    return launch_early(prefill_kernel<KB, KG, VB>, (unsigned)(k_ctas + v_ctas + t_ctas), 256, 0, st, a, kd, vd, rope, p);
 }
 
 // KVQ_ERR_UNSUPPORTED: not for this kernel.
