@@ -16,6 +16,20 @@
 
 namespace kvq {
 
+// Division by a number the host knows (1 .. 2^31), of numbers below 2^31: a high product, an addition and a shift where the compiler's
+// division takes some twenty-five instructions, several of them in a row at the start of every CTA.
+struct FastDiv {
+    uint32_t mul, shr, d;
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(n, mul) + n) >> shr; }
+#endif
+};
+inline FastDiv fast_div(uint32_t d) {
+    uint32_t s = 0;
+    while (s < 31 && (1u << s) < d) ++s;
+    return {(uint32_t)((((uint64_t)1 << 32) * (((uint64_t)1 << s) - d)) / d + 1), s, d};
+}
+
 struct AttnPlan {
     int unit;            // tokens per unit
     int uph;             // units per head
@@ -26,6 +40,9 @@ struct AttnPlan {
     int n_scores;        // most tokens in a segment, rounded up to 32
     int warps;           // warps of a CTA: 8 (two CTAs to an SM) or 4 (three or four)
     int ks_log2;         // the channels of a key tile are shared by 1 << ks_log2 warps (partial scores, summed by the softmax)
+    // how a CTA finds its place (plan_place): heads (or groups of them) per sequence, and those of a kv head
+    FastDiv by_cut, by_seq, by_kv;
+    int rep;             // query heads per kv head
 };
 
 constexpr int kSmCount = 148;
@@ -161,18 +178,41 @@ inline AttnPlan make_attn_plan_mma(int T, int unit, int tile, int max_scores, lo
 
 // CTA index -> (head, segment): whole heads first, then the cut heads segment-major (all first segments, then all
 // second segments, ...), so the shortest segments -- the last of each head -- come last.
-__host__ __device__ inline void plan_cta(const AttnPlan &p, int T, int c, int &head, int &t0, int &t1, int &seg, int &cnt) {
-    if (c < p.n_whole) {
-        head = c; t0 = 0; t1 = T; seg = 0; cnt = 1;
-        return;
+#ifdef __CUDACC__
+__device__ __forceinline__ void plan_head(const AttnPlan &p, int c, int &head, int &seg) {
+    head = c;
+    seg = 0;
+    if (c >= p.n_whole) {
+        const int cc = c - p.n_whole;
+        seg = (int)p.by_cut((uint32_t)cc);
+        head = p.n_whole + cc - seg * p.n_cut;
     }
-    const int cc = c - p.n_whole;
-    seg = cc / p.n_cut;
-    head = p.n_whole + cc - seg * p.n_cut;
-    cnt = p.k;
-    t0 = seg * p.seg_units * p.unit;
-    const int e = t0 + p.seg_units * p.unit;
-    t1 = e < T ? e : T;
+}
+// The tokens of segment `seg` of that head (of T), and how many segments the head has.
+__device__ __forceinline__ void plan_tokens(const AttnPlan &p, int T, int c, int seg, int &t0, int &t1, int &cnt) {
+    t0 = 0;
+    t1 = T;
+    cnt = 1;
+    if (c >= p.n_whole) {
+        cnt = p.k;
+        t0 = seg * p.seg_units * p.unit;
+        t1 = min(t0 + p.seg_units * p.unit, T);
+    }
+}
+// Head s -> sequence, kv head, number within the kv head.
+__device__ __forceinline__ void plan_place(const AttnPlan &p, int s, int &b, int &hk, int &within) {
+    b = (int)p.by_seq((uint32_t)s);
+    const uint32_t r = (uint32_t)s - b * p.by_seq.d;
+    hk = (int)p.by_kv(r);
+    within = (int)(r - hk * p.by_kv.d);
+}
+#endif
+// `per_kv` heads (or groups of them) of one kv head are neighbours.
+inline void plan_set_place(AttnPlan &p, int nh, int nh_kv, int per_kv) {
+    p.rep = nh / nh_kv;
+    p.by_cut = fast_div((uint32_t)(p.n_cut > 0 ? p.n_cut : 1));
+    p.by_kv = fast_div((uint32_t)per_kv);
+    p.by_seq = fast_div((uint32_t)per_kv * (uint32_t)nh_kv);
 }
 
 }  // namespace kvq

@@ -136,8 +136,18 @@ __device__ __forceinline__ int tokens_due(const kvq_attn_args &a, int cur, int g
     return 0;
 }
 
-__device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, kvq_attn_args &b) {
-    // One thread reads the state and counts the CTA in; the others take it from shared memory.  The state may be
+// Asked for by one thread first of all, used after whatever else the CTA can ask for meanwhile (q).
+struct DevState { int v[5]; };
+__device__ __forceinline__ DevState dev_state_load(const kvq_attn_args &a) {
+    DevState s = {};
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) s.v[i] = a.state[i];
+    }
+    return s;
+}
+__device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, const DevState &s, kvq_attn_args &b) {
+    // The thread that read the state counts the CTA in; the others take it from shared memory.  The state may be
     // overwritten once every CTA of the grid has read it: the count is raised only after the reading thread holds the
     // values (the branch on all five loaded values keeps it behind the loads), and the CTA that completes the count -- the last
     // one to START, so nothing is left on the tail of the kernel -- publishes the state after the step (below).
@@ -145,9 +155,10 @@ __device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, kvq_attn_
     int *st = a.state;
     bool publish = false;
     if (threadIdx.x == 0) {
-        const int v0 = st[0], v1 = st[1], v2 = st[2], v3 = st[3], v4 = st[4];
-        s_state[0] = v0; s_state[1] = v1; s_state[2] = v2; s_state[3] = v3; s_state[4] = v4;
-        if ((v0 | v1 | v2 | v3 | v4) >= 0) publish = atomicAdd(reinterpret_cast<unsigned int *>(st + 5), 1u) == gridDim.x - 1;
+        int all = 0;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) { s_state[i] = s.v[i]; all |= s.v[i]; }
+        if (all >= 0) publish = atomicAdd(reinterpret_cast<unsigned int *>(st + 5), 1u) == gridDim.x - 1;
     }
     __syncthreads();
     // (as values the compiler knows to be the same in all lanes: loops over tokens then count in uniform registers)

@@ -54,6 +54,15 @@ constexpr float kMaskFloor = -3.4028234663852886e38f;
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// Counts a CTA in, device-wide: what its threads wrote before the CTA barrier in front of it is visible to whoever reads the last count
+// and synchronises behind it.  One acquire-release atomic; between two __threadfence() (sequentially consistent ones) it took 2700
+// cycles at the end of every CTA, with its SM half idle.
+__device__ __forceinline__ unsigned int count_in(unsigned int *counter) {
+    unsigned int old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;\n" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}
+
 int record_cuda_error(cudaError_t e);
 inline int check_launch() { return record_cuda_error(cudaGetLastError()); }
 template <typename... P, typename... A>

@@ -754,12 +754,13 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of head group s (sequence b, kv head hk, quad of query heads); segment `seg` of `cnt`.
 template <int KB, int VB>
-__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int ks_log2, int qhv, int s, int t0, int t1, int seg,
-                                            int cnt, int n_whole, float *__restrict__ parts,
+__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, __half2 q_mine, const AttnPlan &plan, int qhv, int s, int b, int hk, int h_first, int t0, int t1,
+                                            int seg, int cnt, float *__restrict__ parts,
                                             unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     constexpr int kRegion = gqa_region_bytes<KB, VB>();
+    const int n_scores = plan.n_scores, ks_log2 = plan.ks_log2, n_whole = plan.n_whole;
     GqaSmem sm;
     sm.n_scores = n_scores;
     sm.ks_log2 = ks_log2;
@@ -769,20 +770,12 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     sm.q = reinterpret_cast<__half *>(after_scores + kMmaWarps * kRegion);
     sm.misc = reinterpret_cast<float *>(sm.q + kQH * kHeadDim);
 
-    const int n_rep = a.nh / a.nh_kv, nq = n_rep / qhv;                // quads per kv head
-    const int b = s / (a.nh_kv * nq), hk = (s / nq) % a.nh_kv, h_first = hk * n_rep + (s % nq) * qhv;
-
     const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
     const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
     const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
     prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, kMmaThreads);
     fused_cache_update<KB, VB, kMmaThreads>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
-    // q of the quad (head slots beyond qhv repeat the last head: their columns are computed and dropped)
-    {
-        const int slot = tid >> 6, hs = min(slot, qhv - 1);              // two warps store a head slot
-        const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + hs) * a.q_sH + 2 * (tid & 63);
-        *reinterpret_cast<__half2 *>(sm.q + slot * kHeadDim + 2 * (tid & 63)) = __halves2half2(q[0], q[1]);   // q rows start at any fp16
-    }
+    *reinterpret_cast<__half2 *>(sm.q + (tid >> 6) * kHeadDim + 2 * (tid & 63)) = q_mine;                  // two warps store a head slot
 
     // ---- 1. scores ------------------------------------------------------------------------------
     {
@@ -804,7 +797,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     const int h_mine = h_first + min(hs_mine, qhv - 1);
     float m = kMaskFloor;
     float4 *sc4 = reinterpret_cast<float4 *>(sm.scores + hs_mine * n_scores);
-#pragma unroll 2
+#pragma unroll 4
     for (int i = tid & 63; i < n4; i += 64) {
         float4 v = score_quad(a, sc4 + i, kQH * (n_scores >> 2), ks_log2);
         if (a.mask) mask_quad(a, b, h_mine, t0 + 4 * i, v);
@@ -817,7 +810,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     __syncthreads();
     m = fmaxf(sm.misc[2 * hs_mine], sm.misc[2 * hs_mine + 1]);
     float l = 0.f;
-#pragma unroll 2
+#pragma unroll 4
     for (int i = tid & 63; i < n4; i += 64) {
         float4 v = sc4[i];
         v.x = __expf(v.x - m);
@@ -879,9 +872,7 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     }
     __syncthreads();
     if (tid == 0) {
-        __threadfence();
-        sm.misc[16] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
-        __threadfence();
+        sm.misc[16] = count_in(&counters[s]) == (unsigned)(cnt - 1) ? 1.f : 0.f;
     }
     __syncthreads();
     if (sm.misc[16] == 0.f) return;
@@ -940,17 +931,26 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_gqa_kernel(const _
                                                                      const __grid_constant__ AttnPlan plan, int qhv,
                                                                      float *__restrict__ parts,
                                                                      unsigned int *__restrict__ counters) {
-    int group, t0, t1, seg, cnt;
     grid_wait();
+    DevState state;
+    if constexpr (DEV) state = dev_state_load(a);
+    int group, seg, b, hk, within, t0, t1, cnt;
+    plan_head(plan, blockIdx.x, group, seg);
+    plan_place(plan, group, b, hk, within);
+    const int h_first = hk * plan.rep + within * qhv;
+    // this thread's two channels of q (head slots beyond qhv repeat the last head: their columns are computed and dropped): the key
+    // phase waits for them, and nothing of them depends on the cache's state
+    const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)(h_first + min((int)threadIdx.x >> 6, qhv - 1)) * a.q_sH + 2 * (threadIdx.x & 63);
+    const __half2 q_mine = __halves2half2(q[0], q[1]);         // q rows start at any fp16
     if constexpr (DEV) {                                       // device-resident cache state: see decode_attn_mma_kernel
-        kvq_attn_args b = a;
-        dev_state_step(a, b);
-        plan_cta(plan, b.T, blockIdx.x, group, t0, t1, seg, cnt);
-        if (cnt > 1) cnt = min(cnt, (b.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < b.T) gqa_segment<KB, VB>(b, a, plan.n_scores, plan.ks_log2, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        kvq_attn_args d = a;
+        dev_state_step(a, state, d);
+        plan_tokens(plan, d.T, blockIdx.x, seg, t0, t1, cnt);
+        if (cnt > 1) cnt = min(cnt, (d.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
+        if (t0 < d.T) gqa_segment<KB, VB>(d, a, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
     } else {
-        plan_cta(plan, a.T, blockIdx.x, group, t0, t1, seg, cnt);
-        gqa_segment<KB, VB>(a, a, plan.n_scores, plan.ks_log2, qhv, group, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        plan_tokens(plan, a.T, blockIdx.x, seg, t0, t1, cnt);
+        gqa_segment<KB, VB>(a, a, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
     }
 }
 
@@ -979,8 +979,9 @@ template <int KB, int VB> constexpr int gqa_smem_bytes(int scores) {
 }
 
 template <int KB, int VB>
-static int launch_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, float *parts, unsigned int *counters,
+static int launch_gqa(const kvq_attn_args &a, AttnPlan plan, int qhv, float *parts, unsigned int *counters,
                       cudaStream_t st) {
+    plan_set_place(plan, a.nh, a.nh_kv, a.nh / a.nh_kv / qhv);
     static_assert(gqa_smem_bytes<KB, VB>(KB == 3 ? kGqaMaxScores3 : kGqaMaxScores) <= kMmaSmemMax, "two CTAs to an SM");
     const size_t smem = gqa_smem_bytes<KB, VB>(plan.n_scores << plan.ks_log2);
     static bool attr_set[64] = {};

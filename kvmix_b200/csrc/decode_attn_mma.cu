@@ -31,6 +31,9 @@
 
 namespace kvq {
 
+// Score buffers: of an eight-warp CTA, two to an SM; of a four-warp CTA, three to an SM, and four to an SM.
+constexpr int kWideScores = 6144, kWideScores3 = 7040, kNarrowMax = 8192, kNarrowMax3 = 8096, kNarrowScores = 5216;
+
 struct MmaSmem {
     float *scores;          // [1 << ks_log2][n_scores]
     unsigned char *ring;    // this warp's region
@@ -597,11 +600,11 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of query head (b, h); segment `seg` of the `cnt` the head is cut into.
 template <int KB, int VB, int NW>
-__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, int n_scores, int ks_log2, int s, int t0, int t1, int seg,
-                                             int cnt, int n_whole, float *__restrict__ parts,
-                                             unsigned int *__restrict__ counters) {
+__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, __half q_mine, const AttnPlan &plan, int s, int b, int h, int hk, int t0, int t1,
+                                             int seg, int cnt, float *__restrict__ parts, unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
+    const int n_scores = plan.n_scores, ks_log2 = plan.ks_log2, n_whole = plan.n_whole;
     MmaSmem sm;
     sm.n_scores = n_scores;
     sm.ks_log2 = ks_log2;
@@ -610,18 +613,13 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     sm.ring = after_scores + warp * warp_region_bytes<KB, VB, NW>();
     sm.q = reinterpret_cast<__half *>(after_scores + NW * warp_region_bytes<KB, VB, NW>());
     sm.misc = reinterpret_cast<float *>(sm.q + kHeadDim);
-    const int b = s / a.nh, h = s % a.nh;
-    // grouped queries: each query head is its own segment and reads kv head hk; the heads of one kv head are
-    // neighbouring units of work, so the cache is fetched from HBM once and re-read from L2
-    const int hk = h / (a.nh / a.nh_kv);
 
     const int v_hi = min(t1, a.Tvq), v_lo = max(t0, a.Tvq);
     const __half *vf = static_cast<const __half *>(a.vfull) + (int64_t)b * a.vf_sB + (int64_t)hk * a.vf_sH;
     const __half *kf = static_cast<const __half *>(a.kfull) + (int64_t)b * a.kf_sB + (int64_t)hk * a.kf_sH;
     prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, (32 * NW));
     fused_cache_update<KB, VB, 32 * NW>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
-    const __half *q = static_cast<const __half *>(a.q) + (int64_t)b * a.q_sB + (int64_t)h * a.q_sH;
-    if (tid < kHeadDim) sm.q[tid] = q[tid];
+    if (tid < kHeadDim) sm.q[tid] = q_mine;
 
     // ---- 1. scores ------------------------------------------------------------------------------
     {
@@ -644,12 +642,20 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     const int n = t1 - t0, n4 = (n + 3) >> 2;
     float m = kMaskFloor;                                      // a fully masked range then weighs uniformly, as upstream's does
     float4 *sc4 = reinterpret_cast<float4 *>(sm.scores);
-#pragma unroll 2
-    for (int i = tid; i < n4; i += (32 * NW)) {
-        float4 v = score_quad(a, sc4 + i, n_scores >> 2, ks_log2);
-        if (a.mask) mask_quad(a, b, h, t0 + 4 * i, v);
-        if (4 * i + 3 >= n) pad_quad(v, n - 4 * i);
-        sc4[i] = v;
+    // a thread's scores stay in registers between the maximum and the exponentials
+    constexpr int QN = ((NW == 8 ? kWideScores3 : kNarrowMax) + 128 * NW - 1) / (128 * NW);
+    float4 sv[QN];
+#pragma unroll
+    for (int j = 0; j < QN; ++j) {
+        if (32 * NW * j >= n4) break;
+        const int i = tid + 32 * NW * j;
+        float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        if (i < n4) {
+            v = score_quad(a, sc4 + i, n_scores >> 2, ks_log2);
+            if (a.mask) mask_quad(a, b, h, t0 + 4 * i, v);
+            if (4 * i + 3 >= n) pad_quad(v, n - 4 * i);
+        }
+        sv[j] = v;
         m = fmaxf(fmaxf(m, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
     m = warp_max(m);
@@ -658,14 +664,16 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     m = sm.misc[lane & (NW - 1)];
     m = warp_max(m);
     float l = 0.f;
-#pragma unroll 2
-    for (int i = tid; i < n4; i += (32 * NW)) {
-        float4 v = sc4[i];
+#pragma unroll
+    for (int j = 0; j < QN; ++j) {
+        if (32 * NW * j >= n4) break;
+        const int i = tid + 32 * NW * j;
+        float4 v = sv[j];
         v.x = __expf(v.x - m);
         v.y = __expf(v.y - m);
         v.z = __expf(v.z - m);
         v.w = __expf(v.w - m);
-        sc4[i] = v;
+        if (i < n4) sc4[i] = v;
         l += (v.x + v.y) + (v.z + v.w);
     }
     l = warp_sum(l);
@@ -702,11 +710,9 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     if (tid == 0) { part[kHeadDim] = m; part[kHeadDim + 1] = l_all; }
     __syncthreads();
     if (tid == 0) {
-        // one cumulative device-scope fence after the CTA barrier publishes every thread's partial before the count;
-        // the fence after the count orders the merging CTA's reads (ld.cg, from L2) behind the other CTAs' fences
-        __threadfence();
-        sm.misc[16] = (atomicAdd(&counters[s], 1u) == (unsigned)(cnt - 1)) ? 1.f : 0.f;
-        __threadfence();
+        // the CTA barrier and the count's release publish every thread's partial; its acquire orders the merging CTA's reads
+        // (ld.cg, from L2) behind the other CTAs' counts
+        sm.misc[16] = count_in(&counters[s]) == (unsigned)(cnt - 1) ? 1.f : 0.f;
     }
     __syncthreads();
     if (sm.misc[16] == 0.f) return;
@@ -748,17 +754,26 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) decode_attn_mma_kernel(const
                                                                      const __grid_constant__ AttnPlan plan,
                                                                      float *__restrict__ parts,
                                                                      unsigned int *__restrict__ counters) {
-    int head, t0, t1, seg, cnt;
     grid_wait();
+    DevState state;
+    if constexpr (DEV) state = dev_state_load(a);
+    // grouped queries: each query head is its own segment and reads kv head hk; the heads of one kv head are
+    // neighbouring units of work, so the cache is fetched from HBM once and re-read from L2
+    int head, seg, b, hk, within, t0, t1, cnt;
+    plan_head(plan, blockIdx.x, head, seg);
+    plan_place(plan, head, b, hk, within);
+    const int h = hk * plan.rep + within;
+    // this thread's channel of q: the key phase waits for it, and nothing of it depends on the cache's state
+    const __half q_mine = static_cast<const __half *>(a.q)[(int64_t)b * a.q_sB + (int64_t)h * a.q_sH + (threadIdx.x & (kHeadDim - 1))];
     if constexpr (DEV) {
-        kvq_attn_args b = a;
-        dev_state_step(a, b);
-        plan_cta(plan, b.T, blockIdx.x, head, t0, t1, seg, cnt);
-        if (cnt > 1) cnt = min(cnt, (b.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < b.T) attn_segment<KB, VB, NW>(b, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        kvq_attn_args d = a;
+        dev_state_step(a, state, d);
+        plan_tokens(plan, d.T, blockIdx.x, seg, t0, t1, cnt);
+        if (cnt > 1) cnt = min(cnt, (d.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
+        if (t0 < d.T) attn_segment<KB, VB, NW>(d, a, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
     } else {
-        plan_cta(plan, a.T, blockIdx.x, head, t0, t1, seg, cnt);
-        attn_segment<KB, VB, NW>(a, a, plan.n_scores, plan.ks_log2, head, t0, t1, seg, cnt, plan.n_whole, parts, counters);
+        plan_tokens(plan, a.T, blockIdx.x, seg, t0, t1, cnt);
+        attn_segment<KB, VB, NW>(a, a, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
     }
 }
 
@@ -797,16 +812,15 @@ bool mma_path_eligible(const kvq_attn_args &a) {
     return true;
 }
 
-// Score buffers: of an eight-warp CTA, two to an SM; of a four-warp CTA, three to an SM, and four to an SM.
-constexpr int kWideScores = 6144, kWideScores3 = 7040, kNarrowMax = 8192, kNarrowMax3 = 8096, kNarrowScores = 5216;
 
 template <int KB, int VB, int NW> constexpr int mma_smem_bytes(int scores) {
     return scores * 4 + NW * warp_region_bytes<KB, VB, NW>() + kHeadDim * 2 + 32 * 4;
 }
 
 template <int KB, int VB, int NW>
-static int launch_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,
+static int launch_mma(const kvq_attn_args &a, AttnPlan plan, float *parts, unsigned int *counters,
                       cudaStream_t st) {
+    plan_set_place(plan, a.nh, a.nh_kv, a.nh / a.nh_kv);
     constexpr int kSmSmem = 227 * 1024;                      // of an SM, 1 KB of it taken by every CTA
     static_assert(NW == 4 || mma_smem_bytes<KB, VB, 8>(KB == 3 ? kWideScores3 : kWideScores) <= kMmaSmemMax, "two eight-warp CTAs");
     static_assert(NW == 8 || 3 * (mma_smem_bytes<KB, VB, 4>(KB == 3 ? kNarrowMax3 : kNarrowMax) + 1024) <= kSmSmem, "three four-warp CTAs");
