@@ -146,19 +146,18 @@ __device__ __forceinline__ DevState dev_state_load(const kvq_attn_args &a) {
     }
     return s;
 }
-__device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, const DevState &s, kvq_attn_args &b) {
+// -> what the CTA's count returned to the thread that asked for the state (dev_state_publish).
+__device__ __forceinline__ unsigned int dev_state_step(const kvq_attn_args &a, const DevState &s, kvq_attn_args &b) {
     // The thread that read the state counts the CTA in; the others take it from shared memory.  The state may be
     // overwritten once every CTA of the grid has read it: the count is raised only after the reading thread holds the
-    // values (the branch on all five loaded values keeps it behind the loads), and the CTA that completes the count -- the last
-    // one to START, so nothing is left on the tail of the kernel -- publishes the state after the step (below).
+    // values (the branch on all five loaded values keeps it behind the loads).
     __shared__ int s_state[5];
-    int *st = a.state;
-    bool publish = false;
+    unsigned int before = 0;
     if (threadIdx.x == 0) {
         int all = 0;
 #pragma unroll
         for (int i = 0; i < 5; ++i) { s_state[i] = s.v[i]; all |= s.v[i]; }
-        if (all >= 0) publish = atomicAdd(reinterpret_cast<unsigned int *>(st + 5), 1u) == gridDim.x - 1;
+        if (all >= 0) before = atomicAdd(reinterpret_cast<unsigned int *>(a.state + 5), 1u);
     }
     __syncthreads();
     // (as values the compiler knows to be the same in all lanes: loops over tokens then count in uniform registers)
@@ -175,7 +174,14 @@ __device__ __forceinline__ void dev_state_step(const kvq_attn_args &a, const Dev
     b.v_quant = nv;
     b.k_quant_slot = ks0;
     b.v_quant_slot = vs0;
-    if (publish) {
+    return before;
+}
+
+// The CTA that completed the count -- the last one to START -- publishes the state after the step; not right behind the count, whose
+// answer takes as long as the state did, but when it has long been there.
+__device__ __forceinline__ void dev_state_publish(const kvq_attn_args &a, const kvq_attn_args &b, unsigned int before) {
+    if (threadIdx.x == 0 && before == gridDim.x - 1) {
+        int *st = a.state;
         st[0] = b.T; st[1] = b.Tkq; st[2] = b.Tvq; st[3] = b.kf_start; st[4] = b.vf_start;
         st[5] = 0;
     }

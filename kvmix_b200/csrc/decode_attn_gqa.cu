@@ -754,7 +754,7 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of head group s (sequence b, kv head hk, quad of query heads); segment `seg` of `cnt`.
 template <int KB, int VB>
-__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, __half2 q_mine, const AttnPlan &plan, int qhv, int s, int b, int hk, int h_first, int t0, int t1,
+__device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, unsigned int before, __half2 q_mine, const AttnPlan &plan, int qhv, int s, int b, int hk, int h_first, int t0, int t1,
                                             int seg, int cnt, float *__restrict__ parts,
                                             unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -830,6 +830,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
     __syncwarp();
     if (v_lo < t1) pv_tail<kQH>(a, vf, b, hk, sm.scores, n_scores, t0, v_lo, t1, reinterpret_cast<float *>(sm.ring), warp, kMmaWarps, lane);
     __syncthreads();
+
+    if (ac.state) dev_state_publish(ac, a, before);
 
     launch_next();                                             // what is left is short: the next launch may come
 
@@ -944,13 +946,14 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_gqa_kernel(const _
     const __half2 q_mine = __halves2half2(q[0], q[1]);         // q rows start at any fp16
     if constexpr (DEV) {                                       // device-resident cache state: see decode_attn_mma_kernel
         kvq_attn_args d = a;
-        dev_state_step(a, state, d);
+        const unsigned int before = dev_state_step(a, state, d);
         plan_tokens(plan, d.T, blockIdx.x, seg, t0, t1, cnt);
         if (cnt > 1) cnt = min(cnt, (d.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < d.T) gqa_segment<KB, VB>(d, a, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
+        if (t0 < d.T) gqa_segment<KB, VB>(d, a, before, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
+        else dev_state_publish(a, d, before);
     } else {
         plan_tokens(plan, a.T, blockIdx.x, seg, t0, t1, cnt);
-        gqa_segment<KB, VB>(a, a, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
+        gqa_segment<KB, VB>(a, a, 0u, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
     }
 }
 

@@ -600,7 +600,7 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of query head (b, h); segment `seg` of the `cnt` the head is cut into.
 template <int KB, int VB, int NW>
-__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, __half q_mine, const AttnPlan &plan, int s, int b, int h, int hk, int t0, int t1,
+__device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_attn_args &ac, unsigned int before, __half q_mine, const AttnPlan &plan, int s, int b, int h, int hk, int t0, int t1,
                                              int seg, int cnt, float *__restrict__ parts, unsigned int *__restrict__ counters) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
@@ -620,6 +620,8 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
     prefetch_tails(a, kf, vf, b, hk, t0, t1, tid, (32 * NW));
     fused_cache_update<KB, VB, 32 * NW>(a, b, hk, t0, t1, tid);        // the step's own cache update, when the caller fused it in
     if (tid < kHeadDim) sm.q[tid] = q_mine;
+
+    if (ac.state) dev_state_publish(ac, a, before);
 
     // ---- 1. scores ------------------------------------------------------------------------------
     {
@@ -767,13 +769,14 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) decode_attn_mma_kernel(const
     const __half q_mine = static_cast<const __half *>(a.q)[(int64_t)b * a.q_sB + (int64_t)h * a.q_sH + (threadIdx.x & (kHeadDim - 1))];
     if constexpr (DEV) {
         kvq_attn_args d = a;
-        dev_state_step(a, state, d);
+        const unsigned int before = dev_state_step(a, state, d);
         plan_tokens(plan, d.T, blockIdx.x, seg, t0, t1, cnt);
         if (cnt > 1) cnt = min(cnt, (d.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < d.T) attn_segment<KB, VB, NW>(d, a, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
+        if (t0 < d.T) attn_segment<KB, VB, NW>(d, a, before, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
+        else dev_state_publish(a, d, before);
     } else {
         plan_tokens(plan, a.T, blockIdx.x, seg, t0, t1, cnt);
-        attn_segment<KB, VB, NW>(a, a, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
+        attn_segment<KB, VB, NW>(a, a, 0u, q_mine, plan, head, b, h, hk, t0, t1, seg, cnt, parts, counters);
     }
 }
 
