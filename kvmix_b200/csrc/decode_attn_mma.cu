@@ -15,7 +15,7 @@
 // Keys (codes [D, T/fpi], one word = fpi tokens of one channel; scale/zero [D, T/G]):
 //   A (16x16) = codes, rows = tokens, cols = 16 channels.  q[d]*scale[d,g] is carried as an exact fp16 pair hi + lo.
 //   A 256-token warp tile is worked as two halves whose MMA rows touch at most four groups, so B (16x8) holds
-//   {hi, lo} x 4 groups side by side and one MMA per code tile yields both parts.  3-bit keys (88-token tiles, every
+//   {hi, lo} x 4 groups side by side and one MMA per code tile yields both parts.  3-bit keys (176-token tiles, every
 //   word its own group of 11) multiply each code tile by the hi and by the lo operand instead.  The zero terms
 //   sum_d q[d]*zero[d,g] of all groups of a tile come from one MMA per 16 channels whose A operand is the zero tile
 //   read transposed (row = group) and whose B operand is q.
@@ -34,6 +34,16 @@ namespace kvq {
 // Score buffers: of an eight-warp CTA, two to an SM; of a four-warp CTA, three to an SM, and four to an SM.
 constexpr int kWideScores = 6144, kWideScores3 = 7040, kNarrowMax = 8192, kNarrowMax3 = 8096, kNarrowScores = 5216;
 
+// Key geometry of this kernel.  3 bits: two words (two groups) an octet, a tile of 176 tokens worked 16 channels a stage: with one
+// word an octet, 88 tokens, what a k-step does once -- q, addresses, copies, loop -- was a third of its instructions, and a channel
+// row was fetched 32 bytes at a time (64 x 32 heads of 4096 tokens, 2-bit values, a step: 294 -> 289 us; 8 x 32: 52.9 -> 52.0).
+template <int KB> struct MmaKGeom : KGeom<KB> { static constexpr int SZ = 2 * KGeom<KB>::ROWS * 16; };
+template <> struct MmaKGeom<3> {
+    static constexpr int FPI = 11, WPL = 2, TPO = 11, WT = 176, KSPS = 1, NSTAGE = 8, NMMA = 12;
+    static constexpr int RB = 64, RS = RB + 16, ROWS = 16, CODE_BYTES = ROWS * RS, GPR = RB / 16, GPL = ROWS * GPR / 32, RPI = 32 / GPR;
+    static constexpr int SZ = 2 * ROWS * 32;                           // [half of the tile][scales, zeros][channel][8 groups]
+};
+
 struct MmaSmem {
     float *scores;          // [1 << ks_log2][n_scores]
     unsigned char *ring;    // this warp's region
@@ -43,7 +53,11 @@ struct MmaSmem {
 };
 // Rings of a CTA of NW warps: the scale rows, then the zero rows of a stage, 16 B each, follow its codes.  Four warps: sized so
 // that four CTAs fit an SM next to 5000 scores each.
-template <int KB, int NW> using MmaKRing = KRing<KB, 2 * KGeom<KB>::ROWS * 16, (KB == 2 ? 3 : 4) - (NW == 4)>;
+template <int KB, int NW> struct MmaKRing {
+    static constexpr int NS = (KB == 2 ? 3 : 4) - (NW == 4), P = NS - 1;
+    static constexpr int STAGE_BYTES = MmaKGeom<KB>::CODE_BYTES + MmaKGeom<KB>::SZ;
+    static constexpr int BYTES = NS * STAGE_BYTES;
+};
 template <int VB, int NW> using MmaVGeom = VGeom<VB, (VB == 4 ? 4 : VB == 2 ? 6 : 8) - (NW == 4 && VB != 1)>;
 template <int KB, int VB, int NW> constexpr int warp_region_bytes() {
     return MmaKRing<KB, NW>::BYTES > MmaVGeom<VB, NW>::WARP_BYTES ? MmaKRing<KB, NW>::BYTES : MmaVGeom<VB, NW>::WARP_BYTES;
@@ -64,7 +78,7 @@ template <int KB, int NW, int LGK>
 __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const MmaSmem &sm, int t0, int hi,
                                               const __half *kf, int tail_lo, int t1, int b, int hk) {
-    using G = KGeom<KB>;
+    using G = MmaKGeom<KB>;
     using R = MmaKRing<KB, NW>;
     using F = Fields<KB>;
     const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
@@ -80,7 +94,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     const uint32_t ring_s = smem_u32(sm.ring);
     const int gr = lane % G::GPR, row0 = lane / G::GPR;
     const uint32_t cp_dst = ring_s + row0 * G::RS + gr * 16;                   // + slot*STAGE + i*RPI*RS
-    // 3-bit: octet g owns the word of group g (11 tokens), fetched with plain 32-bit loads.
+    // 3-bit: octet g owns the word of group g (11 tokens) of either half of the tile, fetched with plain 32-bit loads.
     // Other widths: code fragments come from transposing ldmatrix loads.  A channel row of the tile is NBK blocks of
     // 16 bytes; one x4 load covers channel rows 16 ksx + (0..7 | 8..15) x two neighbouring blocks and hands lane
     // (g, tig) the half-word g of each block for the channel pair (2 tig, 2 tig + 1) [+8]: an A-fragment register pair
@@ -97,7 +111,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     // ldmatrix.x4 row addresses: lanes 0-7 scale rows 0..7 of a k-step, 8-15 scale rows 8..15, 16-31 the same of the zero rows
     const uint32_t ldm_s = ring_s + G::CODE_BYTES + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16 + (lane >> 4) * (G::ROWS * 16);
     const uint32_t q_s = smem_u32(sm.q) + (ch0 + 2 * tig) * 2;                 // + 32 per k-step [+16]
-    constexpr int ngw = KB == 3 ? 8 : G::WT >> LGK;                            // groups per warp tile: 8 / 4 / 2
+    constexpr int ngw = KB == 3 ? 16 : G::WT >> LGK;                           // groups per warp tile: 16 / 8 / 4 / 2
     const uint32_t szcp_dst = ring_s + G::CODE_BYTES + lane * 16;                  // one granule per lane (16 channels a stage) or two
     const int tile_words = tile_lanes * G::WT / G::FPI;                        // word-column distance between my tiles
     const int tile_groups = tile_lanes * ngw;
@@ -114,6 +128,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
     uint32_t iss_slot = 0, slot = 0;                                            // byte offsets of the slot being filled / read
     bool iss_ok = iss_col < n_words;
+    int iss_second = n_words - ((t0 + wt * G::WT) / G::FPI + 8);                // 3 bits: > 0: the second half of the tile's groups exists
 
     const char *kc_b = reinterpret_cast<const char *>(kc), *kz_b = reinterpret_cast<const char *>(kz);
     const uint32_t row_step = (uint32_t)(G::RPI * 4) * kc_sD, stage_step = (uint32_t)(G::ROWS * 4) * kc_sD, sz_step = (uint32_t)(G::ROWS * 2) * ks_sD;
@@ -127,7 +142,10 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                     cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, kc_b + (iss + i * row_step));
             }
             const uint32_t d = szcp_dst + iss_slot;
-            if (ngw == 8) { cp_async<16>(d, sz_b + iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, kz_b + iss_s); }
+            if (KB == 3) {
+                cp_async<16>(d, sz_b + iss_s);
+                if (iss_second > 0) cp_async<16>(d + G::SZ / 2, sz_b + (iss_s + 16));
+            } else if (ngw == 8) { cp_async<16>(d, sz_b + iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, kz_b + iss_s); }
             else if (ngw == 4) { cp_async<8>(d, sz_b + iss_s); if (!kOneSz) cp_async<8>(d + G::ROWS * 16, kz_b + iss_s); }
             else { cp_async<4>(d, sz_b + iss_s); if (!kOneSz) cp_async<4>(d + G::ROWS * 16, kz_b + iss_s); }
         }
@@ -141,6 +159,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
             iss_s += tile_sz_step;
             iss_col += tile_words;
             iss_ok = iss_col < n_words;
+            iss_second -= tile_words;
             --iss_tiles;
         }
     };
@@ -162,7 +181,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
         // 3-bit keys: b0 = hi and b1 = lo of the eight groups of the tile, every code tile is multiplied by both.
         // Other widths: b0 / b1 serve the first / second half of the tile; column n carries group (n / 2) of that
         // half, hi in even and lo in odd columns, so one MMA per code tile yields both parts.
-        float zsum = 0.f;
+        float zsum = 0.f, zsum3 = 0.f;                         // (3 bits: of the halves of the tile)
         constexpr int gph = ngw / 2;                           // groups per half tile: 4 / 2 / 1
         const int src0 = 4 * ((g >> 1) % gph) + tig;           // lane holding group (n / 2) of the first half
         const int src1 = src0 + 4 * (ngw / 2);
@@ -174,7 +193,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
 
 #pragma unroll 1
         for (int it = 0; it < steps; ++it) {
-          float accz[4] = {0.f, 0.f, 0.f, 0.f};               // zero terms of two k-steps
+          float accz[4] = {0.f, 0.f, 0.f, 0.f}, accz3[4] = {0.f, 0.f, 0.f, 0.f};      // zero terms of two k-steps
 #pragma unroll
           for (int s2 = 0; s2 < 2 / G::KSPS; ++s2) {
             issue_stage();
@@ -186,6 +205,36 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                 const uint32_t q01u = lds32(q_cur), q89u = lds32(q_cur + 16);
                 q_cur += 32;
                 const __half2 q01 = as_h2(q01u), q89 = as_h2(q89u);
+                if constexpr (KB == 3) {
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        uint32_t r0, r1, r2, r3;               // scales and zeros of this half's eight groups, see below
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(ldm_s + slot + hf * (G::SZ / 2)));
+                        if (hf) mma16816(accz3, r2, 0u, r3, 0u, q01u, q89u);
+                        else mma16816(accz, r2, 0u, r3, 0u, q01u, q89u);
+                        const __half2 s01 = as_h2(r0), s89 = as_h2(r1);
+                        const __half2 p01 = __hmul2(q01, s01), p89 = __hmul2(q89, s89);
+                        const uint32_t hi0 = as_u32(p01), hi1 = as_u32(p89);
+                        const uint32_t lo0 = as_u32(__hfma2(q01, s01, __hneg2(p01))), lo1 = as_u32(__hfma2(q89, s89, __hneg2(p89)));
+                        uint32_t w[4];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) w[r] = lds32(src + 32 * hf + ((r & 1) + (r >> 1) * 8) * G::RS);
+                        uint32_t rlo[F::N], rhi[F::N];
+                        F::unpack(w[0], w[1], rlo);
+                        F::unpack(w[2], w[3], rhi);
+#pragma unroll
+                        for (int i = 0; i < F::N; i += 2) {
+                            const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
+                            mma16816(acc[6 * hf + i / 2], rlo[i], a1, rhi[i], a3, hi0, hi1);
+                        }
+#pragma unroll
+                        for (int i = 0; i < F::N; i += 2) {
+                            const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
+                            mma16816(acc[6 * hf + i / 2], rlo[i], a1, rhi[i], a3, lo0, lo1);
+                        }
+                    }
+                } else {
                 // the tile rows are 8 groups x fp16 = one 8x8 matrix per 8 channels: a transposing ldmatrix hands
                 // lane (g, tig) exactly {row 2tig, row 2tig+1} x column g, i.e. its B-fragment pairs of group g, in one go
                 // (with fewer than 8 groups per tile the columns past the last group are stale and feed unused columns)
@@ -198,37 +247,13 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                 // two MMAs (the tensor core truncates as it accumulates).  A stale group only spoils its own row.
                 mma16816(accz, r2, 0u, r3, 0u, q01u, q89u);
                 uint32_t b0[2], b1[2];
-                if constexpr (KB == 3) {
-                    const __half2 s01 = as_h2(r0), s89 = as_h2(r1);
-                    const __half2 p01 = __hmul2(q01, s01), p89 = __hmul2(q89, s89);
-                    b0[0] = as_u32(p01);
-                    b0[1] = as_u32(p89);
-                    b1[0] = as_u32(__hfma2(q01, s01, __hneg2(p01)));
-                    b1[1] = as_u32(__hfma2(q89, s89, __hneg2(p89)));
-                } else {
+                {
                     b0[0] = hilo(q01, as_h2(__shfl_sync(0xffffffffu, r0, src0)), neg_mask);
                     b0[1] = hilo(q89, as_h2(__shfl_sync(0xffffffffu, r1, src0)), neg_mask);
                     b1[0] = hilo(q01, as_h2(__shfl_sync(0xffffffffu, r0, src1)), neg_mask);
                     b1[1] = hilo(q89, as_h2(__shfl_sync(0xffffffffu, r1, src1)), neg_mask);
                 }
-                if constexpr (KB == 3) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) w[r] = lds32(src + (k * 16 + (r & 1) + (r >> 1) * 8) * G::RS);
-                    uint32_t rlo[F::N], rhi[F::N];
-                    F::unpack(w[0], w[1], rlo);
-                    F::unpack(w[2], w[3], rhi);
-#pragma unroll
-                    for (int i = 0; i < F::N; i += 2) {
-                        const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
-                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b0[0], b0[1]);
-                    }
-#pragma unroll
-                    for (int i = 0; i < F::N; i += 2) {
-                        const uint32_t a1 = (i + 1 < F::N) ? rlo[i + 1] : 0u, a3 = (i + 1 < F::N) ? rhi[i + 1] : 0u;
-                        mma16816(acc[i / 2], rlo[i], a1, rhi[i], a3, b1[0], b1[1]);
-                    }
-                } else if constexpr (KB == 4) {
+                if constexpr (KB == 4) {
                     // 4-bit keys: two words (16 tokens) per octet and half, plain 64-bit loads + byte permutes (measured 1.5 %
                     // faster than the ldmatrix form below for this width: 4 loads of 2 blocks each per k-step)
                     constexpr int NF = F::N;
@@ -275,29 +300,33 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                         }
                     }
                 }
+                }
             }
             __syncwarp();                                      // the slot may be refilled
             slot = slot == (R::NS - 1) * R::STAGE_BYTES ? 0u : slot + R::STAGE_BYTES;
           }
           zsum += accz[0];
+          zsum3 += accz3[0];
         }
 
         float *dst0 = sm.scores + split * sm.n_scores - t0;
         // ---- epilogue ----------------------------------------------------------------------------------
         if constexpr (KB == 3) {
             // the octet's column is n = g, held by the lane with tig == g/2
-            const int tok0 = tile0 + g * G::TPO;               // first token of this octet's chunk
-            if (tok0 < hi && tig == (g >> 1)) {                // chunks are whole or absent (hi is a group multiple)
-                const bool sel = g & 1;
-                const float corr = zsum;                    // row g of the zero-term product = group g = this octet's word
-                float *dst = dst0 + tok0;
 #pragma unroll
-                for (int m = 0; m < G::NMMA; ++m) {
-                    const int i0 = 2 * m, i1 = 2 * m + 1;
-                    float s0 = fmaf(sel ? acc[m][1] : acc[m][0], (float)(1 << (24 - F::pos(i0 % F::N))), corr);
-                    float s1 = (i1 < G::TPO) ? fmaf(sel ? acc[m][3] : acc[m][2], (float)(1 << (24 - F::pos(i1 % F::N))), corr) : 0.f;
-                    dst[i0] = s0;
-                    if (i1 < G::TPO) dst[i1] = s1;
+            for (int hf = 0; hf < 2; ++hf) {
+                const int tok0 = tile0 + 88 * hf + g * G::TPO;     // first token of this octet's word of the half
+                if (tok0 < hi && tig == (g >> 1)) {            // words are whole or absent (hi is a group multiple)
+                    const bool sel = g & 1;
+                    const float corr = hf ? zsum3 : zsum;      // row g of the zero-term product = group g = this octet's word
+                    float *dst = dst0 + tok0;
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) {
+                        const int i0 = 2 * m, i1 = 2 * m + 1;
+                        const float *c = acc[6 * hf + m];
+                        dst[i0] = fmaf(sel ? c[1] : c[0], (float)(1 << (24 - F::pos(i0))), corr);
+                        if (i1 < G::TPO) dst[i1] = fmaf(sel ? c[3] : c[2], (float)(1 << (24 - F::pos(i1 % F::N))), corr);
+                    }
                 }
             }
         } else if constexpr (KB == 4) {
@@ -865,7 +894,7 @@ int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *
 
 // Plan of the tensor-core kernel for B * nh query heads (one head per segment).
 AttnPlan plan_attn_mma(int T, int k_bits, long long heads) {
-    return k_bits == 3 ? make_attn_plan_mma(T, 352, KGeom<3>::WT, kWideScores3, heads, kNarrowMax3, kNarrowScores, 1760)
+    return k_bits == 3 ? make_attn_plan_mma(T, 352, MmaKGeom<3>::WT, kWideScores3, heads, kNarrowMax3, kNarrowScores, 1760)
                        : make_attn_plan_mma(T, 256, KGeom<4>::WT, kWideScores, heads, kNarrowMax, kNarrowScores, 3072);
 }
 
