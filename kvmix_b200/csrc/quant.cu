@@ -24,13 +24,17 @@
 namespace kvq {
 
 // ---------------------------------------------------------------------------------------------
-// Contiguous groups: blockIdx.y = (b, h); inside a (b, h) slab units of WPT words are numbered linearly.
+// Contiguous groups: blockIdx.y = (b, h); inside a (b, h) slab units of WPT words are numbered linearly.  A thread takes `upt` of them
+// where there are CTAs enough: what it does once (addresses, constants in register pairs) is as much as 13 elements' work.
 template <int BITS, typename T, int WPT>
 __global__ void __launch_bounds__(256) quant_contig_kernel(const T *__restrict__ x, int32_t *__restrict__ code,
                                                            T *__restrict__ scale, T *__restrict__ mn, QuantDims d,
-                                                           int tpg, bool vec_ok, bool linear) {
-    quant_contig_unit<BITS, T, WPT>(x, code, scale, mn, d, tpg, vec_ok, linear, blockIdx.y / (int)d.H, blockIdx.y % (int)d.H,
-                                    blockIdx.x * blockDim.x + threadIdx.x);
+                                                           int tpg, bool vec_ok, bool linear, int upt) {
+    const int b = blockIdx.y / (int)d.H, h = blockIdx.y - b * (int)d.H, total = (int)(d.A * (d.S / (fields_per_word(BITS) * WPT)));
+    int idx = blockIdx.x * (256 * upt) + threadIdx.x;
+#pragma unroll 1
+    for (int k = 0; k < upt && idx - (int)threadIdx.x < total; ++k, idx += 256)
+        quant_contig_unit<BITS, T, WPT>(x, code, scale, mn, d, tpg, vec_ok, linear, b, h, idx);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -45,7 +49,9 @@ struct StridedCfg {
     static constexpr int WPAD = WPC + 1;
 };
 
-template <int BITS, int G>
+// ROWS128: tokens lie 128 elements apart (keys as [.., T, 128], back to back), so that the loads of a group differ by immediates: the
+// addresses were an eighth of the kernel's instructions.
+template <int BITS, int G, bool ROWS128>
 __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__restrict__ x, int32_t *__restrict__ code,
                                                             __half *__restrict__ scale, __half *__restrict__ mn,
                                                             QuantDims d) {
@@ -63,7 +69,11 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
     const __half *px = x + b * d.x_sB + h * d.x_sH + (a0 + 2 * pair);
     constexpr int QMAX = (1 << BITS) - 1;
     // element pair (2 pair, 2 pair + 1) of token s of this (b, h) slab
-    auto load = [&](int64_t s) -> __half2 { return __ldg(reinterpret_cast<const __half2 *>(px + s * d.x_sS)); };
+    const int64_t row = ROWS128 ? 128 : d.x_sS;
+    auto load = [&](const __half *pg, int i) -> __half2 {
+        if constexpr (ROWS128) return __ldg(reinterpret_cast<const __half2 *>(pg) + i * 64);
+        else return __ldg(reinterpret_cast<const __half2 *>(pg + i * row));
+    };
 
     // tokens held in registers at a time: a whole group up to 32 tokens; longer groups are walked twice anyway (min/max,
     // then codes from L1/L2), and for them 16 at a time measured 5-10 % faster for 2- and 4-bit codes (fewer live
@@ -72,7 +82,7 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
     constexpr int NCH = G / CH;
     constexpr int WPCH = CH / C::FPI;                         // words per chunk (1 for the 11-token group)
     for (int g = slot; g < groups_here; g += 4) {
-        const int64_t s0 = (g0 + g) * G;                      // first token of the group
+        const __half *pg = px + (g0 + g) * G * row;           // the group's first token
         __half2 raw[CH];
         // min / max of the two channels in fp16x2 (exact: the data are fp16; NaN operands are skipped as by fminf)
         __half2 lo2 = __floats2half2_rn(65504.f, 65504.f), hi2 = __floats2half2_rn(-65504.f, -65504.f);
@@ -80,7 +90,7 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
 #pragma unroll 1
         for (int c = 0; c < NCH; ++c) {
 #pragma unroll
-            for (int i = 0; i < CH; ++i) raw[i] = load(s0 + c * CH + i);
+            for (int i = 0; i < CH; ++i) raw[i] = load(pg + c * CH * row, i);
             if (first) { lo2 = raw[0]; hi2 = raw[0]; first = false; }
 #pragma unroll
             for (int i = 0; i < CH; ++i) { lo2 = __hmin2(lo2, raw[i]); hi2 = __hmax2(hi2, raw[i]); }
@@ -92,7 +102,7 @@ __global__ void __launch_bounds__(256, 3) quant_strided_kernel(const __half *__r
         for (int c = 0; c < NCH; ++c) {
             if (NCH > 1) {                                    // long groups: second pass over the chunk (cache hit)
 #pragma unroll
-                for (int i = 0; i < CH; ++i) raw[i] = load(s0 + c * CH + i);
+                for (int i = 0; i < CH; ++i) raw[i] = load(pg + c * CH * row, i);
             }
 #pragma unroll
             for (int w = 0; w < WPCH; ++w) {
@@ -228,9 +238,11 @@ static int launch_bits(const kvq_quant_args *a, const QuantDims &d, cudaStream_t
         if (tpg <= 32 && (tpg & (tpg - 1)) == 0 && per_slab < (1LL << 31) && d.B * d.H <= 65535) {
             const int64_t wpr = d.S / E;
             const bool linear = d.x_sA == d.S && d.c_sA == wpr && d.z_sA == d.S / G;
-            dim3 grid((unsigned)((per_slab + 255) / 256), (unsigned)(d.B * d.H));
-            if (wide) quant_contig_kernel<BITS, T, WMAX><<<grid, 256, 0, st>>>(x, a->code, sc, mn, d, tpg, vec_ok, linear);
-            else quant_contig_kernel<BITS, T, 1><<<grid, 256, 0, st>>>(x, a->code, sc, mn, d, tpg, vec_ok, linear);
+            // four units a thread from eight waves of CTAs on (eight to an SM)
+            const int upt = (per_slab + 255) / 256 * d.B * d.H >= 8 * 8 * 148 && per_slab >= 4096 && per_slab < (1LL << 30) ? 4 : 1;
+            dim3 grid((unsigned)((per_slab + 256 * upt - 1) / (256 * upt)), (unsigned)(d.B * d.H));
+            if (wide) quant_contig_kernel<BITS, T, WMAX><<<grid, 256, 0, st>>>(x, a->code, sc, mn, d, tpg, vec_ok, linear, upt);
+            else quant_contig_kernel<BITS, T, 1><<<grid, 256, 0, st>>>(x, a->code, sc, mn, d, tpg, vec_ok, linear, upt);
             return check_launch();
         }
     }
@@ -251,7 +263,8 @@ static int launch_bits(const kvq_quant_args *a, const QuantDims &d, cudaStream_t
             grid.x = (unsigned)((ng + RopeCfg<BITS, GG>::GPC - 1) / RopeCfg<BITS, GG>::GPC);       \
             quant_rope_kernel<BITS, GG><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d, *rope);      \
         } else {                                                                                   \
-            quant_strided_kernel<BITS, GG><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d);          \
+            if (d.x_sS == 128) quant_strided_kernel<BITS, GG, true><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d); \
+            else quant_strided_kernel<BITS, GG, false><<<grid, 256, 0, st>>>(xh, a->code, sh, mh, d); \
         }                                                                                          \
         return check_launch();                                                                     \
     }

@@ -86,7 +86,8 @@ __device__ __forceinline__ void quant_contig_unit(const T *__restrict__ x, int32
     const float rinv = __frcp_rn(sc);                          // correctly rounded 1 / sc
     uint32_t word[WPT];
 #pragma unroll
-    for (int k = 0; k < WPT; ++k) word[k] = quant_word<BITS>([&](int i) { return v[k * E + i]; }, lo, sc, rinv);
+    for (int k = 0; k < (BITS == 3 ? WPT : 0); ++k) word[k] = quant_word<BITS>([&](int i) { return v[k * E + i]; }, lo, sc, rinv);
+    if constexpr (BITS != 3) quant_words<BITS, WPT>([&](int k, int i) { return v[k * E + i]; }, lo, sc, rinv, word);
     if (active) {
         int32_t *pc = code + b * d.c_sB + h * d.c_sH + a * d.c_sA + u * WPT;
 #pragma unroll
