@@ -185,7 +185,8 @@ class KVmixLayerCache:
         k_proj, v_proj: the k_proj / v_proj outputs of the prompt, [B, L, Hkv*D] (or [B, L, Hkv, D]) fp16, keys NOT yet
         rotated; cos, sin: the rotary tables [L, D] or [B, L, D] fp16 as HF's rotary embedding returns them (None: the
         keys arrive rotated).  Rotation, the split into packed prefix and fp16 tail, both quantizers and the tail
-        copies run in three launches of the library; no rotated, transposed or sliced temporary is made."""
+        copies run in one launch of the library (three for keys that arrive rotated, for groups other than 32, 64 and 128,
+        and where one part is empty); no rotated, transposed or sliced temporary is made."""
         assert self.kv_seq_len == 0, "prefill needs an empty cache"
         B, L = k_proj.shape[0], k_proj.shape[1]
         k4, v4 = k_proj.reshape(B, L, self.Hkv, self.D), v_proj.reshape(B, L, self.Hkv, self.D)
@@ -218,7 +219,8 @@ class KVmixLayerCache:
         a.kfull, a.kf_sB, a.kf_sH, a.kf_sT = kf.data_ptr(), kf.stride(0), kf.stride(1), kf.stride(2)
         a.vfull, a.vf_sB, a.vf_sH, a.vf_sT = vf.data_ptr(), vf.stride(0), vf.stride(1), vf.stride(2)
         _lib.check(self._lib.kvq_prefill(C.byref(a), ops.raw_stream()))
-        ops.LAUNCHES[0] += (nk > 0) + (nv > 0) + (nk < L or nv < L)
+        at_once = cos is not None and nk and nv and {self.k_group, self.v_cgroup} <= {11, 32, 64, 128}
+        ops.LAUNCHES[0] += 1 if at_once else (nk > 0) + (nv > 0) + (nk < L or nv < L)
         self.tkq, self.tvq = nk, nv
         self.k_start = self.v_start = 0
         self.k_len, self.v_len = L - nk, L - nv

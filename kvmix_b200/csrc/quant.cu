@@ -10,14 +10,14 @@
 //
 // Four kernels, one result:
 //   quant_contig_kernel   groups run along the contiguous axis (values: [.., T, D], groups over D;
-//                         or keys already transposed to [.., D, T]).  A thread owns one or two output
-//                         words; the threads of a group combine min/max with shuffles.
+//                         or keys already transposed to [.., D, T]).  A thread owns one to four output
+//                         words at a time; the threads of a group combine min/max with shuffles.
 //   quant_strided_kernel  groups run along a strided axis while the *other* axis is contiguous
 //                         (keys left as [.., T, D], groups over T).  A thread owns two adjacent
 //                         channels, keeps a whole group in registers (all loads in flight at
 //                         once), and the CTA transposes words through shared memory so global
 //                         writes are contiguous runs per channel.
-//   quant_rope_kernel     the same for keys that still have to be rotated (prefill).
+//   quant_rope_kernel     the same for keys that still have to be rotated (a prompt that prefill.cu does not take in one launch).
 //   quant_generic_kernel  any strides / any group-to-word relation; one thread per word.
 #include "quant_tiles.cuh"
 
