@@ -116,7 +116,8 @@ struct RopeTables {
 // read once -- and then works parts of 32 (11) tokens of a channel pair from there; groups of 64 and 128 tokens meet over
 // shared memory.  Loops stay rolled: with a warp's 32 tokens in registers and every word unrolled, tie path included, the same
 // work took 46 .. 71 us, waiting for instructions; read from global memory twice and rotated twice (a thread per
-// pair and group, four loads an element pair) 38 us.  2 x 8 kv heads x 8191 tokens, group 64, 4 bits: 22 us.
+// pair and group, four loads an element pair) 38 us.  2 x 8 kv heads x 8191 tokens, group 64, 4 bits: 22 us (with values
+// and tails 37.1 us in three launches, 26.7 in one).
 template <int BITS, int G>
 struct RopeCfg {
     static constexpr int FPI = fields_per_word(BITS);
