@@ -82,6 +82,13 @@ inline long long plan_segment_cycles(int n, int tile, int max_scores) {
 // What cutting a head adds to its last CTA: publishing the partials and the merge of k of them.
 inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; }
 
+// Whole heads for more than half of the SMs and no more than there are: a CTA that has its SM to itself takes this percentage of
+// the time, and halves of all heads would only put two on it and a merge behind (us, whole against halves: 128 heads,
+// group 32, 2 bits, 1023 tokens 11.6 and 13.5, 4096 tokens 23.0 and 23.2, 3-bit keys 28.6 and 31.5; 128 groups of 4 heads, 4 bits,
+// 1023 tokens 15.7 and 19.6).
+constexpr int kPlanLone = 77;
+inline bool plan_lone(long long ctas, int k) { return k == 1 && ctas <= kSmCount && 2 * ctas > kSmCount; }
+
 // Pieces a head is cut into where `heads` of them (fewer than SMs) are left behind whole ones: the SM that gets most of the pieces
 // finishes last; a piece costs its tokens and some 600 more, one whole head by itself on its SM `lone` percent of that.
 inline int plan_left_pieces(int T, int unit, int heads, int lone) {
@@ -125,7 +132,8 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
             if (ctas > (long long)kMaxCtaRounds * kPlanSlots && best >= 0) break;
             const long long rounds = (ctas + kPlanSlots - 1) / kPlanSlots;
             const int n = su * unit < T ? su * unit : T;
-            const long long cost = rounds * plan_segment_cycles(n, tile, max_scores) + plan_merge_cycles(k);
+            long long cost = rounds * plan_segment_cycles(n, tile, max_scores) + plan_merge_cycles(k);
+            if (plan_lone(ctas, k)) cost = cost * kPlanLone / 100;
             if (best < 0 || cost < best) {
                 best = cost;
                 p.k = k;

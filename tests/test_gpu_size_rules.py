@@ -131,3 +131,22 @@ def test_attention_group_sizes(cuda, kb, vb, nh, hkv):
                 err = (got.double() - want).norm(dim=-1) / want.norm(dim=-1)
                 # p * scale in fp16 (2^-12 a token) and one fp16 rounding of the result, as everywhere in these tests
                 assert err.max().item() <= REL_TOL, (kg, vg, nk, T, err.max().item())
+
+
+@pytest.mark.parametrize("bits", [(2, 2), (3, 4)])
+@pytest.mark.parametrize("nh", [74, 75, 148, 149])
+def test_whole_heads_alone_on_their_sm(cuda, nh, bits):
+    """75 .. 148 short heads stay whole: as the same heads asked for 30 at a time, which are cut."""
+    import kvmix_b200 as kv
+    g = _gen(cuda, nh)
+    k, v = (torch.randn((1, nh, 1023, 128), generator=g, device=cuda, dtype=torch.float16) for _ in range(2))
+    q = torch.randn((1, nh, 1, 128), generator=g, device=cuda, dtype=torch.float16)
+
+    def attend(sl):
+        c = kv.KVmixLayerCache(1, k[:, sl].shape[1], 128, 1100, *bits, 32, residual_length=128, device=cuda)
+        c.prefill(k[:, sl], v[:, sl])
+        return c.attend(q[:, sl].contiguous(), round_scores=False).double()
+    got = attend(slice(None))
+    want = torch.cat([attend(slice(i, min(i + 30, nh))) for i in range(0, nh, 30)], 1)
+    # both round p * scale to fp16 (2^-12 a token), relative to another segment's maximum
+    assert ((got - want).norm(dim=-1) / want.norm(dim=-1)).max().item() <= REL_TOL
