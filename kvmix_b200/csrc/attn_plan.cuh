@@ -1,7 +1,7 @@
 // Work plan of the tensor-core attention kernels: which tokens of which head a CTA scores.
 //
 // The token axis of every head (a query head, or the group of query heads that share a kv head) is cut into
-// units of `unit` tokens (a warp's key tile: 256, or four of them for 3-bit keys: 352 = 4 x 88); a head has
+// units of `unit` tokens (a warp's key tile: 256, or four of them for 3-bit keys: 352 = 4 x 88, whichever tile the loops load); a head has
 // uph = ceil(T / unit) units, the last one possibly short.  One CTA works one segment = a run of units of one head:
 //   * the first n_whole CTAs take one whole head each (only when a head fits the score buffer); n_whole is a multiple
 //     of the number of SMs, so these CTAs load all SMs alike;

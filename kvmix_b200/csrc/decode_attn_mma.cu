@@ -15,8 +15,8 @@
 // Keys (codes [D, T/fpi], one word = fpi tokens of one channel; scale/zero [D, T/G]):
 //   A (16x16) = codes, rows = tokens, cols = 16 channels.  q[d]*scale[d,g] is carried as an exact fp16 pair hi + lo.
 //   A 256-token warp tile is worked as two halves whose MMA rows touch at most four groups, so B (16x8) holds
-//   {hi, lo} x 4 groups side by side and one MMA per code tile yields both parts.  3-bit keys (176-token tiles, every
-//   word its own group of 11) multiply each code tile by the hi and by the lo operand instead.  The zero terms
+//   {hi, lo} x 4 groups side by side and one MMA per code tile yields both parts.  3-bit keys (tiles of 88 or 176 tokens,
+//   every word its own group of 11) multiply each code tile by the hi and by the lo operand instead.  The zero terms
 //   sum_d q[d]*zero[d,g] of all groups of a tile come from one MMA per 16 channels whose A operand is the zero tile
 //   read transposed (row = group) and whose B operand is q.
 // Values (codes [T, D/fpi], one word = fpi channels of one token; scale/zero [T, D/G]):
@@ -34,15 +34,25 @@ namespace kvq {
 // Score buffers: of an eight-warp CTA, two to an SM; of a four-warp CTA, three to an SM, and four to an SM.
 constexpr int kWideScores = 6144, kWideScores3 = 7040, kNarrowMax = 8192, kNarrowMax3 = 8096, kNarrowScores = 5216;
 
-// Key geometry of this kernel.  3 bits: two words (two groups) an octet, a tile of 176 tokens worked 16 channels a stage: with one
-// word an octet, 88 tokens, what a k-step does once -- q, addresses, copies, loop -- was a third of its instructions, and a channel
-// row was fetched 32 bytes at a time (64 x 32 heads of 4096 tokens, 2-bit values, a step: 294 -> 289 us; 8 x 32: 52.9 -> 52.0).
-template <int KB> struct MmaKGeom : KGeom<KB> { static constexpr int SZ = 2 * KGeom<KB>::ROWS * 16; };
-template <> struct MmaKGeom<3> {
+// Key geometry of this kernel.  3 bits come in two forms with the same sums in the same order.  H = 1: one word (group) an octet, tiles
+// of 88 tokens, 32 channels a stage.  H = 2: two words an octet, tiles of 176 tokens, 16 channels a stage -- what a k-step does once
+// (q, addresses, copies, loop) is a third of the instructions of H = 1, and a channel row is fetched 64 bytes at a time.  But a warp whose
+// last pass is half empty works 88 tokens for nothing.  us, all in tiles of 88 / all in tiles of 176 (laid out as one tile's work) / this
+// choice, 2-bit values: 2048 heads of 4096 tokens 278 / 273 / 272, 1024 of 2000 85.3 / 82.1 / 82.3, 256 of 9000 101 / 102 / 101,
+// 230 of 9000 91 / 100 / 91, 160 of 3001 36.0 / 38.7 / 35.2, 64 of 6000 27.5 / 26.4 / 25.9, 64 of 704 11.2 / 12.2 / 11.4.
+template <int KB, int H> struct MmaKGeom : KGeom<KB> { static constexpr int SZ = 2 * KGeom<KB>::ROWS * 16; };
+template <> struct MmaKGeom<3, 2> {
     static constexpr int FPI = 11, WPL = 2, TPO = 11, WT = 176, KSPS = 1, NSTAGE = 8, NMMA = 12;
     static constexpr int RB = 64, RS = RB + 16, ROWS = 16, CODE_BYTES = ROWS * RS, GPR = RB / 16, GPL = ROWS * GPR / 32, RPI = 32 / GPR;
     static constexpr int SZ = 2 * ROWS * 32;                           // [half of the tile][scales, zeros][channel][8 groups]
 };
+// The form for a segment of n packed tokens: the larger tile where the slowest warp works no more tokens than in tiles of 88, or one tile of
+// 88 more out of sixteen -- out of five where two or four warps share a tile's channels, and what a tile costs once counts double.
+__device__ __forceinline__ bool wide_key_tiles(int n, int warps, int ks_log2) {
+    auto passes = [&](int tile) { return (((n + tile - 1) / tile << ks_log2) + warps - 1) / warps; };
+    const int p = passes(MmaKGeom<3, 1>::WT);
+    return n > 0 && 2 * passes(MmaKGeom<3, 2>::WT) <= p + (p >= (ks_log2 ? 5 : 16));
+}
 
 struct MmaSmem {
     float *scores;          // [1 << ks_log2][n_scores]
@@ -53,14 +63,15 @@ struct MmaSmem {
 };
 // Rings of a CTA of NW warps: the scale rows, then the zero rows of a stage, 16 B each, follow its codes.  Four warps: sized so
 // that four CTAs fit an SM next to 5000 scores each.
-template <int KB, int NW> struct MmaKRing {
+template <int KB, int NW, int H> struct MmaKRing {
     static constexpr int NS = (KB == 2 ? 3 : 4) - (NW == 4), P = NS - 1;
-    static constexpr int STAGE_BYTES = MmaKGeom<KB>::CODE_BYTES + MmaKGeom<KB>::SZ;
+    static constexpr int STAGE_BYTES = MmaKGeom<KB, H>::CODE_BYTES + MmaKGeom<KB, H>::SZ;
     static constexpr int BYTES = NS * STAGE_BYTES;
 };
 template <int VB, int NW> using MmaVGeom = VGeom<VB, (VB == 4 ? 4 : VB == 2 ? 6 : 8) - (NW == 4 && VB != 1)>;
 template <int KB, int VB, int NW> constexpr int warp_region_bytes() {
-    return MmaKRing<KB, NW>::BYTES > MmaVGeom<VB, NW>::WARP_BYTES ? MmaKRing<KB, NW>::BYTES : MmaVGeom<VB, NW>::WARP_BYTES;
+    static_assert(KB != 3 || MmaKRing<3, NW, 2>::BYTES <= MmaKRing<3, NW, 1>::BYTES, "one ring for both forms");
+    return MmaKRing<KB, NW, 1>::BYTES > MmaVGeom<VB, NW>::WARP_BYTES ? MmaKRing<KB, NW, 1>::BYTES : MmaVGeom<VB, NW>::WARP_BYTES;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -74,12 +85,13 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
 
 // If the split also holds fp16 tail keys (tail_lo < t1) they are scored right after the first code stages
 // have been issued, so the tail's global-load latency overlaps the ring fill.
-template <int KB, int NW, int LGK>
+// LGK: log2 of the group size; H: words an octet owns of 3-bit keys (MmaKGeom).
+template <int KB, int NW, int LGK, int H>
 __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const MmaSmem &sm, int t0, int hi,
                                               const __half *kf, int tail_lo, int t1, int b, int hk) {
-    using G = MmaKGeom<KB>;
-    using R = MmaKRing<KB, NW>;
+    using G = MmaKGeom<KB, H>;
+    using R = MmaKRing<KB, NW, H>;
     using F = Fields<KB>;
     const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
     const int n_words = a.Tkq / G::FPI;                       // valid code words per channel row
@@ -94,7 +106,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     const uint32_t ring_s = smem_u32(sm.ring);
     const int gr = lane % G::GPR, row0 = lane / G::GPR;
     const uint32_t cp_dst = ring_s + row0 * G::RS + gr * 16;                   // + slot*STAGE + i*RPI*RS
-    // 3-bit: octet g owns the word of group g (11 tokens) of either half of the tile, fetched with plain 32-bit loads.
+    // 3-bit: octet g owns the word of group g (11 tokens) of each half (H) of the tile, fetched with plain 32-bit loads.
     // Other widths: code fragments come from transposing ldmatrix loads.  A channel row of the tile is NBK blocks of
     // 16 bytes; one x4 load covers channel rows 16 ksx + (0..7 | 8..15) x two neighbouring blocks and hands lane
     // (g, tig) the half-word g of each block for the channel pair (2 tig, 2 tig + 1) [+8]: an A-fragment register pair
@@ -111,7 +123,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     // ldmatrix.x4 row addresses: lanes 0-7 scale rows 0..7 of a k-step, 8-15 scale rows 8..15, 16-31 the same of the zero rows
     const uint32_t ldm_s = ring_s + G::CODE_BYTES + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16 + (lane >> 4) * (G::ROWS * 16);
     const uint32_t q_s = smem_u32(sm.q) + (ch0 + 2 * tig) * 2;                 // + 32 per k-step [+16]
-    constexpr int ngw = KB == 3 ? 16 : G::WT >> LGK;                           // groups per warp tile: 16 / 8 / 4 / 2
+    constexpr int ngw = KB == 3 ? 8 * H : G::WT >> LGK;                        // groups per warp tile: 16 / 8 / 4 / 2
     const uint32_t szcp_dst = ring_s + G::CODE_BYTES + lane * 16;                  // one granule per lane (16 channels a stage) or two
     const int tile_words = tile_lanes * G::WT / G::FPI;                        // word-column distance between my tiles
     const int tile_groups = tile_lanes * ngw;
@@ -128,7 +140,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
     int iss_col = (t0 + wt * G::WT) / G::FPI + 4 * gr, iss_st = 0, iss_tiles = my_tiles;
     uint32_t iss_slot = 0, slot = 0;                                            // byte offsets of the slot being filled / read
     bool iss_ok = iss_col < n_words;
-    int iss_second = n_words - ((t0 + wt * G::WT) / G::FPI + 8);                // 3 bits: > 0: the second half of the tile's groups exists
+    int iss_second = n_words - ((t0 + wt * G::WT) / G::FPI + 8);                // H = 2: > 0: the second half of the tile's groups exists
 
     const char *kc_b = reinterpret_cast<const char *>(kc), *kz_b = reinterpret_cast<const char *>(kz);
     const uint32_t row_step = (uint32_t)(G::RPI * 4) * kc_sD, stage_step = (uint32_t)(G::ROWS * 4) * kc_sD, sz_step = (uint32_t)(G::ROWS * 2) * ks_sD;
@@ -142,7 +154,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                     cp_async<16>(cp_dst + iss_slot + i * G::RPI * G::RS, kc_b + (iss + i * row_step));
             }
             const uint32_t d = szcp_dst + iss_slot;
-            if (KB == 3) {
+            if (KB == 3 && H == 2) {
                 cp_async<16>(d, sz_b + iss_s);
                 if (iss_second > 0) cp_async<16>(d + G::SZ / 2, sz_b + (iss_s + 16));
             } else if (ngw == 8) { cp_async<16>(d, sz_b + iss_s); if (!kOneSz) cp_async<16>(d + G::ROWS * 16, kz_b + iss_s); }
@@ -178,10 +190,10 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
         // ---- B fragments q*scale and the zero term sum_d q[d]*zero[d,g] ----------------------------------
         // q*scale needs 22 bits; it is carried as an fp16 pair hi + lo (lo = fma(q, s, -hi) is exact), so the key
         // side adds no rounding beyond the fp32 accumulation.
-        // 3-bit keys: b0 = hi and b1 = lo of the eight groups of the tile, every code tile is multiplied by both.
+        // 3-bit keys: hi and lo of the eight groups of a half of the tile, every code tile is multiplied by both.
         // Other widths: b0 / b1 serve the first / second half of the tile; column n carries group (n / 2) of that
         // half, hi in even and lo in odd columns, so one MMA per code tile yields both parts.
-        float zsum = 0.f, zsum3 = 0.f;                         // (3 bits: of the halves of the tile)
+        float zsum = 0.f, zsum3 = 0.f;                         // (H = 2: of the halves of the tile)
         constexpr int gph = ngw / 2;                           // groups per half tile: 4 / 2 / 1
         const int src0 = 4 * ((g >> 1) % gph) + tig;           // lane holding group (n / 2) of the first half
         const int src1 = src0 + 4 * (ngw / 2);
@@ -207,10 +219,10 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                 const __half2 q01 = as_h2(q01u), q89 = as_h2(q89u);
                 if constexpr (KB == 3) {
 #pragma unroll
-                    for (int hf = 0; hf < 2; ++hf) {
+                    for (int hf = 0; hf < H; ++hf) {
                         uint32_t r0, r1, r2, r3;               // scales and zeros of this half's eight groups, see below
                         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(ldm_s + slot + hf * (G::SZ / 2)));
+                                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(ldm_s + slot + k * 256 + hf * (G::SZ / 2)));
                         if (hf) mma16816(accz3, r2, 0u, r3, 0u, q01u, q89u);
                         else mma16816(accz, r2, 0u, r3, 0u, q01u, q89u);
                         const __half2 s01 = as_h2(r0), s89 = as_h2(r1);
@@ -219,7 +231,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
                         const uint32_t lo0 = as_u32(__hfma2(q01, s01, __hneg2(p01))), lo1 = as_u32(__hfma2(q89, s89, __hneg2(p89)));
                         uint32_t w[4];
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) w[r] = lds32(src + 32 * hf + ((r & 1) + (r >> 1) * 8) * G::RS);
+                        for (int r = 0; r < 4; ++r) w[r] = lds32(src + 32 * hf + (k * 16 + (r & 1) + (r >> 1) * 8) * G::RS);
                         uint32_t rlo[F::N], rhi[F::N];
                         F::unpack(w[0], w[1], rlo);
                         F::unpack(w[2], w[3], rhi);
@@ -314,7 +326,7 @@ __device__ __forceinline__ void qk_packed_mma(const kvq_attn_args &a, const int3
         if constexpr (KB == 3) {
             // the octet's column is n = g, held by the lane with tig == g/2
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
+            for (int hf = 0; hf < H; ++hf) {
                 const int tok0 = tile0 + 88 * hf + g * G::TPO;     // first token of this octet's word of the half
                 if (tok0 < hi && tig == (g >> 1)) {            // words are whole or absent (hi is a group multiple)
                     const bool sel = g & 1;
@@ -657,10 +669,16 @@ __device__ __forceinline__ void attn_segment(const kvq_attn_args &a, const kvq_a
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
+        const int k_hi = min(t1, a.Tkq), k_tail = max(t0, a.Tkq);
         // the loops for the call's group size: looked up, it cost a compare, a branch or a select per group and k-step
-        if (KB == 3 || a.k_group == 32) qk_packed_mma<KB, NW, 5>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
-        else if (a.k_group == 64) qk_packed_mma<KB, NW, KB == 3 ? 5 : 6>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
-        else qk_packed_mma<KB, NW, KB == 3 ? 5 : 7>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        if constexpr (KB == 3) {
+            if (wide_key_tiles(k_hi - t0, NW, ks_log2)) qk_packed_mma<3, NW, 5, 2>(a, kc, ks, kz, sm, t0, k_hi, kf, k_tail, t1, b, hk);
+            else qk_packed_mma<3, NW, 5, 1>(a, kc, ks, kz, sm, t0, k_hi, kf, k_tail, t1, b, hk);
+        } else {
+            if (a.k_group == 32) qk_packed_mma<KB, NW, 5, 1>(a, kc, ks, kz, sm, t0, k_hi, kf, k_tail, t1, b, hk);
+            else if (a.k_group == 64) qk_packed_mma<KB, NW, 6, 1>(a, kc, ks, kz, sm, t0, k_hi, kf, k_tail, t1, b, hk);
+            else qk_packed_mma<KB, NW, 7, 1>(a, kc, ks, kz, sm, t0, k_hi, kf, k_tail, t1, b, hk);
+        }
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
@@ -894,7 +912,7 @@ int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *
 
 // Plan of the tensor-core kernel for B * nh query heads (one head per segment).
 AttnPlan plan_attn_mma(int T, int k_bits, long long heads) {
-    return k_bits == 3 ? make_attn_plan_mma(T, 352, MmaKGeom<3>::WT, kWideScores3, heads, kNarrowMax3, kNarrowScores, 1760)
+    return k_bits == 3 ? make_attn_plan_mma(T, 352, MmaKGeom<3, 1>::WT, kWideScores3, heads, kNarrowMax3, kNarrowScores, 1760)
                        : make_attn_plan_mma(T, 256, KGeom<4>::WT, kWideScores, heads, kNarrowMax, kNarrowScores, 3072);
 }
 

@@ -150,3 +150,32 @@ def test_whole_heads_alone_on_their_sm(cuda, nh, bits):
     want = torch.cat([attend(slice(i, min(i + 30, nh))) for i in range(0, nh, 30)], 1)
     # both round p * scale to fp16 (2^-12 a token), relative to another segment's maximum
     assert ((got - want).norm(dim=-1) / want.norm(dim=-1)).max().item() <= REL_TOL
+
+
+@pytest.mark.parametrize("nh,nk,T", [(2, 352, 400), (64, 5874, 6000), (256, 3960, 4096), (256, 3971, 4003), (320, 693, 700), (320, 1034, 1050), (1024, 5621, 5700)])
+def test_three_bit_key_tiles(cuda, nh, nk, T):
+    """3-bit keys in tiles of 88 and of 176 tokens: a short segment whose tiles two warps share (88), a long one (176: three passes for five),
+    whole heads on eight warps (176: three passes for six; 88: six passes would be seven) and on four (two passes in one; pieces;
+    nine for seventeen), with ragged last tiles -- against the softmax in 64 bits, heads with the same operands alike."""
+    import kvmix_b200 as kv
+    from kvmix_b200 import ops
+    g = _gen(cuda, nk)
+    k, v = (torch.randn((1, 3, T, 128), generator=g, device=cuda, dtype=torch.float16) for _ in range(2))
+    k[..., 3] *= 8
+    q = torch.randn((1, 3, 1, 128), generator=g, device=cuda, dtype=torch.float16)
+    nv = (T - 1) // 32 * 32
+    kp = ops.quantize_pack_last_dim_cuda(k[:, :, :nk].transpose(2, 3), 11, 3)
+    vp = ops.quantize_pack_last_dim_cuda(v[:, :, :nv].contiguous(), 32, 2)
+    K = torch.cat((_dense(kp, 11, 3).transpose(2, 3), k[:, :, nk:].double()), 2)
+    V = torch.cat((_dense(vp, 32, 2), v[:, :, nv:].double()), 2)
+    want = torch.softmax(q.double() @ K.transpose(2, 3) / 128 ** 0.5, -1) @ V
+    pick = torch.randint(0, 3, (nh,), generator=g, device=cuda)
+    padded = [torch.nn.functional.pad(t, (0, -t.shape[3] % 32 + 32))[:, pick][..., :t.shape[3]] for t in kp]
+    got = kv.decode_attention(q[:, pick].contiguous(), *padded, k[:, pick, nk:].contiguous(), *(t[:, pick].contiguous() for t in vp),
+                              v[:, pick, nv:].contiguous(), 3, 11, 2, 32, Tkq=nk, Tvq=nv, round_scores=False)
+    err = (got.double() - want[:, pick]).norm(dim=-1) / want[:, pick].norm(dim=-1)
+    # p * scale in fp16 (2^-12 a token) and one fp16 rounding of the result, as everywhere in these tests
+    assert err.max().item() <= REL_TOL
+    if nh <= 256:                                              # all heads take the same segments
+        for i in range(3):
+            assert (got[:, pick == i] == got[:, pick == i][:, :1]).all()
