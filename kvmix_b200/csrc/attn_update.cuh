@@ -236,7 +236,7 @@ __device__ __forceinline__ void pv_tail(const kvq_attn_args &a, const __half *vf
         uint4 v[U];
 #pragma unroll
         for (int j = 0; j < U; ++j)
-            if (t + j * step < t1) v[j] = __ldg(reinterpret_cast<const uint4 *>(v_tail_row(a, vf, b, hk, t + j * step)) + l16);
+            if (t + j * step < t1) v[j] = __ldcg(reinterpret_cast<const uint4 *>(v_tail_row(a, vf, b, hk, t + j * step)) + l16);
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             const int tj = t + j * step;

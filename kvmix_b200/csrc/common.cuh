@@ -41,8 +41,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // Additive attention mask value for (sequence b, query head h, key position t); the caller checked a.mask != NULL.
 __device__ __forceinline__ float attn_mask_at(const kvq_attn_args &a, int b, int h, int t) {
     const int64_t off = (int64_t)b * a.mask_sB + (int64_t)h * a.mask_sH + t;
-    return a.mask_is_f32 ? __ldg(static_cast<const float *>(a.mask) + off)
-                         : __half2float(__ldg(static_cast<const __half *>(a.mask) + off));
+    return a.mask_is_f32 ? __ldca(static_cast<const float *>(a.mask) + off)
+                         : __half2float(__ldca(static_cast<const __half *>(a.mask) + off));
 }
 // upstream clamps masked weights from below at torch.finfo(float32).min (models/modeling_llama_KVmix.py:192)
 constexpr float kMaskFloor = -3.4028234663852886e38f;
@@ -50,7 +50,8 @@ constexpr float kMaskFloor = -3.4028234663852886e38f;
 // Programmatic launches: a kernel launched by launch_early() may be put on the GPU while the kernel before it in the stream is still
 // running its last CTAs, as soon as each of those has called launch_next(); grid_wait() then holds it until that kernel
 // is complete and its writes are visible.  Nothing before grid_wait() touches global memory.  Behind a kernel that does not call
-// launch_next() it is an ordinary launch.
+// launch_next() it is an ordinary launch.  Data are read by plain loads, __ldca, __ldcg or cp.async: __ldg(), and whatever the compiler turns into it
+// (const __restrict__), wants memory that nobody writes while the kernel is resident, which here the kernel before may.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 

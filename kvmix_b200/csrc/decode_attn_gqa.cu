@@ -63,25 +63,37 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// fp16 key tail for tokens [lo, t1): 16-token tiles straight from global memory; B column n = query head n.
+// fp16 key tail for tokens [lo, t1): 16-token tiles straight from global memory; B column n = query head n.  EARLY: the first
+// tile is asked for before the CTA barrier behind which q is in shared memory, and every warp passes that barrier in here (four small layers
+// from a host loop 59.8 -> 58.7 us, 32k tokens with 3-bit values 657 -> 643; the device-driven kernels spill for it, 531 -> 535).
+template <bool EARLY>
 __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half *kf, int b, int hk, const GqaSmem &sm,
                                             int t0, int lo, int t1) {
     const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+    const int n_tiles = (t1 - lo + 15) / 16;                   // <= 0: no tail in this segment
+    uint4 ra[4], rb[4];
+    auto load = [&](int tile) {
+        const int ta = lo + 16 * tile + g;
+        const __half *pa = k_tail_row(a, kf, b, hk, min(ta, t1 - 1)) + 8 * tig;
+        const __half *pb = k_tail_row(a, kf, b, hk, min(ta + 8, t1 - 1)) + 8 * tig;
+#pragma unroll
+        for (int S = 0; S < 4; ++S) {
+            ra[S] = __ldcg(reinterpret_cast<const uint4 *>(pa + 32 * S));
+            rb[S] = __ldcg(reinterpret_cast<const uint4 *>(pb + 32 * S));
+        }
+    };
+    if constexpr (EARLY) {
+        if (warp < n_tiles) load(warp);
+        __syncthreads();
+        if (warp >= n_tiles) return;
+    }
     uint4 qf[4];
 #pragma unroll
     for (int S = 0; S < 4; ++S)
         qf[S] = g < kQH ? *reinterpret_cast<const uint4 *>(sm.q + g * kHeadDim + 32 * S + 8 * tig) : make_uint4(0u, 0u, 0u, 0u);
-    const int n_tiles = (t1 - lo + 15) / 16;
     for (int tile = warp; tile < n_tiles; tile += kMmaWarps) {
         const int ta = lo + 16 * tile + g, tb = ta + 8;
-        const __half *pa = k_tail_row(a, kf, b, hk, min(ta, t1 - 1)) + 8 * tig;
-        const __half *pb = k_tail_row(a, kf, b, hk, min(tb, t1 - 1)) + 8 * tig;
-        uint4 ra[4], rb[4];
-#pragma unroll
-        for (int S = 0; S < 4; ++S) {
-            ra[S] = __ldg(reinterpret_cast<const uint4 *>(pa + 32 * S));
-            rb[S] = __ldg(reinterpret_cast<const uint4 *>(pb + 32 * S));
-        }
+        if (!EARLY || tile != warp) load(tile);
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int S = 0; S < 4; ++S) {
@@ -101,7 +113,7 @@ __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same stage geometry, tile order and channel
 // splits as the single-head kernel; scores[split][h][t - t0] receive the raw scores.
-template <int KB, bool WIDE>
+template <int KB, bool WIDE, bool DEV>
 __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const GqaSmem &sm, int t0, int hi, const __half *kf,
                                               int tail_lo, int t1, int b, int hk) {
@@ -188,8 +200,12 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 
 #pragma unroll 1
     for (int q = 0; q < R::P; ++q) issue_stage();
-    __syncthreads();                                           // q is in shared memory (stored by the caller without a barrier)
-    if (tail_lo < t1) gqa_qk_tail(a, kf, b, hk, sm, t0, tail_lo, t1);
+    if constexpr (DEV) {
+        __syncthreads();                                       // q is in shared memory (stored by the caller without a barrier)
+        if (tail_lo < t1) gqa_qk_tail<false>(a, kf, b, hk, sm, t0, tail_lo, t1);
+    } else {
+        gqa_qk_tail<true>(a, kf, b, hk, sm, t0, tail_lo, t1);
+    }
 
     for (int j = 0; j < my_tiles; ++j) {
         const int tile0 = t0 + (j * tile_lanes + wt) * G::WT;
@@ -611,8 +627,8 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
         if (lane < 24) {
 #pragma unroll 3
             for (int q = 0; q < my_blocks; ++q) {
-                const uint4 u = __ldg(reinterpret_cast<const uint4 *>(sz_row + q * sz_step) + lane);
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(sz_row + q * sz_step) + lane + 24);
+                const uint4 u = reinterpret_cast<const uint4 *>(sz_row + q * sz_step)[lane];
+                const uint4 v = reinterpret_cast<const uint4 *>(sz_row + q * sz_step)[lane + 24];
                 mx[0] = __vmaxu2(mx[0], __vmaxu2(u.x & 0x7fff7fffu, v.x & 0x7fff7fffu));
                 mx[1] = __vmaxu2(mx[1], __vmaxu2(u.y & 0x7fff7fffu, v.y & 0x7fff7fffu));
                 mx[2] = __vmaxu2(mx[2], __vmaxu2(u.z & 0x7fff7fffu, v.z & 0x7fff7fffu));
@@ -753,7 +769,7 @@ __device__ __forceinline__ void gqa_pv_packed3(const kvq_attn_args &a, const int
 
 // ---------------------------------------------------------------------------------------------
 // One segment: tokens [t0, t1) of head group s (sequence b, kv head hk, quad of query heads); segment `seg` of `cnt`.
-template <int KB, int VB>
+template <int KB, int VB, bool DEV>
 __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_attn_args &ac, unsigned int before, __half2 q_mine, const AttnPlan &plan, int qhv, int s, int b, int hk, int h_first, int t0, int t1,
                                             int seg, int cnt, float *__restrict__ parts,
                                             unsigned int *__restrict__ counters) {
@@ -782,8 +798,8 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        if (KB != 1 && (KB == 3 || a.k_group == 64)) gqa_qk_packed<KB, false>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
-        else gqa_qk_packed<KB, KB != 3>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        if (KB != 1 && (KB == 3 || a.k_group == 64)) gqa_qk_packed<KB, false, DEV>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        else gqa_qk_packed<KB, KB != 3, DEV>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
@@ -949,11 +965,11 @@ __global__ void __launch_bounds__(kMmaThreads, 2) decode_attn_gqa_kernel(const _
         const unsigned int before = dev_state_step(a, state, d);
         plan_tokens(plan, d.T, blockIdx.x, seg, t0, t1, cnt);
         if (cnt > 1) cnt = min(cnt, (d.T + plan.seg_units * plan.unit - 1) / (plan.seg_units * plan.unit));
-        if (t0 < d.T) gqa_segment<KB, VB>(d, a, before, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
+        if (t0 < d.T) gqa_segment<KB, VB, true>(d, a, before, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
         else dev_state_publish(a, d, before);
     } else {
         plan_tokens(plan, a.T, blockIdx.x, seg, t0, t1, cnt);
-        gqa_segment<KB, VB>(a, a, 0u, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
+        gqa_segment<KB, VB, false>(a, a, 0u, q_mine, plan, qhv, group, b, hk, h_first, t0, t1, seg, cnt, parts, counters);
     }
 }
 

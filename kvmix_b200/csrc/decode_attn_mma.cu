@@ -619,8 +619,8 @@ __device__ __forceinline__ void qk_tail_mma(const kvq_attn_args &a, const __half
         uint4 ra[4], rb[4];
 #pragma unroll
         for (int S = 0; S < 4; ++S) {
-            ra[S] = __ldg(reinterpret_cast<const uint4 *>(pa + 32 * S));
-            rb[S] = __ldg(reinterpret_cast<const uint4 *>(pb + 32 * S));
+            ra[S] = __ldcg(reinterpret_cast<const uint4 *>(pa + 32 * S));
+            rb[S] = __ldcg(reinterpret_cast<const uint4 *>(pb + 32 * S));
         }
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll

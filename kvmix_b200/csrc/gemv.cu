@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
                         const int jj = j & 1;
                         const __half *q = j < 2 ? ps : pz;
                         const bool ok0 = lane < left && 2 * jj < groups, ok1 = lane < left && 2 * jj + 1 < groups;
-                        const uint32_t lo = ok0 ? __half_as_ushort(__ldg(q + 2 * jj)) : 0u, hi = ok1 ? __half_as_ushort(__ldg(q + 2 * jj + 1)) : 0u;
+                        const uint32_t lo = ok0 ? __half_as_ushort(q[2 * jj]) : 0u, hi = ok1 ? __half_as_ushort(q[2 * jj + 1]) : 0u;
                         v[j] = lo | (hi << 16);
                     }
                     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
                         cp_async<kSzBytes>(d, sh_b + o);
                         cp_async<kSzBytes>(d + 8, zh_b + o);
                     } else {
-                        const uint32_t v = __half_as_ushort(__ldg(reinterpret_cast<const __half *>(sh_b + o))), z = __half_as_ushort(__ldg(reinterpret_cast<const __half *>(zh_b + o)));
+                        const uint32_t v = __half_as_ushort(*reinterpret_cast<const __half *>(sh_b + o)), z = __half_as_ushort(*reinterpret_cast<const __half *>(zh_b + o));
                         asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%2};\n" ::"r"(d), "r"(v), "r"(0u), "r"(z));
                     }
                 } else {
@@ -275,7 +275,14 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
         // ---- in * 2^up_e: the largest magnitude to 2^7 .. 2^8, larger ones (and a chunk with an infinity) as they are ----
         if (c0 > k_beg) __syncthreads();                                        // the previous chunk has been read
         float mx = 0.f;
-        for (int i = tid; i < rows; i += kGemvThreads) mx = fmaxf(mx, fabsf(__half2float(__ldg(in + c0 + i))));
+        constexpr int NX = kGemvChunk / kGemvThreads;
+        __half xr[NX];                                                          // asked for in one go, read once
+#pragma unroll
+        for (int j = 0; j < NX; ++j) {
+            const int i = tid + kGemvThreads * j;
+            xr[j] = i < rows ? in[c0 + i] : __float2half_rn(0.f);
+            mx = fmaxf(mx, fabsf(__half2float(xr[j])));
+        }
         mx = warp_max(mx);
         if (lane == 0) misc[warp] = mx;
         __syncthreads();
@@ -285,8 +292,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
         const int up_e = max(8 - in_e, 0);
         const float up = pow2f(up_e), down = pow2f(-up_e);
         const int room = 16 - max(in_e, 8);                                     // scales below 2^room: products below 2^16
-        for (int i = tid; i < n_st * 32; i += kGemvThreads)
-            xs[i] = i < rows ? __float2half_rn(__half2float(__ldg(in + c0 + i)) * up) : __float2half_rn(0.f);
+#pragma unroll
+        for (int j = 0; j < NX; ++j) {
+            const int i = tid + kGemvThreads * j;
+            if (i < n_st * 32) xs[i] = __float2half_rn(__half2float(xr[j]) * up);
+        }
         __syncthreads();
 
         // the window's powers of two: of the group of this lane's B column, undone for the group of its C columns; lanes g < 4 watch

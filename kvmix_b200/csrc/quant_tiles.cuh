@@ -1,5 +1,6 @@
 // Pieces of the quantizer kernels that more than one kernel is made of: a run of contiguous groups, a tile of keys that are
-// rotated on the way in, a word of the short-last-group extension, a chunk of a prompt's fp16 tails.
+// rotated on the way in, a word of the short-last-group extension, a chunk of a prompt's fp16 tails.  Their loads are plain ones and
+// their pointers not __restrict__: see grid_wait().
 #pragma once
 #include "quant_core.cuh"
 
@@ -26,7 +27,7 @@ struct QuantDims {
 // of loads in flight per thread, and the per-thread index arithmetic, division and shuffles spread over enough
 // elements); tpg = group / (E * WPT) threads share a group.
 template <int BITS, typename T, int WPT>
-__device__ __forceinline__ void quant_contig_unit(const T *__restrict__ x, int32_t *__restrict__ code, T *__restrict__ scale, T *__restrict__ mn,
+__device__ __forceinline__ void quant_contig_unit(const T *x, int32_t *code, T *scale, T *mn,
                                                   const QuantDims &d, int tpg, bool vec_ok, bool linear, int b, int h, int idx) {
     constexpr int E = fields_per_word(BITS);
     constexpr int EW = E * WPT;
@@ -49,7 +50,7 @@ __device__ __forceinline__ void quant_contig_unit(const T *__restrict__ x, int32
             __half2 lo2, hi2;
 #pragma unroll
             for (int j = 0; j < EW / 8; ++j) {
-                uint4 q = __ldg(reinterpret_cast<const uint4 *>(px) + j);
+                uint4 q = reinterpret_cast<const uint4 *>(px)[j];
                 const __half2 *hp = reinterpret_cast<const __half2 *>(&q);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -131,7 +132,7 @@ struct RopeCfg {
 };
 
 template <int BITS, int G>
-__device__ __forceinline__ void quant_rope_tile(const __half *__restrict__ x, int32_t *__restrict__ code, __half *__restrict__ scale, __half *__restrict__ mn,
+__device__ __forceinline__ void quant_rope_tile(const __half *x, int32_t *code, __half *scale, __half *mn,
                                                 const QuantDims &d, const RopeTables &rope, int tile, int bh) {
     using C = RopeCfg<BITS, G>;
     constexpr int QMAX = (1 << BITS) - 1;
@@ -156,9 +157,9 @@ __device__ __forceinline__ void quant_rope_tile(const __half *__restrict__ x, in
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
                 const int64_t t = min(t0 + 8 * i, tokens - 1);
-                k[i] = __ldg(reinterpret_cast<const uint2 *>(px + t * d.x_sS));
-                cs[i] = __ldg(reinterpret_cast<const uint2 *>(pc + t * rope.r_sS));
-                sn[i] = __ldg(reinterpret_cast<const uint2 *>(ps + t * rope.r_sS));
+                k[i] = *reinterpret_cast<const uint2 *>(px + t * d.x_sS);
+                cs[i] = *reinterpret_cast<const uint2 *>(pc + t * rope.r_sS);
+                sn[i] = *reinterpret_cast<const uint2 *>(ps + t * rope.r_sS);
             }
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
@@ -247,7 +248,7 @@ __device__ __forceinline__ void quant_rope_tile(const __half *__restrict__ x, in
 // (3-bit values at head_dim 128).  Every group is one word; the last group holds S % 11 elements, its unused fields
 // stay 0.  Upstream's 3-bit group rule otherwise (quantization_cuda.cu:553-596, :612-626).  One thread per word.
 template <typename T>
-__device__ __forceinline__ void quant_ragged3_word(const T *__restrict__ x, int32_t *__restrict__ code, T *__restrict__ scale, T *__restrict__ mn,
+__device__ __forceinline__ void quant_ragged3_word(const T *x, int32_t *code, T *scale, T *mn,
                                                    const QuantDims &d, int64_t idx) {
     const int64_t words_per_row = (d.S + 10) / 11;
     const int64_t total = d.B * d.H * d.A * words_per_row;
@@ -290,19 +291,20 @@ __device__ __forceinline__ void prefill_tail_chunk(const kvq_prefill_args &a, in
     if (is_v) {
         const __half *src = static_cast<const __half *>(a.v) + b * a.v_sB + (a.nv + r) * a.v_sT + h * a.v_sH;
         __half *dst = static_cast<__half *>(a.vfull) + b * a.vf_sB + h * a.vf_sH + r * a.vf_sT;
-        reinterpret_cast<uint4 *>(dst)[j] = __ldg(reinterpret_cast<const uint4 *>(src) + j);
-        reinterpret_cast<uint4 *>(dst)[j + 8] = __ldg(reinterpret_cast<const uint4 *>(src) + j + 8);
+        const uint4 lo = reinterpret_cast<const uint4 *>(src)[j], hi = reinterpret_cast<const uint4 *>(src)[j + 8];
+        reinterpret_cast<uint4 *>(dst)[j] = lo;
+        reinterpret_cast<uint4 *>(dst)[j + 8] = hi;
         return;
     }
     const int64_t t = a.nk + r;
     const __half *src = static_cast<const __half *>(a.k) + b * a.k_sB + t * a.k_sT + h * a.k_sH;
     __half *dst = static_cast<__half *>(a.kfull) + b * a.kf_sB + h * a.kf_sH + r * a.kf_sT;
-    uint4 lo = __ldg(reinterpret_cast<const uint4 *>(src) + j), hi = __ldg(reinterpret_cast<const uint4 *>(src) + j + 8);
+    uint4 lo = reinterpret_cast<const uint4 *>(src)[j], hi = reinterpret_cast<const uint4 *>(src)[j + 8];
     if (a.cos) {
         const __half *pc = static_cast<const __half *>(a.cos) + b * a.r_sB + t * a.r_sT;
         const __half *ps = static_cast<const __half *>(a.sin) + b * a.r_sB + t * a.r_sT;
-        const uint4 cl = __ldg(reinterpret_cast<const uint4 *>(pc) + j), ch = __ldg(reinterpret_cast<const uint4 *>(pc) + j + 8);
-        const uint4 sl = __ldg(reinterpret_cast<const uint4 *>(ps) + j), sh = __ldg(reinterpret_cast<const uint4 *>(ps) + j + 8);
+        const uint4 cl = reinterpret_cast<const uint4 *>(pc)[j], ch = reinterpret_cast<const uint4 *>(pc)[j + 8];
+        const uint4 sl = reinterpret_cast<const uint4 *>(ps)[j], sh = reinterpret_cast<const uint4 *>(ps)[j + 8];
         uint4 ol, oh;
         const __half2 *kl = reinterpret_cast<const __half2 *>(&lo), *kh = reinterpret_cast<const __half2 *>(&hi);
         const __half2 *c0 = reinterpret_cast<const __half2 *>(&cl), *c1 = reinterpret_cast<const __half2 *>(&ch);
