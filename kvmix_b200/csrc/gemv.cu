@@ -115,6 +115,7 @@ struct GemvPlan {
     int fast;            // 16-byte granules and vectors, all rows of a head within 32-bit byte offsets
     int rep;             // query heads per kv head
     int out_vec;         // output rows are 8-byte aligned
+    int early;           // launched early, and lets the next launch in early
 };
 
 template <int CG, int BITS>
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_mma_kernel(const __grid_
     const char *qh_b = reinterpret_cast<const char *>(qh), *sh_b = reinterpret_cast<const char *>(sh), *zh_b = reinterpret_cast<const char *>(zh);
 
     grid_wait();
-    launch_next();
+    if (plan.early) launch_next();
     float acc[8][4], sum[8][2], accz[2][4] = {}, zsum = 0.f;
     auto clear = [&]() {
 #pragma unroll
@@ -461,7 +462,7 @@ static int launch_gemv_mma(const kvq_gemv_args &a, const GemvPlan &p, unsigned g
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;            // see grid_wait()
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = p.early;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = (unsigned)p.kc;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
@@ -497,6 +498,11 @@ static bool gemv_mma_plan(const kvq_gemv_args &a, int64_t n_pack, GemvPlan &p, i
     p.fast = p.code_align == 16 && p.sz_vec && a.q_sK >= 0 && a.s_sK >= 0 && a.K * a.q_sK < (1LL << 30) && a.K * a.s_sK < (1LL << 31) &&
              a.q_sK < (1 << 24) && a.s_sK < (1 << 25);
     p.rep = (int)(a.nh / a.nh_kv);
+    // Clusters of CTAs, where there are many of them, neither come early nor let anybody in early: CTAs that are placed while others still hold
+    // their SMs come to lie two to an SM with SMs left over.  q . K^T and p . V in turn, us, early / ordinary: 32 heads of 4096 tokens 15.7 /
+    // 13.2, of 2048 14.4 / 11.8, 128 heads of 1024 15.4 / 13.4 (15.1, 13.6 and 15.2 before early launches); without clusters: 128 heads of 256
+    // 9.3 / 10.4, 512 of 128 14.4 / 15.0.
+    p.early = p.kc == 1 || jobs * p.kc < 64;
     p.out_vec = (reinterpret_cast<uintptr_t>(a.out) | (uint64_t)(2 * (a.o_sB | a.o_sH))) % 8 == 0;
     grid = jobs * p.kc;
     return grid <= 2147483647LL && a.B * a.nh <= 2147483647LL;
