@@ -64,8 +64,10 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
 
 // ---------------------------------------------------------------------------------------------
 // fp16 key tail for tokens [lo, t1): 16-token tiles straight from global memory; B column n = query head n.  EARLY: the first
-// tile is asked for before the CTA barrier behind which q is in shared memory, and every warp passes that barrier in here (four small layers
-// from a host loop 59.8 -> 58.7 us, 32k tokens with 3-bit values 657 -> 643; the device-driven kernels spill for it, 531 -> 535).
+// tile is asked for before the CTA barrier behind which q is in shared memory, and every warp passes that barrier in here.  For keys
+// and values that together have six bits and more, in calls the host drives (16 .. 160 head groups x 350 .. 8000 tokens: 3-bit keys with 4-bit
+// values 0.964 of the time, 4 and 4 bits 0.989, 4 and 2 bits 0.984; 3 and 2 bits 1.022, 2 and 2 bits 1.014; the device-driven kernels spill
+// for it, 32k tokens 531 -> 535 us).
 template <bool EARLY>
 __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half *kf, int b, int hk, const GqaSmem &sm,
                                             int t0, int lo, int t1) {
@@ -113,7 +115,7 @@ __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half
 // ---------------------------------------------------------------------------------------------
 // q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same stage geometry, tile order and channel
 // splits as the single-head kernel; scores[split][h][t - t0] receive the raw scores.
-template <int KB, bool WIDE, bool DEV>
+template <int KB, bool WIDE, bool EARLY>
 __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const GqaSmem &sm, int t0, int hi, const __half *kf,
                                               int tail_lo, int t1, int b, int hk) {
@@ -200,7 +202,7 @@ __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int3
 
 #pragma unroll 1
     for (int q = 0; q < R::P; ++q) issue_stage();
-    if constexpr (DEV) {
+    if constexpr (!EARLY) {
         __syncthreads();                                       // q is in shared memory (stored by the caller without a barrier)
         if (tail_lo < t1) gqa_qk_tail<false>(a, kf, b, hk, sm, t0, tail_lo, t1);
     } else {
@@ -798,8 +800,9 @@ __device__ __forceinline__ void gqa_segment(const kvq_attn_args &a, const kvq_at
         const int32_t *kc = a.kcode + (int64_t)b * a.kc_sB + (int64_t)hk * a.kc_sH;
         const __half *ks = static_cast<const __half *>(a.kscale) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
         const __half *kz = static_cast<const __half *>(a.kmn) + (int64_t)b * a.ks_sB + (int64_t)hk * a.ks_sH;
-        if (KB != 1 && (KB == 3 || a.k_group == 64)) gqa_qk_packed<KB, false, DEV>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
-        else gqa_qk_packed<KB, KB != 3, DEV>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        constexpr bool kEarly = !DEV && KB + VB >= 6;          // see gqa_qk_tail
+        if (KB != 1 && (KB == 3 || a.k_group == 64)) gqa_qk_packed<KB, false, kEarly>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
+        else gqa_qk_packed<KB, KB != 3, kEarly>(a, kc, ks, kz, sm, t0, min(t1, a.Tkq), kf, max(t0, a.Tkq), t1, b, hk);
     }
     const int32_t *vc = a.vcode + (int64_t)b * a.vc_sB + (int64_t)hk * a.vc_sH;
     const __half *vs = static_cast<const __half *>(a.vscale) + (int64_t)b * a.vs_sB + (int64_t)hk * a.vs_sH;
