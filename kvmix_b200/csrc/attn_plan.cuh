@@ -82,11 +82,17 @@ inline long long plan_segment_cycles(int n, int tile, int max_scores) {
 // What cutting a head adds to its last CTA: publishing the partials and the merge of k of them.
 inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; }
 
-// Whole heads for more than half of the SMs and no more than there are: a CTA that has its SM to itself takes this percentage of
-// the time, and halves of all heads would only put two on it and a merge behind (us, whole against halves: 128 heads,
-// group 32, 2 bits, 1023 tokens 11.6 and 13.5, 4096 tokens 23.0 and 23.2, 3-bit keys 28.6 and 31.5; 128 groups of 4 heads, 4 bits,
-// 1023 tokens 15.7 and 19.6).
-constexpr int kPlanLone = 77;
+// Whole heads for more than half of the SMs and no more than there are: a CTA that has its SM to itself takes this percentage of the time the
+// model gives it, and halves of all heads would only put two on it and a merge behind.  Up to 98 heads three pieces of each also fit one
+// round, the last ones short, which is the better form from some 1200 tokens on (80); 3-bit keys are counted dearer than they are next to
+// what a CTA does once (70).  Every form timed at 75 .. 148 heads x 350 .. 7000 tokens x 2, 4 and 3-bit keys, one head and four a CTA
+// (770 points): 0.942 of the time of the plan without this rule, no point more than 1 % slower, 0.7 % from the best form of each point on
+// average (us, whole and halves, whole taken: 128 heads of 1023 tokens, 2 bits 10.7 and 13.1, 3-bit keys 12.9 and 14.6, of 2000 18.4 and
+// 20.7; 128 groups of 4 heads x 1023, 4 bits 14.2 and 18.1; whole and thirds, thirds taken: 96 groups x 1700, 4 bits 17.0 and 15.3).
+// From some 2500 tokens on halves are taken although whole heads would be up to 4 % faster (128 heads of 4096, 2 bits 22.7 and 23.1, 3-bit
+// keys 28.7 and 30.0): with a long fp16 tail they are the slower form (128 heads on 32 kv heads of 3001 tokens, 600 of them fp16, three
+// layers 79.8 us whole, 76.8 halved).
+inline int plan_lone_percent(long long heads, int unit) { return unit % 11 == 0 ? 70 : 3 * heads <= kPlanSlots ? 80 : 77; }
 inline bool plan_lone(long long ctas, int k) { return k == 1 && ctas <= kSmCount && 2 * ctas > kSmCount; }
 
 // Pieces a head is cut into where `heads` of them (fewer than SMs) are left behind whole ones: the SM that gets most of the pieces
@@ -133,7 +139,7 @@ inline AttnPlan make_attn_plan(int T, int unit, int tile, int max_scores, long l
             const long long rounds = (ctas + kPlanSlots - 1) / kPlanSlots;
             const int n = su * unit < T ? su * unit : T;
             long long cost = rounds * plan_segment_cycles(n, tile, max_scores) + plan_merge_cycles(k);
-            if (plan_lone(ctas, k)) cost = cost * kPlanLone / 100;
+            if (plan_lone(ctas, k)) cost = cost * plan_lone_percent(ctas, unit) / 100;
             if (best < 0 || cost < best) {
                 best = cost;
                 p.k = k;

@@ -191,6 +191,16 @@ def test_split_plan_counts_three_bit_keys_in_tiles_of_88():
         assert _plan(1, heads, T, 3, 1).segments == want, (heads, T)
 
 
+def test_split_plan_lone_heads():
+    """75 .. 148 heads (or groups of them): whole where that was measured faster than pieces, cut where not, in both kernels."""
+    for nh, T, kb, want in [(74, 1023, 2, 4), (75, 1023, 2, 1), (75, 1400, 3, 1), (75, 1700, 2, 3), (98, 2000, 4, 3), (99, 2000, 4, 1), (128, 1023, 2, 1), (128, 1023, 3, 1),
+                            (128, 2000, 3, 1), (128, 3001, 4, 2), (128, 4096, 2, 2), (128, 4096, 3, 2), (98, 3001, 3, 3), (148, 1023, 2, 1), (149, 2000, 3, 3)]:
+        assert _plan(1, nh, T, kb, 1).segments == want, (nh, T, kb)
+    for groups, T, kb, want in [(74, 1023, 4, 4), (75, 1023, 4, 1), (76, 1700, 4, 3), (96, 1700, 2, 3), (96, 1700, 3, 3), (99, 1700, 4, 1), (128, 2000, 3, 1), (148, 1023, 3, 1)]:
+        p = _plan(1, 4 * groups, T, kb, 1, nh_kv=groups, G=64, vb=4)
+        assert p.kernel == 2 and p.segments == want, (groups, T, kb)
+
+
 def test_wide_key_rows_keep_their_kernel():
     """Keys are addressed by unsigned 32-bit byte offsets within a head: 128 rows of up to 2^23 words reach just below 2^32."""
     for words, groups, kernel in [(1 << 20, 1 << 20, 1), ((1 << 23) - 4, 1 << 20, 1), (1 << 23, 1 << 20, 0), (1 << 20, (1 << 24) - 8, 1), (1 << 20, 1 << 24, 0)]:
