@@ -94,6 +94,13 @@ inline long long plan_merge_cycles(int k) { return k > 1 ? 2500 + 40LL * k : 0; 
 // layers 79.8 us whole, 76.8 halved).
 inline int plan_lone_percent(long long heads, int unit) { return unit % 11 == 0 ? 70 : 3 * heads <= kPlanSlots ? 80 : 77; }
 inline bool plan_lone(long long ctas, int k) { return k == 1 && ctas <= kSmCount && 2 * ctas > kSmCount; }
+// Whole heads for all SMs but a few are not launched early: CTAs that are placed while those of the launch before still hold some SMs come to
+// lie two to an SM, and no SM is left over to make up for it (148 heads whole, launched early / ordinarily: 1.11 of the time on average
+// over 350 .. 6000 tokens, 148 groups of four heads 1.17; 144: 1.02; 128: 0.99).
+inline bool plan_early(const AttnPlan &p) {
+    const long long ctas = p.n_whole + (long long)p.n_cut * p.k;
+    return !(p.k == 1 && ctas > kSmCount * 7 / 8 && ctas <= kSmCount);
+}
 
 // Pieces a head is cut into where `heads` of them (fewer than SMs) are left behind whole ones: the SM that gets most of the pieces
 // finishes last; a piece costs its tokens and some 600 more, one whole head by itself on its SM `lone` percent of that.

@@ -67,7 +67,7 @@ __device__ __forceinline__ unsigned int count_in(unsigned int *counter) {
 int record_cuda_error(cudaError_t e);
 inline int check_launch() { return record_cuda_error(cudaGetLastError()); }
 template <typename... P, typename... A>
-inline int launch_early(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+inline int launch_early(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -75,7 +75,7 @@ inline int launch_early(void (*kernel)(P...), unsigned grid, unsigned block, siz
     cfg.stream = st;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    attr.val.programmaticStreamSerializationAllowed = early;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);

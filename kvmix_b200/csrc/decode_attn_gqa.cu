@@ -1020,8 +1020,8 @@ static int launch_gqa(const kvq_attn_args &a, AttnPlan plan, int qhv, float *par
     const unsigned grid = (unsigned)(plan.n_whole + plan.n_cut * plan.k);
     // launched early (grid_wait): four small layers of 4 x 8 kv heads x 1537 tokens from a host loop 69.5 -> 60.2 us, 131k tokens from a graph
     // 407 -> 403; let in at the start of the kernel instead of behind p . V the next launch's CTAs cost more than they gain (66.7)
-    if (VB != 3 && a.state) return launch_early(decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
-    return launch_early(decode_attn_gqa_kernel<KB, VB, false>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
+    if (VB != 3 && a.state) return launch_early(plan_early(plan), decode_attn_gqa_kernel<KB, VB == 3 ? 4 : VB, true>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
+    return launch_early(plan_early(plan), decode_attn_gqa_kernel<KB, VB, false>, grid, kMmaThreads, smem, st, a, plan, qhv, parts, counters);
 }
 
 int launch_decode_attn_gqa(const kvq_attn_args &a, const AttnPlan &plan, int qhv, float *parts, unsigned int *counters,

@@ -894,7 +894,7 @@ static int launch_mma(const kvq_attn_args &a, AttnPlan plan, float *parts, unsig
         decode_attn_mma_kernel<KB, VB, true, NW><<<grid, 32 * NW, smem, st>>>(a, plan, parts, counters);
         return check_launch();
     }
-    return launch_early(decode_attn_mma_kernel<KB, VB, false, NW>, grid, 32 * NW, smem, st, a, plan, parts, counters);
+    return launch_early(plan_early(plan), decode_attn_mma_kernel<KB, VB, false, NW>, grid, 32 * NW, smem, st, a, plan, parts, counters);
 }
 
 int launch_decode_attn_mma(const kvq_attn_args &a, const AttnPlan &plan, float *parts, unsigned int *counters,

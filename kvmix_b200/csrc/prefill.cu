@@ -54,7 +54,7 @@ static int launch_prefill(const kvq_prefill_args &a, const QuantDims &kd, const 
     if (k_ctas + v_ctas + t_ctas > 2147483647LL) return KVQ_ERR_UNSUPPORTED;
     p.k_ctas = (int)k_ctas;
     p.v_ctas = (int)v_ctas;
-    return launch_early(prefill_kernel<KB, KG, VB>, (unsigned)(k_ctas + v_ctas + t_ctas), 256, 0, st, a, kd, vd, rope, p);
+    return launch_early(true, prefill_kernel<KB, KG, VB>, (unsigned)(k_ctas + v_ctas + t_ctas), 256, 0, st, a, kd, vd, rope, p);
 }
 
 // KVQ_ERR_UNSUPPORTED: not for this kernel.

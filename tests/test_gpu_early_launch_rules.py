@@ -57,3 +57,24 @@ def test_mat_vec(cuda, B, nh, T, early):
             ops.quantized_gemm(32, q, *keys, 2)
             ops.quantized_gemm(32, p, *values, 2)
     assert _captured(body) == (5, early)
+
+
+@pytest.mark.parametrize("nh,hkv,T,early", [(128, 128, 700, 3), (144, 144, 700, 1), (148, 148, 700, 1), (149, 149, 700, 3), (592, 148, 700, 1), (32, 32, 700, 3)])
+def test_whole_heads_for_all_sms(cuda, nh, hkv, T, early):
+    """Whole heads for nearly all SMs are launched in the ordinary way; fewer, more, and cut ones early.  Attention
+    twice, with a mat-vec between them, which is early here."""
+    import kvmix_b200 as kv
+    from kvmix_b200 import ops
+    c = kv.KVmixLayerCache(1, hkv, 128, T + 64, 2, 2, 64, residual_length=128, device=cuda)
+    g = torch.Generator(device=cuda).manual_seed(1)
+    c.prefill(*(torch.randn((1, hkv, T, 128), generator=g, device=cuda, dtype=torch.float16) for _ in range(2)))
+    keys = ops.quantize_pack_last_dim_cuda(torch.randn((1, 8, 640, 128), device=cuda, dtype=torch.float16).transpose(2, 3), 32, 2)
+    q, x = torch.randn((1, nh, 1, 128), generator=g, device=cuda, dtype=torch.float16), torch.zeros(4, device=cuda)
+    out = torch.empty_like(q)
+
+    def body():
+        x.add_(1)
+        c.attend(q, out=out)
+        ops.quantized_gemm(32, q[:, :8], *keys, 2)
+        c.attend(q, out=out)
+    assert _captured(body) == (4, early)
