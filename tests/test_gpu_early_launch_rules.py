@@ -78,3 +78,24 @@ def test_whole_heads_for_all_sms(cuda, nh, hkv, T, early):
         ops.quantized_gemm(32, q[:, :8], *keys, 2)
         c.attend(q, out=out)
     assert _captured(body) == (4, early)
+
+
+@pytest.mark.parametrize("kb,vb,G,L,rotate,want", [(2, 2, 32, 600, True, 1), (4, 1, 64, 600, True, 1), (3, 3, 64, 600, True, 1), (1, 4, 128, 600, True, 1),
+                                                   (2, 2, 32, 600, False, 3), (4, 4, 32, 128, True, 1), (3, 2, 32, 140, True, 2)])
+def test_prefill_launches(cuda, kb, vb, G, L, rotate, want):
+    """A prompt is one launch where it is rotated on the way and both packed parts have tokens, three where its keys arrive rotated,
+    one less for each part without tokens.  What LAUNCHES counts is what was launched."""
+    import kvmix_b200 as kv
+    from kvmix_b200 import ops
+    caches = [kv.KVmixLayerCache(2, 3, 128, L + 8, kb, vb, G, residual_length=128, device=cuda) for _ in range(2)]
+    kp, vp = (torch.randn((2, L, 3 * 128), device=cuda, dtype=torch.float16) for _ in range(2))
+    tables = [torch.rand((L, 128), device=cuda).half() for _ in range(2)] if rotate else []
+    counted, x = [], torch.zeros(4, device=cuda)
+
+    def body():
+        x.add_(1)                                              # a graph of one kernel has no edges to look at
+        n = ops.LAUNCHES[0]
+        caches[len(counted)].prefill_projected(kp, vp, *tables)
+        counted.append(ops.LAUNCHES[0] - n)
+    kernels, _ = _captured(body)
+    assert (kernels, counted) == (want + 1, [want, want])
