@@ -173,7 +173,8 @@ int kvq_append_kv(const kvq_append_args *a, kvq_stream_t stream);
  *             and quantized per channel over groups of k_group tokens into kcode / kscale / kmn, values [0, nv) per
  *             token over groups of v_group channels, exactly as kvq_quant_lastdim (scale_by_division = 0) would;
  *             the remaining tokens go, rotated, to rows 0.. of the fp16 tails kfull / vfull.
- * Three launches (key quantizer, value quantizer, tails), no temporary tensors.  D must be 128.
+ * One launch where tables are given, both packed parts have tokens and groups are of 32, 64 or 128 (11 for 3 bits); else
+ * one each for the keys, the values and the tails that have tokens.  No temporary tensors.  D must be 128.
  */
 typedef struct {
     const void *k;

@@ -16,7 +16,7 @@
 
 namespace kvq {
 
-// Division by a number the host knows (1 .. 2^31), of numbers below 2^31: a high product, an addition and a shift where the compiler's
+// Division by an invariant integer (Granlund and Montgomery, 1994), 1 .. 2^31, of numbers below 2^31: a high product, an addition and a shift where the compiler's
 // division takes some twenty-five instructions, several of them in a row at the start of every CTA.
 struct FastDiv {
     uint32_t mul, shr, d;

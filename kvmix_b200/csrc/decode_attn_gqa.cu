@@ -113,8 +113,8 @@ __device__ __forceinline__ void gqa_qk_tail(const kvq_attn_args &a, const __half
 }
 
 // ---------------------------------------------------------------------------------------------
-// q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Same stage geometry, tile order and channel
-// splits as the single-head kernel; scores[split][h][t - t0] receive the raw scores.
+// q . K^T over packed keys, tokens [t0, hi), for the four heads of the quad.  Stage geometry, tile order and channel
+// splits of the single-head kernel, which for 3-bit keys also has tiles of 176 tokens (here always 88); scores[split][h][t - t0] receive the raw scores.
 template <int KB, bool WIDE, bool EARLY>
 __device__ __forceinline__ void gqa_qk_packed(const kvq_attn_args &a, const int32_t *kc, const __half *ks,
                                               const __half *kz, const GqaSmem &sm, int t0, int hi, const __half *kf,

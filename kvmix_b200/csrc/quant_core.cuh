@@ -61,8 +61,9 @@ __device__ __forceinline__ float max_abs(float t, float x, float y) {
 // question are divided: fp16 data tie often enough that some lane of every eighth warp gets here, and dividing for all
 // elements of the word was a fifth of the quantizers' instructions (1, 2 and 4 bits).
 // Elements go in pairs (f32x2), the tie test is one three-input maximum a pair.  16 x 32 x 8192 x 128 fp16:
-// keys (2 bits, groups of 32 tokens) 348 -> 310 us, values (4 bits, groups of 32) 309 -> 296 us; one look for ties a thread and words
-// put together by a byte permute 304 -> 282 us, and with several units a thread 291 -> 252 us.
+// keys (2 bits, groups of 32 tokens) 348 -> 310 us, values (4 bits, groups of 32) 309 -> 296 us; words put together by a byte permute
+// keys 304 -> 282 us (which look for ties once a word and channel); that, one look for ties a thread and several units a thread
+// values 291 -> 252 us.
 // 3-bit words are worked one element at a time and divided whole: eleven fields in two chunks split badly into pairs, and
 // their lone word a group leaves too little between two tie tests (keys 457 us in pairs with single divisions, 426 us so;
 // contiguous groups 464 and 436 us).
