@@ -36,7 +36,7 @@ DTYPE = "f16 data, f32 accumulate, u32 packed codes"
 EAGER_SAMPLE_STEPS = 8
 # dram__bytes_read + dram__bytes_write over algorithmic bytes of one fused-attention launch, from the ncu captures
 # summarised in profiles/decode_attn_mma_kernel_B32_ctx4096.md (one CTA per head there, so the ratio carries over).
-NCU_TRAFFIC_RATIO = {(4, 4): 1.090, (3, 2): 1.117, (2, 2): 1.101}    # fused decode step, device-driven (the bench's launches)
+NCU_TRAFFIC_RATIO = {(4, 4): 1.090, (3, 2): 1.113, (2, 2): 1.107}    # fused decode step, device-driven (the bench's launches)
 
 
 def measured_peak_gbs():
